@@ -13,6 +13,12 @@ namespace kllm {
 std::atomic<uint64_t>& launch_counter();
 inline void count_launch(uint64_t n = 1) { launch_counter().fetch_add(n, std::memory_order_relaxed); }
 
+// The process's flag for waits that ran out inside a kernel: one int of mapped host memory, which kernels write and the host
+// reads without a copy (nullptr: there is no device).  take_wait_error() is 1 when it was raised since the last call; what a
+// stream has noted is certain to be there once that stream has been waited for.
+int* wait_flag();
+int take_wait_error();
+
 // A position that is either a host value or read from device memory at kernel run time; the
 // decoder's CUDA graph uses the device form so ONE captured graph serves every position.
 struct PosArg {

@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <mutex>
 
 #include "kllm_host.h"
 
@@ -11,6 +12,31 @@ namespace kllm {
 std::atomic<uint64_t>& launch_counter() {
   static std::atomic<uint64_t> c{0};
   return c;
+}
+
+int* wait_flag() {
+  static std::atomic<int*> flag{nullptr};
+  if (int* p = flag.load(std::memory_order_acquire)) return p;
+  static std::mutex m;
+  std::lock_guard<std::mutex> lock(m);
+  int* p = flag.load(std::memory_order_relaxed);
+  if (p == nullptr) {
+    void* v = nullptr;
+    if (cudaHostAlloc(&v, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;  // tried again at the next call
+    }
+    p = static_cast<int*>(v);
+    *p = 0;
+    flag.store(p, std::memory_order_release);
+  }
+  return p;
+}
+int take_wait_error() {
+  int* p = wait_flag();
+  if (p == nullptr || __atomic_load_n(p, __ATOMIC_RELAXED) == 0) return 0;
+  __atomic_store_n(p, 0, __ATOMIC_RELAXED);
+  return 1;
 }
 }  // namespace kllm
 

@@ -387,6 +387,7 @@ extern "C" int kllm_seq_create(const kllm_seq_desc* desc, void* stream, kllm_seq
   if (int rc = validate(desc)) return rc;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) return KLLM_E_NODEVICE;
+  if (wait_flag() == nullptr) return KLLM_E_STATE;  // allocated here: a step may be inside a capture
   kllm_seq_engine* e = new (std::nothrow) kllm_seq_engine();
   if (!e) return KLLM_E_STATE;
   e->d = *desc;

@@ -274,7 +274,7 @@ tiled_kernel(const AT* __restrict__ a, const AT* __restrict__ w, void* __restric
 }
 
 template <typename AT>
-int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s, bool* umma_used) {
+int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s) {
   constexpr int V = Vec16<AT>::N;
   if (T <= 8) {
     const bool vec = (K % V) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
@@ -294,7 +294,6 @@ int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K
     return cuda_rc(cudaGetLastError());
   }
   if (umma::usable<AT>(a, w, T, K, N)) {
-    *umma_used = true;
     return umma::launch(a, w, bias, out, T, K, N, s);
   }
   const dim3 grid((N + TN - 1) / TN, (T + TM - 1) / TM);
@@ -305,8 +304,7 @@ int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K
 }
 
 template <typename AT>
-int gemm_gated_t(const AT* a, const AT* w, const float* bias, AT* out, int T, int K, int N, const GatedAct& act, cudaStream_t s,
-                 bool* umma_used) {
+int gemm_gated_t(const AT* a, const AT* w, const float* bias, AT* out, int T, int K, int N, const GatedAct& act, cudaStream_t s) {
   constexpr int V = Vec16<AT>::N;
   if (T <= 8) {
     const bool vec = (K % V) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
@@ -327,7 +325,6 @@ int gemm_gated_t(const AT* a, const AT* w, const float* bias, AT* out, int T, in
     return cuda_rc(cudaGetLastError());
   }
   if (umma::usable<AT>(a, w, T, K, N)) {
-    *umma_used = true;
     return umma::launch_gated(a, w, bias, out, T, K, N, act, s);
   }
   const dim3 grid((N + TN - 1) / TN, (T + TM - 1) / TM);
@@ -355,13 +352,12 @@ int grouped_t(const GroupedArgs& g, cudaStream_t s) {
 
 }  // namespace
 
-static bool g_umma_used;
 int gemm(int dtype, const void* a, const void* w, float* out, int T, int K, int N, cudaStream_t s, const float* bias) {
   if (!a || !w || !out || T <= 0 || K <= 0 || N <= 0) return KLLM_E_INVALID;
   if (dtype == KLLM_SEQ_F32)
-    return gemm_t(static_cast<const float*>(a), static_cast<const float*>(w), bias, out, T, K, N, s, &g_umma_used);
+    return gemm_t(static_cast<const float*>(a), static_cast<const float*>(w), bias, out, T, K, N, s);
   if (dtype == KLLM_SEQ_BF16)
-    return gemm_t(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(w), bias, out, T, K, N, s, &g_umma_used);
+    return gemm_t(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(w), bias, out, T, K, N, s);
   return KLLM_E_INVALID;
 }
 
@@ -369,19 +365,14 @@ int gemm_gated(int dtype, const void* a, const void* w, void* out, int T, int K,
                const float* bias) {
   if (!a || !w || !out || T <= 0 || K <= 0 || ff <= 0) return KLLM_E_INVALID;
   if (dtype == KLLM_SEQ_F32)
-    return gemm_gated_t(static_cast<const float*>(a), static_cast<const float*>(w), bias, static_cast<float*>(out), T, K, ff, act, s,
-                        &g_umma_used);
+    return gemm_gated_t(static_cast<const float*>(a), static_cast<const float*>(w), bias, static_cast<float*>(out), T, K, ff, act, s);
   if (dtype == KLLM_SEQ_BF16)
     return gemm_gated_t(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(w), bias,
-                        static_cast<__nv_bfloat16*>(out), T, K, ff, act, s, &g_umma_used);
+                        static_cast<__nv_bfloat16*>(out), T, K, ff, act, s);
   return KLLM_E_INVALID;
 }
 
-int gemm_take_error() {
-  if (!g_umma_used) return 0;
-  g_umma_used = false;
-  return umma::take_error();
-}
+int gemm_take_error() { return take_wait_error(); }
 
 bool grouped_tensor_core_usable(int dtype, int width, int ff) {
   return dtype == KLLM_SEQ_BF16 && umma::grouped_usable(width, ff) && umma::grouped_usable(ff, width);
@@ -398,7 +389,6 @@ int gather_rows_bf16(const void* a, const int32_t* sorted_pair, int div, void* o
 int gemm_grouped(int dtype, const GroupedArgs& g, cudaStream_t s) {
   if (g.sorted_layout) {
     if (dtype != KLLM_SEQ_BF16 || g.block != umma::GBN) return KLLM_E_INVALID;
-    g_umma_used = true;
     if (g.epilogue == 1)
       return umma::launch_grouped<1>(g.a, g.w, g.out, g.sorted_pair, g.block_expert, g.n_blocks, g.experts, g.K, g.N, s, g.act);
     if (g.epilogue == 2)

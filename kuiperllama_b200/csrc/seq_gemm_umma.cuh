@@ -12,7 +12,7 @@
 //   warps 2-5   epilogue: tcgen05.ld 32 lanes x 32 columns, coalesced stores (a warp's lanes are consecutive features)
 // Rows and columns past the matrices are zero-filled by TMA and never stored.  K needs 16-byte rows (K % 8 == 0).
 //
-// Every mbarrier wait is bounded: a wait that runs out raises a flag in global memory (read by the host after the
+// Every mbarrier wait is bounded: a wait that runs out raises a flag in mapped host memory (read by the host after the
 // step), tells the other roles to stop, lets copies in flight land, frees the TMEM columns and returns.
 #pragma once
 #include <cuda.h>
@@ -36,7 +36,11 @@ constexpr int A_BYTES = BM * BK * 2;
 constexpr int THREADS = 192;
 constexpr uint32_t kWaitLimit = 1u << 24;  // try_wait rounds before a wait gives up (each suspends up to ~1 us)
 
-__device__ int g_error;  // != 0: a wait inside umma_kernel ran out
+// Where a wait that runs out is noted: `here` stops the other roles of the CTA, `report` (kllm::wait_flag) is read by the host.
+struct Stop {
+  volatile int* here;
+  int* report;
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
@@ -46,17 +50,18 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 // false: gave up (limit reached, or another role already did)
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* stop) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const Stop& stop) {
   for (uint32_t i = 0; i < kWaitLimit; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     if (ok) return true;
-    if ((i & 1023u) == 1023u && *stop) return false;
+    if ((i & 1023u) == 1023u && *stop.here) return false;
   }
-  *stop = 1;
-  g_error = 1;
+  *stop.here = 1;
+  *reinterpret_cast<volatile int*>(stop.report) = 1;
+  __threadfence_system();
   return false;
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
@@ -102,7 +107,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 template <int BN, bool GATED, int ST>
 __global__ void __launch_bounds__(THREADS, 1)
 umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
-            void* __restrict__ out_, const float* __restrict__ bias, int T, int N, int K, GatedAct act) {
+            void* __restrict__ out_, const float* __restrict__ bias, int T, int N, int K, GatedAct act, int* report) {
   constexpr int NA = GATED ? 2 : 1;  // weight tiles per stage
   constexpr int W_BYTES = NA * A_BYTES, B_BYTES = BN * BK * 2;
   constexpr uint32_t TMEM_COLS = NA * (BN < 32 ? 32 : BN);
@@ -115,7 +120,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
   uint64_t* empty = bars + ST;
   uint64_t* tmem_full = bars + 2 * ST;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * ST + 1);
-  volatile int* stop = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), report};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * BM, t0 = blockIdx.y * BN;
@@ -127,7 +132,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
       mbar_init(smem_u32(&empty[s]), 1);
     }
     mbar_init(smem_u32(tmem_full), 1);
-    *stop = 0;
+    *stop.here = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -202,7 +207,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
       }
     }
   }
-  if (*stop) {  // a wait ran out: give copies in flight time to land before the shared memory is given up
+  if (*stop.here) {  // a wait ran out: give copies in flight time to land before the shared memory is given up
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -223,7 +228,7 @@ template <int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                     void* __restrict__ out_, const int32_t* __restrict__ sorted_pair,
-                    const int32_t* __restrict__ block_expert, int N, int K, GatedAct act) {
+                    const int32_t* __restrict__ block_expert, int N, int K, GatedAct act, int* report) {
   constexpr int NA = EPI == 1 ? 2 : 1;
   constexpr int B_BYTES = GBN * BK * 2;
   constexpr int STAGE = NA * A_BYTES + B_BYTES;
@@ -237,7 +242,7 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   uint64_t* empty = bars + STAGES;
   uint64_t* tmem_full = bars + 2 * STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
-  volatile int* stop = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), report};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * BM, r0 = blockIdx.y * GBN;
@@ -250,7 +255,7 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       mbar_init(smem_u32(&empty[s]), 1);
     }
     mbar_init(smem_u32(tmem_full), 1);
-    *stop = 0;
+    *stop.here = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -329,7 +334,7 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       }
     }
   }
-  if (*stop) {
+  if (*stop.here) {
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -388,6 +393,8 @@ inline int launch_bn(const void* a, const void* w, const float* bias, void* out,
                      cudaStream_t stream) {
   constexpr int NA = GATED ? 2 : 1;
   CUtensorMap map_w, map_a;
+  int* const report = wait_flag();
+  if (report == nullptr) return KLLM_E_STATE;
   if (int rc = make_map(&map_w, w, NA * N, K, BM)) return rc;
   if (int rc = make_map(&map_a, a, T, K, BN)) return rc;
   const size_t smem = 1024 + static_cast<size_t>(ST) * (NA * A_BYTES + BN * BK * 2) + 256;
@@ -399,7 +406,7 @@ inline int launch_bn(const void* a, const void* w, const float* bias, void* out,
     configured = true;
   }
   const dim3 grid((N + BM - 1) / BM, (T + BN - 1) / BN);
-  umma_kernel<BN, GATED, ST><<<grid, THREADS, smem, stream>>>(map_w, map_a, out, bias, T, N, K, act);
+  umma_kernel<BN, GATED, ST><<<grid, THREADS, smem, stream>>>(map_w, map_a, out, bias, T, N, K, act, report);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }
@@ -447,6 +454,8 @@ inline int launch_grouped(const void* a, const void* w, void* out, const int32_t
                           int n_blocks, int experts, int K, int N, cudaStream_t stream,
                           GatedAct act = GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}) {
   CUtensorMap map_w, map_a;
+  int* const report = wait_flag();
+  if (report == nullptr) return KLLM_E_STATE;
   if (int rc = make_map(&map_w, w, experts * (EPI == 1 ? 2 : 1) * N, K, BM)) return rc;
   if (int rc = make_map(&map_a, a, n_blocks * GBN, K, GBN)) return rc;
   const size_t smem = 1024 + static_cast<size_t>(STAGES) * ((EPI == 1 ? 2 : 1) * A_BYTES + GBN * BK * 2) + 256;
@@ -458,20 +467,9 @@ inline int launch_grouped(const void* a, const void* w, void* out, const int32_t
     configured = true;
   }
   const dim3 grid((N + BM - 1) / BM, n_blocks);
-  umma_grouped_kernel<EPI><<<grid, THREADS, smem, stream>>>(map_w, map_a, out, sorted_pair, block_expert, N, K, act);
+  umma_grouped_kernel<EPI><<<grid, THREADS, smem, stream>>>(map_w, map_a, out, sorted_pair, block_expert, N, K, act, report);
   count_launch();
   return static_cast<int>(cudaGetLastError());
-}
-
-// 1 when a wait inside the kernel ran out since the last call; clears the flag
-inline int take_error() {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_error, sizeof(int)) != cudaSuccess) return 0;
-  if (v) {
-    const int zero = 0;
-    cudaMemcpyToSymbol(g_error, &zero, sizeof(int));
-  }
-  return v;
 }
 
 }  // namespace umma
