@@ -1,0 +1,444 @@
+// Products whose tiles do not fill the chip, on the 5th-generation tensor cores (sm_100a): the same product and the same gated
+// form as seq_gemm_umma.cuh, with K split over the CTAs of a cluster, for three kinds of operands (MODE).
+//
+//   kBf16    bf16 operands
+//   kTf32    fp32 operands read as TF32 (10 mantissa bits): the toleranced prompt path of the single-sequence decoder
+//   kFp32    fp32 operands, products to fp32 accuracy: every operand is hi + lo, hi its leading 11 bits and lo the rest rounded
+//            to 11 bits, and a . w = hi hi + (lo hi + hi lo); what is left out (lo lo, lo's rounding) is below 2^-20 of the
+//            product.  Four warps split each tile in shared memory between its arrival and its use.
+//
+// What bounds it: with a few dozen tokens the weights are read once and every element of them feeds 2 * T multiply-adds, so
+// the time is the weights' way from HBM.  A tile per 128 features leaves most SMs without work (width 4096: 32 tiles), and
+// one CTA's ring does not keep enough bytes on the way.  So K is split over the S CTAs of a cluster: each runs the ring of
+// the large form over its part of K, leaves its partial tile in its own shared memory, and after a cluster barrier every
+// CTA sums BN / S of the tile's tokens over the S partials, read through distributed shared memory in rank order (the
+// result does not depend on timing).  kFp32 on token blocks is bound by shared memory instead: a stage is read and written
+// by the splitting warps (96 KB at BN = 128) and read three times over by the MMAs.
+//
+// Precision: a tcgen05 accumulator is not rounded to nearest at each of its steps, and its error grows with their number.  A
+// CTA hands its accumulator over every SECTION blocks of K to the epilogue warps, which sum the sections in fp32 registers
+// while the tensor core fills the other accumulator.  kFp32 keeps the two small products in an accumulator of their own.
+//
+// Measured, calls back to back with weights from HBM (one B200), the FMA tiles that these shapes took before -> now; error
+// against 64 bits in the 2-norm:
+//   bf16  T = 40, K = 4096, N = 4096    298 -> 14.6 us    6.1e-7 -> 1.4e-7
+//   bf16  T = 24, K = 2048, N = 2048    149 -> 10.4 us    3.9e-7 -> 1.3e-7
+//   bf16  T = 24, K = 2048, N = 32000   382 -> 28.8 us    3.9e-7 -> 1.4e-7
+#pragma once
+#include "seq_gemm_umma.cuh"
+
+namespace kllm {
+namespace seq {
+namespace umma {
+
+// Fewer blocks of K per CTA do not pay for the cluster's barriers and reads (K = 1024, N = 1024, T = 24: 12.4 us unsplit, 8.3 us
+// for 4 and for 8 CTAs).
+constexpr int kMinSplitBlocks = 3;
+
+enum Mode { kBf16 = 0, kTf32 = 1, kFp32 = 2 };
+template <int MODE> struct ModeOf {  // fp32 operands
+  static constexpr int BKE = 32;     // elements of K per 128-byte block
+  static constexpr int SECTION = 2;  // blocks between two hand-overs of the accumulator: 8 steps
+};
+template <> struct ModeOf<kBf16> {
+  static constexpr int BKE = 64;
+  static constexpr int SECTION = 2;  // 8 steps
+};
+
+// instruction descriptor as in instr_desc, A = B = TF32 (2 << 7, 2 << 10)
+__device__ __forceinline__ uint32_t instr_desc_tf32(int n) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
+}
+__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address of `saddr` (a shared-memory address of this CTA) in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t peer_smem(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float ld_peer(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+// hi keeps the sign, the exponent and ten mantissa bits (never rounded up, so it cannot overflow), lo is x - hi, which is exact,
+// rounded to eleven bits.  An infinity has no such form (inf - inf): it is hi alone, and raises `special`.
+__device__ __forceinline__ float split_hi_lo(float x, float* lo, bool* special) {
+  const float hi = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
+  const bool inf = fabsf(x) == INFINITY;
+  uint32_t l;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(x - hi));
+  *lo = inf ? 0.f : __uint_as_float(l);
+  *special = *special || inf;
+  return hi;
+}
+
+// what a product does with its sums
+enum Out {
+  kPlain = 0,  // out = sum + bias (fp32)
+  kGated = 1,  // out = gated_act(sum of w + bias[n], sum of w2 + bias[N + n]) in the operands' type
+  kAdd = 2     // out = add + sum (fp32; add may be out itself)
+};
+
+// operand pointers (kFp32's fallback for infinities reads through them) and what joins the sums
+struct SplitArgs {
+  const void *a, *w, *w2;
+  const float* bias;
+  const float* add;
+  void* out;
+  int T, N, K, S;
+  GatedAct act;
+  int* report;  // wait_flag()
+};
+
+template <int MODE, int OUT>
+__device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, float v, float u) {
+  const size_t at = static_cast<size_t>(t) * p.N + row;
+  if constexpr (OUT == kGated) {
+    const float y = gated_act(p.act, p.bias ? v + p.bias[row] : v, p.bias ? u + p.bias[p.N + row] : u);
+    if constexpr (MODE == kBf16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(y);
+    else static_cast<float*>(p.out)[at] = y;
+  } else if constexpr (OUT == kAdd) {
+    static_cast<float*>(p.out)[at] = p.add[at] + v;
+  } else {
+    static_cast<float*>(p.out)[at] = p.bias ? v + p.bias[row] : v;
+  }
+}
+
+// This CTA's tokens of the tile, summed over the cluster's partial tiles in rank order.  A read from another CTA takes about a
+// microsecond: a group's reads are all on the way before the first is used (T = 40, K = N = 4096: 15.4 us token by token with
+// the sections of 512, 14.6 us with sections of 128).
+template <int MODE, int BN, int OUT, int S>
+__device__ __forceinline__ void split_reduce(const SplitArgs& p, uint32_t mine, int rank, int t0, int row) {
+  constexpr int NA = OUT == kGated ? 2 : 1, PER = BN / S, GROUP = PER < 64 / (S * NA) ? PER : 64 / (S * NA);
+  static_assert(PER >= 1 && PER % GROUP == 0, "tokens of a CTA");
+#pragma unroll 1
+  for (int g = 0; g < PER; g += GROUP) {
+    float v[GROUP][S], u[NA == 2 ? GROUP : 1][S];
+#pragma unroll
+    for (int q = 0; q < S; ++q) {
+      const uint32_t from = peer_smem(mine, static_cast<uint32_t>(q)) + (rank * PER + g) * BM * 4;
+#pragma unroll
+      for (int j = 0; j < GROUP; ++j) {
+        v[j][q] = ld_peer(from + j * BM * 4);
+        if constexpr (NA == 2) u[j][q] = ld_peer(from + (BN + j) * BM * 4);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < GROUP; ++j) {
+      const int t = t0 + rank * PER + g + j;
+      if (t >= p.T) break;
+      float a = v[j][0], b = u[NA == 2 ? j : 0][0];
+#pragma unroll
+      for (int q = 1; q < S; ++q) {
+        a += v[j][q];
+        if constexpr (NA == 2) b += u[j][q];
+      }
+      split_store<MODE, OUT>(p, t, row, a, b);
+    }
+  }
+}
+
+template <int MODE>
+constexpr int split_threads() { return MODE == kFp32 ? THREADS + 128 : THREADS; }
+
+// grid: (feature tiles, S, token tiles), clusters of (1, S, 1)
+template <int MODE, int BN, int OUT, int ST>
+__global__ void __launch_bounds__(split_threads<MODE>())
+umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
+                  const __grid_constant__ CUtensorMap map_a, const SplitArgs p) {
+  using M = ModeOf<MODE>;
+  constexpr int NA = OUT == kGated ? 2 : 1;
+  constexpr int W_BYTES = NA * A_BYTES, B_BYTES = BN * 128;
+  constexpr int HALF = W_BYTES + B_BYTES;                  // the tiles as they arrive (kFp32: then their hi parts)
+  constexpr int STAGE = MODE == kFp32 ? 2 * HALF : HALF;   // kFp32: the lo parts follow
+  constexpr int TILE_COLS = NA * BN;                       // of one sum
+  constexpr int ACC_COLS = MODE == kFp32 ? 2 * TILE_COLS : TILE_COLS;  // of one accumulator; there are two
+  constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
+  static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "columns are given out in powers of two");
+  static_assert(TILE_COLS * BM * 4 <= ST * STAGE, "the partial tile takes the place of the ring");
+  extern __shared__ uint8_t raw_smem[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + ST * STAGE);
+  uint64_t* empty = full + ST;
+  uint64_t* split_done = empty + ST;      // kFp32: the stage holds hi and lo parts
+  uint64_t* acc_full = split_done + ST;   // [2]
+  uint64_t* acc_empty = acc_full + 2;     // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), p.report};
+  float* special = reinterpret_cast<float*>(tmem_slot + 2);  // kFp32: != 0 when an operand of this CTA's part of K is infinite
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * BM, t0 = blockIdx.z * BN;
+  const int S = p.S, rank = S > 1 ? static_cast<int>(cluster_rank()) : 0;
+  const int all_blocks = (p.K + M::BKE - 1) / M::BKE;
+  const int kb0 = static_cast<int>(static_cast<long long>(all_blocks) * rank / S);
+  const int blocks = static_cast<int>(static_cast<long long>(all_blocks) * (rank + 1) / S) - kb0;  // >= 1: S <= all_blocks
+  const int sections = (blocks + M::SECTION - 1) / M::SECTION;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < ST; ++s) {
+      mbar_init(smem_u32(&full[s]), 1);
+      mbar_init(smem_u32(&empty[s]), 1);
+      mbar_init(smem_u32(&split_done[s]), 4);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&acc_full[b]), 1);
+      mbar_init(smem_u32(&acc_empty[b]), 4);
+    }
+    *stop.here = 0;
+    *special = 0.f;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_d = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int i = 0; i < blocks; ++i) {
+        const int s = i % ST, k = (kb0 + i) * M::BKE;
+        if (!mbar_wait(smem_u32(&empty[s]), ((i / ST) & 1) ^ 1u, stop)) break;
+        const uint32_t bar = smem_u32(&full[s]);
+        uint8_t* st = base + s * STAGE;
+        mbar_expect_tx(bar, HALF);
+        tma_load_2d(smem_u32(st), &map_w, bar, k, n0);
+        if (NA == 2) tma_load_2d(smem_u32(st + A_BYTES), &map_w2, bar, k, n0);
+        tma_load_2d(smem_u32(st + W_BYTES), &map_a, bar, k, t0);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = MODE == kBf16 ? instr_desc(BN) : instr_desc_tf32(BN);
+      uint64_t* ready = MODE == kFp32 ? split_done : full;
+      bool ok = true;
+      for (int i = 0; i < blocks && ok; ++i) {
+        const int s = i % ST, sec = i / M::SECTION, b = sec & 1;
+        const bool opens = i % M::SECTION == 0;
+        if (opens) ok = mbar_wait(smem_u32(&acc_empty[b]), ((sec >> 1) & 1) ^ 1u, stop);
+        if (ok) ok = mbar_wait(smem_u32(&ready[s]), (i / ST) & 1, stop);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t st = smem_u32(base + s * STAGE);
+#pragma unroll
+        for (int z = 0; z < NA; ++z) {
+          const uint32_t d = tmem_d + b * ACC_COLS + z * BN;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {  // 32 bytes of K per instruction, inside the swizzle row
+            const uint32_t joins = (!opens || k > 0) ? 1u : 0u;
+            const uint64_t wd = smem_desc(st + z * A_BYTES + k * 32), ad = smem_desc(st + W_BYTES + k * 32);
+            if constexpr (MODE == kBf16) {
+              mma_bf16(d, wd, ad, idesc, joins);
+            } else {
+              mma_tf32(d, wd, ad, idesc, joins);
+              if constexpr (MODE == kFp32) {
+                mma_tf32(d + TILE_COLS, smem_desc(st + HALF + z * A_BYTES + k * 32), ad, idesc, joins);
+                mma_tf32(d + TILE_COLS, wd, smem_desc(st + HALF + W_BYTES + k * 32), idesc, 1u);
+              }
+            }
+          }
+        }
+        mma_commit(smem_u32(&empty[s]));
+        if ((i + 1) % M::SECTION == 0 || i + 1 == blocks) mma_commit(smem_u32(&acc_full[b]));
+      }
+    }
+  } else if (MODE == kFp32 && warp >= 6) {
+    // the splitting warps: both parts keep the tile's layout, so the swizzle needs no thought
+    bool inf = false;
+    for (int i = 0; i < blocks; ++i) {
+      const int s = i % ST;
+      if (!mbar_wait(smem_u32(&full[s]), (i / ST) & 1, stop)) break;
+      float4* hi = reinterpret_cast<float4*>(base + s * STAGE);
+      float4* lo = reinterpret_cast<float4*>(base + s * STAGE + HALF);
+#pragma unroll 8
+      for (int v = threadIdx.x - 192; v < HALF / 16; v += 128) {
+        float4 x = hi[v], l;
+        x.x = split_hi_lo(x.x, &l.x, &inf);
+        x.y = split_hi_lo(x.y, &l.y, &inf);
+        x.z = split_hi_lo(x.z, &l.z, &inf);
+        x.w = split_hi_lo(x.w, &l.w, &inf);
+        hi[v] = x;
+        lo[v] = l;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read what was written here
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&split_done[s])) : "memory");
+    }
+    if (inf) *special = 1.f;
+  }
+  const int quarter = warp & 3, feature = quarter * 32 + lane;  // of the epilogue warps 2 .. 5
+  const bool epilogue = warp >= 2 && warp < 6;
+  const int row = n0 + feature;
+  float* part = reinterpret_cast<float*>(base);                 // [TILE_COLS][BM], in the place of the ring
+  float acc[TILE_COLS];
+  bool ok = true;
+  if (epilogue) {
+#pragma unroll
+    for (int j = 0; j < TILE_COLS; ++j) acc[j] = 0.f;
+    for (int sec = 0; sec < sections && ok; ++sec) {
+      const int b = sec & 1;
+      ok = mbar_wait(smem_u32(&acc_full[b]), (sec >> 1) & 1, stop);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t from = tmem_d + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(b * ACC_COLS);
+#pragma unroll
+      for (int c = 0; c < TILE_COLS; c += 16) {
+        uint32_t r[16], r2[MODE == kFp32 ? 16 : 1];
+        tmem_ld16(from + c, r);
+        if constexpr (MODE == kFp32) tmem_ld16(from + TILE_COLS + c, r2);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if constexpr (MODE == kFp32) acc[c + j] += __uint_as_float(r[j]) + __uint_as_float(r2[j]);
+          else acc[c + j] += __uint_as_float(r[j]);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+    }
+    // the last section's commit covers every MMA of this CTA: nothing reads or writes the ring any more
+    if (S > 1)
+#pragma unroll
+      for (int j = 0; j < TILE_COLS; ++j) part[j * BM + feature] = acc[j];
+  }
+  __syncwarp();
+  if (S > 1) cluster_sync();  // every partial tile of the cluster is in place
+  else if (MODE == kFp32) __syncthreads();  // and `special` is
+  if (epilogue && ok && row < p.N) {
+    bool recompute = false;
+    if constexpr (MODE == kFp32) {
+      for (int q = 0; q < S; ++q)
+        recompute = recompute || (S > 1 ? ld_peer(peer_smem(smem_u32(special), q)) : *special) != 0.f;
+    }
+    if (MODE == kFp32 && recompute) {  // infinities: the sums as a chain of fp32 multiply-adds gives them
+      const int per = BN / S;
+      for (int j = rank * per; j < (rank + 1) * per && t0 + j < p.T; ++j) {
+        const float* ar = static_cast<const float*>(p.a) + static_cast<size_t>(t0 + j) * p.K;
+        const float* wr = static_cast<const float*>(p.w) + static_cast<size_t>(row) * p.K;
+        const float* wr2 = NA == 2 ? static_cast<const float*>(p.w2) + static_cast<size_t>(row) * p.K : wr;
+        float v = 0.f, u = 0.f;
+        for (int k = 0; k < p.K; ++k) {
+          v = fmaf(ar[k], wr[k], v);
+          if (NA == 2) u = fmaf(ar[k], wr2[k], u);
+        }
+        split_store<MODE, OUT>(p, t0 + j, row, v, u);
+      }
+    } else if (S == 1) {
+#pragma unroll
+      for (int j = 0; j < BN; ++j)
+        if (t0 + j < p.T) split_store<MODE, OUT>(p, t0 + j, row, acc[j], acc[NA == 2 ? BN + j : j]);
+    } else {
+      const uint32_t mine = smem_u32(part + feature);
+      if (S == 8) split_reduce<MODE, BN, OUT, 8>(p, mine, rank, t0, row);
+      else if (S == 4) split_reduce<MODE, BN, OUT, 4>(p, mine, rank, t0, row);
+      else split_reduce<MODE, BN, OUT, 2>(p, mine, rank, t0, row);
+    }
+  }
+  __syncwarp();
+  if (S > 1) cluster_sync();  // no CTA leaves while another one still reads its partial tile
+  if (*stop.here) {  // a wait ran out: give copies in flight time to land before the shared memory is given up
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(TMEM_COLS) : "memory");
+  }
+}
+
+// [rows, cols] row-major, box [box_rows x 128 bytes], 128-byte swizzle
+template <int MODE>
+inline int make_map_of(CUtensorMap* map, const void* ptr, int rows, int cols, int box_rows) {
+  if constexpr (MODE == kBf16) return make_map(map, ptr, rows, cols, box_rows);
+  EncodeTiledFn fn = encode_tiled();
+  if (fn == nullptr) return KLLM_E_NODEVICE;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 4};
+  const cuuint32_t box[2] = {32u, static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : KLLM_E_INVALID;
+}
+
+// How many CTAs share a tile's K: as many as one wave of the grid has room for (`room`), each with at least kMinSplitBlocks
+// blocks; a cluster of 8 is the largest portable one.  A second wave costs more than the shorter chains give (bf16, T = 64,
+// K = 4096, N = 11008, 86 tiles, room for 296: S = 1 35.0, 2 24.8, 4 31.2 us; T = 210, K = 1024, N = 4096, 128 tiles: 14.5,
+// 12.4, 18.6 us).
+inline int split_count(int tiles, int blocks, int room) {
+  int S = 1;
+  while (S < 8 && tiles * S * 2 <= room && blocks >= S * 2 * kMinSplitBlocks) S *= 2;
+  return S;
+}
+
+template <int MODE, int BN, int OUT, int ST>
+inline int launch_split(SplitArgs p, cudaStream_t stream) {
+  constexpr int NA = OUT == kGated ? 2 : 1;
+  CUtensorMap map_w, map_w2, map_a;
+  p.report = wait_flag();
+  if (p.report == nullptr) return KLLM_E_STATE;
+  if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, BM)) return rc;
+  if (int rc = make_map_of<MODE>(&map_w2, NA == 2 ? p.w2 : p.w, p.N, p.K, BM)) return rc;
+  if (int rc = make_map_of<MODE>(&map_a, p.a, p.T, p.K, BN)) return rc;
+  constexpr size_t smem = 1024 + static_cast<size_t>(ST) * (MODE == kFp32 ? 2 : 1) * (NA * A_BYTES + BN * 128) + 256;
+  static_assert(smem <= 232448, "shared memory of one CTA");
+  auto kernel = umma_split_kernel<MODE, BN, OUT, ST>;
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = true;
+  }
+  const int feature_tiles = (p.N + BM - 1) / BM, token_tiles = (p.T + BN - 1) / BN;
+  p.S = split_count(feature_tiles * token_tiles, (p.K + ModeOf<MODE>::BKE - 1) / ModeOf<MODE>::BKE, (smem <= 113 * 1024 ? 2 : 1) * kSms);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(feature_tiles, p.S, token_tiles);
+  cfg.blockDim = dim3(split_threads<MODE>());
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = p.S, attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_w2, map_a, p);
+  count_launch();
+  return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+// the narrowest token block that holds the step, up to 64 tokens per tile
+template <bool GATED>
+int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act,
+               cudaStream_t s) {
+  const void* w2 = static_cast<const __nv_bfloat16*>(w) + static_cast<size_t>(N) * K;  // the up rows follow the gate rows
+  const SplitArgs p{a, w, w2, bias, nullptr, out, T, N, K, 1, act, nullptr};
+  constexpr int OUT = GATED ? kGated : kPlain;
+  if (T <= 16) return launch_split<kBf16, 16, OUT, GATED ? 3 : 5>(p, s);
+  if (T <= 32) return launch_split<kBf16, 32, OUT, GATED ? 3 : 5>(p, s);
+  return launch_split<kBf16, 64, OUT, 4>(p, s);
+}
+
+}  // namespace umma
+}  // namespace seq
+}  // namespace kllm

@@ -102,6 +102,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr) : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+}
+
 // ST: stages of the ring.  A ring of at most ~110 KB leaves room for a second CTA on the SM, whose products run under the
 // first one's epilogue.
 template <int BN, bool GATED, int ST>
@@ -411,12 +420,16 @@ inline int launch_bn(const void* a, const void* w, const float* bias, void* out,
   return static_cast<int>(cudaGetLastError());
 }
 
+// products whose tiles do not fill the chip (seq_gemm_split.cuh)
+template <bool GATED>
+int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act, cudaStream_t s);
+
 template <typename AT>
 inline bool usable(const AT*, const AT*, int, int, int) { return false; }
 template <>
 inline bool usable<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* w, int T, int K, int N) {
   static const bool off = [] { const char* e = getenv("KLLM_SEQ_UMMA"); return e != nullptr && e[0] == '0'; }();
-  return !off && T >= 64 && K >= BK && (K % 8) == 0 && N >= 8 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
+  return !off && T > 8 && K >= BK && (K % 8) == 0 && N >= 8 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(w) & 15) == 0;
 }
 
@@ -426,9 +439,9 @@ template <>
 inline int launch<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* w, const float* bias, float* out, int T, int K,
                                  int N, cudaStream_t s) {
   const GatedAct none{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f};
-  // less than one tile of 128 tokens per SM: narrower token blocks give more CTAs; else two CTAs share an SM
+  // less than one tile of 128 tokens per SM: narrower token blocks and K split over CTAs; else two CTAs share an SM
   const int feature_tiles = (N + BM - 1) / BM;
-  if (T <= 64 || feature_tiles * ((T + 127) / 128) < kSms) return launch_bn<64, false, 4>(a, w, bias, out, T, K, N, none, s);
+  if (T <= 64 || feature_tiles * ((T + 127) / 128) < kSms) return launch_few<false>(a, w, bias, out, T, K, N, none, s);
   return launch_bn<128, false, 3>(a, w, bias, out, T, K, N, none, s);
 }
 
@@ -439,7 +452,7 @@ template <>
 inline int launch_gated<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* w, const float* bias, __nv_bfloat16* out, int T,
                                        int K, int N, const GatedAct& act, cudaStream_t s) {
   const int feature_tiles = (N + BM - 1) / BM;
-  if (T <= 64 || feature_tiles * ((T + 127) / 128) < kSms) return launch_bn<64, true, 4>(a, w, bias, out, T, K, N, act, s);
+  if (T <= 64 || feature_tiles * ((T + 127) / 128) < kSms) return launch_few<true>(a, w, bias, out, T, K, N, act, s);
   return launch_bn<128, true, 2>(a, w, bias, out, T, K, N, act, s);
 }
 

@@ -1,0 +1,50 @@
+"""Products of few tokens, K split over a cluster of CTAs (csrc/seq_gemm_split.cuh), against the product in 64 bits.
+
+bf16: the operands are exact, so only the sums differ: a tcgen05 accumulator keeps about 2^-23 of its value per step and is handed
+over every 8 steps of 16 elements of K, the rest is summed in fp32 -- an element's error stays below 2^-19 of the sum of the
+products' magnitudes.
+"""
+import ctypes
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def call(sq, lib, dtype, a, w, out):
+    import torch
+    rc = lib.kllm_seq_gemm(dtype, ctypes.c_void_p(a.data_ptr()), ctypes.c_void_p(w.data_ptr()), ctypes.c_void_p(out.data_ptr()),
+                           a.shape[0], a.shape[1], w.shape[0], ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+
+
+def product(T, K, N, seed, bf16=True):
+    import torch
+    from kuiperllama_b200 import sequence as sq
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    a = torch.randn(T, K, device="cuda", generator=g)
+    w = torch.randn(N, K, device="cuda", generator=g)
+    if bf16:
+        a, w = a.bfloat16(), w.bfloat16()
+    out = torch.full((T + 1, N), 7.0, device="cuda")  # the row behind the result has to stay as it is
+    call(sq, sq.load_seq_library(), sq.BF16 if bf16 else sq.F32, a, w, out)
+    return a.double(), w.double(), out
+
+
+@pytest.mark.parametrize("T,K,N", [
+    (9, 64, 8), (16, 72, 128), (17, 136, 129), (31, 512, 300), (32, 520, 640), (33, 1032, 1000), (40, 4096, 4096),
+    (63, 2048, 2047), (64, 640, 96), (65, 1024, 1024), (127, 8192, 513), (200, 296, 2100), (24, 4104, 32000)])
+def test_split_product(T, K, N):
+    a, w, out = product(T, K, N, T * 7 + K)
+    bound = 2.0 ** -19 * (a.abs() @ w.abs().T)
+    assert ((out[:T].double() - a @ w.T).abs() <= bound).all()
+    assert (out[T] == 7.0).all()
+
+
+def test_split_product_repeats():
+    """The partial tiles are summed in rank order: the same bits every time."""
+    import torch
+    first = product(40, 4096, 1000, 3)[2]
+    for _ in range(3):
+        assert torch.equal(product(40, 4096, 1000, 3)[2], first)
