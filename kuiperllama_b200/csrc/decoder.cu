@@ -128,6 +128,8 @@ struct kllm_decoder {
   // batched tcgen05 prefill (kllm_decoder_prefill_tf32): activations of one block of prompt positions
   float* pf_buf = nullptr;
   PrefillWorkspace pf_ws{};
+  int pf_rows = 0;                // rows it has, and how many were to be had (kPrefillBlock unless memory was short)
+  int pf_cap = kPrefillBlock;
 };
 
 namespace {
@@ -491,25 +493,39 @@ int kllm_decoder_prefill_tf32(kllm_decoder* dc, const int32_t* tokens_host, int3
   const kllm_decoder_desc& d = dc->d;
   if (start_pos + n_tokens > d.seq_len) return KLLM_E_INVALID;
   if (d.group_size != 0 || d.tp_size > 1) return KLLM_E_UNSUPPORTED;  // fp32 checkpoints, one GPU
-  constexpr int kBlock = 256;  // prompt positions per pass = the N of the tcgen05.mma
   const int hs = dc->head_size, q_rows = d.head_num * hs, kvd = dc->kv_dim;
   if ((d.dim & 3) || (d.hidden_dim & 3) || (q_rows & 3)) return KLLM_E_UNSUPPORTED;
-  if (dc->pf_buf == nullptr) {
-    const size_t per_row = static_cast<size_t>(3 * d.dim + 2 * q_rows + 2 * kvd + 2 * d.hidden_dim);
-    if (cudaMalloc(&dc->pf_buf, per_row * kBlock * sizeof(float)) != cudaSuccess)
-      return static_cast<int>(cudaErrorMemoryAllocation);
+  // activations of a block: as many rows as the prompt has, in steps of 128 up to kPrefillBlock, kept for later prompts; where
+  // memory is short, shorter blocks do
+  const int want_rows = std::min(dc->pf_cap, (n_tokens + 127) / 128 * 128);
+  if (dc->pf_rows < want_rows) {
+    const size_t per_row = static_cast<size_t>(2 * d.dim + 2 * q_rows + 2 * kvd + d.hidden_dim);
+    if (dc->pf_buf != nullptr) {  // (nothing of this decoder is in flight: every call waits for its stream)
+      cudaFree(dc->pf_buf);
+      dc->pf_buf = nullptr;
+    }
+    dc->pf_rows = 0;
+    int rows = want_rows;
+    while (cudaMalloc(&dc->pf_buf, per_row * rows * sizeof(float)) != cudaSuccess) {
+      cudaGetLastError();
+      dc->pf_buf = nullptr;
+      if (rows <= 256) return static_cast<int>(cudaErrorMemoryAllocation);
+      rows /= 2;
+    }
+    dc->pf_rows = rows;
+    if (rows < want_rows) dc->pf_cap = rows;
     float* p = dc->pf_buf;
     auto take = [&](size_t n) {
       float* r = p;
-      p += n * kBlock;
+      p += n * rows;
       return r;
     };
-    dc->pf_ws.x = take(d.dim), dc->pf_ws.xn = take(d.dim), dc->pf_ws.tmp = take(d.dim);
+    dc->pf_ws.x = take(d.dim), dc->pf_ws.xn = take(d.dim);
     dc->pf_ws.q = take(q_rows), dc->pf_ws.att = take(q_rows);
     dc->pf_ws.k = take(kvd), dc->pf_ws.v = take(kvd);
-    dc->pf_ws.h1 = take(d.hidden_dim), dc->pf_ws.h3 = take(d.hidden_dim);
+    dc->pf_ws.h1 = take(d.hidden_dim);
   }
-  KLLM_TRY(prefill_attention_smem_opt_in(static_cast<size_t>(start_pos + n_tokens) * sizeof(float)));
+  const int block = dc->pf_rows;
   PrefillModel m{};
   m.dim = d.dim, m.hidden_dim = d.hidden_dim, m.layer_num = d.layer_num, m.head_num = d.head_num;
   m.kv_head_num = d.kv_head_num, m.vocab_size = d.vocab_size, m.seq_len = d.seq_len, m.head_size = hs;
@@ -526,8 +542,8 @@ int kllm_decoder_prefill_tf32(kllm_decoder* dc, const int32_t* tokens_host, int3
   std::memcpy(dc->io_host, tokens_host, sizeof(int32_t) * n_tokens);
   KLLM_TRY(cudaMemcpyAsync(dc->teacher, dc->io_host, sizeof(int32_t) * n_tokens, cudaMemcpyHostToDevice, dc->stream));
   int last_rows = 0;
-  for (int c0 = 0; c0 < n_tokens; c0 += kBlock) {
-    const int T = std::min(kBlock, n_tokens - c0);
+  for (int c0 = 0; c0 < n_tokens; c0 += block) {
+    const int T = std::min(block, n_tokens - c0);
     KLLM_TRY(prefill_block(m, dc->pf_ws, dc->teacher + c0, T, start_pos + c0, dc->stream));
     last_rows = T;
   }
@@ -554,6 +570,7 @@ int kllm_decoder_prefill_tf32(kllm_decoder* dc, const int32_t* tokens_host, int3
   KLLM_TRY(cudaGetLastError());
   KLLM_TRY(cudaMemcpyAsync(hs_state, dc->st, sizeof(StepState), cudaMemcpyDeviceToHost, dc->stream));
   KLLM_TRY(cudaStreamSynchronize(dc->stream));
+  if (take_wait_error()) return KLLM_E_STATE;
   *next_host = hs_state->next;
   return 0;
 }

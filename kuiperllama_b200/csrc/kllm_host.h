@@ -59,12 +59,16 @@ struct PrefillModel {
   float* key_cache; float* value_cache;
   const float* sin_cache; const float* cos_cache;
 };
+constexpr int kPrefillBlock = 1024;  // prompt positions per pass, at most
 struct PrefillWorkspace {  // [block, .] activations
-  float *x, *xn, *q, *k, *v, *att, *h1, *h3, *tmp;
+  float *x, *xn, *q, *k, *v, *att, *h1;
 };
 int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* tokens_dev, int T, int start_pos,
                   cudaStream_t stream);
-int prefill_attention_smem_opt_in(size_t bytes);
+// prefill_gemm.cu: out = x . w^T (+ bias); residual += x . w^T; out = silu(x . w1^T) * (x . w3^T)
+int prefill_product(const float* x, const float* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s);
+int prefill_product_add(const float* x, const float* w, float* residual, int T, int K, int N, cudaStream_t s);
+int prefill_product_gated(const float* x, const float* w1, const float* w3, float* out, int T, int K, int N, cudaStream_t s);
 
 inline float flavour_eps(int flavour) { return flavour == KLLM_FLAVOUR_QWEN2 ? 1e-6f : 1e-5f; }
 }  // namespace kllm

@@ -4,8 +4,8 @@
 //
 // For a block of T prompt positions every projection is ONE GEMM [T, in] x [out, in]^T on the tensor
 // cores (TF32 multiply, fp32 accumulate) instead of T GEMVs, so the weights are streamed once per
-// 256 tokens; the small per-token operators (RMSNorm, RoPE, causal attention over the cache, SiLU*gate,
-// residual adds) are plain fp32 CUDA kernels over the T rows; only the last position runs the
+// block (kPrefillBlock tokens); bias, SiLU*gate and residual adds ride on the products' epilogues; RMSNorm, RoPE and
+// causal attention over the cache are plain fp32 CUDA kernels over the T rows; only the last position runs the
 // classifier (the reference throws the others away, llama3.cpp:738-739).  The K / V rows land in the
 // decoder's cache in the layout of the engine that will continue decoding.
 //
@@ -64,23 +64,16 @@ __global__ void rmsnorm_rows_kernel(const float* __restrict__ x, const float* __
   const float* row = x + static_cast<size_t>(blockIdx.x) * dim;
   float* o = out + static_cast<size_t>(blockIdx.x) * dim;
   float ss = 0.f;
-  for (int i = threadIdx.x; i < dim; i += blockDim.x) ss += row[i] * row[i];
+  for (int i = threadIdx.x * 4; i < dim; i += blockDim.x * 4) {  // dim % 4 == 0: the products need 16-byte rows
+    const float4 v = *reinterpret_cast<const float4*>(row + i);
+    ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+  }
   const float total = block_sum(ss, scratch);
   const float sc = rsqrtf(total / static_cast<float>(dim) + eps);
-  for (int i = threadIdx.x; i < dim; i += blockDim.x) o[i] = (sc * row[i]) * w[i];
-}
-
-__global__ void add_bias_rows_kernel(float* __restrict__ y, const float* __restrict__ b, int n) {
-  float* row = y + static_cast<size_t>(blockIdx.x) * n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) row[i] += b[i];
-}
-__global__ void add_rows_kernel(float* __restrict__ x, const float* __restrict__ y, size_t n) {
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * blockDim.x)
-    x[i] = x[i] + y[i];  // llama3.cpp:683,719: x + out
-}
-__global__ void swiglu_rows_kernel(float* __restrict__ h1, const float* __restrict__ h3, size_t n) {
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * blockDim.x)
-    h1[i] = swiglu_ref(h1[i], h3[i]);
+  for (int i = threadIdx.x * 4; i < dim; i += blockDim.x * 4) {
+    const float4 v = *reinterpret_cast<const float4*>(row + i);
+    *reinterpret_cast<float4*>(o + i) = make_float4((sc * v.x) * w[i], (sc * v.y) * w[i + 1], (sc * v.z) * w[i + 2], (sc * v.w) * w[i + 3]);
+  }
 }
 
 struct CacheLayout {
@@ -135,7 +128,7 @@ __global__ void rope_scatter_kernel(float* __restrict__ q, const float* __restri
     vcache[v_index(c, pos, p / hs, p % hs)] = vrow[p];
 }
 
-// Causal attention of query (t, head) over cache positions 0 .. start_pos + t (mha_kernel.cu:47-110
+// The same for every other head size: causal attention of query (t, head) over cache positions 0 .. start_pos + t (mha_kernel.cu:47-110
 // arithmetic, fp32).  grid = (heads, T); scores in dynamic shared memory.
 __global__ void attn_rows_kernel(const float* __restrict__ q, const float* __restrict__ kcache,
                                  const float* __restrict__ vcache, float* __restrict__ out, CacheLayout c, int heads,
@@ -169,6 +162,149 @@ __global__ void attn_rows_kernel(const float* __restrict__ q, const float* __res
   }
 }
 
+// Causal attention of the block's queries over cache positions 0 .. start_pos + t (mha_kernel.cu:47-110 arithmetic, fp32
+// throughout), in tiles: a CTA takes 64 queries of one head against tiles of 64 keys, scores and running output in registers
+// (4 x 4 scores and 4 x 4 NV outputs per thread), softmax carried on from tile to tile.  The form before it was one CTA per
+// query and head whose threads each walked whole key rows: every key and value was read from L2 once per query, and half the
+// time one thread per column summed the values alone.  Here a key is read once per 64 queries and the FMA pipe bounds it.
+constexpr int kTileRows = 64, kTileKeys = 64, kPad = 4;
+template <int NV>  // head_size <= 64 NV, a multiple of 4
+__global__ void __launch_bounds__(256)
+attn_tile_kernel(const float* __restrict__ q, const float* __restrict__ kcache, const float* __restrict__ vcache,
+                 float* __restrict__ out, CacheLayout c, int heads, int kv_mul, int start_pos, int T) {
+  constexpr int LDR = kTileRows + kPad, LDV = 64 * NV;
+  extern __shared__ __align__(16) float sm[];
+  const int hs = c.head_size, chunks = hs >> 2;
+  float* Qs = sm;                   // [hs][LDR]
+  float* Ks = Qs + hs * LDR;        // [hs][LDR]
+  float* Vs = Ks + hs * LDR;        // [keys][LDV]
+  float* Ps = Vs + kTileKeys * LDV; // [keys][LDR]
+  const int head = blockIdx.y, kvh = head / kv_mul;
+  const int t0 = (gridDim.x - 1 - blockIdx.x) * kTileRows;  // the tiles with the most keys start first
+  const int rows = min(kTileRows, T - t0);
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const float scale = 1.f / sqrtf(static_cast<float>(hs));
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+
+  for (int i = tid; i < kTileRows * chunks; i += 256) {
+    const int ch = i % chunks, r = i / chunks;
+    const float4 v = r < rows ? *reinterpret_cast<const float4*>(q + (static_cast<size_t>(t0 + r) * heads + head) * hs + ch * 4) : zero;
+    Qs[(ch * 4) * LDR + r] = v.x, Qs[(ch * 4 + 1) * LDR + r] = v.y, Qs[(ch * 4 + 2) * LDR + r] = v.z, Qs[(ch * 4 + 3) * LDR + r] = v.w;
+  }
+  if (hs < LDV)  // the columns past the head stay zero
+    for (int i = tid; i < kTileKeys * LDV; i += 256) Vs[i] = 0.f;
+
+  float o[4][4 * NV], mx[4], sum[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    mx[i] = -FLT_MAX, sum[i] = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4 * NV; ++j) o[i][j] = 0.f;
+  }
+  const int last = start_pos + t0 + rows - 1;
+  for (int j0 = 0; j0 <= last; j0 += kTileKeys) {
+    __syncthreads();  // the tile before is done with (and Qs, Vs are filled)
+    for (int i = tid; i < kTileKeys * chunks; i += 256) {
+      const int r = i % kTileKeys, ch = i / kTileKeys, j = j0 + r;
+      const float4 v = j <= last ? *reinterpret_cast<const float4*>(kcache + k_index(c, j, kvh, ch * 4)) : zero;
+      Ks[(ch * 4) * LDR + r] = v.x, Ks[(ch * 4 + 1) * LDR + r] = v.y, Ks[(ch * 4 + 2) * LDR + r] = v.z, Ks[(ch * 4 + 3) * LDR + r] = v.w;
+    }
+    for (int i = tid; i < kTileKeys * chunks; i += 256) {
+      const int ch = i % chunks, r = i / chunks, j = j0 + r;
+      *reinterpret_cast<float4*>(Vs + r * LDV + ch * 4) =
+          j <= last ? *reinterpret_cast<const float4*>(vcache + v_index(c, j, kvh, ch * 4)) : zero;
+    }
+    __syncthreads();
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < hs; ++d) {
+      const float4 a = *reinterpret_cast<const float4*>(Qs + d * LDR + ty * 4);
+      const float4 b = *reinterpret_cast<const float4*>(Ks + d * LDR + tx * 4);
+      const float ar[4] = {a.x, a.y, a.z, a.w}, br[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = __fmaf_rn(ar[i], br[j], s[i][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int seen = start_pos + t0 + ty * 4 + i - j0 - tx * 4;  // keys 0 .. seen of this thread's four are visible
+      float m = mx[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] *= scale;
+        if (j <= seen) m = fmaxf(m, s[i][j]);
+      }
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(kFull, m, off));
+      // the first tile holds key 0, which every row sees: from then on m is a score
+      const float keep = expf(mx[i] - m);
+      mx[i] = m;
+      sum[i] *= keep;
+#pragma unroll
+      for (int j = 0; j < 4 * NV; ++j) o[i][j] *= keep;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] = j <= seen ? expf(s[i][j] - m) : 0.f;
+        sum[i] += s[i][j];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<float4*>(Ps + (tx * 4 + j) * LDR + ty * 4) = make_float4(s[0][j], s[1][j], s[2][j], s[3][j]);
+    __syncthreads();
+#pragma unroll 4
+    for (int r = 0; r < kTileKeys; ++r) {
+      const float4 p = *reinterpret_cast<const float4*>(Ps + r * LDR + ty * 4);
+      const float pr[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+      for (int n = 0; n < NV; ++n) {
+        const float4 v = *reinterpret_cast<const float4*>(Vs + r * LDV + n * 64 + tx * 4);
+        const float vr[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[i][n * 4 + j] = __fmaf_rn(pr[i], vr[j], o[i][n * 4 + j]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) sum[i] += __shfl_xor_sync(kFull, sum[i], off);
+    const int r = ty * 4 + i;
+    if (r >= rows) continue;
+    float* dst = out + (static_cast<size_t>(t0 + r) * heads + head) * hs;
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+      if (n * 64 + tx * 4 < hs)
+        *reinterpret_cast<float4*>(dst + n * 64 + tx * 4) = make_float4(o[i][n * 4] / sum[i], o[i][n * 4 + 1] / sum[i],
+                                                                        o[i][n * 4 + 2] / sum[i], o[i][n * 4 + 3] / sum[i]);
+  }
+}
+
+inline size_t attn_tile_smem(int hs, int nv) {
+  return (static_cast<size_t>(2 * hs + kTileKeys) * (kTileRows + kPad) + kTileKeys * 64 * nv) * sizeof(float);
+}
+// heads of whole 16-byte chunks up to 128 coordinates, whose value slices are whole chunks too
+inline bool attn_tile_usable(const CacheLayout& c) {
+  return c.head_size <= 128 && (c.head_size & 3) == 0 && ((c.head_size / c.split) & 3) == 0 && (c.kv_dim & 3) == 0;
+}
+template <int NV>
+int launch_attn_tile(const float* q, const float* kcache, const float* vcache, float* out, const CacheLayout& c, int heads,
+                     int kv_mul, int start_pos, int T, cudaStream_t s) {
+  const cudaError_t e = cudaFuncSetAttribute(attn_tile_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(attn_tile_smem(64 * NV, NV)));
+  if (e != cudaSuccess) return static_cast<int>(e);
+  attn_tile_kernel<NV><<<dim3((T + kTileRows - 1) / kTileRows, heads), 256, attn_tile_smem(c.head_size, NV), s>>>(
+      q, kcache, vcache, out, c, heads, kv_mul, start_pos, T);
+  return 0;
+}
+
 }  // namespace prefill
 
 using namespace prefill;
@@ -179,18 +315,25 @@ using namespace prefill;
     if (rc_ != 0) return rc_;              \
   } while (0)
 
+static int attention_smem_opt_in(size_t bytes) {
+  static size_t configured = 0;
+  if (bytes <= 48 * 1024 || bytes <= configured) return 0;
+  const cudaError_t e =
+      cudaFuncSetAttribute(attn_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  if (e != cudaSuccess) return static_cast<int>(e);
+  configured = bytes;
+  return 0;
+}
+
 int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* tokens_dev, int T, int start_pos,
                   cudaStream_t s) {
   const int dim = m.dim, hid = m.hidden_dim, hs = m.head_size, heads = m.head_num, kvh = m.kv_head_num;
   const int q_rows = heads * hs, kvd = kvh * hs;
-  auto gemm = [&](const float* x, const void* w, float* out, int K, int N) {
-    return kllm_gemm_tf32(x, static_cast<const float*>(w), out, T, K, N, s);
-  };
+  auto f32 = [](const void* w) { return static_cast<const float*>(w); };
   auto count = [&]() {
     count_launch();
     return static_cast<int>(cudaGetLastError());
   };
-  const int ew_grid = 592;  // 4 x 148 SMs for the grid-stride elementwise kernels
   embed_rows_kernel<<<T, 256, 0, s>>>(tokens_dev, m.tok_emb, ws.x, dim, m.vocab_size);
   PF_TRY(count());
   const CacheLayout cl{m.mega_layout, m.seq_len, kvd, hs, m.attn_split > 0 ? m.attn_split : 1};
@@ -198,46 +341,29 @@ int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* to
     const size_t layer_off = static_cast<size_t>(l) * m.seq_len * kvd;
     rmsnorm_rows_kernel<<<T, 256, 0, s>>>(ws.x, m.attn_norm[l], ws.xn, dim, m.eps);
     PF_TRY(count());
-    PF_TRY(gemm(ws.xn, m.wq[l], ws.q, dim, q_rows));
-    PF_TRY(gemm(ws.xn, m.wk[l], ws.k, dim, kvd));
-    PF_TRY(gemm(ws.xn, m.wv[l], ws.v, dim, kvd));
-    if (m.bq != nullptr) {
-      add_bias_rows_kernel<<<T, 256, 0, s>>>(ws.q, m.bq[l], q_rows);
-      add_bias_rows_kernel<<<T, 256, 0, s>>>(ws.k, m.bk[l], kvd);
-      add_bias_rows_kernel<<<T, 256, 0, s>>>(ws.v, m.bv[l], kvd);
-      count_launch(2);
-      PF_TRY(count());
-    }
+    PF_TRY(prefill_product(ws.xn, f32(m.wq[l]), m.bq ? m.bq[l] : nullptr, ws.q, T, dim, q_rows, s));
+    PF_TRY(prefill_product(ws.xn, f32(m.wk[l]), m.bq ? m.bk[l] : nullptr, ws.k, T, dim, kvd, s));
+    PF_TRY(prefill_product(ws.xn, f32(m.wv[l]), m.bq ? m.bv[l] : nullptr, ws.v, T, dim, kvd, s));
     rope_scatter_kernel<<<T, 256, 0, s>>>(ws.q, ws.k, ws.v, m.sin_cache, m.cos_cache, m.key_cache + layer_off,
                                           m.value_cache + layer_off, cl, heads, kvh, m.flavour, start_pos);
     PF_TRY(count());
-    const size_t sc_bytes = static_cast<size_t>(start_pos + T) * sizeof(float);
-    attn_rows_kernel<<<dim3(heads, T), 128, sc_bytes, s>>>(ws.q, m.key_cache + layer_off, m.value_cache + layer_off,
-                                                           ws.att, cl, heads, heads / kvh, start_pos);
+    const float *kc = m.key_cache + layer_off, *vc = m.value_cache + layer_off;
+    if (!attn_tile_usable(cl)) {
+      const size_t sc_bytes = static_cast<size_t>(start_pos + T) * sizeof(float);
+      PF_TRY(attention_smem_opt_in(sc_bytes));
+      attn_rows_kernel<<<dim3(heads, T), 128, sc_bytes, s>>>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos);
+    } else if (hs <= 64) {
+      PF_TRY(launch_attn_tile<1>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos, T, s));
+    } else {
+      PF_TRY(launch_attn_tile<2>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos, T, s));
+    }
     PF_TRY(count());
-    PF_TRY(gemm(ws.att, m.wo[l], ws.tmp, q_rows, dim));
-    add_rows_kernel<<<ew_grid, 256, 0, s>>>(ws.x, ws.tmp, static_cast<size_t>(T) * dim);
-    PF_TRY(count());
+    PF_TRY(prefill_product_add(ws.att, f32(m.wo[l]), ws.x, T, q_rows, dim, s));  // llama3.cpp:683
     rmsnorm_rows_kernel<<<T, 256, 0, s>>>(ws.x, m.ffn_norm[l], ws.xn, dim, m.eps);
     PF_TRY(count());
-    PF_TRY(gemm(ws.xn, m.w1[l], ws.h1, dim, hid));
-    PF_TRY(gemm(ws.xn, m.w3[l], ws.h3, dim, hid));
-    swiglu_rows_kernel<<<ew_grid, 256, 0, s>>>(ws.h1, ws.h3, static_cast<size_t>(T) * hid);
-    PF_TRY(count());
-    PF_TRY(gemm(ws.h1, m.w2[l], ws.tmp, hid, dim));
-    add_rows_kernel<<<ew_grid, 256, 0, s>>>(ws.x, ws.tmp, static_cast<size_t>(T) * dim);
-    PF_TRY(count());
+    PF_TRY(prefill_product_gated(ws.xn, f32(m.w1[l]), f32(m.w3[l]), ws.h1, T, dim, hid, s));
+    PF_TRY(prefill_product_add(ws.h1, f32(m.w2[l]), ws.x, T, hid, dim, s));  // llama3.cpp:719
   }
-  return 0;
-}
-
-int prefill_attention_smem_opt_in(size_t bytes) {
-  static size_t configured = 0;
-  if (bytes <= 48 * 1024 || bytes <= configured) return 0;
-  const cudaError_t e =
-      cudaFuncSetAttribute(attn_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  if (e != cudaSuccess) return static_cast<int>(e);
-  configured = bytes;
   return 0;
 }
 

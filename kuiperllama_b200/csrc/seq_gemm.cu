@@ -275,6 +275,20 @@ tiled_kernel(const AT* __restrict__ a, const AT* __restrict__ w, void* __restric
   }
 }
 
+// sorted copy of the rows the grouped product reads: row i = a[sorted_pair[i] / div] (zero where sorted_pair[i] < 0)
+__global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ a, const int32_t* __restrict__ sorted_pair, int div,
+                                   __nv_bfloat16* __restrict__ out, int K) {
+  const int i = blockIdx.x;
+  const int p = sorted_pair[i];
+  uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(i) * K);
+  if (p < 0) {
+    for (int k = threadIdx.x; k < K / 8; k += blockDim.x) dst[k] = make_uint4(0, 0, 0, 0);
+  } else {
+    const uint4* src = reinterpret_cast<const uint4*>(a + static_cast<size_t>(p / div) * K);
+    for (int k = threadIdx.x; k < K / 8; k += blockDim.x) dst[k] = src[k];
+  }
+}
+
 template <typename AT>
 int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s) {
   constexpr int V = Vec16<AT>::N;
@@ -382,7 +396,7 @@ bool grouped_tensor_core_usable(int dtype, int width, int ff) {
 
 int gather_rows_bf16(const void* a, const int32_t* sorted_pair, int div, void* out, int rows, int K, cudaStream_t s) {
   if ((K % 8) != 0) return KLLM_E_UNSUPPORTED;
-  umma::gather_rows_kernel<<<rows, 128, 0, s>>>(static_cast<const __nv_bfloat16*>(a), sorted_pair, div,
+  gather_rows_kernel<<<rows, 128, 0, s>>>(static_cast<const __nv_bfloat16*>(a), sorted_pair, div,
                                                static_cast<__nv_bfloat16*>(out), K);
   count_launch();
   return cuda_rc(cudaGetLastError());

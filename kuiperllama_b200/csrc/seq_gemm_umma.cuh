@@ -353,20 +353,6 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   }
 }
 
-// sorted copy of the rows the grouped product reads: row i = a[sorted_pair[i] / div] (zero where sorted_pair[i] < 0)
-__global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ a, const int32_t* __restrict__ sorted_pair, int div,
-                                   __nv_bfloat16* __restrict__ out, int K) {
-  const int i = blockIdx.x;
-  const int p = sorted_pair[i];
-  uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(i) * K);
-  if (p < 0) {
-    for (int k = threadIdx.x; k < K / 8; k += blockDim.x) dst[k] = make_uint4(0, 0, 0, 0);
-  } else {
-    const uint4* src = reinterpret_cast<const uint4*>(a + static_cast<size_t>(p / div) * K);
-    for (int k = threadIdx.x; k < K / 8; k += blockDim.x) dst[k] = src[k];
-  }
-}
-
 // ---- host ---------------------------------------------------------------------------------------------------------
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
