@@ -1,0 +1,175 @@
+// Causal softmax attention in fp32 multiply-adds, in tiles: the inner loop that the sequence engine's fp32 prompts
+// (seq_attention_f32.cu) and the single-sequence decoder's prompts (prefill.cu) share.
+//
+// 256 threads take 64 rows against tiles of 64 keys.  Thread (tx, ty) of 16 x 16 owns rows ty + 16 i and, of the scores, keys
+// tx + 16 j (4 x 4 of them), of the outputs columns 64 n + 4 tx .. + 3.  Queries, keys, values and weights lie row by row in
+// shared memory, rows padded by 16 bytes: with the rows and keys of a thread 16 apart every 16-byte read of a quarter warp falls
+// on different banks, and nothing has to be transposed on its way in, so tiles come by cp.async, the next under the present one.
+// The FMA pipe bounds it: 64 (128) coordinates take 2 x 64 (128) multiply-adds per score for 1/4 + 1/4 (+ 1/8) 16-byte reads.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cmath>
+#include <cstdint>
+
+namespace kllm {
+namespace f32attn {
+
+constexpr int kRows = 64, kKeys = 64, kThreads = 256, kPad = 4;
+constexpr int LDP = kKeys + kPad;
+
+// shared memory in floats: queries, two tiles of keys, two of values, weights
+inline __host__ __device__ size_t smem_floats(int dim, int nv) {
+  return static_cast<size_t>(3 * kRows) * (dim + kPad) + 2 * kKeys * 64 * nv + kRows * LDP;
+}
+
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool in) {  // 16 zero bytes when !in
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src),
+               "r"(in ? 16 : 0));
+}
+
+template <int NV>
+struct Sums {  // of rows ty + 16 i
+  float o[4][4 * NV], m[4], l[4];  // l: this thread's keys only until finish()
+  __device__ __forceinline__ void finish() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], off);
+  }
+};
+
+// Work: q(row) -> the row's query (nullptr: no such row), key(j, c) and value(j, c) -> 16 bytes number c of key / value j (nullptr:
+// zeros), n_tiles, tile(i) -> number of the i-th tile, hidden(row, j) -> row does not see key j, whole(tile) -> every row sees all
+// of it; score(s) -> the score of a product of query and key.
+template <int NV, class Work>
+__device__ __forceinline__ void attend(const Work& w, int dim, int vdim, float* sm, Sums<NV>& r) {
+  constexpr int LDV = 64 * NV;
+  const int LD = dim + kPad, qc = dim >> 2, vc = vdim >> 2;
+  float* Qs = sm;
+  float* Ks = Qs + kRows * LD;          // [2][keys][LD]
+  float* Vs = Ks + 2 * kKeys * LD;      // [2][keys][LDV]
+  float* Ps = Vs + 2 * kKeys * LDV;     // [rows][LDP]
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+
+  auto load = [&](int i, int stage) {
+    const int j0 = w.tile(i) * kKeys;
+    float* kd = Ks + stage * kKeys * LD;
+    float* vd = Vs + stage * kKeys * LDV;
+    for (int z = tid; z < kKeys * qc; z += kThreads) {
+      int j, c;
+      if (w.keys_by_chunk()) j = z % kKeys, c = z / kKeys;
+      else j = z / qc, c = z % qc;
+      const float* src = w.key(j0 + j, c);
+      copy16(kd + j * LD + c * 4, src ? src : w.any(), src != nullptr);
+    }
+    for (int z = tid; z < kKeys * vc; z += kThreads) {
+      const int j = z / vc, c = z % vc;
+      const float* src = w.value(j0 + j, c);
+      copy16(vd + j * LDV + c * 4, src ? src : w.any(), src != nullptr);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  for (int z = tid; z < kRows * qc; z += kThreads) {
+    const int row = z / qc, c = z % qc;
+    const float* src = w.q(row);
+    copy16(Qs + row * LD + c * 4, src ? src + c * 4 : w.any(), src != nullptr);
+  }
+  if (vdim < LDV)  // the columns past the values stay zero
+    for (int z = tid; z < 2 * kKeys * (LDV - vdim); z += kThreads) Vs[(z / (LDV - vdim)) * LDV + vdim + z % (LDV - vdim)] = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    r.m[i] = -INFINITY, r.l[i] = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4 * NV; ++j) r.o[i][j] = 0.f;
+  }
+  if (w.n_tiles > 0) load(0, 0);
+  for (int t = 0; t < w.n_tiles; ++t) {
+    const int stage = t & 1, tile = w.tile(t);
+    if (t + 1 < w.n_tiles) {
+      load(t + 1, stage ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+    const float* qp = Qs + ty * LD;
+    const float* kp = Ks + (stage * kKeys + tx) * LD;
+#pragma unroll 2
+    for (int d = 0; d < dim; d += 4) {
+      float4 a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(qp + i * 16 * LD + d);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(kp + j * 16 * LD + d);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
+          s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
+          s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
+          s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+        }
+    }
+    const bool whole = w.whole(tile);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float m = r.m[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] = w.score(s[i][j]);
+        if (!whole && w.hidden(ty + 16 * i, tile * kKeys + tx + 16 * j)) s[i][j] = -INFINITY;
+        m = fmaxf(m, s[i][j]);
+      }
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+      // a row that has seen nothing yet keeps max = -inf; subtracting 0 instead keeps exp(-inf - 0) = 0 free of NaN
+      const float sub = m > -INFINITY ? m : 0.f, keep = expf(r.m[i] - sub);
+      r.m[i] = m;
+      r.l[i] *= keep;
+#pragma unroll
+      for (int j = 0; j < 4 * NV; ++j) r.o[i][j] *= keep;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float p = expf(s[i][j] - sub);
+        r.l[i] += p;
+        Ps[(ty + 16 * i) * LDP + tx + 16 * j] = p;
+      }
+    }
+    __syncwarp();  // the rows of a warp's two ty are written and read by that warp alone
+    const float* pp = Ps + ty * LDP;
+    const float* vp = Vs + stage * kKeys * LDV + tx * 4;
+#pragma unroll 2
+    for (int j = 0; j < kKeys; j += 4) {
+      float4 p[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(pp + i * 16 * LDP + j);
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float4 v = *reinterpret_cast<const float4*>(vp + (j + k) * LDV + n * 64);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float pk = k == 0 ? p[i].x : k == 1 ? p[i].y : k == 2 ? p[i].z : p[i].w;
+            r.o[i][n * 4] = fmaf(pk, v.x, r.o[i][n * 4]);
+            r.o[i][n * 4 + 1] = fmaf(pk, v.y, r.o[i][n * 4 + 1]);
+            r.o[i][n * 4 + 2] = fmaf(pk, v.z, r.o[i][n * 4 + 2]);
+            r.o[i][n * 4 + 3] = fmaf(pk, v.w, r.o[i][n * 4 + 3]);
+          }
+        }
+    }
+    __syncthreads();  // the stage is loaded again two tiles on
+  }
+  r.finish();
+}
+
+}  // namespace f32attn
+}  // namespace kllm

@@ -18,6 +18,7 @@
 #include <cstdint>
 
 #include "../../include/kllm_b200.h"
+#include "f32_attention.cuh"
 #include "kllm_device.cuh"
 #include "kllm_host.h"
 
@@ -163,133 +164,54 @@ __global__ void attn_rows_kernel(const float* __restrict__ q, const float* __res
 }
 
 // Causal attention of the block's queries over cache positions 0 .. start_pos + t (mha_kernel.cu:47-110 arithmetic, fp32
-// throughout), in tiles: a CTA takes 64 queries of one head against tiles of 64 keys, scores and running output in registers
-// (4 x 4 scores and 4 x 4 NV outputs per thread), softmax carried on from tile to tile.  The form before it was one CTA per
-// query and head whose threads each walked whole key rows: every key and value was read from L2 once per query, and half the
-// time one thread per column summed the values alone.  Here a key is read once per 64 queries and the FMA pipe bounds it.
-constexpr int kTileRows = 64, kTileKeys = 64, kPad = 4;
+// throughout), in tiles: a CTA takes 64 queries of one head against tiles of 64 keys (f32_attention.cuh).  The form before it was
+// one CTA per query and head whose threads each walked whole key rows: every key and value was read from L2 once per query, and
+// half the time one thread per column summed the values alone.  Here a key is read once per 64 queries and the FMA pipe bounds it.
+struct CacheWork {
+  const float *qb, *kb, *vb;
+  CacheLayout c;
+  int heads, head, kvh, start_pos, t0, rows, last, n_tiles;
+  float scale;
+
+  // the persistent engine's keys lie chunk by chunk, the other layout's and all values row by row
+  __device__ __forceinline__ bool keys_by_chunk() const { return c.mega != 0; }
+  __device__ __forceinline__ const float* any() const { return kb; }
+  __device__ __forceinline__ const float* q(int row) const {
+    return row < rows ? qb + (static_cast<size_t>(t0 + row) * heads + head) * c.head_size : nullptr;
+  }
+  __device__ __forceinline__ const float* key(int j, int ch) const { return j <= last ? kb + k_index(c, j, kvh, ch * 4) : nullptr; }
+  __device__ __forceinline__ const float* value(int j, int ch) const { return j <= last ? vb + v_index(c, j, kvh, ch * 4) : nullptr; }
+  __device__ __forceinline__ int tile(int i) const { return i; }
+  __device__ __forceinline__ bool hidden(int row, int j) const { return j > start_pos + t0 + row; }
+  __device__ __forceinline__ bool whole(int t) const { return t * f32attn::kKeys + f32attn::kKeys - 1 <= start_pos + t0; }
+  __device__ __forceinline__ float score(float s) const { return s * scale; }
+};
 template <int NV>  // head_size <= 64 NV, a multiple of 4
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(f32attn::kThreads)
 attn_tile_kernel(const float* __restrict__ q, const float* __restrict__ kcache, const float* __restrict__ vcache,
                  float* __restrict__ out, CacheLayout c, int heads, int kv_mul, int start_pos, int T) {
-  constexpr int LDR = kTileRows + kPad, LDV = 64 * NV;
   extern __shared__ __align__(16) float sm[];
-  const int hs = c.head_size, chunks = hs >> 2;
-  float* Qs = sm;                   // [hs][LDR]
-  float* Ks = Qs + hs * LDR;        // [hs][LDR]
-  float* Vs = Ks + hs * LDR;        // [keys][LDV]
-  float* Ps = Vs + kTileKeys * LDV; // [keys][LDR]
-  const int head = blockIdx.y, kvh = head / kv_mul;
-  const int t0 = (gridDim.x - 1 - blockIdx.x) * kTileRows;  // the tiles with the most keys start first
-  const int rows = min(kTileRows, T - t0);
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const float scale = 1.f / sqrtf(static_cast<float>(hs));
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-
-  for (int i = tid; i < kTileRows * chunks; i += 256) {
-    const int ch = i % chunks, r = i / chunks;
-    const float4 v = r < rows ? *reinterpret_cast<const float4*>(q + (static_cast<size_t>(t0 + r) * heads + head) * hs + ch * 4) : zero;
-    Qs[(ch * 4) * LDR + r] = v.x, Qs[(ch * 4 + 1) * LDR + r] = v.y, Qs[(ch * 4 + 2) * LDR + r] = v.z, Qs[(ch * 4 + 3) * LDR + r] = v.w;
-  }
-  if (hs < LDV)  // the columns past the head stay zero
-    for (int i = tid; i < kTileKeys * LDV; i += 256) Vs[i] = 0.f;
-
-  float o[4][4 * NV], mx[4], sum[4];
+  const int hs = c.head_size, head = blockIdx.y;
+  const int t0 = (gridDim.x - 1 - blockIdx.x) * f32attn::kRows;  // the tiles with the most keys start first
+  const int rows = min(f32attn::kRows, T - t0), last = start_pos + t0 + rows - 1;
+  const CacheWork w{q, kcache, vcache, c, heads, head, head / kv_mul, start_pos, t0, rows, last, last / f32attn::kKeys + 1,
+                    1.f / sqrtf(static_cast<float>(hs))};
+  f32attn::Sums<NV> r;
+  f32attn::attend<NV>(w, hs, hs, sm, r);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    mx[i] = -FLT_MAX, sum[i] = 0.f;
-#pragma unroll
-    for (int j = 0; j < 4 * NV; ++j) o[i][j] = 0.f;
-  }
-  const int last = start_pos + t0 + rows - 1;
-  for (int j0 = 0; j0 <= last; j0 += kTileKeys) {
-    __syncthreads();  // the tile before is done with (and Qs, Vs are filled)
-    for (int i = tid; i < kTileKeys * chunks; i += 256) {
-      const int r = i % kTileKeys, ch = i / kTileKeys, j = j0 + r;
-      const float4 v = j <= last ? *reinterpret_cast<const float4*>(kcache + k_index(c, j, kvh, ch * 4)) : zero;
-      Ks[(ch * 4) * LDR + r] = v.x, Ks[(ch * 4 + 1) * LDR + r] = v.y, Ks[(ch * 4 + 2) * LDR + r] = v.z, Ks[(ch * 4 + 3) * LDR + r] = v.w;
-    }
-    for (int i = tid; i < kTileKeys * chunks; i += 256) {
-      const int ch = i % chunks, r = i / chunks, j = j0 + r;
-      *reinterpret_cast<float4*>(Vs + r * LDV + ch * 4) =
-          j <= last ? *reinterpret_cast<const float4*>(vcache + v_index(c, j, kvh, ch * 4)) : zero;
-    }
-    __syncthreads();
-    float s[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-#pragma unroll 4
-    for (int d = 0; d < hs; ++d) {
-      const float4 a = *reinterpret_cast<const float4*>(Qs + d * LDR + ty * 4);
-      const float4 b = *reinterpret_cast<const float4*>(Ks + d * LDR + tx * 4);
-      const float ar[4] = {a.x, a.y, a.z, a.w}, br[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s[i][j] = __fmaf_rn(ar[i], br[j], s[i][j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int seen = start_pos + t0 + ty * 4 + i - j0 - tx * 4;  // keys 0 .. seen of this thread's four are visible
-      float m = mx[i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        s[i][j] *= scale;
-        if (j <= seen) m = fmaxf(m, s[i][j]);
-      }
-#pragma unroll
-      for (int off = 8; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(kFull, m, off));
-      // the first tile holds key 0, which every row sees: from then on m is a score
-      const float keep = expf(mx[i] - m);
-      mx[i] = m;
-      sum[i] *= keep;
-#pragma unroll
-      for (int j = 0; j < 4 * NV; ++j) o[i][j] *= keep;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        s[i][j] = j <= seen ? expf(s[i][j] - m) : 0.f;
-        sum[i] += s[i][j];
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      *reinterpret_cast<float4*>(Ps + (tx * 4 + j) * LDR + ty * 4) = make_float4(s[0][j], s[1][j], s[2][j], s[3][j]);
-    __syncthreads();
-#pragma unroll 4
-    for (int r = 0; r < kTileKeys; ++r) {
-      const float4 p = *reinterpret_cast<const float4*>(Ps + r * LDR + ty * 4);
-      const float pr[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-      for (int n = 0; n < NV; ++n) {
-        const float4 v = *reinterpret_cast<const float4*>(Vs + r * LDV + n * 64 + tx * 4);
-        const float vr[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) o[i][n * 4 + j] = __fmaf_rn(pr[i], vr[j], o[i][n * 4 + j]);
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-#pragma unroll
-    for (int off = 8; off > 0; off >>= 1) sum[i] += __shfl_xor_sync(kFull, sum[i], off);
-    const int r = ty * 4 + i;
-    if (r >= rows) continue;
-    float* dst = out + (static_cast<size_t>(t0 + r) * heads + head) * hs;
+    const int row = ty + 16 * i;
+    if (row >= rows) continue;
+    float* dst = out + (static_cast<size_t>(t0 + row) * heads + head) * hs;
 #pragma unroll
     for (int n = 0; n < NV; ++n)
       if (n * 64 + tx * 4 < hs)
-        *reinterpret_cast<float4*>(dst + n * 64 + tx * 4) = make_float4(o[i][n * 4] / sum[i], o[i][n * 4 + 1] / sum[i],
-                                                                        o[i][n * 4 + 2] / sum[i], o[i][n * 4 + 3] / sum[i]);
+        *reinterpret_cast<float4*>(dst + n * 64 + tx * 4) =
+            make_float4(r.o[i][n * 4] / r.l[i], r.o[i][n * 4 + 1] / r.l[i], r.o[i][n * 4 + 2] / r.l[i], r.o[i][n * 4 + 3] / r.l[i]);
   }
 }
 
-inline size_t attn_tile_smem(int hs, int nv) {
-  return (static_cast<size_t>(2 * hs + kTileKeys) * (kTileRows + kPad) + kTileKeys * 64 * nv) * sizeof(float);
-}
 // heads of whole 16-byte chunks up to 128 coordinates, whose value slices are whole chunks too
 inline bool attn_tile_usable(const CacheLayout& c) {
   return c.head_size <= 128 && (c.head_size & 3) == 0 && ((c.head_size / c.split) & 3) == 0 && (c.kv_dim & 3) == 0;
@@ -298,9 +220,10 @@ template <int NV>
 int launch_attn_tile(const float* q, const float* kcache, const float* vcache, float* out, const CacheLayout& c, int heads,
                      int kv_mul, int start_pos, int T, cudaStream_t s) {
   const cudaError_t e = cudaFuncSetAttribute(attn_tile_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(attn_tile_smem(64 * NV, NV)));
+                                             static_cast<int>(f32attn::smem_floats(64 * NV, NV) * sizeof(float)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  attn_tile_kernel<NV><<<dim3((T + kTileRows - 1) / kTileRows, heads), 256, attn_tile_smem(c.head_size, NV), s>>>(
+  attn_tile_kernel<NV><<<dim3((T + f32attn::kRows - 1) / f32attn::kRows, heads), f32attn::kThreads,
+                         f32attn::smem_floats(c.head_size, NV) * sizeof(float), s>>>(
       q, kcache, vcache, out, c, heads, kv_mul, start_pos, T);
   return 0;
 }

@@ -1,5 +1,6 @@
 // Matrix products of the sequence-batch engine:  out[T, N] (fp32) = a[T, K] . w[N, K]^T, a and w in the compute type
-// (float: true fp32 multiply-add, no reduced-precision tensor mode; __nv_bfloat16: bf16 operands, fp32 accumulation).
+// (float: fp32 accuracy -- multiply-adds, or tensor-core products of operands in two TF32 parts; __nv_bfloat16: bf16 operands,
+// fp32 accumulation).
 //
 //   rows_kernel     T <= 8 (decode steps): the weights are streamed once, a warp per output feature, all rows of `a`
 //                   against each 16-byte weight vector -- bound by the weight bytes
@@ -8,7 +9,8 @@
 // the activation in its epilogue and writes the compute type.
 //   umma_kernel     bf16, T > 8, K % 8 == 0: 128 weight rows x BN tokens per CTA on tcgen05.mma (kind::f16, operands
 //                   by TMA with 128-byte swizzle, accumulator in TMEM)                      [seq_gemm_umma.cuh]
-//   umma_split_kernel  the same where the tiles are fewer than the SMs: K split over a cluster  [seq_gemm_split.cuh]
+//   umma_split_kernel  the same where the tiles are fewer than the SMs: K split over a cluster; fp32 with T > 8 and
+//                   K % 4 == 0, each operand as two TF32 parts                              [seq_gemm_split.cuh]
 //   grouped_kernel  the tiled kernel over row blocks that each belong to one expert (rows gathered by index, the
 //                   SiLU-gate product as an optional epilogue)
 #include <cuda_bf16.h>
@@ -16,6 +18,7 @@
 
 #include <cstdint>
 #include <cstdlib>
+#include <type_traits>
 
 #include "seq_engine.h"
 #include "seq_gemm_split.cuh"
@@ -312,6 +315,9 @@ int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K
   if (umma::usable<AT>(a, w, T, K, N)) {
     return umma::launch(a, w, bias, out, T, K, N, s);
   }
+  if constexpr (std::is_same_v<AT, float>)
+    if (umma::fp32_usable(a, w, T, K))
+      return umma::launch_fp32<false>(a, w, bias, out, T, K, N, GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}, s);
   const dim3 grid((N + TN - 1) / TN, (T + TM - 1) / TM);
   tiled_kernel<AT, false, 0><<<grid, 256, 0, s>>>(a, w, out, T, K, N, nullptr, nullptr, 1,
                                                  GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}, bias);
@@ -343,6 +349,8 @@ int gemm_gated_t(const AT* a, const AT* w, const float* bias, AT* out, int T, in
   if (umma::usable<AT>(a, w, T, K, N)) {
     return umma::launch_gated(a, w, bias, out, T, K, N, act, s);
   }
+  if constexpr (std::is_same_v<AT, float>)
+    if (umma::fp32_usable(a, w, T, K)) return umma::launch_fp32<true>(a, w, bias, out, T, K, N, act, s);
   const dim3 grid((N + TN - 1) / TN, (T + TM - 1) / TM);
   tiled_kernel<AT, false, 1><<<grid, 256, 0, s>>>(a, w, out, T, K, N, nullptr, nullptr, 1, act, bias);
   count_launch();

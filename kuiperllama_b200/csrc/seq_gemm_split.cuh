@@ -24,6 +24,9 @@
 //   bf16  T = 40, K = 4096, N = 4096    298 -> 14.6 us    6.1e-7 -> 1.4e-7
 //   bf16  T = 24, K = 2048, N = 2048    149 -> 10.4 us    3.9e-7 -> 1.3e-7
 //   bf16  T = 24, K = 2048, N = 32000   382 -> 28.8 us    3.9e-7 -> 1.4e-7
+//   fp32  T = 16, K = 2048, N = 2048    158 -> 17.7 us    8.1e-7 -> 2.9e-7
+//   fp32  T = 64, K = 4096, N = 4096    314 -> 39.1 us    1.1e-6 -> 2.9e-7
+//   fp32  T = 517, K = 1024, N = 3072   161 -> 47.2 us    5.7e-7 -> 2.9e-7
 #pragma once
 #include "seq_gemm_umma.cuh"
 
@@ -437,6 +440,24 @@ int launch_few(const void* a, const void* w, const float* bias, void* out, int T
   if (T <= 16) return launch_split<kBf16, 16, OUT, GATED ? 3 : 5>(p, s);
   if (T <= 32) return launch_split<kBf16, 32, OUT, GATED ? 3 : 5>(p, s);
   return launch_split<kBf16, 64, OUT, 4>(p, s);
+}
+
+// fp32 operands, fp32 accuracy: whole 16-byte rows, and more rows than the kernel that streams weights once takes
+inline bool fp32_usable(const void* a, const void* w, int T, int K) {
+  static const bool off = [] { const char* e = getenv("KLLM_SEQ_UMMA"); return e != nullptr && e[0] == '0'; }();
+  return !off && T > 8 && K >= 32 && (K % 4) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
+         (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+}
+template <bool GATED>
+int launch_fp32(const float* a, const float* w, const float* bias, float* out, int T, int K, int N, const GatedAct& act,
+                cudaStream_t s) {
+  const SplitArgs p{a, w, w + static_cast<size_t>(N) * K, bias, nullptr, out, T, N, K, 1, act, nullptr};
+  constexpr int OUT = GATED ? kGated : kPlain;
+  if (T <= 16) return launch_split<kFp32, 16, OUT, 3>(p, s);
+  if (T <= 32) return launch_split<kFp32, 32, OUT, 3>(p, s);
+  if (GATED || T <= 64) return launch_split<kFp32, 64, OUT, GATED ? 2 : 4>(p, s);
+  if constexpr (!GATED) return launch_split<kFp32, 128, OUT, 3>(p, s);
+  return KLLM_E_UNSUPPORTED;
 }
 
 }  // namespace umma

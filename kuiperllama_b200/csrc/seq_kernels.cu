@@ -1633,6 +1633,9 @@ int launch_attention(int dtype, const AttnShape& a, const void* q, const float* 
     rc = launch_attention_mma(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws,
                               out, s);
     if (rc || (splits == 1 && !a.no_merge)) return rc;
+  } else if (attention_f32_usable(dtype, a, kv, max_count)) {
+    rc = launch_attention_f32(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, s);
+    if (rc || (splits == 1 && !a.no_merge)) return rc;
   } else if (attention_rows_mma_usable(dtype, a, kv, n_entries)) {
     rc = launch_attention_rows_mma(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, s);
   } else if (a.vdim > 4 * kAttnKeys || a.dim > kAttnMaxDim || attention_tile_bytes(a) > kAttnMaxTileBytes) {

@@ -48,3 +48,36 @@ def test_split_product_repeats():
     first = product(40, 4096, 1000, 3)[2]
     for _ in range(3):
         assert torch.equal(product(40, 4096, 1000, 3)[2], first)
+
+
+@pytest.mark.parametrize("T,K,N", [
+    (9, 32, 8), (16, 36, 128), (17, 100, 129), (32, 2048, 300), (33, 1028, 640), (64, 4096, 1000), (65, 288, 96),
+    (128, 512, 2047), (129, 1024, 1024), (517, 1024, 513)])
+def test_split_product_fp32(T, K, N):
+    """fp32 operands as two TF32 parts: left out are products of two low parts (2^-20 of the product at most) and the low
+    parts' rounding (2^-22 each); with the sums' 2^-20 an element stays within 2^-18 of the sum of the products' magnitudes."""
+    a, w, out = product(T, K, N, T * 5 + K, bf16=False)
+    bound = 2.0 ** -18 * (a.abs() @ w.abs().T)
+    assert ((out[:T].double() - a @ w.T).abs() <= bound).all()
+    assert (out[T] == 7.0).all()
+
+
+@pytest.mark.parametrize("T", [12, 40, 200])
+def test_split_product_fp32_keeps_infinities_and_nans(T):
+    """An infinity has no low part: such tiles are summed by multiply-adds, so inf stays inf and only inf * 0, inf - inf and NaN
+    give NaN; the largest finite value does not become infinite."""
+    import torch
+    from kuiperllama_b200 import sequence as sq
+    g = torch.Generator(device="cuda").manual_seed(T)
+    a, w = torch.randn(T, 256, device="cuda", generator=g), torch.randn(300, 256, device="cuda", generator=g)
+    a[1, 5], a[3, 200], a[7, 9], w[4, 70], w[250, 5] = float("inf"), -float("inf"), float("nan"), float("inf"), 0.0
+    a[5], w[9] = 0.0, 0.0
+    a[5, 3], w[9, 3] = torch.finfo(torch.float32).max, 0.5
+    out = torch.empty(T, 300, device="cuda")
+    call(sq, sq.load_seq_library(), sq.F32, a, w, out)
+    ref = (a.double() @ w.double().T).float()
+    assert torch.equal(out.isnan(), ref.isnan())
+    assert torch.equal(out == float("inf"), ref == float("inf"))
+    assert torch.equal(out == -float("inf"), ref == -float("inf"))
+    fine = ref.isfinite()
+    assert torch.allclose(out[fine], ref[fine], rtol=1e-5, atol=1e-4)
