@@ -430,7 +430,7 @@ inline int launch_split(SplitArgs p, cudaStream_t stream) {
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 
-// the narrowest token block that holds the step, up to 64 tokens per tile
+// the narrowest token block that holds the step; more than 128 tokens (gated: 64) in tiles of 64
 template <bool GATED>
 int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act,
                cudaStream_t s) {
@@ -439,6 +439,8 @@ int launch_few(const void* a, const void* w, const float* bias, void* out, int T
   constexpr int OUT = GATED ? kGated : kPlain;
   if (T <= 16) return launch_split<kBf16, 16, OUT, GATED ? 3 : 5>(p, s);
   if (T <= 32) return launch_split<kBf16, 32, OUT, GATED ? 3 : 5>(p, s);
+  if constexpr (!GATED)
+    if (T > 64 && T <= 128) return launch_split<kBf16, 128, OUT, 3>(p, s);  // one tile: the weights are read once
   return launch_split<kBf16, 64, OUT, 4>(p, s);
 }
 
