@@ -5,15 +5,16 @@
 //   kTf32    fp32 operands read as TF32 (10 mantissa bits): the toleranced prompt path of the single-sequence decoder
 //   kFp32    fp32 operands, products to fp32 accuracy: every operand is hi + lo, hi its leading 11 bits and lo the rest rounded
 //            to 11 bits, and a . w = hi hi + (lo hi + hi lo); what is left out (lo lo, lo's rounding) is below 2^-20 of the
-//            product.  Four warps split each tile in shared memory between its arrival and its use.
+//            product.  hi is the operand as it arrived -- kind::tf32 reads 11 bits of it, truncating --, four warps write lo
+//            beside it between the tile's arrival and its use.
 //
 // What bounds it: with a few dozen tokens the weights are read once and every element of them feeds 2 * T multiply-adds, so
 // the time is the weights' way from HBM.  A tile per 128 features leaves most SMs without work (width 4096: 32 tiles), and
 // one CTA's ring does not keep enough bytes on the way.  So K is split over the S CTAs of a cluster: each runs the ring of
 // the large form over its part of K, leaves its partial tile in its own shared memory, and after a cluster barrier every
 // CTA sums BN / S of the tile's tokens over the S partials, read through distributed shared memory in rank order (the
-// result does not depend on timing).  kFp32 on token blocks is bound by shared memory instead: a stage is read and written
-// by the splitting warps (96 KB at BN = 128) and read three times over by the MMAs.
+// result does not depend on timing).  kFp32 on token blocks is bound by shared memory instead: a stage is read by the splitting
+// warps and its lo part written (64 KB at BN = 128), and the MMAs read it three times over (96 KB).
 //
 // Precision: a tcgen05 accumulator is not rounded to nearest at each of its steps, and its error grows with their number.  A
 // CTA hands its accumulator over every SECTION blocks of K to the epilogue warps, which sum the sections in fp32 registers
@@ -77,16 +78,13 @@ __device__ __forceinline__ float ld_peer(uint32_t addr) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
   return v;
 }
-// hi keeps the sign, the exponent and ten mantissa bits (never rounded up, so it cannot overflow), lo is x - hi, which is exact,
-// rounded to eleven bits.  An infinity has no such form (inf - inf): it is hi alone, and raises `special`.
-__device__ __forceinline__ float split_hi_lo(float x, float* lo, bool* special) {
-  const float hi = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
-  const bool inf = fabsf(x) == INFINITY;
-  uint32_t l;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(x - hi));
-  *lo = inf ? 0.f : __uint_as_float(l);
-  *special = *special || inf;
-  return hi;
+// x - hi, hi being what kind::tf32 reads of x: sign, exponent and ten mantissa bits, never rounded up, so it cannot overflow.  The
+// difference is exact and holds 13 bits; half of the 11th one's unit is added to its magnitude, so that reading it in the same way
+// rounds it to nearest.  An infinity has no such form (inf - inf): `check` becomes NaN for it, as for a NaN.
+__device__ __forceinline__ float low_part(float x, float& check) {
+  const float lo = x - __uint_as_float(__float_as_uint(x) & 0xffffe000u);
+  check = fmaf(lo, 0.f, check);
+  return __uint_as_float(__float_as_uint(lo) + 0x1000u);
 }
 
 // what a product does with its sums
@@ -166,7 +164,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   using M = ModeOf<MODE>;
   constexpr int NA = OUT == kGated ? 2 : 1;
   constexpr int W_BYTES = NA * A_BYTES, B_BYTES = BN * 128;
-  constexpr int HALF = W_BYTES + B_BYTES;                  // the tiles as they arrive (kFp32: then their hi parts)
+  constexpr int HALF = W_BYTES + B_BYTES;                  // the tiles as they arrive
   constexpr int STAGE = MODE == kFp32 ? 2 * HALF : HALF;   // kFp32: the lo parts follow
   constexpr int TILE_COLS = NA * BN;                       // of one sum
   constexpr int ACC_COLS = MODE == kFp32 ? 2 * TILE_COLS : TILE_COLS;  // of one accumulator; there are two
@@ -177,12 +175,12 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(base + ST * STAGE);
   uint64_t* empty = full + ST;
-  uint64_t* split_done = empty + ST;      // kFp32: the stage holds hi and lo parts
+  uint64_t* split_done = empty + ST;      // kFp32: the stage holds the lo parts too
   uint64_t* acc_full = split_done + ST;   // [2]
   uint64_t* acc_empty = acc_full + 2;     // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), p.report};
-  float* special = reinterpret_cast<float*>(tmem_slot + 2);  // kFp32: != 0 when an operand of this CTA's part of K is infinite
+  float* special = reinterpret_cast<float*>(tmem_slot + 2);  // kFp32: != 0 when an operand of this CTA's part of K is not finite
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * BM, t0 = blockIdx.z * BN;
@@ -266,27 +264,22 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
   } else if (MODE == kFp32 && warp >= 6) {
     // the splitting warps: both parts keep the tile's layout, so the swizzle needs no thought
-    bool inf = false;
+    float check = 0.f;
     for (int i = 0; i < blocks; ++i) {
       const int s = i % ST;
       if (!mbar_wait(smem_u32(&full[s]), (i / ST) & 1, stop)) break;
-      float4* hi = reinterpret_cast<float4*>(base + s * STAGE);
+      const float4* tile = reinterpret_cast<const float4*>(base + s * STAGE);
       float4* lo = reinterpret_cast<float4*>(base + s * STAGE + HALF);
 #pragma unroll 8
       for (int v = threadIdx.x - 192; v < HALF / 16; v += 128) {
-        float4 x = hi[v], l;
-        x.x = split_hi_lo(x.x, &l.x, &inf);
-        x.y = split_hi_lo(x.y, &l.y, &inf);
-        x.z = split_hi_lo(x.z, &l.z, &inf);
-        x.w = split_hi_lo(x.w, &l.w, &inf);
-        hi[v] = x;
-        lo[v] = l;
+        const float4 x = tile[v];
+        lo[v] = make_float4(low_part(x.x, check), low_part(x.y, check), low_part(x.z, check), low_part(x.w, check));
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read what was written here
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&split_done[s])) : "memory");
     }
-    if (inf) *special = 1.f;
+    if (check != check) *special = 1.f;
   }
   const int quarter = warp & 3, feature = quarter * 32 + lane;  // of the epilogue warps 2 .. 5
   const bool epilogue = warp >= 2 && warp < 6;
@@ -333,7 +326,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       for (int q = 0; q < S; ++q)
         recompute = recompute || (S > 1 ? ld_peer(peer_smem(smem_u32(special), q)) : *special) != 0.f;
     }
-    if (MODE == kFp32 && recompute) {  // infinities: the sums as a chain of fp32 multiply-adds gives them
+    if (MODE == kFp32 && recompute) {  // infinities, NaN: the sums as a chain of fp32 multiply-adds gives them
       const int per = BN / S;
       for (int j = rank * per; j < (rank + 1) * per && t0 + j < p.T; ++j) {
         const float* ar = static_cast<const float*>(p.a) + static_cast<size_t>(t0 + j) * p.K;
