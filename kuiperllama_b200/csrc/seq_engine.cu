@@ -703,7 +703,7 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
   if (d.streams > 0) RC(e->xs.reserve(Ts * d.streams * W * 4));
   if (e->max_blend > 0) RC(e->vfirst.reserve(Ts * e->max_blend * 4));
   RC(e->h.reserve(Ts * W * es));
-  RC(e->proj.reserve(Ts * std::max({e->max_proj, 2 * e->max_sff, W}) * 4));
+  RC(e->proj.reserve(Ts * std::max(e->max_proj, W) * 4));
   RC(e->q.reserve(Ts * std::max(1, e->max_q) * es));
   RC(e->gates.reserve(Ts * std::max(1, e->max_gates) * 4));
   RC(e->att.reserve(Ts * std::max(e->max_att, e->max_sff) * es));
@@ -1041,14 +1041,17 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
       const int n_pairs = T * M.top;
       const int cap = ((n_pairs + kGroupBlock - 1) / kGroupBlock + M.experts) * kGroupBlock;
       const int n_blocks = cap / kGroupBlock;
-      RC(e->sort.reserve((static_cast<size_t>(M.experts) + 1 + cap + n_blocks) * 4));
-      int32_t* counts_d = static_cast<int32_t*>(e->sort.p);
+      // the tile list (entries of 16 bytes) and its length, then counts, sorted pairs, and the experts of blocks
+      RC(e->sort.reserve((static_cast<size_t>(n_blocks) * 4 + 4 + M.experts + 1 + cap + n_blocks) * 4));
+      int32_t* tiles = static_cast<int32_t*>(e->sort.p);
+      int32_t* n_tiles = tiles + static_cast<size_t>(n_blocks) * 4;
+      int32_t* counts_d = n_tiles + 4;
       int32_t* sorted = counts_d + M.experts + 1;
       int32_t* block_expert = sorted + cap;
-      RC(launch_sort_pairs(top_idx, n_pairs, M.experts, kGroupBlock, counts_d, sorted, block_expert, cap, st));
+      RC(launch_sort_pairs(top_idx, n_pairs, M.experts, kGroupBlock, counts_d, sorted, block_expert, cap, tiles, n_tiles, st));
       GroupedArgs g{};
       g.sorted_pair = sorted, g.block_expert = block_expert, g.n_blocks = n_blocks, g.block = kGroupBlock;
-      g.experts = M.experts, g.act = act;
+      g.experts = M.experts, g.act = act, g.tiles = tiles, g.n_tiles = n_tiles;
       const int inner_epilogue = M.act == KLLM_SEQ_ACT_RELU2 ? 2 : 1;
       if (grouped_tensor_core_usable(dtype, W, M.ff)) {
         // rows in sorted order: a gathered copy of h, the expert's inner activations, then scattered back by pair
@@ -1070,8 +1073,7 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
     }
     e->mark(KLLM_SEQ_PHASE_EXPERTS);
     if (M.shared_ff > 0 && !shared_done) {
-      RC(gemm(dtype, e->h.p, M.shared_gate_up, proj, T, W, 2 * M.shared_ff, st));
-      RC(launch_gated_act(dtype, GatedAct{M.act, M.shared_act_limit, M.act_alpha}, proj, e->att.p, T, M.shared_ff, st));
+      RC(gemm_gated(dtype, e->h.p, M.shared_gate_up, e->att.p, T, W, M.shared_ff, GatedAct{M.act, M.shared_act_limit, M.act_alpha}, st));
       RC(gemm(dtype, e->att.p, M.shared_down, y2, T, M.shared_ff, W, st));
       e->mark(KLLM_SEQ_PHASE_SHARED);
       *shared_out = true;

@@ -321,13 +321,12 @@ int launch_expert_down(int dtype, const void* inter, const void* down, const int
 // y[t] = sum_k w[t, k] * yp[t * top + k]   (fp32 [T * top, width] -> [T, width])
 int launch_combine_pairs(const float* yp, const float* top_w, float* y, int T, int top, int width, cudaStream_t s);
 
-// out[t, f] = act(gu[t, f], gu[t, ff + f])   (gu fp32 [T, 2*ff], out compute type [T, ff]; silu(g) * u for KLLM_SEQ_ACT_SWIGLU)
-int launch_gated_act(int dtype, const GatedAct& act, const float* gu, void* out, int T, int ff, cudaStream_t s);
-
 // Routed experts over token blocks (prefill): rows grouped by expert.  sort_pairs builds, on the device, the list of
 // pairs ordered by expert in blocks of `block` rows (padded with -1), and the expert of every block.
+// tiles (16-byte aligned, [cap / block] entries of 4) and n_tiles: the lists of GroupedArgs
 int launch_sort_pairs(const int32_t* top_idx, int n_pairs, int experts, int block, int32_t* counts /*[experts+1]*/,
-                      int32_t* sorted_pair /*[cap]*/, int32_t* block_expert /*[cap/block]*/, int cap, cudaStream_t s);
+                      int32_t* sorted_pair /*[cap]*/, int32_t* block_expert /*[cap / block]*/, int cap, int32_t* tiles, int32_t* n_tiles,
+                      cudaStream_t s);
 
 // ---- seq_streams.cu: residual streams joined by hyper-connections -------------------------------------------------------
 // Row t of S streams [T, S, width]: x_t <- sum_s mix[s][t] x_s + out_w[t] y (when y is given), then u = sum_s in_w[s] x_s (in_w
@@ -451,6 +450,8 @@ struct GroupedArgs {
   // tensor-core form (bf16): `a` is already in sorted order [n_blocks * block, K] and epilogue 1 writes its result in
   // sorted order too; `experts` sizes the weight map
   int sorted_layout;
+  // ... and the tiles: {expert, first row, rows, 0} of up to 256 rows of one expert, *n_tiles of them, in device memory
+  const int32_t *tiles, *n_tiles;
   int experts;
 };
 int gemm_grouped(int dtype, const GroupedArgs& g, cudaStream_t s);

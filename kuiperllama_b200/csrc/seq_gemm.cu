@@ -412,12 +412,12 @@ int gather_rows_bf16(const void* a, const int32_t* sorted_pair, int div, void* o
 
 int gemm_grouped(int dtype, const GroupedArgs& g, cudaStream_t s) {
   if (g.sorted_layout) {
-    if (dtype != KLLM_SEQ_BF16 || g.block != umma::GBN) return KLLM_E_INVALID;
+    if (dtype != KLLM_SEQ_BF16 || g.block != umma::GBN || !g.tiles || !g.n_tiles) return KLLM_E_INVALID;
     if (g.epilogue == 1)
-      return umma::launch_grouped<1>(g.a, g.w, g.out, g.sorted_pair, g.block_expert, g.n_blocks, g.experts, g.K, g.N, s, g.act);
+      return umma::launch_grouped<1>(g.a, g.w, g.out, g.sorted_pair, g.tiles, g.n_tiles, g.n_blocks, g.experts, g.K, g.N, s, g.act);
     if (g.epilogue == 2)
-      return umma::launch_grouped<2>(g.a, g.w, g.out, g.sorted_pair, g.block_expert, g.n_blocks, g.experts, g.K, g.N, s);
-    return umma::launch_grouped<0>(g.a, g.w, g.out, g.sorted_pair, g.block_expert, g.n_blocks, g.experts, g.K, g.N, s);
+      return umma::launch_grouped<2>(g.a, g.w, g.out, g.sorted_pair, g.tiles, g.n_tiles, g.n_blocks, g.experts, g.K, g.N, s);
+    return umma::launch_grouped<0>(g.a, g.w, g.out, g.sorted_pair, g.tiles, g.n_tiles, g.n_blocks, g.experts, g.K, g.N, s);
   }
   if (dtype == KLLM_SEQ_F32) return grouped_t<float>(g, s);
   if (dtype == KLLM_SEQ_BF16) return grouped_t<__nv_bfloat16>(g, s);

@@ -30,7 +30,6 @@ namespace umma {
 constexpr int BM = 128;    // weight rows per CTA = MMA M
 constexpr int BK = 64;     // bf16 elements per K block = 128 bytes = one swizzle row
 constexpr int UK = 16;     // K of one tcgen05.mma.kind::f16
-constexpr int STAGES = 4;   // of the grouped form
 constexpr int kSms = 148;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int THREADS = 192;
@@ -298,44 +297,51 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
   }
 }
 
-// ---- grouped form: blocks of 64 rows, each block against the weights of one expert ---------------------------------
-// `a` holds the rows in sorted order ([n_blocks * 64, K], padding rows are zero), `w` the experts stacked along the rows.
-// EPI 1: the weights of an expert are N gate rows followed by N up rows; both accumulate side by side in TMEM and
-//        out[block row, n] = silu(gate) * up in bf16, still in sorted order (the next product reads it as its `a`).
-// EPI 0: out[pair, n] = acc in fp32, pair = sorted_pair[block row] (rows of padding are skipped).
+// ---- grouped form: rows in the order of their experts, each tile against the weights of one expert ---------------------
+// `a` holds the rows in sorted order, every expert's rows from a multiple of 64 on (padding rows are zero), `w` the experts stacked
+// along the rows.  `tiles` lists {expert, first row, rows} of up to 256 rows of one expert; *n_tiles of them (both from
+// sort_pairs_kernel, in device memory).  The persistent loop of umma_kernel over (list entry, feature tile); the MMA's N is the
+// entry's rows rounded up to 16, and only the 64-row boxes that hold some are loaded.
+// What bounds it: an expert's weights are read from L2 once per tile of its rows; in tiles of 64 rows that traffic was the bound.
+// EPI 1: the weights of an expert are N gate rows followed by N up rows (a tile: 64 features, gate rows above up rows);
+//        out[row, n] = gated_act(gate, up) in bf16, still in sorted order (the next product reads it as its `a`).
+// EPI 0: out[pair, n] = acc in fp32, pair = sorted_pair[row].
 // EPI 2: one product; max(acc, 0)^2 in bf16, written in sorted order like EPI 1.
-constexpr int GBN = 64;
+// 1501 tokens, 4 of 32 experts, K = 2048, N = 768 gated and back: 114 + 54 us in tiles of 64 rows, 82 + 34 us in tiles of up to 256.
+constexpr int GBN = 64;  // rows per box, and what the sorted order is padded to
+constexpr int kGroupRows = 256;
 template <int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
-umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
-                    void* __restrict__ out_, const int32_t* __restrict__ sorted_pair,
-                    const int32_t* __restrict__ block_expert, int N, int K, GatedAct act, int* report) {
-  constexpr int NA = EPI == 1 ? 2 : 1;
-  constexpr int B_BYTES = GBN * BK * 2;
-  constexpr int STAGE = NA * A_BYTES + B_BYTES;
-  constexpr uint32_t TMEM_COLS = NA * GBN;
-  const int ex = block_expert[blockIdx.y];
-  if (ex < 0) return;  // a block of padding only
+umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, void* __restrict__ out_,
+                    const int32_t* __restrict__ sorted_pair, const int4* __restrict__ list, const int32_t* __restrict__ n_tiles, int N,
+                    int K, GatedAct act, int* report) {
+  constexpr bool GATED = EPI == 1;
+  constexpr int ST = kPersistentStages<256>, STAGE = A_BYTES + kGroupRows * BK * 2;
+  constexpr int FEATURES = GATED ? BM / 2 : BM;
+  constexpr uint32_t TMEM_COLS = 2 * kGroupRows;
   extern __shared__ uint8_t raw_smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(base + STAGES * STAGE);
-  uint64_t* full = bars;
-  uint64_t* empty = bars + STAGES;
-  uint64_t* tmem_full = bars + 2 * STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
+  float* exchange = reinterpret_cast<float*>(base + ST * STAGE);  // gated: [pair of warps][buffer][column][lane]
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + ST * STAGE + (GATED ? 2 * 2 * kPairCols * 32 * 4 : 0));
+  uint64_t* empty = full + ST;
+  uint64_t* acc_full = empty + ST;     // [2]
+  uint64_t* acc_empty = acc_full + 2;  // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), report};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * BM, r0 = blockIdx.y * GBN;
   const int kblocks = (K + BK - 1) / BK;
-  const int wrow = ex * NA * N + n0;
+  const int feature_tiles = (N + FEATURES - 1) / FEATURES, tiles = feature_tiles * *n_tiles;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < ST; ++s) {
       mbar_init(smem_u32(&full[s]), 1);
       mbar_init(smem_u32(&empty[s]), 1);
     }
-    mbar_init(smem_u32(tmem_full), 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&acc_full[b]), 1);
+      mbar_init(smem_u32(&acc_empty[b]), 4);
+    }
     *stop.here = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -351,68 +357,116 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
   if (warp == 0) {
     if (lane == 0) {
-      for (int kb = 0; kb < kblocks; ++kb) {
-        const int s = kb % STAGES;
-        if (!mbar_wait(smem_u32(&empty[s]), ((kb / STAGES) & 1) ^ 1u, stop)) break;
-        const uint32_t bar = smem_u32(&full[s]);
-        uint8_t* st = base + s * STAGE;
-        mbar_expect_tx(bar, STAGE);
-        tma_load_2d(smem_u32(st), &map_w, bar, kb * BK, wrow);
-        if (NA == 2) tma_load_2d(smem_u32(st + A_BYTES), &map_w, bar, kb * BK, wrow + N);
-        tma_load_2d(smem_u32(st + NA * A_BYTES), &map_a, bar, kb * BK, r0);
+      int i = 0;  // blocks of K so far, over all tiles
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        const int n0 = (tile % feature_tiles) * FEATURES;
+        const int4 g = list[tile / feature_tiles];
+        const int wrow = g.x * (GATED ? 2 : 1) * N + n0, boxes = (g.z + GBN - 1) / GBN;
+        for (int kb = 0; kb < kblocks; ++kb, ++i) {
+          const int s = i % ST;
+          ok = mbar_wait(smem_u32(&empty[s]), ((i / ST) & 1) ^ 1u, stop);
+          if (!ok) break;
+          const uint32_t bar = smem_u32(&full[s]);
+          uint8_t* st = base + s * STAGE;
+          mbar_expect_tx(bar, A_BYTES + boxes * (GBN * BK * 2));
+          tma_load_2d(smem_u32(st), &map_w, bar, kb * BK, wrow);
+          if (GATED) tma_load_2d(smem_u32(st + A_BYTES / 2), &map_w, bar, kb * BK, wrow + N);
+          for (int x = 0; x < boxes; ++x)
+            tma_load_2d(smem_u32(st + A_BYTES + x * (GBN * BK * 2)), &map_a, bar, kb * BK, g.y + x * GBN);
+        }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc = instr_desc(GBN);
+      int i = 0, done = 0;  // blocks of K and tiles so far
       bool ok = true;
-      for (int kb = 0; kb < kblocks && ok; ++kb) {
-        const int s = kb % STAGES;
-        ok = mbar_wait(smem_u32(&full[s]), (kb / STAGES) & 1, stop);
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t st = smem_u32(base + s * STAGE);
-        const uint32_t b_addr = st + NA * A_BYTES;
-#pragma unroll
-        for (int z = 0; z < NA; ++z)
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++done) {
+        const int b = done & 1;
+        const uint32_t idesc = instr_desc((list[tile / feature_tiles].z + 15) & ~15);
+        ok = mbar_wait(smem_u32(&acc_empty[b]), ((done >> 1) & 1) ^ 1u, stop);
+        for (int kb = 0; kb < kblocks && ok; ++kb, ++i) {
+          const int s = i % ST;
+          ok = mbar_wait(smem_u32(&full[s]), (i / ST) & 1, stop);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a_addr = smem_u32(base + s * STAGE), b_addr = a_addr + A_BYTES;
 #pragma unroll
           for (int k = 0; k < BK / UK; ++k)
-            mma_bf16(tmem_d + z * GBN, smem_desc(st + z * A_BYTES + k * UK * 2), smem_desc(b_addr + k * UK * 2), idesc,
+            mma_bf16(tmem_d + b * kGroupRows, smem_desc(a_addr + k * UK * 2), smem_desc(b_addr + k * UK * 2), idesc,
                      (kb > 0 || k > 0) ? 1u : 0u);
-        mma_commit(smem_u32(&empty[s]));
+          mma_commit(smem_u32(&empty[s]));
+        }
+        if (ok) mma_commit(smem_u32(&acc_full[b]));
       }
-      if (ok) mma_commit(smem_u32(tmem_full));
     }
   } else {
     const int quarter = warp & 3;
-    if (mbar_wait(smem_u32(tmem_full), 0u, stop)) {
+    int done = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++done) {
+      const int n0 = (tile % feature_tiles) * FEATURES, b = done & 1;
+      const int4 g = list[tile / feature_tiles];
+      // a warp whose wait ran out stores nothing more, but still meets its partner at every barrier below
+      ok = ok && mbar_wait(smem_u32(&acc_full[b]), (done >> 1) & 1, stop);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int row = n0 + quarter * 32 + lane;
+      const uint32_t from = tmem_d + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(b * kGroupRows);
+      const int pair = quarter & 1, row = n0 + (GATED ? pair * 32 : quarter * 32) + lane;
+      const bool up = quarter >= 2;  // gated: quarters 0, 1 hold gate rows; 2, 3 up rows of the same features
+      float* buf = exchange + pair * (2 * kPairCols * 32) + lane;
 #pragma unroll 1
-      for (int c = 0; c < GBN; c += 32) {
-        uint32_t r[32], u[32];
-        const uint32_t taddr = tmem_d + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c);
-        tmem_ld32(taddr, r);
-        if (NA == 2) tmem_ld32(taddr + GBN, u);
+      for (int c = 0; c < g.z; c += kPairCols) {
+        uint32_t r[32];
+        tmem_ld32(from + c, r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (row < N) {
+        if (c + kPairCols >= g.z) {
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+        }
+        const int here = min(kPairCols, g.z - c);
+        if constexpr (EPI == 0) {
+          const int mine = lane < here ? sorted_pair[g.y + c + lane] : -1;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            const int br = r0 + c + j;
-            if (EPI == 1) {
-              const float g = __uint_as_float(r[j]), up = __uint_as_float(u[j]);
-              static_cast<__nv_bfloat16*>(out_)[static_cast<size_t>(br) * N + row] =
-                  __float2bfloat16_rn(gated_act(act, g, up));
-            } else if (EPI == 2) {
-              const float up = fmaxf(__uint_as_float(r[j]), 0.f);
-              static_cast<__nv_bfloat16*>(out_)[static_cast<size_t>(br) * N + row] = __float2bfloat16_rn(up * up);
+            const int to = __shfl_sync(0xffffffffu, mine, j);
+            if (ok && to >= 0 && row < N) static_cast<float*>(out_)[static_cast<size_t>(to) * N + row] = __uint_as_float(r[j]);
+          }
+        } else if constexpr (EPI == 2) {
+          __nv_bfloat16* out = static_cast<__nv_bfloat16*>(out_) + static_cast<size_t>(g.y + c) * N + row;
+          if (ok && row < N) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const float v = fmaxf(__uint_as_float(r[j]), 0.f);
+              if (j < here) out[static_cast<size_t>(j) * N] = __float2bfloat16_rn(v * v);
+            }
+          }
+        } else {
+          // as in umma_kernel: of 32 columns the gate's warp finishes 16 and the up rows' warp 16
+          __nv_bfloat16* out = static_cast<__nv_bfloat16*>(out_) + static_cast<size_t>(g.y + c) * N + row;
+          float* x = buf + ((c / kPairCols) & 1) * (kPairCols * 32);
+          if (up) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j * 32] = __uint_as_float(r[j]);
+          } else {
+#pragma unroll
+            for (int j = 16; j < 32; ++j) x[j * 32] = __uint_as_float(r[j]);
+          }
+          asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
+          if (ok && row < N) {
+            if (up) {
+#pragma unroll
+              for (int j = 16; j < 32; ++j)
+                if (j < here) out[static_cast<size_t>(j) * N] = __float2bfloat16_rn(gated_act(act, x[j * 32], __uint_as_float(r[j])));
             } else {
-              const int pair = sorted_pair[br];
-              if (pair >= 0) static_cast<float*>(out_)[static_cast<size_t>(pair) * N + row] = __uint_as_float(r[j]);
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                if (j < here) out[static_cast<size_t>(j) * N] = __float2bfloat16_rn(gated_act(act, __uint_as_float(r[j]), x[j * 32]));
             }
           }
         }
       }
+      if constexpr (GATED) asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");  // the next tile starts with the first buffer again
     }
   }
   if (*stop.here) {
@@ -530,17 +584,18 @@ inline bool grouped_usable(int K, int N) {
   return !off && K >= BK && (K % 8) == 0 && N >= 8;
 }
 
-// a: [n_blocks * 64, K] bf16 in sorted order; w: [experts * (EPI ? 2 : 1) * N, K]
+// a: [n_blocks * 64, K] bf16 in sorted order; w: [experts * (EPI ? 2 : 1) * N, K]; at most n_blocks entries in the list
 template <int EPI>
-inline int launch_grouped(const void* a, const void* w, void* out, const int32_t* sorted_pair, const int32_t* block_expert,
-                          int n_blocks, int experts, int K, int N, cudaStream_t stream,
+inline int launch_grouped(const void* a, const void* w, void* out, const int32_t* sorted_pair, const int32_t* list,
+                          const int32_t* n_tiles, int n_blocks, int experts, int K, int N, cudaStream_t stream,
                           GatedAct act = GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}) {
+  constexpr int FEATURES = EPI == 1 ? BM / 2 : BM;
   CUtensorMap map_w, map_a;
   int* const report = wait_flag();
   if (report == nullptr) return KLLM_E_STATE;
-  if (int rc = make_map(&map_w, w, experts * (EPI == 1 ? 2 : 1) * N, K, BM)) return rc;
+  if (int rc = make_map(&map_w, w, experts * (EPI == 1 ? 2 : 1) * N, K, FEATURES)) return rc;
   if (int rc = make_map(&map_a, a, n_blocks * GBN, K, GBN)) return rc;
-  const size_t smem = 1024 + static_cast<size_t>(STAGES) * ((EPI == 1 ? 2 : 1) * A_BYTES + GBN * BK * 2) + 256;
+  constexpr size_t smem = persistent_smem<256, EPI == 1>();
   static bool configured = false;
   if (!configured) {
     const cudaError_t e = cudaFuncSetAttribute(umma_grouped_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -548,8 +603,9 @@ inline int launch_grouped(const void* a, const void* w, void* out, const int32_t
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
-  const dim3 grid((N + BM - 1) / BM, n_blocks);
-  umma_grouped_kernel<EPI><<<grid, THREADS, smem, stream>>>(map_w, map_a, out, sorted_pair, block_expert, N, K, act, report);
+  const int most = n_blocks * ((N + FEATURES - 1) / FEATURES);
+  umma_grouped_kernel<EPI><<<most < kSms ? most : kSms, THREADS, smem, stream>>>(
+      map_w, map_a, out, sorted_pair, reinterpret_cast<const int4*>(list), n_tiles, N, K, act, report);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }

@@ -207,9 +207,10 @@ __global__ void embed_kernel(const AT* __restrict__ table, const int32_t* __rest
 // ---- router ---------------------------------------------------------------------------------------------------------
 // The warps of a CTA share the experts' logits of ONE token whose row `xs` is in shared memory in fp32 (a warp per
 // expert row, fp32 weights); warp 0 then does the softmax over all experts and picks the top-k.  `z`: [experts] shared.
+__device__ void choose_experts(const RouterArgs& r, float* z, int t);
 __device__ void route_token(const RouterArgs& r, const float* xs, float* z, int t, int width) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int experts = r.experts, top = r.top;
+  const int experts = r.experts;
   for (int e = warp; e < experts + (r.w_sg ? 1 : 0); e += nw) {
     const float* w = e < experts ? r.w_router + static_cast<size_t>(e) * width : r.w_sg;
     const float acc = warp_dot<float>(w, xs, width, lane);
@@ -219,7 +220,11 @@ __device__ void route_token(const RouterArgs& r, const float* xs, float* z, int 
     }
   }
   __syncthreads();
-  if (warp != 0) return;
+  if (warp == 0) choose_experts(r, z, t);
+}
+// One warp: the logits z of token t (and the scratch behind them, router_smem_floats) become its experts and their weights.
+__device__ void choose_experts(const RouterArgs& r, float* z, int t) {
+  const int lane = threadIdx.x & 31, experts = r.experts, top = r.top;
   if (r.kind == KLLM_SEQ_ROUTER_SIGMOID) {
     // z: scores s;  c: choice scores (s + correction, -inf outside the kept groups and once chosen);  gs: group scores
     float* c = z + experts;
@@ -366,6 +371,67 @@ __global__ void router_kernel(const AT* __restrict__ h, RouterArgs r, int width)
   for (int k = threadIdx.x; k < width; k += blockDim.x) xs[k] = to_f(x[k]);
   __syncthreads();
   route_token(r, xs, z, t, width);
+}
+
+// Blocks of tokens: a CTA routes kRouteRows of them.  A router of 32 experts at width 2048 is 256 KB of fp32 weights; a CTA per token
+// reads all of it from L2 for one row of multiply-adds.  Here a warp holds kRouteExperts experts against the rows in shared memory,
+// so a weight is read once per 8 rows, and each sum keeps the order of warp_dot.  Warp r then chooses for row r.
+// (32 experts, width 2048, 1501 tokens: norm and router in one kernel per token 65 us, 10 + 36 us here.)
+constexpr int kRouteRows = 8, kRouteExperts = 4, kRouteThreads = 32 * kRouteRows;
+inline size_t route_rows_smem(const RouterArgs& r, int width) {
+  return (kRouteRows * (static_cast<size_t>(width) + router_smem_floats(r))) * sizeof(float);
+}
+template <typename AT>
+__global__ void __launch_bounds__(kRouteThreads) route_rows_kernel(const AT* __restrict__ h, RouterArgs r, int width, int T) {
+  extern __shared__ __align__(16) float sm[];  // the rows in fp32, then the router's scratch of each
+  const int scratch = static_cast<int>(router_smem_floats(r));
+  float* z = sm + kRouteRows * width;
+  const int t0 = blockIdx.x * kRouteRows, rows = min(kRouteRows, T - t0);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int k = threadIdx.x; k < kRouteRows * width; k += kRouteThreads)
+    sm[k] = k < rows * width ? to_f(h[static_cast<size_t>(t0) * width + k]) : 0.f;
+  __syncthreads();
+  const int n = r.experts + (r.w_sg ? 1 : 0);
+  for (int e0 = warp * kRouteExperts; e0 < n; e0 += kRouteRows * kRouteExperts) {
+    const float* w[kRouteExperts];
+#pragma unroll
+    for (int e = 0; e < kRouteExperts; ++e)  // experts past the last repeat it
+      w[e] = min(e0 + e, n - 1) < r.experts ? r.w_router + static_cast<size_t>(min(e0 + e, n - 1)) * width : r.w_sg;
+    float acc[kRouteExperts][kRouteRows];
+#pragma unroll
+    for (int e = 0; e < kRouteExperts; ++e)
+#pragma unroll
+      for (int i = 0; i < kRouteRows; ++i) acc[e][i] = 0.f;
+#pragma unroll 2
+    for (int k = lane * 4; k < width; k += 128) {
+      float4 f[kRouteExperts];
+#pragma unroll
+      for (int e = 0; e < kRouteExperts; ++e) f[e] = *reinterpret_cast<const float4*>(w[e] + k);
+#pragma unroll
+      for (int i = 0; i < kRouteRows; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(sm + i * width + k);
+#pragma unroll
+        for (int e = 0; e < kRouteExperts; ++e)
+          acc[e][i] = fmaf(f[e].w, x.w, fmaf(f[e].z, x.z, fmaf(f[e].y, x.y, fmaf(f[e].x, x.x, acc[e][i]))));
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < kRouteExperts; ++e)
+#pragma unroll
+      for (int i = 0; i < kRouteRows; ++i) {
+        const float v = warp_sum(acc[e][i]);
+        if (lane != 0 || i >= rows || e0 + e >= n) continue;
+        if (e0 + e < r.experts) z[i * scratch + e0 + e] = v + (r.bias ? r.bias[e0 + e] : 0.f);
+        else r.sgate[t0 + i] = 1.0f / (1.0f + expf(-v));
+      }
+  }
+  __syncthreads();
+  if (warp < rows) choose_experts(r, z + warp * scratch, t0 + warp);
+}
+// From about two rows per SM on; 16-byte weight rows.
+inline bool route_rows_usable(const RouterArgs& r, int width, int T) {
+  return T >= 256 && width % 4 == 0 && route_rows_smem(r, width) <= 200 * 1024 &&
+         ((reinterpret_cast<uintptr_t>(r.w_router) | reinterpret_cast<uintptr_t>(r.w_sg)) & 15) == 0;
 }
 
 // ---- residual + norms -----------------------------------------------------------------------------------------------
@@ -1344,16 +1410,6 @@ __global__ void combine_pairs_kernel(const float* __restrict__ yp, const float* 
   }
 }
 
-template <typename AT>
-__global__ void gated_act_kernel(GatedAct act, const float* __restrict__ gu, AT* __restrict__ out, int ff, size_t total) {
-  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const size_t t = i / ff;
-  const int f = static_cast<int>(i % ff);
-  const float g = gu[t * 2 * ff + f], u = gu[t * 2 * ff + ff + f];
-  out[i] = from_f<AT>(gated_act(act, g, u));
-}
-
 // ---- greedy id of each logits row (lowest index on ties) ------------------------------------------------------------
 __global__ void argmax_rows_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, int vocab) {
   __shared__ float bv[32];
@@ -1392,12 +1448,19 @@ __global__ void argmax_rows_kernel(const float* __restrict__ logits, int32_t* __
 }
 
 // ---- pairs grouped by expert (one CTA) --------------------------------------------------------
-__global__ void sort_pairs_kernel(const int32_t* __restrict__ top_idx, int n_pairs, int experts, int block,
+constexpr int kGroupTileRows = 256;  // rows of a tile of the grouped product
+__global__ void sort_pairs_kernel(const int32_t* top_idx, int n_pairs, int experts, int block,
                                   int32_t* __restrict__ counts, int32_t* __restrict__ sorted_pair,
-                                  int32_t* __restrict__ block_expert, int cap) {
-  extern __shared__ int32_t sh[];  // [experts] counts, [experts + 1] block offsets
+                                  int32_t* __restrict__ block_expert, int cap, int4* __restrict__ tiles, int32_t* __restrict__ n_tiles,
+                                  int staged) {
+  extern __shared__ int32_t sh[];  // [experts] counts, [experts + 1] block offsets, [n_pairs] the chosen experts when `staged`
   int32_t* cnt = sh;
   int32_t* off = sh + experts;
+  if (staged) {  // every warp walks the whole list below: from shared memory instead of L2
+    int32_t* copy = off + experts + 1;
+    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) copy[p] = top_idx[p];
+    top_idx = copy;
+  }
   for (int e = threadIdx.x; e < experts; e += blockDim.x) cnt[e] = 0;
   __syncthreads();
   for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) atomicAdd(&cnt[top_idx[p]], 1);
@@ -1411,6 +1474,10 @@ __global__ void sort_pairs_kernel(const int32_t* __restrict__ top_idx, int n_pai
     }
     off[experts] = o;
     counts[experts] = o;
+    int n = 0;
+    for (int e = 0; e < experts; ++e)
+      for (int r = 0; r < cnt[e]; r += kGroupTileRows) tiles[n++] = make_int4(e, off[e] + r, min(kGroupTileRows, cnt[e] - r), 0);
+    *n_tiles = n;
   }
   __syncthreads();
   const int used = off[experts];
@@ -1429,6 +1496,7 @@ __global__ void sort_pairs_kernel(const int32_t* __restrict__ top_idx, int n_pai
   for (int e = warp; e < experts; e += nw) {
     int o = off[e];
     if (cnt[e] == 0) continue;
+#pragma unroll 4
     for (int base = 0; base < n_pairs; base += 32) {
       const int p = base + lane;
       const bool mine = p < n_pairs && top_idx[p] == e;
@@ -1482,6 +1550,17 @@ int launch_resid_norm(const ResidNormArgs& a, cudaStream_t s) {
   if (smem > 200 * 1024) return KLLM_E_UNSUPPORTED;
   if (a.router.w_router && (a.router.top > a.router.experts || a.router.experts <= 0 || a.router.top <= 0 || !a.pre.w))
     return KLLM_E_INVALID;
+  if (a.router.w_router && a.out && !a.out_f32 && !a.rows && route_rows_usable(a.router, a.width, a.T)) {
+    ResidNormArgs rows = a;  // the rows first, without the router, then the router on blocks of them
+    rows.router = RouterArgs{};
+    if (const int rc = launch_resid_norm(rows, s)) return rc;
+    const size_t bytes = route_rows_smem(a.router, a.width);
+    KLLM_SEQ_DISPATCH(a.dtype, (cudaFuncSetAttribute(route_rows_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     static_cast<int>(bytes))));
+    KLLM_SEQ_DISPATCH(a.dtype, (route_rows_kernel<AT><<<(a.T + kRouteRows - 1) / kRouteRows, kRouteThreads, bytes, s>>>(
+                                   static_cast<const AT*>(a.out), a.router, a.width, a.T)));
+    return done();
+  }
   auto aligned = [](std::initializer_list<const void*> ps) {
     uintptr_t bits = 0;
     for (const void* p : ps) bits |= reinterpret_cast<uintptr_t>(p);
@@ -1709,23 +1788,19 @@ int launch_combine_pairs(const float* yp, const float* top_w, float* y, int T, i
   return done();
 }
 
-int launch_gated_act(int dtype, const GatedAct& act, const float* gu, void* out, int T, int ff, cudaStream_t s) {
-  const size_t total = static_cast<size_t>(T) * ff;
-  const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-  KLLM_SEQ_DISPATCH(dtype, (gated_act_kernel<AT><<<blocks, 256, 0, s>>>(act, gu, static_cast<AT*>(out), ff, total)));
-  return done();
-}
-
 int launch_argmax_rows(const float* logits, int32_t* out, int rows, int vocab, cudaStream_t s) {
   argmax_rows_kernel<<<rows, 1024, 0, s>>>(logits, out, vocab);
   return done();
 }
 
 int launch_sort_pairs(const int32_t* top_idx, int n_pairs, int experts, int block, int32_t* counts,
-                      int32_t* sorted_pair, int32_t* block_expert, int cap, cudaStream_t s) {
-  const size_t smem = (2 * static_cast<size_t>(experts) + 1) * sizeof(int32_t);
+                      int32_t* sorted_pair, int32_t* block_expert, int cap, int32_t* tiles, int32_t* n_tiles, cudaStream_t s) {
+  size_t smem = (static_cast<size_t>(2) * experts + 1) * sizeof(int32_t);
   if (smem > 48 * 1024) return KLLM_E_UNSUPPORTED;
-  sort_pairs_kernel<<<1, 1024, smem, s>>>(top_idx, n_pairs, experts, block, counts, sorted_pair, block_expert, cap);
+  const size_t with_pairs = smem + static_cast<size_t>(n_pairs) * sizeof(int32_t);
+  const int staged = with_pairs <= 48 * 1024;
+  sort_pairs_kernel<<<1, 1024, staged ? with_pairs : smem, s>>>(top_idx, n_pairs, experts, block, counts, sorted_pair, block_expert, cap,
+                                                                reinterpret_cast<int4*>(tiles), n_tiles, staged);
   return done();
 }
 
