@@ -66,7 +66,9 @@ struct PrefillWorkspace {  // [block, .] activations
 int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* tokens_dev, int T, int start_pos,
                   cudaStream_t stream);
 // prefill_gemm.cu: out = x . w^T (+ bias); residual += x . w^T; out = silu(x . w1^T) * (x . w3^T)
-int prefill_product(const float* x, const float* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s);
+// (ahead: may read its weights before the kernels ahead of it on the stream have finished)
+int prefill_product(const float* x, const float* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s,
+                    bool ahead = true);
 int prefill_product_add(const float* x, const float* w, float* residual, int T, int K, int N, cudaStream_t s);
 int prefill_product_gated(const float* x, const float* w1, const float* w3, float* out, int T, int K, int N, cudaStream_t s);
 

@@ -28,13 +28,13 @@ namespace {
 // The narrowest token block that holds the rows.  Two weight matrices share a token tile, whose sums have to fit the epilogue's
 // registers: at most 64 tokens there, else 128.
 template <int OUT>
-int product(const seq::umma::SplitArgs& p, cudaStream_t s) {
+int product(const seq::umma::SplitArgs& p, cudaStream_t s, bool ahead = true) {
   using namespace seq::umma;
   constexpr bool two = OUT == kGated;
-  if (p.T <= 16) return launch_split<kTf32, 16, OUT, two ? 3 : 5>(p, s);
-  if (p.T <= 32) return launch_split<kTf32, 32, OUT, two ? 3 : 5>(p, s);
-  if (two || p.T <= 64) return launch_split<kTf32, 64, OUT, two ? 2 : 4>(p, s);
-  if constexpr (!two) return launch_split<kTf32, 128, OUT, 3>(p, s);
+  if (p.T <= 16) return launch_split<kTf32, 16, OUT, two ? 3 : 5>(p, s, ahead);
+  if (p.T <= 32) return launch_split<kTf32, 32, OUT, two ? 3 : 5>(p, s, ahead);
+  if (two || p.T <= 64) return launch_split<kTf32, 64, OUT, two ? 2 : 4>(p, s, ahead);
+  if constexpr (!two) return launch_split<kTf32, 128, OUT, 3>(p, s, ahead);
   return KLLM_E_UNSUPPORTED;
 }
 // TMA needs 16-byte aligned bases and row pitches
@@ -45,9 +45,9 @@ constexpr seq::GatedAct kSwiglu{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f};
 
 }  // namespace
 
-int prefill_product(const float* x, const float* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s) {
+int prefill_product(const float* x, const float* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s, bool ahead) {
   if (!aligned(x, w, K)) return KLLM_E_UNSUPPORTED;
-  return product<seq::umma::kPlain>({x, w, nullptr, bias, nullptr, out, T, N, K, 1, kSwiglu, nullptr}, s);
+  return product<seq::umma::kPlain>({x, w, nullptr, bias, nullptr, out, T, N, K, 1, kSwiglu, nullptr}, s, ahead);
 }
 int prefill_product_add(const float* x, const float* w, float* residual, int T, int K, int N, cudaStream_t s) {
   if (!aligned(x, w, K)) return KLLM_E_UNSUPPORTED;
@@ -63,5 +63,5 @@ int prefill_product_gated(const float* x, const float* w1, const float* w3, floa
 extern "C" int kllm_gemm_tf32(const float* x, const float* w, float* out, int n_tokens, int in_dim, int out_dim,
                               void* stream) {
   if (!x || !w || !out || n_tokens <= 0 || in_dim <= 0 || out_dim <= 0) return KLLM_E_INVALID;
-  return kllm::prefill_product(x, w, nullptr, out, n_tokens, in_dim, out_dim, static_cast<cudaStream_t>(stream));
+  return kllm::prefill_product(x, w, nullptr, out, n_tokens, in_dim, out_dim, static_cast<cudaStream_t>(stream), false);
 }

@@ -33,6 +33,7 @@
 #include <cstdlib>
 
 #include "seq_engine.h"
+#include "seq_launch.cuh"
 #include "seq_mma.cuh"
 
 namespace kllm {
@@ -353,6 +354,8 @@ __global__ void __launch_bounds__(kFewThreads)
 attention_rows_mma_kernel(AttnShape a, const void* __restrict__ q_, PagedKV kv, const int32_t* __restrict__ ent_first,
                           const int32_t* __restrict__ ent_count, const int32_t* __restrict__ ent_seq,
                           const int32_t* __restrict__ ent_pos0, int splits, float* __restrict__ ws) {
+  next_may_start();
+  after_previous();
   const int e = blockIdx.y / a.kv_heads, g = blockIdx.y % a.kv_heads, split = blockIdx.z;
   const int gv = g / v_share_of(a);
   const int rep = a.heads / a.kv_heads, dim = a.dim, vdim = a.vdim;
@@ -553,7 +556,7 @@ int launch_few(const AttnShape& a, const void* q, const PagedKV& kv, int n_entri
   }
   const dim3 grid((max_count * (a.heads / a.kv_heads) + kFewRows - 1) / kFewRows, n_entries * a.kv_heads, splits);
   if (grid.y > 65535u) return KLLM_E_UNSUPPORTED;
-  attention_rows_mma_kernel<NBW, SAME, QF32><<<grid, kFewThreads, smem, s>>>(a, q, kv, ent_first, ent_count, ent_seq, ent_pos0,
+  launch_ahead(attention_rows_mma_kernel<NBW, SAME, QF32>, dim3(grid), dim3(kFewThreads), smem, s, a, q, kv, ent_first, ent_count, ent_seq, ent_pos0,
                                                                             splits, ws);
   count_launch();
   return cuda_rc(cudaGetLastError());

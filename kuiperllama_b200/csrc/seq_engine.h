@@ -427,7 +427,9 @@ int launch_ssd_out(int dtype, const kllm_seq_ssd& m, const float* y, const float
 
 // ---- seq_gemm.cu --------------------------------------------------------------------------------------------------
 // out[T, N] (fp32) = a[T, K] . w[N, K]^T (+ bias[N]), a and w in the compute type, fp32 accumulation.
-int gemm(int dtype, const void* a, const void* w, float* out, int T, int K, int N, cudaStream_t s, const float* bias = nullptr);
+// ahead: the kernel may read weights before the kernels ahead of it on the stream have finished (seq_launch.cuh)
+int gemm(int dtype, const void* a, const void* w, float* out, int T, int K, int N, cudaStream_t s, const float* bias = nullptr,
+         bool ahead = true);
 // out[T, ff] (compute type) = gated_act(a . wg^T + bias[f], a . wu^T + bias[ff + f]), w = [ff gate rows, then ff up rows][K]
 int gemm_gated(int dtype, const void* a, const void* w, void* out, int T, int K, int ff, const GatedAct& act, cudaStream_t s,
                const float* bias = nullptr);

@@ -23,6 +23,7 @@
 #include "seq_engine.h"
 #include "seq_gemm_split.cuh"
 #include "seq_gemm_umma.cuh"
+#include "seq_launch.cuh"
 
 namespace kllm {
 namespace seq {
@@ -74,6 +75,7 @@ __global__ void __launch_bounds__(256)
 rows_kernel(const AT* __restrict__ a, const AT* __restrict__ w, const float* __restrict__ bias, float* __restrict__ out, int T,
             int K, int N) {
   constexpr int V = Vec16<AT>::N;
+  next_may_start();
   const int lane = threadIdx.x & 31;
   const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (n >= N) return;
@@ -88,6 +90,7 @@ rows_kernel(const AT* __restrict__ a, const AT* __restrict__ w, const float* __r
 #pragma unroll
       for (int u = 0; u < U; ++u)
         if (k0 + u * 32 * V < K) Vec16<AT>::load_stream(wr + k0 + u * 32 * V, wf[u]);
+      if (k0 == lane * V) after_previous();  // the first weights are on their way before the rows they meet are there
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int k = k0 + u * 32 * V;
@@ -104,6 +107,7 @@ rows_kernel(const AT* __restrict__ a, const AT* __restrict__ w, const float* __r
       }
     }
   } else {
+    after_previous();
     for (int k = lane; k < K; k += 32) {
       const float wv = ld_f(wr + k);
 #pragma unroll
@@ -126,6 +130,7 @@ __global__ void __launch_bounds__(256)
 rows_gated_kernel(const AT* __restrict__ a, const AT* __restrict__ w, const float* __restrict__ bias, AT* __restrict__ out, int T,
                   int K, int N, GatedAct act) {
   constexpr int V = Vec16<AT>::N;
+  next_may_start();
   const int lane = threadIdx.x & 31;
   const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (n >= N) return;
@@ -144,6 +149,7 @@ rows_gated_kernel(const AT* __restrict__ a, const AT* __restrict__ w, const floa
           Vec16<AT>::load_stream(wg + k0 + z * 32 * V, gf[z]);
           Vec16<AT>::load_stream(wu + k0 + z * 32 * V, uf[z]);
         }
+      if (k0 == lane * V) after_previous();
 #pragma unroll
       for (int z = 0; z < U; ++z) {
         const int k = k0 + z * 32 * V;
@@ -160,6 +166,7 @@ rows_gated_kernel(const AT* __restrict__ a, const AT* __restrict__ w, const floa
       }
     }
   } else {
+    after_previous();
     for (int k = lane; k < K; k += 32) {
       const float gv = ld_f(wg + k), uv = ld_f(wu + k);
 #pragma unroll
@@ -293,7 +300,7 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ a, const in
 }
 
 template <typename AT>
-int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s) {
+int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s, bool ahead) {
   constexpr int V = Vec16<AT>::N;
   if (T <= 8) {
     const bool vec = (K % V) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
@@ -301,8 +308,8 @@ int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K
     const dim3 grid((N + warps - 1) / warps);
 #define KLLM_ROWS(R)                                                                  \
   do {                                                                                \
-    if (vec) rows_kernel<AT, R, true><<<grid, warps * 32, 0, s>>>(a, w, bias, out, T, K, N); \
-    else rows_kernel<AT, R, false><<<grid, warps * 32, 0, s>>>(a, w, bias, out, T, K, N);    \
+    if (vec) launch_maybe_ahead(ahead, rows_kernel<AT, R, true>, dim3(grid), dim3(warps * 32), 0, s, a, w, bias, out, T, K, N); \
+    else launch_maybe_ahead(ahead, rows_kernel<AT, R, false>, dim3(grid), dim3(warps * 32), 0, s, a, w, bias, out, T, K, N);    \
   } while (0)
     if (T <= 1) KLLM_ROWS(1);
     else if (T <= 2) KLLM_ROWS(2);
@@ -313,11 +320,11 @@ int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K
     return cuda_rc(cudaGetLastError());
   }
   if (umma::usable<AT>(a, w, T, K, N)) {
-    return umma::launch(a, w, bias, out, T, K, N, s);
+    return umma::launch(a, w, bias, out, T, K, N, s, ahead);
   }
   if constexpr (std::is_same_v<AT, float>)
     if (umma::fp32_usable(a, w, T, K))
-      return umma::launch_fp32<false>(a, w, bias, out, T, K, N, GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}, s);
+      return umma::launch_fp32<false>(a, w, bias, out, T, K, N, GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}, s, ahead);
   const dim3 grid((N + TN - 1) / TN, (T + TM - 1) / TM);
   tiled_kernel<AT, false, 0><<<grid, 256, 0, s>>>(a, w, out, T, K, N, nullptr, nullptr, 1,
                                                  GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}, bias);
@@ -335,8 +342,8 @@ int gemm_gated_t(const AT* a, const AT* w, const float* bias, AT* out, int T, in
     const dim3 grid((N + warps - 1) / warps);
 #define KLLM_ROWS(R)                                                                                \
   do {                                                                                              \
-    if (vec) rows_gated_kernel<AT, R, true><<<grid, warps * 32, 0, s>>>(a, w, bias, out, T, K, N, act);    \
-    else rows_gated_kernel<AT, R, false><<<grid, warps * 32, 0, s>>>(a, w, bias, out, T, K, N, act);       \
+    if (vec) launch_ahead(rows_gated_kernel<AT, R, true>, dim3(grid), dim3(warps * 32), 0, s, a, w, bias, out, T, K, N, act);    \
+    else launch_ahead(rows_gated_kernel<AT, R, false>, dim3(grid), dim3(warps * 32), 0, s, a, w, bias, out, T, K, N, act);       \
   } while (0)
     if (T <= 1) KLLM_ROWS(1);
     else if (T <= 2) KLLM_ROWS(2);
@@ -350,7 +357,7 @@ int gemm_gated_t(const AT* a, const AT* w, const float* bias, AT* out, int T, in
     return umma::launch_gated(a, w, bias, out, T, K, N, act, s);
   }
   if constexpr (std::is_same_v<AT, float>)
-    if (umma::fp32_usable(a, w, T, K)) return umma::launch_fp32<true>(a, w, bias, out, T, K, N, act, s);
+    if (umma::fp32_usable(a, w, T, K)) return umma::launch_fp32<true>(a, w, bias, out, T, K, N, act, s, true);
   const dim3 grid((N + TN - 1) / TN, (T + TM - 1) / TM);
   tiled_kernel<AT, false, 1><<<grid, 256, 0, s>>>(a, w, out, T, K, N, nullptr, nullptr, 1, act, bias);
   count_launch();
@@ -376,12 +383,12 @@ int grouped_t(const GroupedArgs& g, cudaStream_t s) {
 
 }  // namespace
 
-int gemm(int dtype, const void* a, const void* w, float* out, int T, int K, int N, cudaStream_t s, const float* bias) {
+int gemm(int dtype, const void* a, const void* w, float* out, int T, int K, int N, cudaStream_t s, const float* bias, bool ahead) {
   if (!a || !w || !out || T <= 0 || K <= 0 || N <= 0) return KLLM_E_INVALID;
   if (dtype == KLLM_SEQ_F32)
-    return gemm_t(static_cast<const float*>(a), static_cast<const float*>(w), bias, out, T, K, N, s);
+    return gemm_t(static_cast<const float*>(a), static_cast<const float*>(w), bias, out, T, K, N, s, ahead);
   if (dtype == KLLM_SEQ_BF16)
-    return gemm_t(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(w), bias, out, T, K, N, s);
+    return gemm_t(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(w), bias, out, T, K, N, s, ahead);
   return KLLM_E_INVALID;
 }
 

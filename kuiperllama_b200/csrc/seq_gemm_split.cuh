@@ -30,6 +30,7 @@
 //   fp32  T = 517, K = 1024, N = 3072   161 -> 47.2 us    5.7e-7 -> 2.9e-7
 #pragma once
 #include "seq_gemm_umma.cuh"
+#include "seq_launch.cuh"
 
 namespace kllm {
 namespace seq {
@@ -213,18 +214,27 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_d = *tmem_slot;
+  next_may_start();
 
   if (warp == 0) {
     if (lane == 0) {
-      for (int i = 0; i < blocks; ++i) {
-        const int s = i % ST, k = (kb0 + i) * M::BKE;
-        if (!mbar_wait(smem_u32(&empty[s]), ((i / ST) & 1) ^ 1u, stop)) break;
-        const uint32_t bar = smem_u32(&full[s]);
-        uint8_t* st = base + s * STAGE;
+      auto weights = [&](int i) {
+        const uint32_t bar = smem_u32(&full[i % ST]);
+        uint8_t* st = base + (i % ST) * STAGE;
         mbar_expect_tx(bar, HALF);
-        tma_load_2d(smem_u32(st), &map_w, bar, k, n0);
-        if (NA == 2) tma_load_2d(smem_u32(st + A_BYTES), &map_w2, bar, k, n0);
-        tma_load_2d(smem_u32(st + W_BYTES), &map_a, bar, k, t0);
+        tma_load_2d(smem_u32(st), &map_w, bar, (kb0 + i) * M::BKE, n0);
+        if (NA == 2) tma_load_2d(smem_u32(st + A_BYTES), &map_w2, bar, (kb0 + i) * M::BKE, n0);
+      };
+      // the ring's first weights are on their way before the rows they meet are there
+      for (int i = 0; i < ST && i < blocks; ++i) weights(i);
+      after_previous();
+      for (int i = 0; i < blocks; ++i) {
+        const int s = i % ST;
+        if (i >= ST) {
+          if (!mbar_wait(smem_u32(&empty[s]), ((i / ST) & 1) ^ 1u, stop)) break;
+          weights(i);
+        }
+        tma_load_2d(smem_u32(base + s * STAGE + W_BYTES), &map_a, smem_u32(&full[s]), (kb0 + i) * M::BKE, t0);
       }
     }
   } else if (warp == 1) {
@@ -288,6 +298,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   float acc[TILE_COLS];
   bool ok = true;
   if (epilogue) {
+    after_previous();  // (it writes, and kAdd reads, what earlier kernels may still use)
 #pragma unroll
     for (int j = 0; j < TILE_COLS; ++j) acc[j] = 0.f;
     for (int sec = 0; sec < sections && ok; ++sec) {
@@ -389,7 +400,7 @@ inline int split_count(int tiles, int blocks, int room) {
 }
 
 template <int MODE, int BN, int OUT, int ST>
-inline int launch_split(SplitArgs p, cudaStream_t stream) {
+inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
   constexpr int NA = OUT == kGated ? 2 : 1;
   CUtensorMap map_w, map_w2, map_a;
   p.report = wait_flag();
@@ -413,11 +424,13 @@ inline int launch_split(SplitArgs p, cudaStream_t stream) {
   cfg.blockDim = dim3(split_threads<MODE>());
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = p.S, attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = ahead ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_w2, map_a, p);
   count_launch();
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
@@ -426,15 +439,15 @@ inline int launch_split(SplitArgs p, cudaStream_t stream) {
 // the narrowest token block that holds the step; more than 128 tokens (gated: 64) in tiles of 64
 template <bool GATED>
 int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act,
-               cudaStream_t s) {
+               cudaStream_t s, bool ahead) {
   const void* w2 = static_cast<const __nv_bfloat16*>(w) + static_cast<size_t>(N) * K;  // the up rows follow the gate rows
   const SplitArgs p{a, w, w2, bias, nullptr, out, T, N, K, 1, act, nullptr};
   constexpr int OUT = GATED ? kGated : kPlain;
-  if (T <= 16) return launch_split<kBf16, 16, OUT, GATED ? 3 : 5>(p, s);
-  if (T <= 32) return launch_split<kBf16, 32, OUT, GATED ? 3 : 5>(p, s);
+  if (T <= 16) return launch_split<kBf16, 16, OUT, GATED ? 3 : 5>(p, s, ahead);
+  if (T <= 32) return launch_split<kBf16, 32, OUT, GATED ? 3 : 5>(p, s, ahead);
   if constexpr (!GATED)
-    if (T > 64 && T <= 128) return launch_split<kBf16, 128, OUT, 3>(p, s);  // one tile: the weights are read once
-  return launch_split<kBf16, 64, OUT, 4>(p, s);
+    if (T > 64 && T <= 128) return launch_split<kBf16, 128, OUT, 3>(p, s, ahead);  // one tile: the weights are read once
+  return launch_split<kBf16, 64, OUT, 4>(p, s, ahead);
 }
 
 // fp32 operands, fp32 accuracy: whole 16-byte rows, and more rows than the kernel that streams weights once takes
@@ -445,13 +458,13 @@ inline bool fp32_usable(const void* a, const void* w, int T, int K) {
 }
 template <bool GATED>
 int launch_fp32(const float* a, const float* w, const float* bias, float* out, int T, int K, int N, const GatedAct& act,
-                cudaStream_t s) {
+                cudaStream_t s, bool ahead) {
   const SplitArgs p{a, w, w + static_cast<size_t>(N) * K, bias, nullptr, out, T, N, K, 1, act, nullptr};
   constexpr int OUT = GATED ? kGated : kPlain;
-  if (T <= 16) return launch_split<kFp32, 16, OUT, 3>(p, s);
-  if (T <= 32) return launch_split<kFp32, 32, OUT, 3>(p, s);
-  if (GATED || T <= 64) return launch_split<kFp32, 64, OUT, GATED ? 2 : 4>(p, s);
-  if constexpr (!GATED) return launch_split<kFp32, 128, OUT, 3>(p, s);
+  if (T <= 16) return launch_split<kFp32, 16, OUT, 3>(p, s, ahead);
+  if (T <= 32) return launch_split<kFp32, 32, OUT, 3>(p, s, ahead);
+  if (GATED || T <= 64) return launch_split<kFp32, 64, OUT, GATED ? 2 : 4>(p, s, ahead);
+  if constexpr (!GATED) return launch_split<kFp32, 128, OUT, 3>(p, s, ahead);
   return KLLM_E_UNSUPPORTED;
 }
 

@@ -536,15 +536,16 @@ inline int launch_persistent(const void* a, const void* w, const float* bias, vo
 
 // products whose tiles do not fill the chip (seq_gemm_split.cuh)
 template <bool GATED>
-int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act, cudaStream_t s);
+int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act, cudaStream_t s,
+               bool ahead);
 
 // One token tile (which two CTAs on an SM stream through better: T = 100, K = 2048, N = 32000 31 us, one persistent CTA 32.4), or less
 // than one tile of 128 tokens per SM: narrower token blocks and K split over CTAs.  Else the wider tile, unless its last wave is
 // so empty that the narrower one, whose tiles take 0.65 of the time, is done sooner.
 template <bool GATED>
 inline int launch_block(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act,
-                        cudaStream_t s) {
-  if (T <= (GATED ? 64 : 128) || ((N + BM - 1) / BM) * ((T + 127) / 128) < kSms) return launch_few<GATED>(a, w, bias, out, T, K, N, act, s);
+                        cudaStream_t s, bool ahead) {
+  if (T <= (GATED ? 64 : 128) || ((N + BM - 1) / BM) * ((T + 127) / 128) < kSms) return launch_few<GATED>(a, w, bias, out, T, K, N, act, s, ahead);
   const int feature_tiles = GATED ? (N + BM / 2 - 1) / (BM / 2) : (N + BM - 1) / BM;
   const int waves_wide = (feature_tiles * ((T + 255) / 256) + kSms - 1) / kSms;
   const int waves = (feature_tiles * ((T + 127) / 128) + kSms - 1) / kSms;
@@ -562,12 +563,12 @@ inline bool usable<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* w
 }
 
 template <typename AT>
-inline int launch(const AT*, const AT*, const float*, float*, int, int, int, cudaStream_t) { return KLLM_E_UNSUPPORTED; }
+inline int launch(const AT*, const AT*, const float*, float*, int, int, int, cudaStream_t, bool) { return KLLM_E_UNSUPPORTED; }
 template <>
 inline int launch<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* w, const float* bias, float* out, int T, int K,
-                                 int N, cudaStream_t s) {
+                                 int N, cudaStream_t s, bool ahead) {
   const GatedAct none{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f};
-  return launch_block<false>(a, w, bias, out, T, K, N, none, s);
+  return launch_block<false>(a, w, bias, out, T, K, N, none, s, ahead);
 }
 
 // w: [2 * N, K], gate rows then up rows
@@ -576,7 +577,7 @@ inline int launch_gated(const AT*, const AT*, const float*, AT*, int, int, int, 
 template <>
 inline int launch_gated<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* w, const float* bias, __nv_bfloat16* out, int T,
                                        int K, int N, const GatedAct& act, cudaStream_t s) {
-  return launch_block<true>(a, w, bias, out, T, K, N, act, s);
+  return launch_block<true>(a, w, bias, out, T, K, N, act, s, true);
 }
 
 inline bool grouped_usable(int K, int N) {

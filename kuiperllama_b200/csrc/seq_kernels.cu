@@ -17,6 +17,7 @@
 #include <initializer_list>
 
 #include "seq_engine.h"
+#include "seq_launch.cuh"
 #include "seq_merge.cuh"
 
 namespace kllm {
@@ -438,6 +439,8 @@ inline bool route_rows_usable(const RouterArgs& r, int width, int T) {
 // Layer norm: (v - mean) / sqrt(var + eps) * w + b, var = mean of squared deviations.  RMS norm: v / sqrt(mean(v^2) + eps) * w.
 template <typename AT>
 __global__ void resid_norm_kernel(ResidNormArgs a) {
+  next_may_start();
+  after_previous();
   extern __shared__ float buf[];  // [width], then the router's scratch when the kernel also routes
   __shared__ float red[33];
   const int W = a.width;
@@ -557,6 +560,8 @@ __device__ __forceinline__ void put4(__nv_bfloat16* dst, const float4& v) {
 
 template <typename AT, int NV>
 __global__ void __launch_bounds__(512) resid_rows_kernel(ResidNormArgs a) {
+  next_may_start();
+  after_previous();
   __shared__ float red_post[32], red_pre[32];
   const int W = a.width, r = blockIdx.x;
   const size_t src = static_cast<size_t>(a.rows ? a.rows[r] : r) * W, dst = static_cast<size_t>(r) * W;
@@ -643,6 +648,8 @@ __global__ void qk_prepare_kernel(AttnShape a, RopeArgs rope, const float* __res
                                   const float* __restrict__ qnorm_w, const float* __restrict__ knorm_w, float eps,
                                   const int32_t* __restrict__ tok_seq, const int32_t* __restrict__ tok_pos,
                                   AT* __restrict__ q, float* __restrict__ gates, PagedKV kv, ValueBlend blend) {
+  next_may_start();
+  after_previous();
   extern __shared__ float head_rows[];  // [warps][dim]
   __shared__ float red[33];
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -726,6 +733,8 @@ __global__ void __launch_bounds__(512)
 qk_turn_kernel(AttnShape a, RopeArgs rope, const float* __restrict__ qkvg, int stride, const float* __restrict__ qnorm_w,
                const float* __restrict__ knorm_w, float eps, const int32_t* __restrict__ tok_seq,
                const int32_t* __restrict__ tok_pos, AT* __restrict__ q, float* __restrict__ gates, PagedKV kv) {
+  next_may_start();
+  after_previous();
   extern __shared__ __align__(16) float turn[];  // [half] cos, [half] sin
   __shared__ float red[2][32];
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -840,6 +849,8 @@ __global__ void qk_rows_kernel(AttnShape a, const float* __restrict__ qkvg, int 
                                const float* __restrict__ knorm_w, float eps, const int32_t* __restrict__ tok_seq,
                                const int32_t* __restrict__ tok_pos, AT* __restrict__ q, float* __restrict__ gates, PagedKV kv,
                                ValueBlend blend) {
+  next_may_start();
+  after_previous();
   __shared__ float red[2][32];
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int qn = a.heads * a.dim, kn = a.kv_heads * a.dim, vn = a.kv_heads * a.vdim, gn = gate_floats(a);
@@ -917,6 +928,8 @@ __global__ void __launch_bounds__(kAttnThreads)
 attention_kernel(AttnShape a, const void* __restrict__ q_, PagedKV kv, const int32_t* __restrict__ ent_first,
                  const int32_t* __restrict__ ent_count, const int32_t* __restrict__ ent_seq,
                  const int32_t* __restrict__ ent_pos0, int splits, float* __restrict__ ws) {
+  next_may_start();
+  after_previous();
   const int e = blockIdx.y / a.kv_heads, g = blockIdx.y % a.kv_heads, split = blockIdx.z;
   const int gv = g / v_share_of(a);  // the value head this key head reads
   const int rep = a.heads / a.kv_heads;
@@ -1211,6 +1224,8 @@ template <typename AT>
 __global__ void attention_merge_kernel(int heads, int vdim, int splits, const float* __restrict__ ws,
                                        const float* __restrict__ gates, int gate_kind, const float* __restrict__ sink,
                                        int out_f32, void* __restrict__ out_) {
+  next_may_start();
+  after_previous();
   extern __shared__ float weight[];  // [splits]
   const size_t th = blockIdx.x;  // t * heads + h
   const int pstride = vdim + 2;
@@ -1340,6 +1355,8 @@ template <typename AT>
 __global__ void expert_gate_up_kernel(const AT* __restrict__ h, const AT* __restrict__ gate_up,
                                       const int32_t* __restrict__ top_idx, AT* __restrict__ inter, int T, int top, int ff,
                                       int width, SharedExpert sh, GatedAct ga) {
+  next_may_start();
+  after_previous();
   const int act = ga.kind;
   extern __shared__ float xs[];  // [width]
   const int pair = blockIdx.x;
@@ -1376,6 +1393,8 @@ template <typename AT>
 __global__ void expert_down_kernel(const AT* __restrict__ inter, const AT* __restrict__ down,
                                    const int32_t* __restrict__ top_idx, const float* __restrict__ top_w,
                                    float* __restrict__ y, int top, int ff, int width, SharedExpert sh) {
+  next_may_start();
+  after_previous();
   extern __shared__ float xs[];  // [top][ff], then [sh.ff]
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -1574,7 +1593,7 @@ int launch_resid_norm(const ResidNormArgs& a, cudaStream_t s) {
     int threads = std::min((n4 + 31) / 32 * 32, a.T <= 64 ? 512 : 256);
     const int nv = (n4 + threads - 1) / threads;
     if (nv > 4) threads = 512;
-#define KLLM_RESID_ROWS(N) KLLM_SEQ_DISPATCH(a.dtype, (resid_rows_kernel<AT, N><<<a.T, threads, 0, s>>>(a)))
+#define KLLM_RESID_ROWS(N) KLLM_SEQ_DISPATCH(a.dtype, (launch_ahead(resid_rows_kernel<AT, N>, dim3(a.T), dim3(threads), 0, s, a)))
     if (nv <= 1) KLLM_RESID_ROWS(1);
     else if (nv <= 2) KLLM_RESID_ROWS(2);
     else KLLM_RESID_ROWS(4);
@@ -1586,7 +1605,7 @@ int launch_resid_norm(const ResidNormArgs& a, cudaStream_t s) {
     KLLM_SEQ_DISPATCH(a.dtype, (cudaFuncSetAttribute(resid_norm_kernel<AT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      static_cast<int>(smem))));
   }
-  KLLM_SEQ_DISPATCH(a.dtype, (resid_norm_kernel<AT><<<a.T, threads, smem, s>>>(a)));
+  KLLM_SEQ_DISPATCH(a.dtype, (launch_ahead(resid_norm_kernel<AT>, dim3(a.T), dim3(threads), smem, s, a)));
   return done();
 }
 
@@ -1604,10 +1623,10 @@ int launch_qk_prepare(int dtype, const AttnShape& a, const RopeArgs& rope_, cons
     const bool vec = qn % 4 == 0 && kn % 4 == 0 && vn % 4 == 0 && stride % 4 == 0 && (reinterpret_cast<uintptr_t>(qkvg) & 15) == 0;
     const int threads = T <= 16 ? 512 : 256;
     if (vec)
-      KLLM_SEQ_DISPATCH(dtype, (qk_rows_kernel<AT, 4><<<T, threads, 0, s>>>(a, qkvg, stride, qnorm_w, knorm_w, eps, tok_seq, tok_pos,
+      KLLM_SEQ_DISPATCH(dtype, (launch_ahead(qk_rows_kernel<AT, 4>, dim3(T), dim3(threads), 0, s, a, qkvg, stride, qnorm_w, knorm_w, eps, tok_seq, tok_pos,
                                                                             static_cast<AT*>(q), gates, kv, blend)));
     else
-      KLLM_SEQ_DISPATCH(dtype, (qk_rows_kernel<AT, 1><<<T, threads, 0, s>>>(a, qkvg, stride, qnorm_w, knorm_w, eps, tok_seq, tok_pos,
+      KLLM_SEQ_DISPATCH(dtype, (launch_ahead(qk_rows_kernel<AT, 1>, dim3(T), dim3(threads), 0, s, a, qkvg, stride, qnorm_w, knorm_w, eps, tok_seq, tok_pos,
                                                                             static_cast<AT*>(q), gates, kv, blend)));
     return done();
   }
@@ -1618,7 +1637,7 @@ int launch_qk_prepare(int dtype, const AttnShape& a, const RopeArgs& rope_, cons
     const int threads = T <= 64 ? 512 : 256;
     const size_t smem = std::max<size_t>(16, 2 * static_cast<size_t>(half) * sizeof(float));
 #define KLLM_QK_TURN(G)                                                                                                   \
-  KLLM_SEQ_DISPATCH(dtype, (qk_turn_kernel<AT, G><<<T, threads, smem, s>>>(a, rope, qkvg, stride, qnorm_w, knorm_w, eps, tok_seq, \
+  KLLM_SEQ_DISPATCH(dtype, (launch_ahead(qk_turn_kernel<AT, G>, dim3(T), dim3(threads), smem, s, a, rope, qkvg, stride, qnorm_w, knorm_w, eps, tok_seq, \
                                                                           tok_pos, static_cast<AT*>(q), gates, kv)))
     if (units <= 8) KLLM_QK_TURN(8);
     else if (units <= 16) KLLM_QK_TURN(16);
@@ -1631,7 +1650,7 @@ int launch_qk_prepare(int dtype, const AttnShape& a, const RopeArgs& rope_, cons
   int warps = T <= 64 ? std::min(16, std::max(4, a.heads + a.kv_heads)) : 4;
   warps = std::max(1, std::min(warps, 48 * 1024 / (4 * a.dim)));
   const size_t smem = static_cast<size_t>(warps) * a.dim * sizeof(float);
-  KLLM_SEQ_DISPATCH(dtype, (qk_prepare_kernel<AT><<<T, 32 * warps, smem, s>>>(a, rope, qkvg, stride, qnorm_w, knorm_w, eps, tok_seq,
+  KLLM_SEQ_DISPATCH(dtype, (launch_ahead(qk_prepare_kernel<AT>, dim3(T), dim3(32 * warps), smem, s, a, rope, qkvg, stride, qnorm_w, knorm_w, eps, tok_seq,
                                                                              tok_pos, static_cast<AT*>(q), gates, kv, blend)));
   return done();
 }
@@ -1681,7 +1700,7 @@ static int launch_attention_cs(const AttnShape& a, const void* q, const PagedKV&
   }
   const int rep = a.heads / a.kv_heads;
   const dim3 grid((max_count * rep + kAttnRows - 1) / kAttnRows, n_entries * a.kv_heads, splits);
-  attention_kernel<AT, C, SPARSE, RS><<<grid, kAttnThreads, smem, s>>>(a, q, kv, ent_first, ent_count, ent_seq, ent_pos0, splits,
+  launch_ahead(attention_kernel<AT, C, SPARSE, RS>, dim3(grid), dim3(kAttnThreads), smem, s, a, q, kv, ent_first, ent_count, ent_seq, ent_pos0, splits,
                                                                        ws);
   return done();
 }
@@ -1736,7 +1755,7 @@ int launch_attention(int dtype, const AttnShape& a, const void* q, const float* 
 #undef KLLM_ATTN_C
   }
   if (rc || a.no_merge) return rc;
-  KLLM_SEQ_DISPATCH(dtype, (attention_merge_kernel<AT><<<T * a.heads, a.vdim <= 64 ? 64 : 128, splits * sizeof(float), s>>>(a.heads, a.vdim, splits, ws,
+  KLLM_SEQ_DISPATCH(dtype, (launch_ahead(attention_merge_kernel<AT>, dim3(T * a.heads), dim3(a.vdim <= 64 ? 64 : 128), splits * sizeof(float), s, a.heads, a.vdim, splits, ws,
                                                                                  a.gate ? gates : nullptr, a.gate, a.sink,
                                                                                  a.out_f32, out)));
   return done();
@@ -1764,7 +1783,7 @@ int launch_expert_gate_up(int dtype, const void* h, const void* gate_up, const i
   if (smem > 48 * 1024) return KLLM_E_UNSUPPORTED;
   const int kPairRows = pair_rows(T * top);
   const dim3 grid(T * top + (sh.ff > 0 ? T : 0), (std::max(ff, sh.ff) + kPairRows - 1) / kPairRows);
-  KLLM_SEQ_DISPATCH(dtype, (expert_gate_up_kernel<AT><<<grid, 128, smem, s>>>(static_cast<const AT*>(h),
+  KLLM_SEQ_DISPATCH(dtype, (launch_ahead(expert_gate_up_kernel<AT>, dim3(grid), dim3(128), smem, s, static_cast<const AT*>(h),
                                                                              static_cast<const AT*>(gate_up), top_idx,
                                                                              static_cast<AT*>(inter), T, top, ff, width,
                                                                              sh, act)));
@@ -1777,7 +1796,7 @@ int launch_expert_down(int dtype, const void* inter, const void* down, const int
   if (smem > 48 * 1024) return KLLM_E_UNSUPPORTED;
   const int kPairRows = pair_rows(T * top);
   const dim3 grid(T, (width + kPairRows - 1) / kPairRows);
-  KLLM_SEQ_DISPATCH(dtype, (expert_down_kernel<AT><<<grid, 128, smem, s>>>(static_cast<const AT*>(inter),
+  KLLM_SEQ_DISPATCH(dtype, (launch_ahead(expert_down_kernel<AT>, dim3(grid), dim3(128), smem, s, static_cast<const AT*>(inter),
                                                                           static_cast<const AT*>(down), top_idx, top_w,
                                                                           y, top, ff, width, sh)));
   return done();

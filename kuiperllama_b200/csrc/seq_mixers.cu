@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "seq_engine.h"
+#include "seq_launch.cuh"
 #include "seq_linear.cuh"
 #include "seq_merge.cuh"
 
@@ -128,6 +129,8 @@ __global__ void latent_prepare_kernel(LatentShape a, const float* __restrict__ p
                                       const float* __restrict__ kv_norm_w, float eps, const int32_t* __restrict__ tok_seq,
                                       const int32_t* __restrict__ tok_pos, AT* __restrict__ cq, float* __restrict__ gates,
                                       PagedKV kv, AT* __restrict__ c_rows, float* __restrict__ kr_rows) {
+  next_may_start();
+  after_previous();
   __shared__ float red[33];
   const int t = blockIdx.x;
   const int stride = latent_proj_rows(a);
@@ -207,6 +210,8 @@ template <typename AT, int NT>
 __global__ void __launch_bounds__(kFewWarps * 32)
 latent_absorb_few_kernel(LatentShape a, const float* __restrict__ q, int q_row, const AT* __restrict__ w_uk,
                          const int32_t* __restrict__ tok_pos, float* __restrict__ qa, int T) {
+  next_may_start();
+  after_previous();
   constexpr int V = Wide<AT>::N, LPR = kFewCols / V, RPW = 32 / LPR;  // values per lane, lanes per row, rows per warp
   constexpr int kStep = kFewWarps * RPW;
   extern __shared__ float qs[];                 // [NT][dim + rot_dim]
@@ -374,6 +379,8 @@ template <typename AT, bool VEC>
 __global__ void __launch_bounds__(kExpandWarps * 32)
 latent_merge_expand_kernel(LatentShape a, int splits, const float* __restrict__ ws, const float* __restrict__ gates,
                            const float* __restrict__ sink, const AT* __restrict__ w_uv, AT* __restrict__ out) {
+  next_may_start();
+  after_previous();
   extern __shared__ __align__(16) float ls[];  // [kv_rank], then [splits] weights
   float* weight = ls + a.kv_rank;
   constexpr int V = VEC ? Wide<AT>::N : 1;
@@ -779,6 +786,8 @@ __global__ void __launch_bounds__(512)
 linear_token_kernel(int heads, int dim, int vdim, const float* __restrict__ decay, LinearRot rot, int silu,
                     const float* __restrict__ proj, int stride, int gate_act, float eps, float* __restrict__ state,
                     const int32_t* __restrict__ tok_seq, const int32_t* __restrict__ tok_pos, AT* __restrict__ out) {
+  next_may_start();
+  after_previous();
   extern __shared__ __align__(16) float sm[];
   __shared__ float red[33];
   const int h = blockIdx.x, t = blockIdx.y, tid = threadIdx.x;
@@ -939,7 +948,7 @@ inline int done() {
 int launch_latent_prepare(int dtype, const LatentShape& a, const float* proj, const float* q_norm_w, const float* kv_norm_w,
                           float eps, const int32_t* tok_seq, const int32_t* tok_pos, void* cq, float* gates,
                           const PagedKV& kv, void* c_rows, float* kr_rows, int T, cudaStream_t s) {
-  KLLM_SEQ_DISPATCH(dtype, (latent_prepare_kernel<AT><<<T, 128, 0, s>>>(a, proj, q_norm_w, kv_norm_w, eps, tok_seq, tok_pos,
+  KLLM_SEQ_DISPATCH(dtype, (launch_ahead(latent_prepare_kernel<AT>, dim3(T), dim3(128), 0, s, a, proj, q_norm_w, kv_norm_w, eps, tok_seq, tok_pos,
                                                                        static_cast<AT*>(cq), gates, kv,
                                                                        static_cast<AT*>(c_rows), kr_rows)));
   return done();
@@ -970,7 +979,7 @@ int launch_latent_absorb(int dtype, const LatentShape& a, const float* q, int q_
     const dim3 grid(a.heads, (a.kv_rank + kFewCols - 1) / kFewCols);
     const size_t few = static_cast<size_t>(T) * (a.dim + a.rot_dim) * sizeof(float);
 #define KLLM_ABSORB(NT)                                                                                                   \
-  KLLM_SEQ_DISPATCH(dtype, (latent_absorb_few_kernel<AT, NT><<<grid, kFewWarps * 32, few, s>>>(a, q, q_row,               \
+  KLLM_SEQ_DISPATCH(dtype, (launch_ahead(latent_absorb_few_kernel<AT, NT>, dim3(grid), dim3(kFewWarps * 32), few, s, a, q, q_row,               \
                                                                                                static_cast<const AT*>(w_uk), \
                                                                                                tok_pos, qa, T)))
     if (T == 1) KLLM_ABSORB(1);
@@ -994,10 +1003,10 @@ int launch_latent_merge_expand(int dtype, const LatentShape& a, int splits, cons
   const dim3 grid(T * a.heads, (a.vdim + kExpandRows - 1) / kExpandRows);
   const bool vec = a.kv_rank % 8 == 0 && (reinterpret_cast<uintptr_t>(w_uv) & 15) == 0;
   if (vec)
-    KLLM_SEQ_DISPATCH(dtype, (latent_merge_expand_kernel<AT, true><<<grid, kExpandWarps * 32, smem, s>>>(
+    KLLM_SEQ_DISPATCH(dtype, (launch_ahead(latent_merge_expand_kernel<AT, true>, dim3(grid), dim3(kExpandWarps * 32), smem, s, 
                                  a, splits, ws, gates, sink, static_cast<const AT*>(w_uv), static_cast<AT*>(out))));
   else
-    KLLM_SEQ_DISPATCH(dtype, (latent_merge_expand_kernel<AT, false><<<grid, kExpandWarps * 32, smem, s>>>(
+    KLLM_SEQ_DISPATCH(dtype, (launch_ahead(latent_merge_expand_kernel<AT, false>, dim3(grid), dim3(kExpandWarps * 32), smem, s, 
                                  a, splits, ws, gates, sink, static_cast<const AT*>(w_uv), static_cast<AT*>(out))));
   return done();
 }
@@ -1105,11 +1114,11 @@ int launch_linear_token(int dtype, const kllm_seq_linear& m, const float* proj, 
   const LinearRot rot = linear_rot(m);
   const int silu = m.qkv_act == KLLM_SEQ_QKV_SILU;
   if (vec)
-    KLLM_SEQ_DISPATCH(dtype, (linear_token_kernel<AT, 4><<<grid, threads, smem, s>>>(m.heads, m.dim, m.vdim, m.decay, rot, silu, proj, row,
+    KLLM_SEQ_DISPATCH(dtype, (launch_ahead(linear_token_kernel<AT, 4>, dim3(grid), dim3(threads), smem, s, m.heads, m.dim, m.vdim, m.decay, rot, silu, proj, row,
                                                                                     m.gate_act, eps, state, tok_seq, tok_pos,
                                                                                     static_cast<AT*>(out))));
   else
-    KLLM_SEQ_DISPATCH(dtype, (linear_token_kernel<AT, 1><<<grid, threads, smem, s>>>(m.heads, m.dim, m.vdim, m.decay, rot, silu, proj, row,
+    KLLM_SEQ_DISPATCH(dtype, (launch_ahead(linear_token_kernel<AT, 1>, dim3(grid), dim3(threads), smem, s, m.heads, m.dim, m.vdim, m.decay, rot, silu, proj, row,
                                                                                     m.gate_act, eps, state, tok_seq, tok_pos,
                                                                                     static_cast<AT*>(out))));
   return done();

@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "seq_engine.h"
+#include "seq_launch.cuh"
 
 namespace kllm {
 namespace seq {
@@ -64,6 +65,8 @@ template <> struct Cols<1> {
 template <typename AT, int S, int V, bool EXACT>
 __global__ void __launch_bounds__(512)
 streams_kernel(StreamArgs a) {
+  next_may_start();
+  after_previous();
   extern __shared__ __align__(16) float us[];  // [width]
   __shared__ float red[33];
   const int W = a.width, n = EXACT ? S : a.streams;
@@ -170,8 +173,8 @@ int launch_s(const StreamArgs& a, cudaStream_t s) {
   // few rows: as many loads in flight as a row has; many rows: several CTAs per SM, so that one's reduction hides behind the
   // others' loads
   const int threads = std::max(64, std::min(a.T <= 16 ? 512 : 256, (per + 31) / 32 * 32));
-  if (vec) streams_kernel<AT, S, 4, EXACT><<<a.T, threads, smem, s>>>(a);
-  else streams_kernel<AT, S, 1, EXACT><<<a.T, threads, smem, s>>>(a);
+  if (vec) launch_ahead(streams_kernel<AT, S, 4, EXACT>, dim3(a.T), dim3(threads), smem, s, a);
+  else launch_ahead(streams_kernel<AT, S, 1, EXACT>, dim3(a.T), dim3(threads), smem, s, a);
   count_launch();
   return cuda_rc(cudaGetLastError());
 }
