@@ -25,17 +25,15 @@
 namespace kllm {
 namespace {
 
-// The narrowest token block that holds the rows.  Two weight matrices share a token tile, whose sums have to fit the epilogue's
-// registers: at most 64 tokens there, else 128.
+// The narrowest token block that holds the rows; where 128-token tiles fill the chip, persistent CTAs.
 template <int OUT>
 int product(const seq::umma::SplitArgs& p, cudaStream_t s, bool ahead = true) {
   using namespace seq::umma;
-  constexpr bool two = OUT == kGated;
-  if (p.T <= 16) return launch_split<kTf32, 16, OUT, two ? 3 : 5>(p, s, ahead);
-  if (p.T <= 32) return launch_split<kTf32, 32, OUT, two ? 3 : 5>(p, s, ahead);
-  if (two || p.T <= 64) return launch_split<kTf32, 64, OUT, two ? 2 : 4>(p, s, ahead);
-  if constexpr (!two) return launch_split<kTf32, 128, OUT, 3>(p, s, ahead);
-  return KLLM_E_UNSUPPORTED;
+  if (fills_chip(p.T, p.N)) return launch_wide<kTf32, OUT>(p, s);
+  if (p.T <= 16) return launch_split<kTf32, 16, OUT, 5>(p, s, ahead);
+  if (p.T <= 32) return launch_split<kTf32, 32, OUT, 5>(p, s, ahead);
+  if (p.T <= 64) return launch_split<kTf32, 64, OUT, 4>(p, s, ahead);
+  return launch_split<kTf32, 128, OUT, 3>(p, s, ahead);
 }
 // TMA needs 16-byte aligned bases and row pitches
 bool aligned(const void* x, const void* w, int K) {

@@ -20,6 +20,8 @@
 // CTA hands its accumulator over every SECTION blocks of K to the epilogue warps, which sum the sections in fp32 registers
 // while the tensor core fills the other accumulator.  kFp32 keeps the two small products in an accumulator of their own.
 //
+// Gated: as in umma_kernel a tile is 64 features, their gate rows above their up rows; the two meet in the partial tile.
+//
 // Measured, calls back to back with weights from HBM (one B200), the FMA tiles that these shapes took before -> now; error
 // against 64 bits in the 2-norm:
 //   bf16  T = 40, K = 4096, N = 4096    298 -> 14.6 us    6.1e-7 -> 1.4e-7
@@ -40,26 +42,6 @@ namespace umma {
 // for 4 and for 8 CTAs).
 constexpr int kMinSplitBlocks = 3;
 
-enum Mode { kBf16 = 0, kTf32 = 1, kFp32 = 2 };
-template <int MODE> struct ModeOf {  // fp32 operands
-  static constexpr int BKE = 32;     // elements of K per 128-byte block
-  static constexpr int SECTION = 2;  // blocks between two hand-overs of the accumulator: 8 steps
-};
-template <> struct ModeOf<kBf16> {
-  static constexpr int BKE = 64;
-  static constexpr int SECTION = 2;  // 8 steps
-};
-
-// instruction descriptor as in instr_desc, A = B = TF32 (2 << 7, 2 << 10)
-__device__ __forceinline__ uint32_t instr_desc_tf32(int n) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
-}
-__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
-}
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -68,6 +50,8 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
 // the address of `saddr` (a shared-memory address of this CTA) in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t peer_smem(uint32_t saddr, uint32_t rank) {
   uint32_t r;
@@ -88,66 +72,41 @@ __device__ __forceinline__ float low_part(float x, float& check) {
   return __uint_as_float(__float_as_uint(lo) + 0x1000u);
 }
 
-// what a product does with its sums
-enum Out {
-  kPlain = 0,  // out = sum + bias (fp32)
-  kGated = 1,  // out = gated_act(sum of w + bias[n], sum of w2 + bias[N + n]) in the operands' type
-  kAdd = 2     // out = add + sum (fp32; add may be out itself)
-};
-
-// operand pointers (kFp32's fallback for infinities reads through them) and what joins the sums
-struct SplitArgs {
-  const void *a, *w, *w2;
-  const float* bias;
-  const float* add;
-  void* out;
-  int T, N, K, S;
-  GatedAct act;
-  int* report;  // wait_flag()
-};
-
-template <int MODE, int OUT>
-__device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, float v, float u) {
-  const size_t at = static_cast<size_t>(t) * p.N + row;
-  if constexpr (OUT == kGated) {
-    const float y = gated_act(p.act, p.bias ? v + p.bias[row] : v, p.bias ? u + p.bias[p.N + row] : u);
-    if constexpr (MODE == kBf16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(y);
-    else static_cast<float*>(p.out)[at] = y;
-  } else if constexpr (OUT == kAdd) {
-    static_cast<float*>(p.out)[at] = p.add[at] + v;
-  } else {
-    static_cast<float*>(p.out)[at] = p.bias ? v + p.bias[row] : v;
-  }
-}
-
-// This CTA's tokens of the tile, summed over the cluster's partial tiles in rank order.  A read from another CTA takes about a
-// microsecond: a group's reads are all on the way before the first is used (T = 40, K = N = 4096: 15.4 us token by token with
-// the sections of 512, 14.6 us with sections of 128).
+// This CTA's tokens of the tile, summed over the cluster's S partial tiles in rank order: column rank * BN / S + j for the j that
+// this thread has (gated: the threads of the upper 64 rows take every other column of the lower ones' features).  A read from
+// another CTA takes about a microsecond: a group's reads are all on the way before the first is used (T = 40, K = N = 4096: 15.4 us
+// token by token, 14.6 us).
 template <int MODE, int BN, int OUT, int S>
-__device__ __forceinline__ void split_reduce(const SplitArgs& p, uint32_t mine, int rank, int t0, int row) {
-  constexpr int NA = OUT == kGated ? 2 : 1, PER = BN / S, GROUP = PER < 64 / (S * NA) ? PER : 64 / (S * NA);
+__device__ __forceinline__ void split_reduce(const SplitArgs& p, const float* part, int rank, int t0, int n0, int thread) {
+  constexpr bool two = OUT == kGated;
+  constexpr int FEATURES = two ? BM / 2 : BM, STEP = two ? 2 : 1, PER = BN / S / STEP;  // columns of a thread
+  constexpr int GROUP = PER < 32 / S ? PER : 32 / S;
   static_assert(PER >= 1 && PER % GROUP == 0, "tokens of a CTA");
+  const int feature = thread % FEATURES, row = n0 + feature;
+  if (row >= p.N) return;
+  const uint32_t mine = smem_u32(part + feature);
+  const int c0 = rank * (BN / S) + (two ? thread / FEATURES : 0);
 #pragma unroll 1
   for (int g = 0; g < PER; g += GROUP) {
-    float v[GROUP][S], u[NA == 2 ? GROUP : 1][S];
+    float v[GROUP][S], u[two ? GROUP : 1][S];
 #pragma unroll
     for (int q = 0; q < S; ++q) {
-      const uint32_t from = peer_smem(mine, static_cast<uint32_t>(q)) + (rank * PER + g) * BM * 4;
+      const uint32_t from = (S > 1 ? peer_smem(mine, static_cast<uint32_t>(q)) : mine) + (c0 + g * STEP) * BM * 4;
 #pragma unroll
       for (int j = 0; j < GROUP; ++j) {
-        v[j][q] = ld_peer(from + j * BM * 4);
-        if constexpr (NA == 2) u[j][q] = ld_peer(from + (BN + j) * BM * 4);
+        v[j][q] = ld_peer(from + j * STEP * BM * 4);
+        if constexpr (two) u[j][q] = ld_peer(from + j * STEP * BM * 4 + FEATURES * 4);
       }
     }
 #pragma unroll
     for (int j = 0; j < GROUP; ++j) {
-      const int t = t0 + rank * PER + g + j;
+      const int t = t0 + c0 + (g + j) * STEP;
       if (t >= p.T) break;
-      float a = v[j][0], b = u[NA == 2 ? j : 0][0];
+      float a = v[j][0], b = u[two ? j : 0][0];
 #pragma unroll
       for (int q = 1; q < S; ++q) {
         a += v[j][q];
-        if constexpr (NA == 2) b += u[j][q];
+        if constexpr (two) b += u[j][q];
       }
       split_store<MODE, OUT>(p, t, row, a, b);
     }
@@ -163,13 +122,15 @@ __global__ void __launch_bounds__(split_threads<MODE>())
 umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
                   const __grid_constant__ CUtensorMap map_a, const SplitArgs p) {
   using M = ModeOf<MODE>;
-  constexpr int NA = OUT == kGated ? 2 : 1;
-  constexpr int W_BYTES = NA * A_BYTES, B_BYTES = BN * 128;
+  constexpr bool two = OUT == kGated;
+  constexpr int FEATURES = two ? BM / 2 : BM;
+  constexpr int W_BYTES = A_BYTES, B_BYTES = BN * 128;
   constexpr int HALF = W_BYTES + B_BYTES;                  // the tiles as they arrive
   constexpr int STAGE = MODE == kFp32 ? 2 * HALF : HALF;   // kFp32: the lo parts follow
-  constexpr int TILE_COLS = NA * BN;                       // of one sum
+  constexpr int TILE_COLS = BN;                            // of one sum
   constexpr int ACC_COLS = MODE == kFp32 ? 2 * TILE_COLS : TILE_COLS;  // of one accumulator; there are two
   constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
+  constexpr int AT_ONCE = BN < 32 || (MODE == kFp32 && BN > 64) ? 16 : 32;  // columns on the way from TMEM before the first is added
   static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "columns are given out in powers of two");
   static_assert(TILE_COLS * BM * 4 <= ST * STAGE, "the partial tile takes the place of the ring");
   extern __shared__ uint8_t raw_smem[];
@@ -184,7 +145,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   float* special = reinterpret_cast<float*>(tmem_slot + 2);  // kFp32: != 0 when an operand of this CTA's part of K is not finite
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * BM, t0 = blockIdx.z * BN;
+  const int n0 = blockIdx.x * FEATURES, t0 = blockIdx.z * BN;
   const int S = p.S, rank = S > 1 ? static_cast<int>(cluster_rank()) : 0;
   const int all_blocks = (p.K + M::BKE - 1) / M::BKE;
   const int kb0 = static_cast<int>(static_cast<long long>(all_blocks) * rank / S);
@@ -223,7 +184,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         uint8_t* st = base + (i % ST) * STAGE;
         mbar_expect_tx(bar, HALF);
         tma_load_2d(smem_u32(st), &map_w, bar, (kb0 + i) * M::BKE, n0);
-        if (NA == 2) tma_load_2d(smem_u32(st + A_BYTES), &map_w2, bar, (kb0 + i) * M::BKE, n0);
+        if (two) tma_load_2d(smem_u32(st + A_BYTES / 2), &map_w2, bar, (kb0 + i) * M::BKE, n0);
       };
       // the ring's first weights are on their way before the rows they meet are there
       for (int i = 0; i < ST && i < blocks; ++i) weights(i);
@@ -250,21 +211,18 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t st = smem_u32(base + s * STAGE);
+        const uint32_t d = tmem_d + b * ACC_COLS;
 #pragma unroll
-        for (int z = 0; z < NA; ++z) {
-          const uint32_t d = tmem_d + b * ACC_COLS + z * BN;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {  // 32 bytes of K per instruction, inside the swizzle row
-            const uint32_t joins = (!opens || k > 0) ? 1u : 0u;
-            const uint64_t wd = smem_desc(st + z * A_BYTES + k * 32), ad = smem_desc(st + W_BYTES + k * 32);
-            if constexpr (MODE == kBf16) {
-              mma_bf16(d, wd, ad, idesc, joins);
-            } else {
-              mma_tf32(d, wd, ad, idesc, joins);
-              if constexpr (MODE == kFp32) {
-                mma_tf32(d + TILE_COLS, smem_desc(st + HALF + z * A_BYTES + k * 32), ad, idesc, joins);
-                mma_tf32(d + TILE_COLS, wd, smem_desc(st + HALF + W_BYTES + k * 32), idesc, 1u);
-              }
+        for (int k = 0; k < 4; ++k) {  // 32 bytes of K per instruction, inside the swizzle row
+          const uint32_t joins = (!opens || k > 0) ? 1u : 0u;
+          const uint64_t wd = smem_desc(st + k * 32), ad = smem_desc(st + W_BYTES + k * 32);
+          if constexpr (MODE == kBf16) {
+            mma_bf16(d, wd, ad, idesc, joins);
+          } else {
+            mma_tf32(d, wd, ad, idesc, joins);
+            if constexpr (MODE == kFp32) {
+              mma_tf32(d + TILE_COLS, smem_desc(st + HALF + k * 32), ad, idesc, joins);
+              mma_tf32(d + TILE_COLS, wd, smem_desc(st + HALF + W_BYTES + k * 32), idesc, 1u);
             }
           }
         }
@@ -291,9 +249,8 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
     if (check != check) *special = 1.f;
   }
-  const int quarter = warp & 3, feature = quarter * 32 + lane;  // of the epilogue warps 2 .. 5
+  const int quarter = warp & 3, mine = quarter * 32 + lane;  // the tile row of a thread of the epilogue warps 2 .. 5
   const bool epilogue = warp >= 2 && warp < 6;
-  const int row = n0 + feature;
   float* part = reinterpret_cast<float*>(base);                 // [TILE_COLS][BM], in the place of the ring
   float acc[TILE_COLS];
   bool ok = true;
@@ -308,13 +265,13 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t from = tmem_d + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(b * ACC_COLS);
 #pragma unroll
-      for (int c = 0; c < TILE_COLS; c += 16) {
-        uint32_t r[16], r2[MODE == kFp32 ? 16 : 1];
-        tmem_ld16(from + c, r);
-        if constexpr (MODE == kFp32) tmem_ld16(from + TILE_COLS + c, r2);
+      for (int c = 0; c < TILE_COLS; c += AT_ONCE) {
+        uint32_t r[AT_ONCE], r2[MODE == kFp32 ? AT_ONCE : 1];
+        tmem_ld(from + c, r);
+        if constexpr (MODE == kFp32) tmem_ld(from + TILE_COLS + c, r2);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
+        for (int j = 0; j < AT_ONCE; ++j) {
           if constexpr (MODE == kFp32) acc[c + j] += __uint_as_float(r[j]) + __uint_as_float(r2[j]);
           else acc[c + j] += __uint_as_float(r[j]);
         }
@@ -324,41 +281,45 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
     }
     // the last section's commit covers every MMA of this CTA: nothing reads or writes the ring any more
-    if (S > 1)
+    if (S > 1 || two)
 #pragma unroll
-      for (int j = 0; j < TILE_COLS; ++j) part[j * BM + feature] = acc[j];
+      for (int j = 0; j < TILE_COLS; ++j) part[j * BM + mine] = acc[j];
   }
   __syncwarp();
   if (S > 1) cluster_sync();  // every partial tile of the cluster is in place
-  else if (MODE == kFp32) __syncthreads();  // and `special` is
-  if (epilogue && ok && row < p.N) {
+  else if (two || MODE == kFp32) __syncthreads();  // the partial tile is, and `special`
+  if (epilogue && ok) {
     bool recompute = false;
     if constexpr (MODE == kFp32) {
       for (int q = 0; q < S; ++q)
         recompute = recompute || (S > 1 ? ld_peer(peer_smem(smem_u32(special), q)) : *special) != 0.f;
     }
     if (MODE == kFp32 && recompute) {  // infinities, NaN: the sums as a chain of fp32 multiply-adds gives them
-      const int per = BN / S;
-      for (int j = rank * per; j < (rank + 1) * per && t0 + j < p.T; ++j) {
-        const float* ar = static_cast<const float*>(p.a) + static_cast<size_t>(t0 + j) * p.K;
-        const float* wr = static_cast<const float*>(p.w) + static_cast<size_t>(row) * p.K;
-        const float* wr2 = NA == 2 ? static_cast<const float*>(p.w2) + static_cast<size_t>(row) * p.K : wr;
-        float v = 0.f, u = 0.f;
-        for (int k = 0; k < p.K; ++k) {
-          v = fmaf(ar[k], wr[k], v);
-          if (NA == 2) u = fmaf(ar[k], wr2[k], u);
+      const int per = BN / S, row = n0 + mine;
+      if (mine < FEATURES && row < p.N) {
+        for (int j = rank * per; j < (rank + 1) * per && t0 + j < p.T; ++j) {
+          const float* ar = static_cast<const float*>(p.a) + static_cast<size_t>(t0 + j) * p.K;
+          const float* wr = static_cast<const float*>(p.w) + static_cast<size_t>(row) * p.K;
+          const float* wr2 = two ? static_cast<const float*>(p.w2) + static_cast<size_t>(row) * p.K : wr;
+          float v = 0.f, u = 0.f;
+          for (int k = 0; k < p.K; ++k) {
+            v = fmaf(ar[k], wr[k], v);
+            if (two) u = fmaf(ar[k], wr2[k], u);
+          }
+          split_store<MODE, OUT>(p, t0 + j, row, v, u);
         }
-        split_store<MODE, OUT>(p, t0 + j, row, v, u);
       }
-    } else if (S == 1) {
+    } else if (!two && S == 1) {
+      if (n0 + mine < p.N) {
 #pragma unroll
-      for (int j = 0; j < BN; ++j)
-        if (t0 + j < p.T) split_store<MODE, OUT>(p, t0 + j, row, acc[j], acc[NA == 2 ? BN + j : j]);
+        for (int j = 0; j < BN; ++j)
+          if (t0 + j < p.T) split_store<MODE, OUT>(p, t0 + j, n0 + mine, acc[j], 0.f);
+      }
     } else {
-      const uint32_t mine = smem_u32(part + feature);
-      if (S == 8) split_reduce<MODE, BN, OUT, 8>(p, mine, rank, t0, row);
-      else if (S == 4) split_reduce<MODE, BN, OUT, 4>(p, mine, rank, t0, row);
-      else split_reduce<MODE, BN, OUT, 2>(p, mine, rank, t0, row);
+      if (S == 8) split_reduce<MODE, BN, OUT, 8>(p, part, rank, t0, n0, mine);
+      else if (S == 4) split_reduce<MODE, BN, OUT, 4>(p, part, rank, t0, n0, mine);
+      else if (S == 2) split_reduce<MODE, BN, OUT, 2>(p, part, rank, t0, n0, mine);
+      else if constexpr (two) split_reduce<MODE, BN, OUT, 1>(p, part, rank, t0, n0, mine);
     }
   }
   __syncwarp();
@@ -373,22 +334,6 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   }
 }
 
-// [rows, cols] row-major, box [box_rows x 128 bytes], 128-byte swizzle
-template <int MODE>
-inline int make_map_of(CUtensorMap* map, const void* ptr, int rows, int cols, int box_rows) {
-  if constexpr (MODE == kBf16) return make_map(map, ptr, rows, cols, box_rows);
-  EncodeTiledFn fn = encode_tiled();
-  if (fn == nullptr) return KLLM_E_NODEVICE;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 4};
-  const cuuint32_t box[2] = {32u, static_cast<cuuint32_t>(box_rows)};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : KLLM_E_INVALID;
-}
-
 // How many CTAs share a tile's K: as many as one wave of the grid has room for (`room`), each with at least kMinSplitBlocks
 // blocks; a cluster of 8 is the largest portable one.  A second wave costs more than the shorter chains give (bf16, T = 64,
 // K = 4096, N = 11008, 86 tiles, room for 296: S = 1 35.0, 2 24.8, 4 31.2 us; T = 210, K = 1024, N = 4096, 128 tiles: 14.5,
@@ -401,14 +346,15 @@ inline int split_count(int tiles, int blocks, int room) {
 
 template <int MODE, int BN, int OUT, int ST>
 inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
-  constexpr int NA = OUT == kGated ? 2 : 1;
+  constexpr bool two = OUT == kGated;
+  constexpr int FEATURES = two ? BM / 2 : BM;
   CUtensorMap map_w, map_w2, map_a;
   p.report = wait_flag();
   if (p.report == nullptr) return KLLM_E_STATE;
-  if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, BM)) return rc;
-  if (int rc = make_map_of<MODE>(&map_w2, NA == 2 ? p.w2 : p.w, p.N, p.K, BM)) return rc;
+  if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, FEATURES)) return rc;
+  if (int rc = make_map_of<MODE>(&map_w2, two ? p.w2 : p.w, p.N, p.K, FEATURES)) return rc;
   if (int rc = make_map_of<MODE>(&map_a, p.a, p.T, p.K, BN)) return rc;
-  constexpr size_t smem = 1024 + static_cast<size_t>(ST) * (MODE == kFp32 ? 2 : 1) * (NA * A_BYTES + BN * 128) + 256;
+  constexpr size_t smem = 1024 + static_cast<size_t>(ST) * (MODE == kFp32 ? 2 : 1) * (A_BYTES + BN * 128) + 256;
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kernel = umma_split_kernel<MODE, BN, OUT, ST>;
   static bool configured = false;
@@ -417,7 +363,7 @@ inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
-  const int feature_tiles = (p.N + BM - 1) / BM, token_tiles = (p.T + BN - 1) / BN;
+  const int feature_tiles = (p.N + FEATURES - 1) / FEATURES, token_tiles = (p.T + BN - 1) / BN;
   p.S = split_count(feature_tiles * token_tiles, (p.K + ModeOf<MODE>::BKE - 1) / ModeOf<MODE>::BKE, (smem <= 113 * 1024 ? 2 : 1) * kSms);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(feature_tiles, p.S, token_tiles);
@@ -436,17 +382,16 @@ inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 
-// the narrowest token block that holds the step; more than 128 tokens (gated: 64) in tiles of 64
+// the narrowest token block that holds the step; more than 128 tokens in tiles of 64
 template <bool GATED>
 int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act,
                cudaStream_t s, bool ahead) {
   const void* w2 = static_cast<const __nv_bfloat16*>(w) + static_cast<size_t>(N) * K;  // the up rows follow the gate rows
   const SplitArgs p{a, w, w2, bias, nullptr, out, T, N, K, 1, act, nullptr};
   constexpr int OUT = GATED ? kGated : kPlain;
-  if (T <= 16) return launch_split<kBf16, 16, OUT, GATED ? 3 : 5>(p, s, ahead);
-  if (T <= 32) return launch_split<kBf16, 32, OUT, GATED ? 3 : 5>(p, s, ahead);
-  if constexpr (!GATED)
-    if (T > 64 && T <= 128) return launch_split<kBf16, 128, OUT, 3>(p, s, ahead);  // one tile: the weights are read once
+  if (T <= 16) return launch_split<kBf16, 16, OUT, 5>(p, s, ahead);
+  if (T <= 32) return launch_split<kBf16, 32, OUT, 5>(p, s, ahead);
+  if (T > 64 && T <= 128) return launch_split<kBf16, 128, OUT, 3>(p, s, ahead);  // one tile: the weights are read once
   return launch_split<kBf16, 64, OUT, 4>(p, s, ahead);
 }
 
@@ -463,9 +408,8 @@ int launch_fp32(const float* a, const float* w, const float* bias, float* out, i
   constexpr int OUT = GATED ? kGated : kPlain;
   if (T <= 16) return launch_split<kFp32, 16, OUT, 3>(p, s, ahead);
   if (T <= 32) return launch_split<kFp32, 32, OUT, 3>(p, s, ahead);
-  if (GATED || T <= 64) return launch_split<kFp32, 64, OUT, GATED ? 2 : 4>(p, s, ahead);
-  if constexpr (!GATED) return launch_split<kFp32, 128, OUT, 3>(p, s, ahead);
-  return KLLM_E_UNSUPPORTED;
+  if (T <= 64) return launch_split<kFp32, 64, OUT, 4>(p, s, ahead);
+  return launch_split<kFp32, 128, OUT, 3>(p, s, ahead);
 }
 
 }  // namespace umma

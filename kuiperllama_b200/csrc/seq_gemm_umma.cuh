@@ -85,6 +85,30 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
 }
+enum Mode { kBf16 = 0, kTf32 = 1, kFp32 = 2 };
+template <int MODE> struct ModeOf {  // fp32 operands
+  static constexpr int BKE = 32;     // elements of K per 128-byte block
+  static constexpr int SECTION = 2;  // blocks between two hand-overs of the accumulator: 8 steps
+};
+template <> struct ModeOf<kTf32> {
+  static constexpr int BKE = 32;
+  static constexpr int SECTION = 1 << 20;  // the operands' ten bits bound the error: one section
+};
+template <> struct ModeOf<kBf16> {
+  static constexpr int BKE = 64;
+  static constexpr int SECTION = 2;  // 8 steps
+};
+
+// instruction descriptor as in instr_desc, A = B = TF32 (2 << 7, 2 << 10)
+__device__ __forceinline__ uint32_t instr_desc_tf32(int n) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
+}
+__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
+}
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -110,6 +134,38 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr) : "memory");
 }
 
+// what a product does with its sums
+enum Out {
+  kPlain = 0,  // out = sum + bias (fp32)
+  kGated = 1,  // out = gated_act(sum of w + bias[n], sum of w2 + bias[N + n]) in the operands' type
+  kAdd = 2     // out = add + sum (fp32; add may be out itself)
+};
+
+// operand pointers (kFp32's fallback for infinities reads through them) and what joins the sums
+struct SplitArgs {
+  const void *a, *w, *w2;
+  const float* bias;
+  const float* add;
+  void* out;
+  int T, N, K, S;
+  GatedAct act;
+  int* report;  // wait_flag()
+};
+
+template <int MODE, int OUT>
+__device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, float v, float u) {
+  const size_t at = static_cast<size_t>(t) * p.N + row;
+  if constexpr (OUT == kGated) {
+    const float y = gated_act(p.act, p.bias ? v + p.bias[row] : v, p.bias ? u + p.bias[p.N + row] : u);
+    if constexpr (MODE == kBf16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(y);
+    else static_cast<float*>(p.out)[at] = y;
+  } else if constexpr (OUT == kAdd) {
+    static_cast<float*>(p.out)[at] = p.add[at] + v;
+  } else {
+    static_cast<float*>(p.out)[at] = p.bias ? v + p.bias[row] : v;
+  }
+}
+
 // ---- token blocks: persistent CTAs ----------------------------------------------------------------------------------
 // One CTA per SM walks tiles of 128 weight rows x BN tokens.  The tile's accumulator alternates between two sets of BN TMEM columns,
 // so the epilogue of a tile runs under the products of the next, and the ring never drains between tiles.
@@ -129,11 +185,14 @@ constexpr size_t persistent_smem() {
   return 1024 + static_cast<size_t>(kPersistentStages<BN>) * (A_BYTES + BN * BK * 2) + (GATED ? kExchangeBytes : 0) + 256;
 }
 
-template <int BN, bool GATED>
+template <int MODE, int BN, int OUT>
 __global__ void __launch_bounds__(kPersistentThreads, 1)
 umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_up,
-            const __grid_constant__ CUtensorMap map_a, void* __restrict__ out_, const float* __restrict__ bias, int T, int N, int K,
-            GatedAct act, int* report) {
+            const __grid_constant__ CUtensorMap map_a, const SplitArgs p) {
+  static_assert(MODE != kFp32, "operands are taken as they arrive");
+  constexpr bool GATED = OUT == kGated;
+  constexpr int BKE = ModeOf<MODE>::BKE;
+  const int T = p.T, N = p.N, K = p.K;
   constexpr int ST = kPersistentStages<BN>, B_BYTES = BN * BK * 2, STAGE = A_BYTES + B_BYTES;
   constexpr int FEATURES = GATED ? BM / 2 : BM;  // of a tile
   constexpr uint32_t TMEM_COLS = 2 * BN;
@@ -145,10 +204,10 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
   uint64_t* acc_full = empty + ST;     // [2]
   uint64_t* acc_empty = acc_full + 2;  // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), report};
+  const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), p.report};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kblocks = (K + BK - 1) / BK;
+  const int kblocks = (K + BKE - 1) / BKE;
   const int feature_tiles = (N + FEATURES - 1) / FEATURES, tiles = feature_tiles * ((T + BN - 1) / BN);
 
   if (threadIdx.x == 0) {
@@ -186,15 +245,15 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
           const uint32_t bar = smem_u32(&full[s]);
           uint8_t* st = base + s * STAGE;
           mbar_expect_tx(bar, STAGE);
-          tma_load_2d(smem_u32(st), &map_w, bar, kb * BK, n0);
-          if (GATED) tma_load_2d(smem_u32(st + A_BYTES / 2), &map_up, bar, kb * BK, n0);
-          tma_load_2d(smem_u32(st + A_BYTES), &map_a, bar, kb * BK, t0);
+          tma_load_2d(smem_u32(st), &map_w, bar, kb * BKE, n0);
+          if (GATED) tma_load_2d(smem_u32(st + A_BYTES / 2), &map_up, bar, kb * BKE, n0);
+          tma_load_2d(smem_u32(st + A_BYTES), &map_a, bar, kb * BKE, t0);
         }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc = instr_desc(BN);
+      const uint32_t idesc = MODE == kBf16 ? instr_desc(BN) : instr_desc_tf32(BN);
       int i = 0, done = 0;  // blocks of K and tiles so far
       bool ok = true;
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++done) {
@@ -207,9 +266,11 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a_addr = smem_u32(base + s * STAGE), b_addr = a_addr + A_BYTES;
 #pragma unroll
-          for (int k = 0; k < BK / UK; ++k)  // 32 bytes of K per instruction, inside the swizzle row
-            mma_bf16(tmem_d + b * BN, smem_desc(a_addr + k * UK * 2), smem_desc(b_addr + k * UK * 2), idesc,
-                     (kb > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < 4; ++k) {  // 32 bytes of K per instruction, inside the swizzle row
+            const uint32_t joins = (kb > 0 || k > 0) ? 1u : 0u;
+            if constexpr (MODE == kBf16) mma_bf16(tmem_d + b * BN, smem_desc(a_addr + k * 32), smem_desc(b_addr + k * 32), idesc, joins);
+            else mma_tf32(tmem_d + b * BN, smem_desc(a_addr + k * 32), smem_desc(b_addr + k * 32), idesc, joins);
+          }
           mma_commit(smem_u32(&empty[s]));
         }
         if (ok) mma_commit(smem_u32(&acc_full[b]));
@@ -233,8 +294,6 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
       };
       if constexpr (!GATED) {
         const int row = n0 + quarter * 32 + lane;
-        const float add = bias != nullptr && row < N ? bias[row] : 0.f;
-        float* out = static_cast<float*>(out_) + row;
 #pragma unroll 1
         for (int c = c_begin; c < c_end; c += 32) {
           uint32_t r[32];
@@ -244,14 +303,12 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
           if (ok && row < N) {
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (t0 + c + j < T) out[static_cast<size_t>(t0 + c + j) * N] = __uint_as_float(r[j]) + add;
+              if (t0 + c + j < T) split_store<MODE, OUT>(p, t0 + c + j, row, __uint_as_float(r[j]), 0.f);
           }
         }
       } else {
         const int pair = quarter & 1, row = n0 + pair * 32 + lane;  // quarters 0, 1: gate rows; 2, 3: up rows of the same features
         const bool up = quarter >= 2;
-        const float add = bias != nullptr && row < N ? bias[row] : 0.f, add_up = bias != nullptr && row < N ? bias[N + row] : 0.f;
-        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(out_) + row;
         float* buf = exchange + (2 * half + pair) * (2 * kPairCols * 32) + lane;
 #pragma unroll 1
         for (int c = c_begin; c < c_end; c += kPairCols) {
@@ -274,13 +331,11 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
             if (up) {
 #pragma unroll
               for (int j = 16; j < 32; ++j)
-                if (t0 + c + j < T)
-                  out[static_cast<size_t>(t0 + c + j) * N] = __float2bfloat16_rn(gated_act(act, x[j * 32] + add, __uint_as_float(r[j]) + add_up));
+                if (t0 + c + j < T) split_store<MODE, OUT>(p, t0 + c + j, row, x[j * 32], __uint_as_float(r[j]));
             } else {
 #pragma unroll
               for (int j = 0; j < 16; ++j)
-                if (t0 + c + j < T)
-                  out[static_cast<size_t>(t0 + c + j) * N] = __float2bfloat16_rn(gated_act(act, __uint_as_float(r[j]) + add, x[j * 32] + add_up));
+                if (t0 + c + j < T) split_store<MODE, OUT>(p, t0 + c + j, row, __uint_as_float(r[j]), x[j * 32]);
             }
           }
         }
@@ -509,29 +564,55 @@ inline int make_map(CUtensorMap* map, const void* ptr, int rows, int cols, int b
   return r == CUDA_SUCCESS ? 0 : KLLM_E_INVALID;
 }
 
-template <int BN, bool GATED>
-inline int launch_persistent(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act,
-                             cudaStream_t stream) {
-  constexpr int FEATURES = GATED ? BM / 2 : BM;
+// [rows, cols] row-major, box [box_rows x 128 bytes], 128-byte swizzle
+template <int MODE>
+inline int make_map_of(CUtensorMap* map, const void* ptr, int rows, int cols, int box_rows) {
+  if constexpr (MODE == kBf16) return make_map(map, ptr, rows, cols, box_rows);
+  EncodeTiledFn fn = encode_tiled();
+  if (fn == nullptr) return KLLM_E_NODEVICE;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 4};
+  const cuuint32_t box[2] = {32u, static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : KLLM_E_INVALID;
+}
+
+template <int MODE, int BN, int OUT>
+inline int launch_persistent(SplitArgs p, cudaStream_t stream) {
+  constexpr int FEATURES = OUT == kGated ? BM / 2 : BM;
   CUtensorMap map_w, map_up, map_a;
-  int* const report = wait_flag();
-  if (report == nullptr) return KLLM_E_STATE;
-  const __nv_bfloat16* up = static_cast<const __nv_bfloat16*>(w) + (GATED ? static_cast<size_t>(N) * K : 0);  // 16-byte rows: K % 8 == 0
-  if (int rc = make_map(&map_w, w, N, K, FEATURES)) return rc;
-  if (int rc = make_map(&map_up, up, N, K, FEATURES)) return rc;
-  if (int rc = make_map(&map_a, a, T, K, BN)) return rc;
-  constexpr size_t smem = persistent_smem<BN, GATED>();
+  p.report = wait_flag();
+  if (p.report == nullptr) return KLLM_E_STATE;
+  if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, FEATURES)) return rc;
+  if (int rc = make_map_of<MODE>(&map_up, OUT == kGated ? p.w2 : p.w, p.N, p.K, FEATURES)) return rc;
+  if (int rc = make_map_of<MODE>(&map_a, p.a, p.T, p.K, BN)) return rc;
+  constexpr size_t smem = persistent_smem<BN, OUT == kGated>();
   static_assert(smem <= 232448, "shared memory of one CTA");
+  auto kernel = umma_kernel<MODE, BN, OUT>;
   static bool configured = false;
   if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(umma_kernel<BN, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
-  const int tiles = ((N + FEATURES - 1) / FEATURES) * ((T + BN - 1) / BN);
-  umma_kernel<BN, GATED><<<tiles < kSms ? tiles : kSms, kPersistentThreads, smem, stream>>>(map_w, map_up, map_a, out, bias, T, N, K, act, report);
+  const int tiles = ((p.N + FEATURES - 1) / FEATURES) * ((p.T + BN - 1) / BN);
+  kernel<<<tiles < kSms ? tiles : kSms, kPersistentThreads, smem, stream>>>(map_w, map_up, map_a, p);
   count_launch();
   return static_cast<int>(cudaGetLastError());
+}
+// whether a product has a tile of 128 tokens for every SM
+inline bool fills_chip(int T, int N) { return T > 64 && ((N + BM - 1) / BM) * ((T + 127) / 128) >= kSms; }
+// The wider tile, unless its last wave is so empty that the narrower one, whose tiles take 0.65 of the time, is done sooner.
+template <int MODE, int OUT>
+inline int launch_wide(const SplitArgs& p, cudaStream_t s) {
+  const int feature_tiles = OUT == kGated ? (p.N + BM / 2 - 1) / (BM / 2) : (p.N + BM - 1) / BM;
+  const int waves_wide = (feature_tiles * ((p.T + 255) / 256) + kSms - 1) / kSms;
+  const int waves = (feature_tiles * ((p.T + 127) / 128) + kSms - 1) / kSms;
+  if (100 * waves_wide <= 65 * waves) return launch_persistent<MODE, 256, OUT>(p, s);
+  return launch_persistent<MODE, 128, OUT>(p, s);
 }
 
 // products whose tiles do not fill the chip (seq_gemm_split.cuh)
@@ -539,18 +620,13 @@ template <bool GATED>
 int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act, cudaStream_t s,
                bool ahead);
 
-// One token tile (which two CTAs on an SM stream through better: T = 100, K = 2048, N = 32000 31 us, one persistent CTA 32.4), or less
-// than one tile of 128 tokens per SM: narrower token blocks and K split over CTAs.  Else the wider tile, unless its last wave is
-// so empty that the narrower one, whose tiles take 0.65 of the time, is done sooner.
+// less than one tile of 128 tokens per SM: narrower token blocks and K split over CTAs
 template <bool GATED>
 inline int launch_block(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act,
                         cudaStream_t s, bool ahead) {
-  if (T <= (GATED ? 64 : 128) || ((N + BM - 1) / BM) * ((T + 127) / 128) < kSms) return launch_few<GATED>(a, w, bias, out, T, K, N, act, s, ahead);
-  const int feature_tiles = GATED ? (N + BM / 2 - 1) / (BM / 2) : (N + BM - 1) / BM;
-  const int waves_wide = (feature_tiles * ((T + 255) / 256) + kSms - 1) / kSms;
-  const int waves = (feature_tiles * ((T + 127) / 128) + kSms - 1) / kSms;
-  if (100 * waves_wide <= 65 * waves) return launch_persistent<256, GATED>(a, w, bias, out, T, K, N, act, s);
-  return launch_persistent<128, GATED>(a, w, bias, out, T, K, N, act, s);
+  if (!fills_chip(T, N)) return launch_few<GATED>(a, w, bias, out, T, K, N, act, s, ahead);
+  const void* w2 = static_cast<const __nv_bfloat16*>(w) + (GATED ? static_cast<size_t>(N) * K : 0);  // 16-byte rows: K % 8 == 0
+  return launch_wide<kBf16, GATED ? kGated : kPlain>(SplitArgs{a, w, w2, bias, nullptr, out, T, N, K, 1, act, nullptr}, s);
 }
 
 template <typename AT>
