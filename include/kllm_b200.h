@@ -132,7 +132,7 @@ int kllm_gemv_fused(const kllm_gemv_job* job, void* stream);
  * out[n_tokens, out_dim] = x[n_tokens, in_dim] . w[out_dim, in_dim]^T, all fp32 row-major device memory.
  * Replaces the n_tokens single-row GEMVs the reference issues for a prompt, one full forward per
  * prompt token (demo/main.cpp:18-23 -> LLama2Model::predict, llama3.cpp:147-167; MatmulLayer::forward,
- * matmul.cpp:57-80): the weight matrix is streamed once per 256 tokens instead of once per token.
+ * matmul.cpp:57-80): the weight matrix is streamed once per block of tokens instead of once per token.
  * TMA tensor-map loads (cp.async.bulk.tensor, 128-byte swizzle) feed tcgen05.mma.kind::tf32 with the
  * accumulator in TMEM.  Results agree with the fp32 GEMV to ~1e-3 relative (10-bit mantissas), NOT
  * bit for bit: the decode path never uses it.  in_dim % 4 == 0, 16-byte aligned x and w. */
@@ -241,8 +241,8 @@ int kllm_decoder_prompt(kllm_decoder* dec, const int32_t* tokens_host, int32_t n
                         int32_t* next_host);
 /* TOLERANCED batched prefill: the same contract as kllm_decoder_prompt, but the prompt positions go
  * through every layer together -- each projection one GEMM [n, in] x [out, in]^T on the tcgen05
- * tensor cores (TF32 multiply, fp32 accumulate, kllm_gemm_tf32), the weights streamed once per 256
- * positions instead of once per position; classifier only for the last position.  KV-cache rows and
+ * tensor cores (TF32 multiply, fp32 accumulate, kllm_gemm_tf32), the weights streamed once per
+ * block of up to 1024 positions instead of once per position; classifier only for the last position.  KV-cache rows and
  * logits agree with the position-by-position path to ~1e-3 relative, NOT bit for bit (TF32 keeps 10
  * mantissa bits).  fp32 checkpoints on one GPU; KLLM_E_UNSUPPORTED otherwise (use kllm_decoder_prompt). */
 int kllm_decoder_prefill_tf32(kllm_decoder* dec, const int32_t* tokens_host, int32_t n_tokens, int32_t start_pos,

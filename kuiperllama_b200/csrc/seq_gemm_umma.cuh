@@ -87,14 +87,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
 }
 enum Mode { kBf16 = 0, kTf32 = 1, kFp32 = 2 };
 template <int MODE> struct ModeOf {  // fp32 operands
+  using T = float;
   static constexpr int BKE = 32;     // elements of K per 128-byte block
   static constexpr int SECTION = 2;  // blocks between two hand-overs of the accumulator: 8 steps
 };
 template <> struct ModeOf<kTf32> {
+  using T = float;
   static constexpr int BKE = 32;
   static constexpr int SECTION = 1 << 20;  // the operands' ten bits bound the error: one section
 };
 template <> struct ModeOf<kBf16> {
+  using T = __nv_bfloat16;
   static constexpr int BKE = 64;
   static constexpr int SECTION = 2;  // 8 steps
 };
@@ -152,6 +155,8 @@ struct SplitArgs {
   int* report;  // wait_flag()
 };
 
+template <typename OT> __device__ __forceinline__ OT to_type(float v) { return v; }
+template <> __device__ __forceinline__ __nv_bfloat16 to_type<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <int MODE, int OUT>
 __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, float v, float u) {
   const size_t at = static_cast<size_t>(t) * p.N + row;
@@ -294,6 +299,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
       };
       if constexpr (!GATED) {
         const int row = n0 + quarter * 32 + lane;
+        const float add = OUT == kPlain && p.bias != nullptr && row < N ? p.bias[row] : 0.f;
 #pragma unroll 1
         for (int c = c_begin; c < c_end; c += 32) {
           uint32_t r[32];
@@ -301,14 +307,22 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if (c + 32 == c_end) release();
           if (ok && row < N) {
+            const size_t at = static_cast<size_t>(t0 + c) * N + row;
+            float* out = static_cast<float*>(p.out) + at;
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (t0 + c + j < T) split_store<MODE, OUT>(p, t0 + c + j, row, __uint_as_float(r[j]), 0.f);
+              if (t0 + c + j < T) {
+                if constexpr (OUT == kAdd) out[static_cast<size_t>(j) * N] = p.add[at + static_cast<size_t>(j) * N] + __uint_as_float(r[j]);
+                else out[static_cast<size_t>(j) * N] = __uint_as_float(r[j]) + add;
+              }
           }
         }
       } else {
         const int pair = quarter & 1, row = n0 + pair * 32 + lane;  // quarters 0, 1: gate rows; 2, 3: up rows of the same features
         const bool up = quarter >= 2;
+        const float add = p.bias != nullptr && row < N ? p.bias[row] : 0.f, add_up = p.bias != nullptr && row < N ? p.bias[N + row] : 0.f;
+        using OT = typename ModeOf<MODE>::T;
+        const GatedAct act = p.act;
         float* buf = exchange + (2 * half + pair) * (2 * kPairCols * 32) + lane;
 #pragma unroll 1
         for (int c = c_begin; c < c_end; c += kPairCols) {
@@ -328,14 +342,15 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
           }
           asm volatile("bar.sync %0, 64;" ::"r"(1 + 2 * half + pair) : "memory");
           if (ok && row < N) {
+            OT* out = static_cast<OT*>(p.out) + static_cast<size_t>(t0 + c) * N + row;
             if (up) {
 #pragma unroll
               for (int j = 16; j < 32; ++j)
-                if (t0 + c + j < T) split_store<MODE, OUT>(p, t0 + c + j, row, x[j * 32], __uint_as_float(r[j]));
+                if (t0 + c + j < T) out[static_cast<size_t>(j) * N] = to_type<OT>(gated_act(act, x[j * 32] + add, __uint_as_float(r[j]) + add_up));
             } else {
 #pragma unroll
               for (int j = 0; j < 16; ++j)
-                if (t0 + c + j < T) split_store<MODE, OUT>(p, t0 + c + j, row, __uint_as_float(r[j]), x[j * 32]);
+                if (t0 + c + j < T) out[static_cast<size_t>(j) * N] = to_type<OT>(gated_act(act, __uint_as_float(r[j]) + add, x[j * 32] + add_up));
             }
           }
         }
@@ -603,8 +618,10 @@ inline int launch_persistent(SplitArgs p, cudaStream_t stream) {
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }
-// whether a product has a tile of 128 tokens for every SM
-inline bool fills_chip(int T, int N) { return T > 64 && ((N + BM - 1) / BM) * ((T + 127) / 128) >= kSms; }
+// whether there is about a tile of 128 tokens for every SM: below that, splitting K over CTAs gives more (T = 1501, K = 2048, 1536
+// gated features, 144 tiles: 57 us split, 41 us here; TF32, T = 900, N = 2048, 128 tiles, K = 2048 and 5632: 26 and 104 us split,
+// 29 and 117 us here)
+inline bool fills_chip(int T, int N) { return T > 64 && ((N + BM - 1) / BM) * ((T + 127) / 128) >= kSms * 19 / 20; }
 // The wider tile, unless its last wave is so empty that the narrower one, whose tiles take 0.65 of the time, is done sooner.
 template <int MODE, int OUT>
 inline int launch_wide(const SplitArgs& p, cudaStream_t s) {

@@ -81,3 +81,59 @@ def test_split_product_fp32_keeps_infinities_and_nans(T):
     assert torch.equal(out == -float("inf"), ref == -float("inf"))
     fine = ref.isfinite()
     assert torch.allclose(out[fine], ref[fine], rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("T,K,N", [(129, 72, 18945), (300, 64, 8193), (1501, 520, 2050), (2048, 2048, 2561), (4000, 136, 640)])
+def test_persistent_product(T, K, N):
+    """Token blocks with a tile of 128 tokens per SM: persistent CTAs with tiles of 256 or 128 tokens, one accumulation over K (K / 16
+    steps of about 2^-24 each: within 2^-19 of the products' magnitudes up to K = 2048)."""
+    a, w, out = product(T, K, N, T + K)
+    bound = 2.0 ** -19 * (a.abs() @ w.abs().T)
+    assert ((out[:T].double() - a @ w.T).abs() <= bound).all()
+    assert (out[T] == 7.0).all()
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("tokens", [2500, 2432])
+def test_gated_block_against_portions(bf16, tokens):
+    """A gated feed-forward on a block that fills the chip against the same tokens in portions of 100, which take split tiles.  fp32:
+    other orders of sums only; bf16: rows round at 2^-9 behind other sums."""
+    import ctypes as ct
+
+    import numpy as np
+    from kuiperllama_b200.sequence import BF16, F32, BifazenShape, SeqEngine
+    shape = BifazenShape("b", 256, 300, (("attention", 1000),), 4, 4, 32, 16, 32, 64, 64, 4, 2, 32, 32, 96)
+    eng = SeqEngine(shape, BF16 if bf16 else F32, max_tokens=4096, max_seqs=2, seed=3)
+    ids = [int(x) for x in np.random.default_rng(tokens).integers(0, 300, tokens)]
+
+    def run(portions):
+        seq, rows = eng.open(), []
+        for p in portions:
+            n, buf = len(p), np.empty((len(p), 300), np.float32)
+            arr = ct.c_int32 * n
+            assert eng.lib.kllm_seq_step(eng.handle, 1, (ct.c_int32 * 1)(seq), (ct.c_int32 * 1)(n), arr(*p), n, arr(*range(n)),
+                                         buf.ctypes.data_as(ct.c_void_p), None) == 0
+            rows.append(buf)
+        eng.close_seq(seq)
+        return np.concatenate(rows)
+
+    whole, parts = run([ids]), run([ids[i:i + 100] for i in range(0, tokens, 100)])
+    eng.close()
+    off = np.abs(whole - parts).max(axis=1) / np.abs(parts).max()
+    assert off.max() < (4e-2 if bf16 else 1e-4)
+
+
+def test_prefill_block_that_fills_the_chip():
+    """460 tokens of a TinyLlama-wide model: the gated TF32 product runs on persistent CTAs; logits as close to the exact prompt path as
+    tests/test_prefill_gpu.py asks of shorter prompts."""
+    import numpy as np
+    from dataclasses import replace
+    from kuiperllama_b200 import SHAPES, Decoder, synth_weights
+    shape = replace(SHAPES["tinyllama-1.1b"], layer_num=2)
+    dec = Decoder(shape, synth_weights(shape, "cuda", 5))
+    toks = [1] + [int(t) for t in np.random.default_rng(1).integers(2, 32000, 459)]
+    dec.prompt(toks)
+    exact = dec.logits()
+    dec.prefill_tf32(toks)
+    assert np.abs(dec.logits() - exact).max() <= 2e-2 * np.abs(exact).max()
+    dec.close()
