@@ -23,8 +23,8 @@
 // at most 16 (token, query head) rows, one split of the keys, and walks tiles of 32 keys.  The queries enter as two bf16
 // terms when they are fp32, the weights always do, so both products see their left operand to about 2^-17.
 //
-// tcgen05 is not used here: at head sizes of 64..128 a 64-row tile is small against TMEM's 128-lane accumulators, and
-// the softmax between the two products wants the scores in registers anyway.
+// Long prompts take attention_umma_kernel (seq_attention_umma.cu); these kernels stay for short ones, where 128-key tiles are
+// mostly diagonal, and for key sizes past 128.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 

@@ -1,0 +1,458 @@
+// Prompt attention of the sequence-batch engine on the 5th-generation tensor cores (sm_100a): the problem of attention_mma_kernel
+// (seq_attention_mma.cu) for long prompts -- a CTA takes two groups of 128 consecutive rows of one entry and one key/value head, row
+// r = token r / rep, query head g * rep + r % rep, against tiles of 128 keys.
+//
+//   warps 0-3, 4-7  softmax of a group: thread t owns row t (TMEM lane t).  Reads its scores from TMEM, keeps maximum and sum in
+//                   registers, writes the weights over the scores as two bf16 terms, p = hi + lo, and rescales the output accumulator
+//                   where a maximum grew
+//   warps 8-11      loader: keys and values by 16-byte cp.async into tiles with the 128-byte swizzle (rows are scattered over pages)
+//   warp 12         one thread issues tcgen05.mma: S = Q K^T (both K-major in shared memory) and O += (hi + lo) V (weights from TMEM,
+//                   values with the head's coordinates contiguous: MN-major)
+//
+// TMEM: 128 columns of scores (then weights) and 128 of output for each group.  One group's products run under the other's softmax, and
+// both share a tile of keys and values.  The softmax bounds it.  On mma.sync with 16 rows a warp every 16 rows read all keys and values
+// from shared memory again, and the rate of the legacy tensor path bounded it.
+// Measured, a whole step of one layer (width 512) over 6001 tokens of four entries, heads / key heads x size: 16 / 4 x 128 538 -> 376 us,
+// 32 / 4 x 64 511 -> 428, 8 / 1 x 128 366 -> 314, 16 / 16 x 64 383 -> 371.  With one group of 128 rows a CTA 440, 515, 324, 404; with the
+// loader waiting for its copies before it announces them (its fence then waits for those just issued too) another 35 us.
+//
+// The maximum that a row subtracts follows the true one only when that is more than 8 (a factor of 256) ahead: the output in TMEM is
+// rescaled a few times instead of at every tile, and sums and weights keep their relative precision.  Keys and values come one tile
+// ahead, their pool rows three.
+//
+// Scores in units of log2 and ex2.approx, as in attention_mma_kernel; weights enter the second product to about 2^-17.  Every
+// mbarrier wait is bounded (seq_gemm_umma.cuh); a thread whose wait ran out keeps taking part in the warps' collective steps.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <cmath>
+#include <cstdint>
+#include <type_traits>
+
+#include "seq_engine.h"
+#include "seq_gemm_umma.cuh"
+#include "seq_mma.cuh"
+
+namespace kllm {
+namespace seq {
+namespace {
+
+constexpr int kTile = 128;                     // rows of a group, keys of a tile
+constexpr int kRows = 2 * kTile;               // rows of a CTA
+constexpr int kLoaders = 128, kAttnUmmaThreads = 256 + kLoaders + 32;
+constexpr int kHalfTile = kTile * 128;         // bytes of 128 rows x 64 coordinates
+constexpr int kColS = 0, kColO = 256;          // + 128 for the second group
+
+__device__ __forceinline__ float ex2(float x) {  // 2^x, relative error about 2^-22; 2^-inf = 0
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  uint32_t a[16], b[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) a[j] = r[j], b[j] = r[16 + j];
+  tmem_st16(taddr, a), tmem_st16(taddr + 16, b);
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// MN-major tile, 128-byte swizzle: 64 coordinates of a key are one 128-byte row; leading byte offset = the next 64 coordinates
+// (kHalfTile on), stride byte offset = the next 8 keys (1024 B)
+__device__ __forceinline__ uint64_t value_desc(uint32_t saddr) {
+  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(kHalfTile >> 4) << 16) | (64ull << 32) | (1ull << 46) |
+         (2ull << 61);
+}
+// A from TMEM (two bf16 per column and lane), B MN-major: bit 16 of the instruction descriptor
+__device__ __forceinline__ void mma_weights(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
+}
+// arrives when the thread's cp.async so far have landed
+__device__ __forceinline__ void arrive_copied(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(umma::smem_u32(bar)) : "memory");
+}
+// what the barriers waited for -- accumulators, and operands written by cp.async -- is the tensor core's to read
+__device__ __forceinline__ void after_wait() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(bar)) : "memory");
+}
+
+// KC, VC: 16-byte chunks of a key and of a value, 8 or 16
+template <int KC, int VC>
+__global__ void __launch_bounds__(kAttnUmmaThreads, 1)
+attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV kv, const int32_t* __restrict__ ent_first,
+                      const int32_t* __restrict__ ent_count, const int32_t* __restrict__ ent_seq,
+                      const int32_t* __restrict__ ent_pos0, int splits, float* __restrict__ ws, const float* __restrict__ gates,
+                      __nv_bfloat16* __restrict__ out, int* report) {
+  using namespace umma;
+  const int e = blockIdx.x / a.kv_heads, g = blockIdx.x % a.kv_heads, split = blockIdx.z;
+  const int gv = g / v_share_of(a), rep = a.heads / a.kv_heads, dim = a.dim, vdim = a.vdim;
+  const int first = ent_first[e], pos0 = ent_pos0[e], n_rows = ent_count[e] * rep;
+  const int r0 = (gridDim.y - 1 - blockIdx.y) * kRows;  // the tiles with the most keys start first
+  if (r0 >= n_rows) return;
+  const int pmax = pos0 + (min(r0 + kRows, n_rows) - 1) / rep;  // last position any row of the CTA sees
+  const int groups = r0 + kTile < n_rows ? 2 : 1;
+  // with a window or chunks no row sees anything before what the first row sees; tiles before that which hold kept
+  // first positions come ahead: this CTA's list of tiles is [0, keep_tiles) then [tile_first, last], cut into `splits` parts
+  const int tile_first = first_seen(a, pos0 + r0 / rep) / kTile;
+  const int keep_tiles = min(tile_first, (a.keep_first + kTile - 1) / kTile);
+  const int list_n = keep_tiles + pmax / kTile + 1 - tile_first, per = (list_n + splits - 1) / splits;
+  const int tile_lo = split * per, n = max(0, min(list_n, tile_lo + per) - tile_lo);
+  auto tile_of = [&](int i) {
+    const int li = tile_lo + i;
+    return li < keep_tiles ? li : tile_first + (li - keep_tiles);
+  };
+
+  extern __shared__ uint8_t raw_smem[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
+  uint8_t* Qs = base;                    // [2 groups][2 blocks of 64 coordinates][128 rows][128 bytes]
+  uint8_t* Ks = Qs + 4 * kHalfTile;      // [2 stages][2 blocks of 64 coordinates][128 keys][128 bytes]
+  uint8_t* Vs = Ks + 4 * kHalfTile;      // [2 stages] the same
+  uint64_t* bars = reinterpret_cast<uint64_t*>(Vs + 4 * kHalfTile);
+  uint64_t *k_full = bars, *k_empty = bars + 2, *v_full = bars + 4, *v_empty = bars + 6, *s_full = bars + 8, *p_full = bars + 10;
+  uint64_t *o_done = bars + 12, *q_full = bars + 14;
+  int32_t* slots = reinterpret_cast<int32_t*>(bars + 16);  // [4][128] rows of a tile's keys in the pool
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(slots + 4 * kTile);
+  const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), report};
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&k_full[s]), kLoaders);
+      mbar_init(smem_u32(&v_full[s]), kLoaders);
+      mbar_init(smem_u32(&k_empty[s]), 1);
+      mbar_init(smem_u32(&v_empty[s]), 1);
+      mbar_init(smem_u32(&s_full[s]), 1);
+      mbar_init(smem_u32(&p_full[s]), 4);
+      mbar_init(smem_u32(&o_done[s]), 1);
+    }
+    mbar_init(smem_u32(q_full), kLoaders);
+    *stop.here = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 12) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp >= 8 && warp < 12) {
+    // ---- loader ----
+    const int t = threadIdx.x - 256;
+    const __nv_bfloat16* kbase = static_cast<const __nv_bfloat16*>(kv.k) + g * dim;
+    const __nv_bfloat16* vbase = static_cast<const __nv_bfloat16*>(kv.v) + gv * vdim;
+    const int32_t* table = kv.table ? kv.table + static_cast<size_t>(ent_seq[e]) * kv.table_stride : nullptr;
+    auto lookup = [&](int i) {  // the pool row of this thread's key of tile i, -1: none
+      const int kj = i < n ? tile_of(i) * kTile + t : pmax + 1;
+      if (kj > pmax) return -1;
+      // no page table: the keys and values are the step's own rows, row of position p = first + p - pos0
+      return table ? table[kj / kv.page] * kv.page + kj % kv.page : first + max(kj - pos0, 0);
+    };
+    // A tile by 16-byte copies, C chunks to a row: this thread has chunk t % C of rows t / C, t / C + 128 / C, ...  Those rows agree in
+    // their last three bits, so the swizzled place of the chunk inside the row is the same in all of them.  Chunks past the head and
+    // keys past the last are zero.  The barrier counts a thread when its copies have landed: the loader itself never waits for them.
+    auto load = [&](auto chunks, int i, uint8_t* tiles, const __nv_bfloat16* src, int row_elems, int used, uint64_t* full, bool go) {
+      constexpr int C = decltype(chunks)::value, STEP = kLoaders / C;
+      static_assert(STEP % 8 == 0, "rows of a thread agree in their last three bits");
+      if (i < n && go) {
+        const int c = t % C, row = t / C;
+        const bool wanted = c * 8 < used;
+        const int32_t* at = slots + (i & 3) * kTile + row;
+        const uint32_t dst = smem_u32(tiles) + (i & 1) * 2 * kHalfTile + (c >> 3) * kHalfTile + row * 128 + (((c & 7) ^ (row & 7)) << 4);
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+          const int slot = at[j * STEP];
+          const bool in = wanted && slot >= 0;
+          cp_async16(dst + j * STEP * 128, in ? src + static_cast<size_t>(slot) * row_elems + c * 8 : src, in);
+        }
+        arrive_copied(&full[i & 1]);
+      }
+    };
+    auto load_keys = [&](int i, bool go) { load(std::integral_constant<int, KC>{}, i, Ks, kbase, kv.k_row, dim, k_full, go); };
+    auto load_values = [&](int i, bool go) { load(std::integral_constant<int, VC>{}, i, Vs, vbase, kv.v_row, vdim, v_full, go); };
+    auto sync_loaders = [] { asm volatile("bar.sync 1, %0;" ::"n"(kLoaders) : "memory"); };
+    bool ok = true;
+    {
+      const int c = t % KC;
+      for (int row = t / KC; row < kRows; row += kLoaders / KC) {
+        const int r = r0 + row;
+        const bool in = r < n_rows && c * 8 < dim;
+        const size_t th = in ? static_cast<size_t>(first + r / rep) * a.heads + g * rep + r % rep : 0;
+        cp_async16(smem_u32(Qs) + ((row / kTile) * 2 + (c >> 3)) * kHalfTile + (row % kTile) * 128 + (((c & 7) ^ (row & 7)) << 4), in ? q + th * dim + c * 8 : q, in);
+      }
+    }
+    arrive_copied(q_full);
+    for (int i = 0; i < 3; ++i) slots[i * kTile + t] = lookup(i);
+    sync_loaders();
+    load_keys(0, true), load_values(0, true), load_keys(1, true);
+    for (int i = 0; i < n; ++i) {
+      const int ahead = lookup(i + 3);
+      // tile i + 2's keys take the place of tile i's, tile i + 1's values that of tile i - 1's
+      if (i + 2 < n) ok = mbar_wait(smem_u32(&k_empty[i & 1]), (((i + 2) >> 1) & 1) ^ 1u, stop) && ok;
+      load_keys(i + 2, ok);
+      if (i + 1 < n) ok = mbar_wait(smem_u32(&v_empty[(i + 1) & 1]), (((i + 1) >> 1) & 1) ^ 1u, stop) && ok;
+      load_values(i + 1, ok);
+      slots[((i + 3) & 3) * kTile + t] = ahead;  // in the place of tile i - 1's, which every loader is done with
+      sync_loaders();
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (warp == 12) {
+    // ---- tensor core ----
+    if (lane == 0 && n > 0) {
+      const uint32_t idesc_s = instr_desc(kTile), idesc_o = instr_desc((vdim + 15) / 16 * 16) | (1u << 16);
+      const int ksteps = (dim + 15) / 16;
+      auto scores = [&](int i, int grp) {  // over the weights of tile i - 1, which the product issued before reads
+        const uint32_t qa = smem_u32(Qs) + grp * 2 * kHalfTile, ka = smem_u32(Ks) + (i & 1) * 2 * kHalfTile;
+        for (int k = 0; k < ksteps; ++k) {
+          const uint32_t off = (k >> 2) * kHalfTile + (k & 3) * 32;  // 16 coordinates, inside the swizzle row
+          umma::mma_bf16(tmem + kColS + grp * kTile, smem_desc(qa + off), smem_desc(ka + off), idesc_s, k > 0);
+        }
+        if (grp == groups - 1) mma_commit(smem_u32(&k_empty[i & 1]));
+        mma_commit(smem_u32(&s_full[grp]));
+      };
+      bool ok = mbar_wait(smem_u32(q_full), 0, stop) && mbar_wait(smem_u32(&k_full[0]), 0, stop);
+      if (ok) {
+        after_wait();
+        for (int grp = 0; grp < groups; ++grp) scores(0, grp);
+      }
+      for (int i = 0; i < n && ok; ++i) {
+        ok = mbar_wait(smem_u32(&v_full[i & 1]), (i >> 1) & 1, stop) &&
+             (i + 1 >= n || mbar_wait(smem_u32(&k_full[(i + 1) & 1]), ((i + 1) >> 1) & 1, stop));
+        const uint32_t va = smem_u32(Vs) + (i & 1) * 2 * kHalfTile;
+        for (int grp = 0; grp < groups && ok; ++grp) {
+          ok = mbar_wait(smem_u32(&p_full[grp]), i & 1, stop);
+          if (!ok) break;
+          after_wait();
+          const uint32_t weights = tmem + kColS + grp * kTile;
+#pragma unroll
+          for (int term = 0; term < 2; ++term)
+            for (int k = 0; k < kTile / 16; ++k)  // 16 keys: 8 columns of weights, 16 rows of values
+              mma_weights(tmem + kColO + grp * kTile, weights + (k >> 1) * 32 + term * 16 + (k & 1) * 8, value_desc(va + k * 2048), idesc_o,
+                          (i > 0 || term > 0 || k > 0) ? 1u : 0u);
+          if (grp == groups - 1) mma_commit(smem_u32(&v_empty[i & 1]));
+          if (i + 1 < n) scores(i + 1, grp);
+          else mma_commit(smem_u32(&o_done[grp]));
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp < 4 * groups) {
+    // ---- softmax: one row per thread ----
+    const int grp = warp >> 2, r = r0 + warp * 32 + lane;
+    const bool exists = r < n_rows;
+    const int pos = exists ? pos0 + r / rep : -1;             // -1: sees nothing
+    const int lo = exists ? first_seen(a, pos) : 0x7fffffff;  // the first key it sees
+    const uint32_t lanes = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const uint32_t scores = lanes + kColS + grp * kTile, output = lanes + kColO + grp * kTile;
+    const float scale2 = (a.softcap > 0.f ? 1.0f : a.scale) * 1.4426950408889634f, cap_in = a.softcap > 0.f ? a.scale / a.softcap : 0.f;
+    // the largest product is the largest score only when they are scaled by a positive number
+    const bool rewrite = a.softcap > 0.f || scale2 <= 0.f;
+    const float factor = scale2 > 0.f ? scale2 : 1.0f;
+    float m = -INFINITY, l = 0.f;
+    bool ok = true;
+    for (int i = 0; i < n; ++i) {
+      const int k0 = tile_of(i) * kTile;
+      // the tile's scores; the tile before has been added to the output
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&s_full[grp]), i & 1, stop));
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const bool edge = !__all_sync(0xffffffffu, k0 + kTile - 1 <= pos && k0 >= lo);  // else every row of the warp sees the whole tile
+      auto mask = [&](uint32_t(&v)[32], int c) {
+        if (edge) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const int kj = k0 + c * 32 + j;
+            if (!(kj <= pos && (kj >= lo || kj < a.keep_first))) v[j] = __float_as_uint(-INFINITY);
+          }
+        }
+      };
+      uint32_t s0[32], s1[32];
+      if (rewrite) {
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          tmem_ld32(scores + c * 32, s0);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const float x = __uint_as_float(s0[j]), y = a.softcap > 0.f ? a.softcap * tanhf(x * cap_in) : x;
+            s0[j] = __float_as_uint(scale2 > 0.f ? y : y * scale2);
+          }
+          tmem_st32(scores + c * 32, s0);
+        }
+        tmem_wait_st();
+      }
+      float part4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < 4; c += 2) {  // the last two chunks stay in registers
+        tmem_ld32(scores + c * 32, s0);
+        tmem_ld32(scores + c * 32 + 32, s1);
+        tmem_wait_ld();
+        mask(s0, c), mask(s1, c + 1);
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          part4[0] = fmaxf(part4[0], __uint_as_float(s0[j])), part4[1] = fmaxf(part4[1], __uint_as_float(s0[j + 1]));
+          part4[2] = fmaxf(part4[2], __uint_as_float(s1[j])), part4[3] = fmaxf(part4[3], __uint_as_float(s1[j + 1]));
+        }
+      }
+      const float top = fmaxf(m, fmaxf(fmaxf(part4[0], part4[1]), fmaxf(part4[2], part4[3])) * factor);
+      const bool grows = __any_sync(0xffffffffu, top > m + 8.0f);  // (m = -inf: the row's first key)
+      if (grows) {
+        const float keep = ex2(m - (top > -INFINITY ? top : 0.f));
+        m = top;
+        l *= keep;
+        if (i > 0) {
+#pragma unroll 1
+          for (int c = 0; c < vdim; c += 16) {
+            uint32_t o[16];
+            tmem_ld16(output + c, o);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * keep);
+            tmem_st16(output + c, o);
+          }
+        }
+      }
+      // a row that has seen nothing yet keeps m = -inf; subtracting 0 instead keeps 2^(-inf - 0) = 0 free of NaN
+      const float sub = m > -INFINITY ? m : 0.f;
+      float sum0 = 0.f, sum1 = 0.f;
+      auto weigh = [&](const uint32_t(&v)[32], int c) {  // 32 columns of scores become 16 of high and 16 of low terms
+        uint32_t hi[16], low[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float p0 = ex2(fmaf(__uint_as_float(v[2 * j]), factor, -sub)), p1 = ex2(fmaf(__uint_as_float(v[2 * j + 1]), factor, -sub));
+          sum0 += p0, sum1 += p1;
+          split_pack(p0, p1, hi[j], low[j]);
+        }
+        tmem_st16(scores + c * 32, hi);
+        tmem_st16(scores + c * 32 + 16, low);
+      };
+      weigh(s0, 2);
+      tmem_ld32(scores, s0);
+      weigh(s1, 3);
+      tmem_ld32(scores + 32, s1);
+      tmem_wait_ld();
+      mask(s0, 0), mask(s1, 1);
+      weigh(s0, 0);
+      weigh(s1, 1);
+      l += sum0 + sum1;
+      tmem_wait_st();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) arrive(&p_full[grp]);
+    }
+    if (n > 0) {
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&o_done[grp]), 0, stop));
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    const size_t th = exists ? static_cast<size_t>(first + r / rep) * a.heads + g * rep + r % rep : 0;
+    const bool whole = splits == 1 && !a.no_merge, per_element = gates != nullptr && a.gate == KLLM_SEQ_GATE_ELEMENT;
+    if (whole && a.sink != nullptr && exists) {  // exp(sink) joins the denominator; scores are in units of log2
+      l = m > -INFINITY ? l + ex2(a.sink[th % a.heads] * 1.4426950408889634f - m) : 1.0f;
+    }
+    const float inv = 1.0f / l;
+    const float gate = whole && exists && gates && !per_element ? gates[th] : 1.0f;
+    float* part = ws + (th * splits + split) * (vdim + 2);
+    if (!whole && exists && ok) part[0] = m * 0.6931471805599453f, part[1] = l;  // the merge works with natural logarithms
+#pragma unroll 1
+    for (int c = 0; c < vdim; c += 16) {
+      uint32_t o[16];
+      if (n > 0) {
+        tmem_ld16(output + c, o);
+        tmem_wait_ld();
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = 0u;
+      }
+      if (!exists || !ok) continue;
+      const int here = min(16, vdim - c);  // 16 or 8
+      if (whole) {
+        uint32_t y[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float v0 = __uint_as_float(o[2 * j]) * inv * gate, v1 = __uint_as_float(o[2 * j + 1]) * inv * gate;
+          if (per_element && 2 * j < here) v0 *= gates[th * vdim + c + 2 * j], v1 *= gates[th * vdim + c + 2 * j + 1];
+          const __nv_bfloat162 two = __floats2bfloat162_rn(v0, v1);
+          y[j] = *reinterpret_cast<const uint32_t*>(&two);
+        }
+        uint4* dst = reinterpret_cast<uint4*>(out + th * vdim + c);
+        dst[0] = make_uint4(y[0], y[1], y[2], y[3]);
+        if (here > 8) dst[1] = make_uint4(y[4], y[5], y[6], y[7]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (j < here) part[2 + c + j] = __uint_as_float(o[j]);
+      }
+    }
+  }
+  if (*stop.here) {
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 12) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+}
+
+constexpr size_t kAttnUmmaSmem = 1024 + 12 * kHalfTile + 16 * 8 + 4 * kTile * 4 + 64;
+static_assert(kAttnUmmaSmem <= 232448, "shared memory of one CTA");
+
+}  // namespace
+
+// bf16 heads of whole 16-byte chunks up to 128 coordinates, entries long enough that most tiles are not on the diagonal.  Steps as above,
+// mma.sync -> here: 16 / 4 x 128, 3 entries of up to 667 171 -> 165 us, one of 640 132 -> 130, 1600 221 -> 186, 3000 451 -> 316; one of 384
+// with 8 / 1 x 128 104 -> 110.  Where each key head has one query head a group spans 128 tokens, and the line lies later: 16 / 16 x 64,
+// 8 entries of up to 533 240 -> 262, 3 of up to 667 165 -> 164, one of 1000 147 -> 146, 1600 187 -> 182, 3000 339 -> 285.
+bool attention_umma_usable(int dtype, const AttnShape& a, int max_count) {
+  if (dtype != KLLM_SEQ_BF16 || a.kv_heads <= 0 || a.heads % a.kv_heads || a.q_f32 || a.out_f32) return false;
+  return a.dim % 8 == 0 && a.dim <= 128 && a.vdim % 8 == 0 && a.vdim <= 128 && max_count >= (a.heads > a.kv_heads ? 640 : 1280);
+}
+
+template <int KC, int VC>
+static int launch_umma(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries, const int32_t* ent_first,
+                       const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0, int max_count, int splits, float* ws,
+                       void* out, int* report, cudaStream_t s) {
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(attention_umma_kernel<KC, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(kAttnUmmaSmem));
+    if (e != cudaSuccess) return cuda_rc(e);
+    configured = true;
+  }
+  const int rep = a.heads / a.kv_heads;
+  const dim3 grid(n_entries * a.kv_heads, (max_count * rep + kRows - 1) / kRows, splits);
+  if (grid.y > 65535u) return KLLM_E_UNSUPPORTED;
+  attention_umma_kernel<KC, VC><<<grid, kAttnUmmaThreads, kAttnUmmaSmem, s>>>(
+      a, static_cast<const __nv_bfloat16*>(q), kv, ent_first, ent_count, ent_seq, ent_pos0, splits, ws, a.gate ? gates : nullptr,
+      static_cast<__nv_bfloat16*>(out), report);
+  count_launch();
+  return cuda_rc(cudaGetLastError());
+}
+int launch_attention_umma(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
+                          const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0,
+                          int max_count, int splits, float* ws, void* out, cudaStream_t s) {
+  int* const report = wait_flag();
+  if (report == nullptr) return KLLM_E_STATE;
+#define KLLM_ATTN_UMMA(K, V) \
+  return launch_umma<K, V>(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, report, s)
+  if (a.dim <= 64 && a.vdim <= 64) KLLM_ATTN_UMMA(8, 8);
+  if (a.dim <= 64) KLLM_ATTN_UMMA(8, 16);
+  if (a.vdim <= 64) KLLM_ATTN_UMMA(16, 8);
+  KLLM_ATTN_UMMA(16, 16);
+#undef KLLM_ATTN_UMMA
+}
+
+}  // namespace seq
+}  // namespace kllm
