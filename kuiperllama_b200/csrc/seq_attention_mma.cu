@@ -351,9 +351,9 @@ __host__ __device__ inline FewLayout few_layout(const AttnShape& a, bool same, b
 
 template <int NBW, bool SAME, bool QF32>
 __global__ void __launch_bounds__(kFewThreads)
-attention_rows_mma_kernel(AttnShape a, const void* __restrict__ q_, PagedKV kv, const int32_t* __restrict__ ent_first,
-                          const int32_t* __restrict__ ent_count, const int32_t* __restrict__ ent_seq,
-                          const int32_t* __restrict__ ent_pos0, int splits, float* __restrict__ ws) {
+attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t* ent_first,
+                          const int32_t* ent_count, const int32_t* ent_seq,
+                          const int32_t* ent_pos0, int splits, float* ws) {
   next_may_start();
   after_previous();
   const int e = blockIdx.y / a.kv_heads, g = blockIdx.y % a.kv_heads, split = blockIdx.z;

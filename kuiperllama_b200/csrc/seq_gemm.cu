@@ -34,11 +34,12 @@ __device__ __forceinline__ float ld_f(const __nv_bfloat16* p) { return __bfloat1
 __device__ __forceinline__ void st_t(float* p, float v) { *p = v; }
 __device__ __forceinline__ void st_t(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
+// load: rows that an earlier kernel wrote (coherent); load_stream: weights, which no kernel writes
 template <typename AT> struct Vec16;
 template <> struct Vec16<float> {
   static constexpr int N = 4;
   __device__ static __forceinline__ void load(const float* p, float* f) {
-    const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+    const float4 v = *reinterpret_cast<const float4*>(p);
     f[0] = v.x, f[1] = v.y, f[2] = v.z, f[3] = v.w;
   }
   __device__ static __forceinline__ void load_stream(const float* p, float* f) {
@@ -59,7 +60,7 @@ template <> struct Vec16<__nv_bfloat16> {
     }
   }
   __device__ static __forceinline__ void load(const __nv_bfloat16* p, float* f) {
-    widen(__ldg(reinterpret_cast<const uint4*>(p)), f);
+    widen(*reinterpret_cast<const uint4*>(p), f);
   }
   __device__ static __forceinline__ void load_stream(const __nv_bfloat16* p, float* f) {
     uint4 v;
@@ -72,7 +73,7 @@ template <> struct Vec16<__nv_bfloat16> {
 // ---- a few rows against every weight row ----------------------------------------------------------------------------
 template <typename AT, int R, bool VEC>
 __global__ void __launch_bounds__(256)
-rows_kernel(const AT* __restrict__ a, const AT* __restrict__ w, const float* __restrict__ bias, float* __restrict__ out, int T,
+rows_kernel(const AT* a, const AT* __restrict__ w, const float* __restrict__ bias, float* out, int T,
             int K, int N) {
   constexpr int V = Vec16<AT>::N;
   next_may_start();
@@ -127,7 +128,7 @@ rows_kernel(const AT* __restrict__ a, const AT* __restrict__ w, const float* __r
 // The gated form: a warp owns feature f and streams its gate row and its up row together.
 template <typename AT, int R, bool VEC>
 __global__ void __launch_bounds__(256)
-rows_gated_kernel(const AT* __restrict__ a, const AT* __restrict__ w, const float* __restrict__ bias, AT* __restrict__ out, int T,
+rows_gated_kernel(const AT* a, const AT* __restrict__ w, const float* __restrict__ bias, AT* out, int T,
                   int K, int N, GatedAct act) {
   constexpr int V = Vec16<AT>::N;
   next_may_start();

@@ -645,10 +645,10 @@ __device__ __forceinline__ AT* page_row(AT* base, const PagedKV& kv, int seq, in
 // it), temperature -- and leaves as a query row or as the key row of the token's page.  Angles, cos and sin are fp32.
 // One norm over all query rows (and one over all key rows) takes its two sums of squares over the CTA first.
 template <typename AT>
-__global__ void qk_prepare_kernel(AttnShape a, RopeArgs rope, const float* __restrict__ qkvg, int stride,
+__global__ void qk_prepare_kernel(AttnShape a, RopeArgs rope, const float* qkvg, int stride,
                                   const float* __restrict__ qnorm_w, const float* __restrict__ knorm_w, float eps,
-                                  const int32_t* __restrict__ tok_seq, const int32_t* __restrict__ tok_pos,
-                                  AT* __restrict__ q, float* __restrict__ gates, PagedKV kv, ValueBlend blend) {
+                                  const int32_t* tok_seq, const int32_t* tok_pos,
+                                  AT* q, float* gates, PagedKV kv, ValueBlend blend) {
   next_may_start();
   after_previous();
   extern __shared__ float head_rows[];  // [warps][dim]
@@ -731,9 +731,9 @@ __global__ void qk_prepare_kernel(AttnShape a, RopeArgs rope, const float* __res
 // token's position are taken once, into shared memory; all heads read them from there.
 template <typename AT, int G>
 __global__ void __launch_bounds__(512)
-qk_turn_kernel(AttnShape a, RopeArgs rope, const float* __restrict__ qkvg, int stride, const float* __restrict__ qnorm_w,
-               const float* __restrict__ knorm_w, float eps, const int32_t* __restrict__ tok_seq,
-               const int32_t* __restrict__ tok_pos, AT* __restrict__ q, float* __restrict__ gates, PagedKV kv) {
+qk_turn_kernel(AttnShape a, RopeArgs rope, const float* qkvg, int stride, const float* __restrict__ qnorm_w,
+               const float* __restrict__ knorm_w, float eps, const int32_t* tok_seq,
+               const int32_t* tok_pos, AT* q, float* gates, PagedKV kv) {
   next_may_start();
   after_previous();
   extern __shared__ __align__(16) float turn[];  // [half] cos, [half] sin
@@ -846,9 +846,9 @@ template <> __device__ __forceinline__ void get_cols<4>(const float* src, float*
 template <> __device__ __forceinline__ void get_cols<1>(const float* src, float* v) { v[0] = *src; }
 
 template <typename AT, int V>
-__global__ void qk_rows_kernel(AttnShape a, const float* __restrict__ qkvg, int stride, const float* __restrict__ qnorm_w,
-                               const float* __restrict__ knorm_w, float eps, const int32_t* __restrict__ tok_seq,
-                               const int32_t* __restrict__ tok_pos, AT* __restrict__ q, float* __restrict__ gates, PagedKV kv,
+__global__ void qk_rows_kernel(AttnShape a, const float* qkvg, int stride, const float* __restrict__ qnorm_w,
+                               const float* __restrict__ knorm_w, float eps, const int32_t* tok_seq,
+                               const int32_t* tok_pos, AT* q, float* gates, PagedKV kv,
                                ValueBlend blend) {
   next_may_start();
   after_previous();
@@ -926,9 +926,9 @@ __global__ void qk_rows_kernel(AttnShape a, const float* __restrict__ qkvg, int 
 // the unrolled row loops do not issue twelve predicated-off iterations per step.
 template <typename AT, int C, bool SPARSE, int RS>
 __global__ void __launch_bounds__(kAttnThreads)
-attention_kernel(AttnShape a, const void* __restrict__ q_, PagedKV kv, const int32_t* __restrict__ ent_first,
-                 const int32_t* __restrict__ ent_count, const int32_t* __restrict__ ent_seq,
-                 const int32_t* __restrict__ ent_pos0, int splits, float* __restrict__ ws) {
+attention_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t* ent_first,
+                 const int32_t* ent_count, const int32_t* ent_seq,
+                 const int32_t* ent_pos0, int splits, float* ws) {
   next_may_start();
   after_previous();
   const int e = blockIdx.y / a.kv_heads, g = blockIdx.y % a.kv_heads, split = blockIdx.z;
@@ -1222,9 +1222,9 @@ attention_wide_kernel(AttnShape a, const void* __restrict__ q_, PagedKV kv, cons
 
 // One CTA per (token, head): the splits' weights (warp 0), the weighted sum of their outputs, the output gate, the conversion.
 template <typename AT>
-__global__ void attention_merge_kernel(int heads, int vdim, int splits, const float* __restrict__ ws,
-                                       const float* __restrict__ gates, int gate_kind, const float* __restrict__ sink,
-                                       int out_f32, void* __restrict__ out_) {
+__global__ void attention_merge_kernel(int heads, int vdim, int splits, const float* ws,
+                                       const float* gates, int gate_kind, const float* __restrict__ sink,
+                                       int out_f32, void* out_) {
   next_may_start();
   after_previous();
   extern __shared__ float weight[];  // [splits]
@@ -1353,8 +1353,8 @@ __host__ __device__ inline int pair_rows(int pairs) { return pairs <= 32 ? 4 : 1
 // With a shared expert riding along (sh.ff > 0) the grid has T more "pairs": pair T * top + t is token t's pass
 // through the shared expert, whose inner activations go to sh.inter [T, sh.ff].
 template <typename AT>
-__global__ void expert_gate_up_kernel(const AT* __restrict__ h, const AT* __restrict__ gate_up,
-                                      const int32_t* __restrict__ top_idx, AT* __restrict__ inter, int T, int top, int ff,
+__global__ void expert_gate_up_kernel(const AT* h, const AT* __restrict__ gate_up,
+                                      const int32_t* top_idx, AT* inter, int T, int top, int ff,
                                       int width, SharedExpert sh, GatedAct ga) {
   next_may_start();
   after_previous();
@@ -1391,9 +1391,9 @@ __global__ void expert_gate_up_kernel(const AT* __restrict__ h, const AT* __rest
 }
 
 template <typename AT>
-__global__ void expert_down_kernel(const AT* __restrict__ inter, const AT* __restrict__ down,
-                                   const int32_t* __restrict__ top_idx, const float* __restrict__ top_w,
-                                   float* __restrict__ y, int top, int ff, int width, SharedExpert sh) {
+__global__ void expert_down_kernel(const AT* inter, const AT* __restrict__ down,
+                                   const int32_t* top_idx, const float* top_w,
+                                   float* y, int top, int ff, int width, SharedExpert sh) {
   next_may_start();
   after_previous();
   extern __shared__ float xs[];  // [top][ff], then [sh.ff]

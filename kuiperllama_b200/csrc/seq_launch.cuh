@@ -7,6 +7,12 @@
 // following kernel's CTAs take up what room is left; a kernel that allocates TMEM calls it after the allocation, so that a CTA which
 // waits for this kernel never holds columns that this kernel still needs.
 //
+// Such a kernel is alive while earlier ones still write.  Loads through the read-only path (__ldg, ld.global.nc, a
+// `const __restrict__` parameter) are allowed only for data that nothing writes during the kernel's whole life, and the compiler may
+// move them, and accesses through any `__restrict__` parameter, across after_previous().  So in these kernels weights alone are
+// `__restrict__` or read that way; whatever a kernel of the step reads or writes besides goes through plain pointers
+// (tests/test_launch_rules.py).
+//
 // Only inside a step: its weights are not written by any kernel on the stream.  A product that a caller enqueues by itself begins
 // after everything the caller enqueued before, which may have written its weights.
 #pragma once

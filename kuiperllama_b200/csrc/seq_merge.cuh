@@ -9,7 +9,7 @@ namespace {
 
 // Run by one whole warp: weight[s] = exp(m_s - M) / L, so that the joined output is sum_s weight[s] * o_s.  A sink adds
 // exp(sink) to L (no key, no value).  Splits that saw no key get weight 0.
-__device__ __forceinline__ void split_weights(const float* __restrict__ p, int splits, int pstride, bool has_sink, float sink,
+__device__ __forceinline__ void split_weights(const float* p, int splits, int pstride, bool has_sink, float sink,
                                               float* weight) {
   const int lane = threadIdx.x & 31;
   float M = has_sink ? sink : -INFINITY;
@@ -33,11 +33,11 @@ __device__ __forceinline__ void split_weights(const float* __restrict__ p, int s
 constexpr int kMergeAhead = 16;
 struct MergeColumn {
   float v[kMergeAhead];
-  __device__ __forceinline__ void load(const float* __restrict__ p, int splits, int pstride, int d) {
+  __device__ __forceinline__ void load(const float* p, int splits, int pstride, int d) {
 #pragma unroll
     for (int s = 0; s < kMergeAhead; ++s) v[s] = s < splits ? p[s * pstride + 2 + d] : 0.f;
   }
-  __device__ __forceinline__ float join(const float* __restrict__ p, int splits, int pstride, int d, const float* weight) const {
+  __device__ __forceinline__ float join(const float* p, int splits, int pstride, int d, const float* weight) const {
     float o = 0.f;
 #pragma unroll
     for (int s = 0; s < kMergeAhead; ++s)

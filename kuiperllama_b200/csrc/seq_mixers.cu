@@ -51,7 +51,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 __device__ __forceinline__ float sigmoidf(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float siluf(float z) { return z / (1.0f + expf(-z)); }
 
-// V consecutive values of the compute type (16 bytes, or one value), widened to fp32
+// V consecutive weights of the compute type (16 bytes, or one value), widened to fp32
 template <typename AT> struct Wide;
 template <> struct Wide<float> {
   static constexpr int N = 4;
@@ -125,10 +125,10 @@ __device__ __forceinline__ float rotated(const LatentShape& a, const float* v, i
 
 // ---- latent attention: down-projections -> normed query latent, cache row, gates -----------------------------------------
 template <typename AT>
-__global__ void latent_prepare_kernel(LatentShape a, const float* __restrict__ proj, const float* __restrict__ q_norm_w,
-                                      const float* __restrict__ kv_norm_w, float eps, const int32_t* __restrict__ tok_seq,
-                                      const int32_t* __restrict__ tok_pos, AT* __restrict__ cq, float* __restrict__ gates,
-                                      PagedKV kv, AT* __restrict__ c_rows, float* __restrict__ kr_rows) {
+__global__ void latent_prepare_kernel(LatentShape a, const float* proj, const float* __restrict__ q_norm_w,
+                                      const float* __restrict__ kv_norm_w, float eps, const int32_t* tok_seq,
+                                      const int32_t* tok_pos, AT* cq, float* gates,
+                                      PagedKV kv, AT* c_rows, float* kr_rows) {
   next_may_start();
   after_previous();
   __shared__ float red[33];
@@ -208,8 +208,8 @@ __global__ void latent_absorb_kernel(LatentShape a, const float* __restrict__ q,
 constexpr int kFewCols = 64, kFewWarps = 8, kFewAhead = 4;
 template <typename AT, int NT>
 __global__ void __launch_bounds__(kFewWarps * 32)
-latent_absorb_few_kernel(LatentShape a, const float* __restrict__ q, int q_row, const AT* __restrict__ w_uk,
-                         const int32_t* __restrict__ tok_pos, float* __restrict__ qa, int T) {
+latent_absorb_few_kernel(LatentShape a, const float* q, int q_row, const AT* __restrict__ w_uk,
+                         const int32_t* tok_pos, float* qa, int T) {
   next_may_start();
   after_previous();
   constexpr int V = Wide<AT>::N, LPR = kFewCols / V, RPW = 32 / LPR;  // values per lane, lanes per row, rows per warp
@@ -377,8 +377,8 @@ __global__ void latent_expand_kernel(LatentShape a, const float* __restrict__ ol
 constexpr int kExpandWarps = 8, kExpandRowsPerWarp = 4, kExpandRows = kExpandWarps * kExpandRowsPerWarp;
 template <typename AT, bool VEC>
 __global__ void __launch_bounds__(kExpandWarps * 32)
-latent_merge_expand_kernel(LatentShape a, int splits, const float* __restrict__ ws, const float* __restrict__ gates,
-                           const float* __restrict__ sink, const AT* __restrict__ w_uv, AT* __restrict__ out) {
+latent_merge_expand_kernel(LatentShape a, int splits, const float* ws, const float* gates,
+                           const float* __restrict__ sink, const AT* __restrict__ w_uv, AT* out) {
   next_may_start();
   after_previous();
   extern __shared__ __align__(16) float ls[];  // [kv_rank], then [splits] weights
@@ -784,8 +784,8 @@ constexpr int kLinTokenLoads = 8;
 template <typename AT, int V>
 __global__ void __launch_bounds__(512)
 linear_token_kernel(int heads, int dim, int vdim, const float* __restrict__ decay, LinearRot rot, int silu,
-                    const float* __restrict__ proj, int stride, int gate_act, float eps, float* __restrict__ state,
-                    const int32_t* __restrict__ tok_seq, const int32_t* __restrict__ tok_pos, AT* __restrict__ out) {
+                    const float* proj, int stride, int gate_act, float eps, float* state,
+                    const int32_t* tok_seq, const int32_t* tok_pos, AT* out) {
   next_may_start();
   after_previous();
   extern __shared__ __align__(16) float sm[];

@@ -1,0 +1,58 @@
+"""Kernels that begin before the ones ahead of them have ended (csrc/seq_launch.cuh): what an earlier kernel writes must not be read
+through the read-only path or through `__restrict__` parameters, which the compiler may move across the wait.  Read from the sources,
+since a wrong value would depend on timing."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "kuiperllama_b200" / "csrc"
+WEIGHTS = {"w", "bias", "qnorm_w", "knorm_w", "q_norm_w", "kv_norm_w", "sink", "w_uk", "w_uv", "decay", "gate_up", "down"}
+WEIGHT_POINTERS = WEIGHTS | {"wr", "wg", "wu", "a.in_w", "a.out_w", "a.mix", "a.rope_freq"}
+
+
+def body(text, start):
+    depth, i = 1, start
+    while depth:
+        depth += (text[i] == "{") - (text[i] == "}")
+        i += 1
+    return text[start:i]
+
+
+def early_kernels():
+    out = []
+    for path in sorted(CSRC.glob("seq_*.cu*")):
+        text = path.read_text()
+        for m in re.finditer(r"__global__[^{;]*?\b(\w+_kernel)\(([^{]*)\)\s*\{", text):
+            code = body(text, m.end())
+            if "after_previous()" in code:
+                out.append((m.group(1), m.group(2), code))
+    return out
+
+
+KERNELS = early_kernels()
+
+
+def test_kernels_were_found():
+    assert len(KERNELS) >= 18
+    assert {"rows_kernel", "qk_turn_kernel", "attention_kernel", "umma_split_kernel", "streams_kernel"} <= {k[0] for k in KERNELS}
+
+
+@pytest.mark.parametrize("name,parameters,code", KERNELS, ids=[k[0] for k in KERNELS])
+def test_only_weights_take_the_read_only_path(name, parameters, code):
+    assert set(re.findall(r"__restrict__ (\w+)", parameters)) <= WEIGHTS
+    assert "__restrict__" not in code
+    read_only = r"(?:__ldg|Vec16<AT>::load_stream|Wide<AT>::template load<\w+>)\((?:reinterpret_cast<[^>]*>\()?([\w.]+)"
+    assert set(re.findall(read_only, code)) <= WEIGHT_POINTERS
+    assert "ld.global.nc" not in code
+
+
+def test_rows_are_loaded_coherently():
+    """Vec16::load, by which the products of few rows read their rows."""
+    text = (CSRC / "seq_gemm.cu").read_text()
+    loads = [body(text, m.end()) for m in re.finditer(r" load\(const \w+\* p, float\* f\) \{", text)]
+    assert len(loads) == 2 and not any("__ldg" in x or ".nc" in x for x in loads)
+
+
+def test_joining_splits_reads_plain_pointers():
+    assert "__restrict__" not in (CSRC / "seq_merge.cuh").read_text()
