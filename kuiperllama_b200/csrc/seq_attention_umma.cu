@@ -49,6 +49,7 @@ __device__ __forceinline__ float ex2(float x) {  // 2^x, relative error about 2^
   return y;
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
@@ -185,7 +186,7 @@ attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV 
     };
     auto load_keys = [&](int i, bool go) { load(std::integral_constant<int, KC>{}, i, Ks, kbase, kv.k_row, dim, k_full, go); };
     auto load_values = [&](int i, bool go) { load(std::integral_constant<int, VC>{}, i, Vs, vbase, kv.v_row, vdim, v_full, go); };
-    auto sync_loaders = [] { asm volatile("bar.sync 1, %0;" ::"n"(kLoaders) : "memory"); };
+    auto sync_loaders = [] { named_sync<kLoaders>(1); };
     bool ok = true;
     {
       const int c = t % KC;
@@ -268,7 +269,7 @@ attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV 
     for (int i = 0; i < n; ++i) {
       const int k0 = tile_of(i) * kTile;
       // the tile's scores; the tile before has been added to the output
-      ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&s_full[grp]), i & 1, stop));
+      ok = warp_wait(ok, smem_u32(&s_full[grp]), i & 1, stop);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const bool edge = !__all_sync(0xffffffffu, k0 + kTile - 1 <= pos && k0 >= lo);  // else every row of the warp sees the whole tile
       auto mask = [&](uint32_t(&v)[32], int c) {
@@ -355,7 +356,7 @@ attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV 
       if (lane == 0) arrive(&p_full[grp]);
     }
     if (n > 0) {
-      ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&o_done[grp]), 0, stop));
+      ok = warp_wait(ok, smem_u32(&o_done[grp]), 0, stop);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     const size_t th = exists ? static_cast<size_t>(first + r / rep) * a.heads + g * rep + r % rep : 0;
@@ -377,30 +378,32 @@ attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV 
 #pragma unroll
         for (int j = 0; j < 16; ++j) o[j] = 0u;
       }
-      if (!exists || !ok) continue;
-      const int here = min(16, vdim - c);  // 16 or 8
-      if (whole) {
-        uint32_t y[8];
+      if (exists && ok) {
+        const int here = min(16, vdim - c);  // 16 or 8
+        if (whole) {
+          uint32_t y[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float v0 = __uint_as_float(o[2 * j]) * inv * gate, v1 = __uint_as_float(o[2 * j + 1]) * inv * gate;
-          if (per_element && 2 * j < here) v0 *= gates[th * vdim + c + 2 * j], v1 *= gates[th * vdim + c + 2 * j + 1];
-          const __nv_bfloat162 two = __floats2bfloat162_rn(v0, v1);
-          y[j] = *reinterpret_cast<const uint32_t*>(&two);
+          for (int j = 0; j < 8; ++j) {
+            float v0 = __uint_as_float(o[2 * j]) * inv * gate, v1 = __uint_as_float(o[2 * j + 1]) * inv * gate;
+            if (per_element && 2 * j < here) v0 *= gates[th * vdim + c + 2 * j], v1 *= gates[th * vdim + c + 2 * j + 1];
+            const __nv_bfloat162 two = __floats2bfloat162_rn(v0, v1);
+            y[j] = *reinterpret_cast<const uint32_t*>(&two);
+          }
+          uint4* dst = reinterpret_cast<uint4*>(out + th * vdim + c);
+          dst[0] = make_uint4(y[0], y[1], y[2], y[3]);
+          if (here > 8) dst[1] = make_uint4(y[4], y[5], y[6], y[7]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (j < here) part[2 + c + j] = __uint_as_float(o[j]);
         }
-        uint4* dst = reinterpret_cast<uint4*>(out + th * vdim + c);
-        dst[0] = make_uint4(y[0], y[1], y[2], y[3]);
-        if (here > 8) dst[1] = make_uint4(y[4], y[5], y[6], y[7]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (j < here) part[2 + c + j] = __uint_as_float(o[j]);
       }
     }
   }
   if (*stop.here) {
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   }
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 12) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");

@@ -235,7 +235,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     float check = 0.f;
     for (int i = 0; i < blocks; ++i) {
       const int s = i % ST;
-      if (!mbar_wait(smem_u32(&full[s]), (i / ST) & 1, stop)) break;
+      if (!warp_wait(true, smem_u32(&full[s]), (i / ST) & 1, stop)) break;
       const float4* tile = reinterpret_cast<const float4*>(base + s * STAGE);
       float4* lo = reinterpret_cast<float4*>(base + s * STAGE + HALF);
 #pragma unroll 8
@@ -260,7 +260,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     for (int j = 0; j < TILE_COLS; ++j) acc[j] = 0.f;
     for (int sec = 0; sec < sections && ok; ++sec) {
       const int b = sec & 1;
-      ok = mbar_wait(smem_u32(&acc_full[b]), (sec >> 1) & 1, stop);
+      ok = warp_wait(ok, smem_u32(&acc_full[b]), (sec >> 1) & 1, stop);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t from = tmem_d + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(b * ACC_COLS);
@@ -327,6 +327,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   if (*stop.here) {  // a wait ran out: give copies in flight time to land before the shared memory is given up
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   }
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1) {

@@ -63,6 +63,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const S
   __threadfence_system();
   return false;
 }
+// The steps that a warp takes as one (.sync.aligned: TMEM loads and stores, named barriers) need its lanes together.  Lanes part at
+// every row that does not exist and every wait that only some of them gave up, so each helper brings them together first, and a warp
+// that takes such steps after a wait goes on, or gives up, as a whole: false when any lane's wait ran out or `ok` was false before.
+__device__ __forceinline__ bool warp_wait(bool ok, uint32_t bar, uint32_t parity, const Stop& stop) {
+  return __all_sync(0xffffffffu, ok && mbar_wait(bar, parity, stop));
+}
+template <int THREADS_IN>
+__device__ __forceinline__ void named_sync(int id) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(THREADS_IN) : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -117,6 +128,7 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
 }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -129,6 +141,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -289,7 +302,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++done) {
       const int n0 = (tile % feature_tiles) * FEATURES, t0 = (tile / feature_tiles) * BN, b = done & 1;
       // a warp whose wait ran out stores nothing more, but still meets its partner at every barrier below
-      ok = ok && mbar_wait(smem_u32(&acc_full[b]), (done >> 1) & 1, stop);
+      ok = warp_wait(ok, smem_u32(&acc_full[b]), (done >> 1) & 1, stop);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t from = tmem_d + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(b * BN);
       auto release = [&]() {
@@ -340,7 +353,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
 #pragma unroll
             for (int j = 16; j < 32; ++j) x[j * 32] = __uint_as_float(r[j]);
           }
-          asm volatile("bar.sync %0, 64;" ::"r"(1 + 2 * half + pair) : "memory");
+          named_sync<64>(1 + 2 * half + pair);
           if (ok && row < N) {
             OT* out = static_cast<OT*>(p.out) + static_cast<size_t>(t0 + c) * N + row;
             if (up) {
@@ -360,6 +373,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
   if (*stop.here) {  // a wait ran out: give copies in flight time to land before the shared memory is given up
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   }
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1) {
@@ -478,7 +492,7 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       const int n0 = (tile % feature_tiles) * FEATURES, b = done & 1;
       const int4 g = list[tile / feature_tiles];
       // a warp whose wait ran out stores nothing more, but still meets its partner at every barrier below
-      ok = ok && mbar_wait(smem_u32(&acc_full[b]), (done >> 1) & 1, stop);
+      ok = warp_wait(ok, smem_u32(&acc_full[b]), (done >> 1) & 1, stop);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t from = tmem_d + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(b * kGroupRows);
       const int pair = quarter & 1, row = n0 + (GATED ? pair * 32 : quarter * 32) + lane;
@@ -522,7 +536,7 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
             for (int j = 16; j < 32; ++j) x[j * 32] = __uint_as_float(r[j]);
           }
-          asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
+          named_sync<64>(1 + pair);
           if (ok && row < N) {
             if (up) {
 #pragma unroll
@@ -536,12 +550,13 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           }
         }
       }
-      if constexpr (GATED) asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");  // the next tile starts with the first buffer again
+      if constexpr (GATED) named_sync<64>(1 + pair);  // the next tile starts with the first buffer again
     }
   }
   if (*stop.here) {
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   }
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1) {

@@ -1,0 +1,43 @@
+"""Steps that a warp takes as one (tcgen05.ld / st, named barriers) in the tcgen05 kernels: undefined when its lanes are apart.  Lanes part
+in epilogues at rows that do not exist and at waits that ran out, so every helper with such a step first brings them together, and
+waits of whole warps end for all lanes alike.  Read from the sources: what an apart warp does is not defined, so no run can show it."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "kuiperllama_b200" / "csrc"
+FILES = ["seq_gemm_umma.cuh", "seq_gemm_split.cuh", "seq_attention_umma.cu"]
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_collective_steps_follow_a_join(name):
+    lines = (CSRC / name).read_text().splitlines()
+    steps = [i for i, line in enumerate(lines) if re.search(r'"(tcgen05\.(ld|st)\.sync\.aligned|bar\.sync|barrier\.sync)', line)]
+    for i in steps:
+        assert any("__syncwarp();" in line for line in lines[max(0, i - 2):i]), f"{name}:{i + 1}"
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_the_last_barrier_follows_a_join(name):
+    """Before TMEM is given back, the roles of a warp (one lane loads or multiplies, the others wait) meet again."""
+    text = (CSRC / name).read_text()
+    for m in re.finditer(r"tcgen05\.dealloc", text):
+        tail = text[:m.start()].splitlines()[-6:]
+        assert any("__syncwarp();" in line for line in tail)
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_waits_of_whole_warps_end_alike(name):
+    """acc_full, s_full and o_done are waited for by whole warps that load TMEM next; the splitting warps vote on `full`."""
+    for line in (CSRC / name).read_text().splitlines():
+        if re.search(r"_wait\([^;]*(acc_full|s_full|o_done)", line):
+            assert "warp_wait(" in line
+    if name == "seq_gemm_split.cuh":
+        assert "if (!warp_wait(true, smem_u32(&full[s])" in (CSRC / name).read_text()
+
+
+def test_no_lane_leaves_the_output_loop_of_the_attention():
+    text = (CSRC / "seq_attention_umma.cu").read_text()
+    loop = text[text.index("for (int c = 0; c < vdim; c += 16) {", text.index("o_done[grp]), 0")):]
+    assert "continue" not in loop[:loop.index("if (*stop.here)")]
