@@ -135,7 +135,8 @@ int kllm_gemv_fused(const kllm_gemv_job* job, void* stream);
  * matmul.cpp:57-80): the weight matrix is streamed once per block of tokens instead of once per token.
  * TMA tensor-map loads (cp.async.bulk.tensor, 128-byte swizzle) feed tcgen05.mma.kind::tf32 with the
  * accumulator in TMEM.  Results agree with the fp32 GEMV to ~1e-3 relative (10-bit mantissas), NOT
- * bit for bit: the decode path never uses it.  in_dim % 4 == 0, 16-byte aligned x and w. */
+ * bit for bit: the decode path never uses it.  in_dim % 4 == 0, 16-byte aligned x and w.  Enqueues and returns; a bounded wait
+ * inside it that ran out (KLLM_E_STATE) is reported by kllm_product_status (kllm_seq.h) or by a later product on the stream. */
 int kllm_gemm_tf32(const float* x, const float* w, float* out, int n_tokens, int in_dim, int out_dim,
                    void* stream);
 

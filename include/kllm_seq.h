@@ -370,10 +370,15 @@ int kllm_seq_profile(kllm_seq_engine* eng, float* phase_ms);
 int kllm_seq_last_launches(const kllm_seq_engine* eng);
 
 /* The engine's token-block product on its own: out[T, N] (fp32) = a[T, K] . w[N, K]^T with a and w in the compute
- * type `dtype` (device pointers).  Picks the kernel the engine would pick for this shape.  Enqueues and returns; a wait that
- * ran out inside a tensor-core kernel (KLLM_E_STATE) is reported by the first call after it was noted. */
+ * type `dtype` (device pointers).  Picks the kernel the engine would pick for this shape.  Enqueues and returns. */
 int kllm_seq_gemm(int32_t dtype, const void* a, const void* w, float* out, int32_t n_tokens, int32_t in_dim,
                   int32_t out_dim, void* stream);
+
+/* Whether the products enqueued on `stream` through this library (kllm_seq_gemm, kllm_gemm_tf32) are complete: waits for the
+ * stream, then returns KLLM_E_STATE if a bounded wait inside one of them ran out since the last report (its result is not
+ * valid), else 0.  A later product on the same stream reports such a wait too, and leaves nothing to report here.  A captured
+ * product reports under the stream it was captured on.  Engines and decoders report their own waits from their own calls. */
+int kllm_product_status(void* stream);
 
 #ifdef __cplusplus
 }

@@ -27,6 +27,7 @@
 #include "kllm_device.cuh"
 #include "kllm_host.h"
 #include "megakernel.h"
+#include "wait_flag.h"
 
 namespace kllm {
 
@@ -130,6 +131,7 @@ struct kllm_decoder {
   PrefillWorkspace pf_ws{};
   int pf_rows = 0;                // rows it has, and how many were to be had (kPrefillBlock unless memory was short)
   int pf_cap = kPrefillBlock;
+  WaitFlag wait;                  // of its products
 };
 
 namespace {
@@ -526,6 +528,7 @@ int kllm_decoder_prefill_tf32(kllm_decoder* dc, const int32_t* tokens_host, int3
     dc->pf_ws.h1 = take(d.hidden_dim);
   }
   const int block = dc->pf_rows;
+  if (dc->wait.get() == nullptr) return KLLM_E_STATE;
   PrefillModel m{};
   m.dim = d.dim, m.hidden_dim = d.hidden_dim, m.layer_num = d.layer_num, m.head_num = d.head_num;
   m.kv_head_num = d.kv_head_num, m.vocab_size = d.vocab_size, m.seq_len = d.seq_len, m.head_size = hs;
@@ -544,7 +547,7 @@ int kllm_decoder_prefill_tf32(kllm_decoder* dc, const int32_t* tokens_host, int3
   int last_rows = 0;
   for (int c0 = 0; c0 < n_tokens; c0 += block) {
     const int T = std::min(block, n_tokens - c0);
-    KLLM_TRY(prefill_block(m, dc->pf_ws, dc->teacher + c0, T, start_pos + c0, dc->stream));
+    KLLM_TRY(prefill_block(m, dc->pf_ws, dc->teacher + c0, T, start_pos + c0, dc->stream, dc->wait.get()));
     last_rows = T;
   }
   // last prompt position only: final RMSNorm + classifier (cls_logits, llama3.cpp:722-731) and the
@@ -570,7 +573,7 @@ int kllm_decoder_prefill_tf32(kllm_decoder* dc, const int32_t* tokens_host, int3
   KLLM_TRY(cudaGetLastError());
   KLLM_TRY(cudaMemcpyAsync(hs_state, dc->st, sizeof(StepState), cudaMemcpyDeviceToHost, dc->stream));
   KLLM_TRY(cudaStreamSynchronize(dc->stream));
-  if (take_wait_error()) return KLLM_E_STATE;
+  if (dc->wait.take()) return KLLM_E_STATE;
   *next_host = hs_state->next;
   return 0;
 }

@@ -13,12 +13,6 @@ namespace kllm {
 std::atomic<uint64_t>& launch_counter();
 inline void count_launch(uint64_t n = 1) { launch_counter().fetch_add(n, std::memory_order_relaxed); }
 
-// The process's flag for waits that ran out inside a kernel: one int of mapped host memory, which kernels write and the host
-// reads without a copy (nullptr: there is no device).  take_wait_error() is 1 when it was raised since the last call; what a
-// stream has noted is certain to be there once that stream has been waited for.
-int* wait_flag();
-int take_wait_error();
-
 // A position that is either a host value or read from device memory at kernel run time; the
 // decoder's CUDA graph uses the device form so ONE captured graph serves every position.
 struct PosArg {
@@ -63,14 +57,16 @@ constexpr int kPrefillBlock = 1024;  // prompt positions per pass, at most
 struct PrefillWorkspace {  // [block, .] activations
   float *x, *xn, *q, *k, *v, *att, *h1;
 };
+// wait: where its products note a wait that ran out (wait_flag.h)
 int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* tokens_dev, int T, int start_pos,
-                  cudaStream_t stream);
+                  cudaStream_t stream, int* wait);
 // prefill_gemm.cu: out = x . w^T (+ bias); residual += x . w^T; out = silu(x . w1^T) * (x . w3^T)
 // (ahead: may read its weights before the kernels ahead of it on the stream have finished)
 int prefill_product(const float* x, const float* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s,
-                    bool ahead = true);
-int prefill_product_add(const float* x, const float* w, float* residual, int T, int K, int N, cudaStream_t s);
-int prefill_product_gated(const float* x, const float* w1, const float* w3, float* out, int T, int K, int N, cudaStream_t s);
+                    int* wait, bool ahead = true);
+int prefill_product_add(const float* x, const float* w, float* residual, int T, int K, int N, cudaStream_t s, int* wait);
+int prefill_product_gated(const float* x, const float* w1, const float* w3, float* out, int T, int K, int N, cudaStream_t s,
+                          int* wait);
 
 inline float flavour_eps(int flavour) { return flavour == KLLM_FLAVOUR_QWEN2 ? 1e-6f : 1e-5f; }
 }  // namespace kllm

@@ -249,7 +249,7 @@ static int attention_smem_opt_in(size_t bytes) {
 }
 
 int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* tokens_dev, int T, int start_pos,
-                  cudaStream_t s) {
+                  cudaStream_t s, int* wait) {
   const int dim = m.dim, hid = m.hidden_dim, hs = m.head_size, heads = m.head_num, kvh = m.kv_head_num;
   const int q_rows = heads * hs, kvd = kvh * hs;
   auto f32 = [](const void* w) { return static_cast<const float*>(w); };
@@ -264,9 +264,9 @@ int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* to
     const size_t layer_off = static_cast<size_t>(l) * m.seq_len * kvd;
     rmsnorm_rows_kernel<<<T, 256, 0, s>>>(ws.x, m.attn_norm[l], ws.xn, dim, m.eps);
     PF_TRY(count());
-    PF_TRY(prefill_product(ws.xn, f32(m.wq[l]), m.bq ? m.bq[l] : nullptr, ws.q, T, dim, q_rows, s));
-    PF_TRY(prefill_product(ws.xn, f32(m.wk[l]), m.bq ? m.bk[l] : nullptr, ws.k, T, dim, kvd, s));
-    PF_TRY(prefill_product(ws.xn, f32(m.wv[l]), m.bq ? m.bv[l] : nullptr, ws.v, T, dim, kvd, s));
+    PF_TRY(prefill_product(ws.xn, f32(m.wq[l]), m.bq ? m.bq[l] : nullptr, ws.q, T, dim, q_rows, s, wait));
+    PF_TRY(prefill_product(ws.xn, f32(m.wk[l]), m.bq ? m.bk[l] : nullptr, ws.k, T, dim, kvd, s, wait));
+    PF_TRY(prefill_product(ws.xn, f32(m.wv[l]), m.bq ? m.bv[l] : nullptr, ws.v, T, dim, kvd, s, wait));
     rope_scatter_kernel<<<T, 256, 0, s>>>(ws.q, ws.k, ws.v, m.sin_cache, m.cos_cache, m.key_cache + layer_off,
                                           m.value_cache + layer_off, cl, heads, kvh, m.flavour, start_pos);
     PF_TRY(count());
@@ -281,11 +281,11 @@ int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* to
       PF_TRY(launch_attn_tile<2>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos, T, s));
     }
     PF_TRY(count());
-    PF_TRY(prefill_product_add(ws.att, f32(m.wo[l]), ws.x, T, q_rows, dim, s));  // llama3.cpp:683
+    PF_TRY(prefill_product_add(ws.att, f32(m.wo[l]), ws.x, T, q_rows, dim, s, wait));  // llama3.cpp:683
     rmsnorm_rows_kernel<<<T, 256, 0, s>>>(ws.x, m.ffn_norm[l], ws.xn, dim, m.eps);
     PF_TRY(count());
-    PF_TRY(prefill_product_gated(ws.xn, f32(m.w1[l]), f32(m.w3[l]), ws.h1, T, dim, hid, s));
-    PF_TRY(prefill_product_add(ws.h1, f32(m.w2[l]), ws.x, T, hid, dim, s));  // llama3.cpp:719
+    PF_TRY(prefill_product_gated(ws.xn, f32(m.w1[l]), f32(m.w3[l]), ws.h1, T, dim, hid, s, wait));
+    PF_TRY(prefill_product_add(ws.h1, f32(m.w2[l]), ws.x, T, hid, dim, s, wait));  // llama3.cpp:719
   }
   return 0;
 }

@@ -21,6 +21,7 @@
 #include "kllm_host.h"
 #include "seq_engine.h"
 #include "seq_gemm_split.cuh"
+#include "wait_flag.h"
 
 namespace kllm {
 namespace {
@@ -43,17 +44,19 @@ constexpr seq::GatedAct kSwiglu{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f};
 
 }  // namespace
 
-int prefill_product(const float* x, const float* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s, bool ahead) {
+int prefill_product(const float* x, const float* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s,
+                    int* wait, bool ahead) {
   if (!aligned(x, w, K)) return KLLM_E_UNSUPPORTED;
-  return product<seq::umma::kPlain>({x, w, nullptr, bias, nullptr, out, T, N, K, 1, kSwiglu, nullptr}, s, ahead);
+  return product<seq::umma::kPlain>({x, w, nullptr, bias, nullptr, out, T, N, K, 1, kSwiglu, wait}, s, ahead);
 }
-int prefill_product_add(const float* x, const float* w, float* residual, int T, int K, int N, cudaStream_t s) {
+int prefill_product_add(const float* x, const float* w, float* residual, int T, int K, int N, cudaStream_t s, int* wait) {
   if (!aligned(x, w, K)) return KLLM_E_UNSUPPORTED;
-  return product<seq::umma::kAdd>({x, w, nullptr, nullptr, residual, residual, T, N, K, 1, kSwiglu, nullptr}, s);
+  return product<seq::umma::kAdd>({x, w, nullptr, nullptr, residual, residual, T, N, K, 1, kSwiglu, wait}, s);
 }
-int prefill_product_gated(const float* x, const float* w1, const float* w3, float* out, int T, int K, int N, cudaStream_t s) {
+int prefill_product_gated(const float* x, const float* w1, const float* w3, float* out, int T, int K, int N, cudaStream_t s,
+                          int* wait) {
   if (!aligned(x, w1, K) || !aligned(x, w3, K)) return KLLM_E_UNSUPPORTED;
-  return product<seq::umma::kGated>({x, w1, w3, nullptr, nullptr, out, T, N, K, 1, kSwiglu, nullptr}, s);
+  return product<seq::umma::kGated>({x, w1, w3, nullptr, nullptr, out, T, N, K, 1, kSwiglu, wait}, s);
 }
 
 }  // namespace kllm
@@ -61,5 +64,9 @@ int prefill_product_gated(const float* x, const float* w1, const float* w3, floa
 extern "C" int kllm_gemm_tf32(const float* x, const float* w, float* out, int n_tokens, int in_dim, int out_dim,
                               void* stream) {
   if (!x || !w || !out || n_tokens <= 0 || in_dim <= 0 || out_dim <= 0) return KLLM_E_INVALID;
-  return kllm::prefill_product(x, w, nullptr, out, n_tokens, in_dim, out_dim, static_cast<cudaStream_t>(stream), false);
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  int* const wait = kllm::stream_wait_flag(s);
+  if (wait == nullptr) return KLLM_E_STATE;
+  if (const int rc = kllm::prefill_product(x, w, nullptr, out, n_tokens, in_dim, out_dim, s, wait, false)) return rc;
+  return kllm::take_wait_flag(wait) ? KLLM_E_STATE : 0;
 }

@@ -1,12 +1,13 @@
 // Process-wide pieces every library built from this directory carries: the launch counter behind
-// kllm_launch_count(), the version string and the error names of include/kllm_b200.h.
+// kllm_launch_count(), the flags of products enqueued by themselves, the version string and the error names of include/kllm_b200.h.
 #include <cuda_runtime.h>
 
 #include <atomic>
 #include <cstdint>
-#include <mutex>
 
+#include "../../include/kllm_seq.h"
 #include "kllm_host.h"
+#include "wait_flag.h"
 
 namespace kllm {
 std::atomic<uint64_t>& launch_counter() {
@@ -14,29 +15,19 @@ std::atomic<uint64_t>& launch_counter() {
   return c;
 }
 
-int* wait_flag() {
-  static std::atomic<int*> flag{nullptr};
-  if (int* p = flag.load(std::memory_order_acquire)) return p;
-  static std::mutex m;
-  std::lock_guard<std::mutex> lock(m);
-  int* p = flag.load(std::memory_order_relaxed);
-  if (p == nullptr) {
-    void* v = nullptr;
-    if (cudaHostAlloc(&v, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;  // tried again at the next call
-    }
-    p = static_cast<int*>(v);
-    *p = 0;
-    flag.store(p, std::memory_order_release);
-  }
-  return p;
+namespace {
+StreamWaitFlags& stream_flags() {
+  static StreamWaitFlags f;
+  return f;
 }
-int take_wait_error() {
-  int* p = wait_flag();
-  if (p == nullptr || __atomic_load_n(p, __ATOMIC_RELAXED) == 0) return 0;
-  __atomic_store_n(p, 0, __ATOMIC_RELAXED);
-  return 1;
+}  // namespace
+int* stream_wait_flag(cudaStream_t stream) {
+  unsigned long long id = 0;
+  if (cudaStreamGetId(stream, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return stream_flags().get(id);
 }
 }  // namespace kllm
 
@@ -53,6 +44,12 @@ const char* kllm_error_string(int code) {
     case KLLM_E_COMM: return "tensor-parallel transport unavailable or failed";
     default: return code > 0 ? cudaGetErrorString(static_cast<cudaError_t>(code)) : "unknown";
   }
+}
+
+int kllm_product_status(void* stream) {
+  const cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return static_cast<int>(e);
+  return kllm::take_wait_flag(kllm::stream_wait_flag(static_cast<cudaStream_t>(stream))) ? KLLM_E_STATE : 0;
 }
 
 uint64_t kllm_launch_count(void) { return kllm::launch_counter().load(); }

@@ -445,8 +445,7 @@ static int launch_umma(const AttnShape& a, const void* q, const float* gates, co
 }
 int launch_attention_umma(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
                           const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0,
-                          int max_count, int splits, float* ws, void* out, cudaStream_t s) {
-  int* const report = wait_flag();
+                          int max_count, int splits, float* ws, void* out, cudaStream_t s, int* report) {
   if (report == nullptr) return KLLM_E_STATE;
 #define KLLM_ATTN_UMMA(K, V) \
   return launch_umma<K, V>(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, report, s)

@@ -73,6 +73,7 @@
 
 #include "../../include/kllm_seq.h"
 #include "seq_engine.h"
+#include "wait_flag.h"
 
 namespace kllm {
 namespace seq {
@@ -120,6 +121,7 @@ struct kllm_seq_engine {
   std::vector<kllm_seq_layer> layers;
   std::vector<int32_t> run_layer, run_add;
   cudaStream_t stream = nullptr;
+  WaitFlag wait;  // of the step's kernels
   // cache
   int page = 0, n_pages = 0, table_stride = 0;
   std::vector<void*> k_pool, v_pool;  // per run (null for runs without a cache; a latent run has keys only)
@@ -387,9 +389,12 @@ extern "C" int kllm_seq_create(const kllm_seq_desc* desc, void* stream, kllm_seq
   if (int rc = validate(desc)) return rc;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) return KLLM_E_NODEVICE;
-  if (wait_flag() == nullptr) return KLLM_E_STATE;  // allocated here: a step may be inside a capture
   kllm_seq_engine* e = new (std::nothrow) kllm_seq_engine();
   if (!e) return KLLM_E_STATE;
+  if (e->wait.get() == nullptr) {  // allocated here: a step may be inside a capture
+    delete e;
+    return KLLM_E_STATE;
+  }
   e->d = *desc;
   e->layers.assign(desc->layers, desc->layers + desc->n_layers);
   e->run_layer.assign(desc->run_layer, desc->run_layer + desc->n_runs);
@@ -608,6 +613,7 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
   const int W = d.width, dtype = d.dtype;
   const size_t es = elt(dtype);
   cudaStream_t st = e->stream;
+  int* const wait = e->wait.get();
   const uint64_t launches_before = launch_counter().load();
 
   // ---- host: validate, pages, index arrays ------------------------------------------------------------------------
@@ -836,7 +842,7 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
                        A.kv_heads * A.vdim};
       const int n_proj = attn_proj_rows(A), row = room.row > 0 ? room.row : n_proj;
       // the filtered form adds its bias in its own preparation
-      if (room.row == 0) RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, n_proj, st, A.values_are_keys ? nullptr : A.in_bias));
+      if (room.row == 0) RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, n_proj, st, wait, A.values_are_keys ? nullptr : A.in_bias));
       mark(KLLM_SEQ_PHASE_IN_PROJ);
       if (A.values_are_keys) {
         const AttnPrep prep{std::max(1, A.conv_taps), A.conv_w, e->attn_conv[r], A.in_bias, A.rope_dims, A.rope_pairing,
@@ -851,13 +857,13 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
       mark(KLLM_SEQ_PHASE_QK_PREPARE);
       RC(launch_attention(dtype, shape, room.q, static_cast<const float*>(e->gates.p), kv, n_entries, d_first, d_count,
                           d_eseq, d_pos0, max_count, max_ctx, attn_splits(A),
-                          room.ws, room.att, T, d_seq, d_pos, st));
+                          room.ws, room.att, T, d_seq, d_pos, st, wait));
       if (A.differential)
         RC(launch_diff_merge(dtype, shape, attn_splits(A), room.ws,
                              static_cast<const float*>(e->gates.p), A.diff_lambda, A.diff_out_scale, d.norm_eps, room.att, T,
                              st));
       mark(KLLM_SEQ_PHASE_ATTENTION);
-      RC(gemm(dtype, room.att, A.w_out, yout, T, A.heads * A.vdim, W, st, A.out_bias));
+      RC(gemm(dtype, room.att, A.w_out, yout, T, A.heads * A.vdim, W, st, wait, A.out_bias));
       mark(KLLM_SEQ_PHASE_OUT_PROJ);
     } else if (kind == KLLM_SEQ_MIXER_LATENT) {
       const kllm_seq_latent& A = L.latent;
@@ -866,13 +872,13 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
       const PagedKV kv{e->k_pool[r], e->k_pool[r], e->table_dev, e->table_stride, e->page, krow, krow};
       float* gates = A.gate ? static_cast<float*>(e->gates.p) : nullptr;
       const int n_proj = latent_proj_rows(ls);
-      RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, n_proj, st));
+      RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, n_proj, st, wait));
       mark(KLLM_SEQ_PHASE_IN_PROJ);
       // the queries: expanded from their own latent, or rows of the input projection
       const float* queries = A.q_rank > 0 ? static_cast<const float*>(e->qf.p) : proj;
       const int q_row = A.q_rank > 0 ? A.heads * (A.dim + A.rot_dim) : n_proj;
       auto expand_queries = [&]() -> int {
-        return A.q_rank > 0 ? gemm(dtype, room.q, A.w_uq, static_cast<float*>(e->qf.p), T, A.q_rank, q_row, st) : 0;
+        return A.q_rank > 0 ? gemm(dtype, room.q, A.w_uq, static_cast<float*>(e->qf.p), T, A.q_rank, q_row, st, wait) : 0;
       };
       // Prompt steps whose sequences all start here: the step's own latents are all the keys there are, so they are
       // expanded into per-head keys and values (two products) and the tensor-core attention runs on those rows.  Every
@@ -894,17 +900,17 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
                                  e->lat_c.p, static_cast<float*>(e->lat_kr.p), T, st));
         RC(expand_queries());
         float* kp = static_cast<float*>(e->lat_kp.p);
-        RC(gemm(dtype, e->lat_c.p, A.w_uk, kp, T, A.kv_rank, stacked ? kn + vn : kn, st));
-        if (!stacked) RC(gemm(dtype, e->lat_c.p, A.w_uv, static_cast<float*>(e->lat_vp.p), T, A.kv_rank, vn, st));
+        RC(gemm(dtype, e->lat_c.p, A.w_uk, kp, T, A.kv_rank, stacked ? kn + vn : kn, st, wait));
+        if (!stacked) RC(gemm(dtype, e->lat_c.p, A.w_uv, static_cast<float*>(e->lat_vp.p), T, A.kv_rank, vn, st, wait));
         RC(launch_latent_pack(dtype, ls, queries, q_row, kp, stacked ? kn + vn : kn, static_cast<const float*>(e->lat_kr.p),
                               stacked ? kp + kn : static_cast<const float*>(e->lat_vp.p), stacked ? kn + vn : vn, d_pos,
                               e->lat_q.p, e->lat_k.p, e->lat_v.p, T, st));
         mark(KLLM_SEQ_PHASE_QK_PREPARE);
         const PagedKV rows{e->lat_k.p, e->lat_v.p, nullptr, 0, 1, A.heads * dqk, A.heads * A.vdim};
         RC(launch_attention(dtype, eshape, e->lat_q.p, gates, rows, n_entries, d_first, d_count, d_eseq, d_pos0, max_count,
-                            max_ctx, 1, room.ws, room.att, T, d_seq, d_pos, st));
+                            max_ctx, 1, room.ws, room.att, T, d_seq, d_pos, st, wait));
         mark(KLLM_SEQ_PHASE_ATTENTION);
-        RC(gemm(dtype, room.att, A.w_out, yout, T, A.heads * A.vdim, W, st));
+        RC(gemm(dtype, room.att, A.w_out, yout, T, A.heads * A.vdim, W, st, wait));
         mark(KLLM_SEQ_PHASE_OUT_PROJ);
       } else {
       RC(launch_latent_prepare(dtype, ls, proj, A.q_norm_w, A.kv_norm_w, d.norm_eps, d_seq, d_pos, room.q, gates, kv, nullptr,
@@ -918,20 +924,20 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
       const AttnShape shape{A.heads, 1, krow, A.kv_rank, A.scale, 0.f, 0, 0, A.gate, A.window, A.sink, 1, 1, fused_merge ? 1 : 0};
       const int lsplits = reach_splits(A.window);
       RC(launch_attention(dtype, shape, e->qa.p, gates, kv, n_entries, d_first, d_count, d_eseq, d_pos0, max_count, max_ctx,
-                          lsplits, room.ws, e->ol.p, T, d_seq, d_pos, st));
+                          lsplits, room.ws, e->ol.p, T, d_seq, d_pos, st, wait));
       if (fused_merge)
         RC(launch_latent_merge_expand(dtype, ls, lsplits, room.ws, gates, A.sink, A.w_uv,
                                       room.att, T, st));
       else
         RC(launch_latent_expand(dtype, ls, static_cast<const float*>(e->ol.p), A.w_uv, room.att, T, st));
       mark(KLLM_SEQ_PHASE_ATTENTION);
-      RC(gemm(dtype, room.att, A.w_out, yout, T, A.heads * A.vdim, W, st));
+      RC(gemm(dtype, room.att, A.w_out, yout, T, A.heads * A.vdim, W, st, wait));
       mark(KLLM_SEQ_PHASE_OUT_PROJ);
       }
     } else if (kind == KLLM_SEQ_MIXER_LINEAR) {
       const kllm_seq_linear& A = L.linear;
       const int n_proj = linear_proj_rows(A), row = room.row > 0 ? room.row : n_proj;
-      if (room.row == 0) RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, n_proj, st));
+      if (room.row == 0) RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, n_proj, st, wait));
       mark(KLLM_SEQ_PHASE_IN_PROJ);
       const bool by_head = A.out_norm == KLLM_SEQ_OUTNORM_HEAD;
       float* o = static_cast<float*>(e->ol.p);
@@ -953,52 +959,52 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
       }
       if (!normed) RC(launch_linear_out(dtype, A, o, proj, row, d.norm_eps, room.att, T, st));
       mark(KLLM_SEQ_PHASE_ATTENTION);
-      RC(gemm(dtype, room.att, A.w_out, yout, T, A.heads * A.vdim, W, st));
+      RC(gemm(dtype, room.att, A.w_out, yout, T, A.heads * A.vdim, W, st, wait));
       mark(KLLM_SEQ_PHASE_OUT_PROJ);
     } else if (kind == KLLM_SEQ_MIXER_SSM) {
       const kllm_seq_ssm& A = L.ssm;
       float* uc = static_cast<float*>(e->rec_a.p);
       float* low = static_cast<float*>(e->rec_b.p);
-      RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, 2 * A.inner, st));
+      RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, 2 * A.inner, st, wait));
       mark(KLLM_SEQ_PHASE_IN_PROJ);
       RC(launch_ssm_conv(dtype, A, proj, e->ssm_conv[r], step_rows, uc, room.att, T, st));
-      RC(gemm(dtype, room.att, A.w_x, low, T, A.inner, A.dt_rank + 2 * A.state, st));
+      RC(gemm(dtype, room.att, A.w_x, low, T, A.inner, A.dt_rank + 2 * A.state, st, wait));
       mark(KLLM_SEQ_PHASE_QK_PREPARE);
       RC(launch_ssm_scan(dtype, A, proj, uc, low, e->ssm_state[r], step_rows, d_eseq, max_count, T,
                          room.ws, room.att, st));
       mark(KLLM_SEQ_PHASE_ATTENTION);
-      RC(gemm(dtype, room.att, A.w_out, yout, T, A.inner, W, st));
+      RC(gemm(dtype, room.att, A.w_out, yout, T, A.inner, W, st, wait));
       mark(KLLM_SEQ_PHASE_OUT_PROJ);
     } else if (kind == KLLM_SEQ_MIXER_SSD) {
       const kllm_seq_ssd& A = L.ssd;
       float* xbc = static_cast<float*>(e->rec_a.p);
       float* yr = static_cast<float*>(e->rec_b.p);
-      RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, ssd_proj_row(A), st));
+      RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, ssd_proj_row(A), st, wait));
       mark(KLLM_SEQ_PHASE_IN_PROJ);
       RC(launch_ssd_conv(A, proj, e->ssd_conv[r], step_rows, xbc, T, st));
       mark(KLLM_SEQ_PHASE_QK_PREPARE);
       RC(launch_ssd_scan(A, proj, xbc, e->ssd_state[r], step_rows, d_eseq, max_count, T, room.ws, yr, st));
       RC(launch_ssd_out(dtype, A, yr, proj, d.norm_eps, room.att, T, st));
       mark(KLLM_SEQ_PHASE_ATTENTION);
-      RC(gemm(dtype, room.att, A.w_out, yout, T, ssd_inner(A), W, st));
+      RC(gemm(dtype, room.att, A.w_out, yout, T, ssd_inner(A), W, st, wait));
       mark(KLLM_SEQ_PHASE_OUT_PROJ);
     } else {
       const kllm_seq_delta& A = L.delta;
       float* prep = static_cast<float*>(e->rec_a.p);
       float* o = static_cast<float*>(e->rec_b.p);
       const int n_proj = 2 * A.kv_heads * A.dim + A.heads * A.vdim + A.heads + A.decay_rank + A.gate_rank;
-      RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, n_proj, st));
+      RC(gemm(dtype, e->h.p, A.w_in, proj, T, W, n_proj, st, wait));
       mark(KLLM_SEQ_PHASE_IN_PROJ);
       // the second low-rank projections of the decays and the gates: one product on the low-rank rows in the compute type
       float* low2 = static_cast<float*>(e->rec_c.p);
       RC(launch_delta_low(dtype, A, proj, room.q, T, st));
-      RC(gemm(dtype, room.q, A.w_low2, low2, T, A.decay_rank + A.gate_rank, A.heads * (A.dim + A.vdim), st));
+      RC(gemm(dtype, room.q, A.w_low2, low2, T, A.decay_rank + A.gate_rank, A.heads * (A.dim + A.vdim), st, wait));
       RC(launch_delta_prepare(A, proj, low2, e->delta_conv[r], step_rows, prep, T, st));
       mark(KLLM_SEQ_PHASE_QK_PREPARE);
       RC(launch_delta_rule(A, prep, e->delta_state[r], step_rows, d_eseq, max_count, T, room.ws, o, st));
       RC(launch_delta_out(dtype, A, o, prep, d.norm_eps, room.att, T, st));
       mark(KLLM_SEQ_PHASE_ATTENTION);
-      RC(gemm(dtype, room.att, A.w_out, yout, T, A.heads * A.vdim, W, st));
+      RC(gemm(dtype, room.att, A.w_out, yout, T, A.heads * A.vdim, W, st, wait));
       mark(KLLM_SEQ_PHASE_OUT_PROJ);
     }
     return 0;
@@ -1012,12 +1018,12 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
     if (L.ff_kind == KLLM_SEQ_FF_DENSE) {
       const kllm_seq_dense& F = L.dense;
       if (dense_gated(F)) {
-        RC(gemm_gated(dtype, e->h.p, F.up, e->att.p, T, W, F.ff, GatedAct{F.act, F.act_a, F.act_b}, st, F.up_bias));
+        RC(gemm_gated(dtype, e->h.p, F.up, e->att.p, T, W, F.ff, GatedAct{F.act, F.act_a, F.act_b}, st, wait, F.up_bias));
       } else {
-        RC(gemm(dtype, e->h.p, F.up, proj, T, W, F.ff, st, F.up_bias));
+        RC(gemm(dtype, e->h.p, F.up, proj, T, W, F.ff, st, wait, F.up_bias));
         RC(launch_activation(dtype, F.act, F.act_a, F.act_b, proj, e->att.p, Ts * F.ff, st));
       }
-      RC(gemm(dtype, e->att.p, F.down, yout, T, F.ff, W, st, F.down_bias));
+      RC(gemm(dtype, e->att.p, F.down, yout, T, F.ff, W, st, wait, F.down_bias));
       e->mark(KLLM_SEQ_PHASE_EXPERTS);
       return 0;
     }
@@ -1051,7 +1057,7 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
       RC(launch_sort_pairs(top_idx, n_pairs, M.experts, kGroupBlock, counts_d, sorted, block_expert, cap, tiles, n_tiles, st));
       GroupedArgs g{};
       g.sorted_pair = sorted, g.block_expert = block_expert, g.n_blocks = n_blocks, g.block = kGroupBlock;
-      g.experts = M.experts, g.act = act, g.tiles = tiles, g.n_tiles = n_tiles;
+      g.experts = M.experts, g.act = act, g.tiles = tiles, g.n_tiles = n_tiles, g.report = wait;
       const int inner_epilogue = M.act == KLLM_SEQ_ACT_RELU2 ? 2 : 1;
       if (grouped_tensor_core_usable(dtype, W, M.ff)) {
         // rows in sorted order: a gathered copy of h, the expert's inner activations, then scattered back by pair
@@ -1073,8 +1079,8 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
     }
     e->mark(KLLM_SEQ_PHASE_EXPERTS);
     if (M.shared_ff > 0 && !shared_done) {
-      RC(gemm_gated(dtype, e->h.p, M.shared_gate_up, e->att.p, T, W, M.shared_ff, GatedAct{M.act, M.shared_act_limit, M.act_alpha}, st));
-      RC(gemm(dtype, e->att.p, M.shared_down, y2, T, M.shared_ff, W, st));
+      RC(gemm_gated(dtype, e->h.p, M.shared_gate_up, e->att.p, T, W, M.shared_ff, GatedAct{M.act, M.shared_act_limit, M.act_alpha}, st, wait));
+      RC(gemm(dtype, e->att.p, M.shared_down, y2, T, M.shared_ff, W, st, wait));
       e->mark(KLLM_SEQ_PHASE_SHARED);
       *shared_out = true;
     }
@@ -1134,7 +1140,7 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
       MixerRoom a1 = room1, a2 = room2;
       if (const int n1 = stacked_rows(d, L); n1 > 0) {
         const int row = n1 + linear_proj_rows(L.linear);
-        RC(gemm(dtype, e->h.p, L.attn.w_in, a1.proj, T, W, row, st));
+        RC(gemm(dtype, e->h.p, L.attn.w_in, a1.proj, T, W, row, st, wait));
         e->mark(KLLM_SEQ_PHASE_IN_PROJ);
         a1.row = a2.row = row, a2.proj = a1.proj + n1;
       }
@@ -1213,7 +1219,7 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
       RC(launch_resid_norm(a, st));
     }
     float* lg = static_cast<float*>(e->logits.p);
-    RC(gemm(dtype, e->hw.p, d.head, lg, n_want, W, d.vocab, st));
+    RC(gemm(dtype, e->hw.p, d.head, lg, n_want, W, d.vocab, st, wait));
     if ((d.logit_scale != 0.f && d.logit_scale != 1.f) || d.logit_softcap > 0.f)
       RC(launch_scale(lg, d.logit_scale, d.logit_softcap, static_cast<size_t>(n_want) * d.vocab, st));
     if (argmax_host) RC(launch_argmax_rows(lg, static_cast<int32_t*>(e->amax.p), n_want, d.vocab, st));
@@ -1274,14 +1280,14 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
     }
     e->prof_out = nullptr;
   }
-  if (gemm_take_error()) return KLLM_E_STATE;
+  if (e->wait.take()) return KLLM_E_STATE;
   return 0;
 }
 
 extern "C" int kllm_seq_gemm(int32_t dtype, const void* a, const void* w, float* out, int32_t n_tokens, int32_t in_dim,
                              int32_t out_dim, void* stream) {
-  const int rc = gemm(dtype, a, w, out, n_tokens, in_dim, out_dim, static_cast<cudaStream_t>(stream), nullptr, false);
-  if (rc != 0) return rc;
-  if (gemm_take_error()) return KLLM_E_STATE;
-  return 0;
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  int* const wait = stream_wait_flag(s);  // (kernels that wait for nothing run without it)
+  if (const int rc = gemm(dtype, a, w, out, n_tokens, in_dim, out_dim, s, wait, nullptr, false)) return rc;
+  return take_wait_flag(wait) ? KLLM_E_STATE : 0;
 }

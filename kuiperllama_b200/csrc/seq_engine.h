@@ -196,7 +196,7 @@ size_t attention_workspace_bytes(const AttnShape& a, int T, int splits);
 int launch_attention(int dtype, const AttnShape& a, const void* q, const float* gates, const PagedKV& kv,
                      int n_entries, const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq,
                      const int32_t* ent_pos0, int max_count, int max_ctx, int splits, float* ws, void* out, int T,
-                     const int32_t* tok_seq, const int32_t* tok_pos, cudaStream_t s);
+                     const int32_t* tok_seq, const int32_t* tok_pos, cudaStream_t s, int* report);
 
 // Prompt steps in bf16 with head sizes up to 128 (multiples of 8): the same attention on the tensor cores (seq_attention_mma.cu).
 // With splits == 1 it writes `out` itself (gate applied); otherwise it leaves partial results in `ws` for the merge.
@@ -204,11 +204,11 @@ bool attention_mma_usable(int dtype, const AttnShape& a, int max_count);
 int launch_attention_mma(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
                          const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq,
                          const int32_t* ent_pos0, int max_count, int splits, float* ws, void* out, cudaStream_t s);
-// the same on tcgen05, for long prompts (seq_attention_umma.cu)
+// the same on tcgen05, for long prompts (seq_attention_umma.cu); report: where a wait that ran out is noted (wait_flag.h)
 bool attention_umma_usable(int dtype, const AttnShape& a, int max_count);
 int launch_attention_umma(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
                           const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0,
-                          int max_count, int splits, float* ws, void* out, cudaStream_t s);
+                          int max_count, int splits, float* ws, void* out, cudaStream_t s, int* report);
 // the same to fp32 accuracy (seq_attention_f32.cu)
 bool attention_f32_usable(int dtype, const AttnShape& a, const PagedKV& kv, int max_count);
 int launch_attention_f32(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
@@ -432,14 +432,13 @@ int launch_ssd_out(int dtype, const kllm_seq_ssd& m, const float* y, const float
 
 // ---- seq_gemm.cu --------------------------------------------------------------------------------------------------
 // out[T, N] (fp32) = a[T, K] . w[N, K]^T (+ bias[N]), a and w in the compute type, fp32 accumulation.
-// ahead: the kernel may read weights before the kernels ahead of it on the stream have finished (seq_launch.cuh)
-int gemm(int dtype, const void* a, const void* w, float* out, int T, int K, int N, cudaStream_t s, const float* bias = nullptr,
-         bool ahead = true);
+// report: where a wait that ran out is noted (wait_flag.h); ahead: the kernel may read weights before the kernels ahead of it on the
+// stream have finished (seq_launch.cuh)
+int gemm(int dtype, const void* a, const void* w, float* out, int T, int K, int N, cudaStream_t s, int* report,
+         const float* bias = nullptr, bool ahead = true);
 // out[T, ff] (compute type) = gated_act(a . wg^T + bias[f], a . wu^T + bias[ff + f]), w = [ff gate rows, then ff up rows][K]
 int gemm_gated(int dtype, const void* a, const void* w, void* out, int T, int K, int ff, const GatedAct& act, cudaStream_t s,
-               const float* bias = nullptr);
-// != 0 when a bounded wait inside a tensor-core product ran out since the last call (checked after a step's sync)
-int gemm_take_error();
+               int* report, const float* bias = nullptr);
 // Grouped form for the routed experts: block b (of `block` rows) multiplies rows a[row_of(b, i)] with the weights of
 // expert block_expert[b]; see seq_gemm.cu.
 struct GroupedArgs {
@@ -460,6 +459,7 @@ struct GroupedArgs {
   // ... and the tiles: {expert, first row, rows, 0} of up to 256 rows of one expert, *n_tiles of them, in device memory
   const int32_t *tiles, *n_tiles;
   int experts;
+  int* report;  // where a wait that ran out is noted
 };
 int gemm_grouped(int dtype, const GroupedArgs& g, cudaStream_t s);
 // bf16 only: can the grouped products of an expert layer (K = width, then K = ff) run on the tensor cores?

@@ -301,7 +301,8 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ a, const in
 }
 
 template <typename AT>
-int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s, bool ahead) {
+int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s, int* report,
+           bool ahead) {
   constexpr int V = Vec16<AT>::N;
   if (T <= 8) {
     const bool vec = (K % V) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
@@ -321,11 +322,11 @@ int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K
     return cuda_rc(cudaGetLastError());
   }
   if (umma::usable<AT>(a, w, T, K, N)) {
-    return umma::launch(a, w, bias, out, T, K, N, s, ahead);
+    return umma::launch(a, w, bias, out, T, K, N, s, report, ahead);
   }
   if constexpr (std::is_same_v<AT, float>)
     if (umma::fp32_usable(a, w, T, K))
-      return umma::launch_fp32<false>(a, w, bias, out, T, K, N, GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}, s, ahead);
+      return umma::launch_fp32<false>(a, w, bias, out, T, K, N, GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}, s, report, ahead);
   const dim3 grid((N + TN - 1) / TN, (T + TM - 1) / TM);
   tiled_kernel<AT, false, 0><<<grid, 256, 0, s>>>(a, w, out, T, K, N, nullptr, nullptr, 1,
                                                  GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}, bias);
@@ -334,7 +335,8 @@ int gemm_t(const AT* a, const AT* w, const float* bias, float* out, int T, int K
 }
 
 template <typename AT>
-int gemm_gated_t(const AT* a, const AT* w, const float* bias, AT* out, int T, int K, int N, const GatedAct& act, cudaStream_t s) {
+int gemm_gated_t(const AT* a, const AT* w, const float* bias, AT* out, int T, int K, int N, const GatedAct& act, cudaStream_t s,
+                 int* report) {
   constexpr int V = Vec16<AT>::N;
   if (T <= 8) {
     const bool vec = (K % V) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
@@ -355,10 +357,10 @@ int gemm_gated_t(const AT* a, const AT* w, const float* bias, AT* out, int T, in
     return cuda_rc(cudaGetLastError());
   }
   if (umma::usable<AT>(a, w, T, K, N)) {
-    return umma::launch_gated(a, w, bias, out, T, K, N, act, s);
+    return umma::launch_gated(a, w, bias, out, T, K, N, act, s, report);
   }
   if constexpr (std::is_same_v<AT, float>)
-    if (umma::fp32_usable(a, w, T, K)) return umma::launch_fp32<true>(a, w, bias, out, T, K, N, act, s, true);
+    if (umma::fp32_usable(a, w, T, K)) return umma::launch_fp32<true>(a, w, bias, out, T, K, N, act, s, report, true);
   const dim3 grid((N + TN - 1) / TN, (T + TM - 1) / TM);
   tiled_kernel<AT, false, 1><<<grid, 256, 0, s>>>(a, w, out, T, K, N, nullptr, nullptr, 1, act, bias);
   count_launch();
@@ -384,27 +386,28 @@ int grouped_t(const GroupedArgs& g, cudaStream_t s) {
 
 }  // namespace
 
-int gemm(int dtype, const void* a, const void* w, float* out, int T, int K, int N, cudaStream_t s, const float* bias, bool ahead) {
+int gemm(int dtype, const void* a, const void* w, float* out, int T, int K, int N, cudaStream_t s, int* report, const float* bias,
+         bool ahead) {
   if (!a || !w || !out || T <= 0 || K <= 0 || N <= 0) return KLLM_E_INVALID;
   if (dtype == KLLM_SEQ_F32)
-    return gemm_t(static_cast<const float*>(a), static_cast<const float*>(w), bias, out, T, K, N, s, ahead);
+    return gemm_t(static_cast<const float*>(a), static_cast<const float*>(w), bias, out, T, K, N, s, report, ahead);
   if (dtype == KLLM_SEQ_BF16)
-    return gemm_t(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(w), bias, out, T, K, N, s, ahead);
+    return gemm_t(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(w), bias, out, T, K, N, s, report,
+                  ahead);
   return KLLM_E_INVALID;
 }
 
 int gemm_gated(int dtype, const void* a, const void* w, void* out, int T, int K, int ff, const GatedAct& act, cudaStream_t s,
-               const float* bias) {
+               int* report, const float* bias) {
   if (!a || !w || !out || T <= 0 || K <= 0 || ff <= 0) return KLLM_E_INVALID;
   if (dtype == KLLM_SEQ_F32)
-    return gemm_gated_t(static_cast<const float*>(a), static_cast<const float*>(w), bias, static_cast<float*>(out), T, K, ff, act, s);
+    return gemm_gated_t(static_cast<const float*>(a), static_cast<const float*>(w), bias, static_cast<float*>(out), T, K, ff, act, s,
+                        report);
   if (dtype == KLLM_SEQ_BF16)
     return gemm_gated_t(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(w), bias,
-                        static_cast<__nv_bfloat16*>(out), T, K, ff, act, s);
+                        static_cast<__nv_bfloat16*>(out), T, K, ff, act, s, report);
   return KLLM_E_INVALID;
 }
-
-int gemm_take_error() { return take_wait_error(); }
 
 bool grouped_tensor_core_usable(int dtype, int width, int ff) {
   return dtype == KLLM_SEQ_BF16 && umma::grouped_usable(width, ff) && umma::grouped_usable(ff, width);
@@ -422,10 +425,11 @@ int gemm_grouped(int dtype, const GroupedArgs& g, cudaStream_t s) {
   if (g.sorted_layout) {
     if (dtype != KLLM_SEQ_BF16 || g.block != umma::GBN || !g.tiles || !g.n_tiles) return KLLM_E_INVALID;
     if (g.epilogue == 1)
-      return umma::launch_grouped<1>(g.a, g.w, g.out, g.sorted_pair, g.tiles, g.n_tiles, g.n_blocks, g.experts, g.K, g.N, s, g.act);
+      return umma::launch_grouped<1>(g.a, g.w, g.out, g.sorted_pair, g.tiles, g.n_tiles, g.n_blocks, g.experts, g.K, g.N, s, g.report,
+                                     g.act);
     if (g.epilogue == 2)
-      return umma::launch_grouped<2>(g.a, g.w, g.out, g.sorted_pair, g.tiles, g.n_tiles, g.n_blocks, g.experts, g.K, g.N, s);
-    return umma::launch_grouped<0>(g.a, g.w, g.out, g.sorted_pair, g.tiles, g.n_tiles, g.n_blocks, g.experts, g.K, g.N, s);
+      return umma::launch_grouped<2>(g.a, g.w, g.out, g.sorted_pair, g.tiles, g.n_tiles, g.n_blocks, g.experts, g.K, g.N, s, g.report);
+    return umma::launch_grouped<0>(g.a, g.w, g.out, g.sorted_pair, g.tiles, g.n_tiles, g.n_blocks, g.experts, g.K, g.N, s, g.report);
   }
   if (dtype == KLLM_SEQ_F32) return grouped_t<float>(g, s);
   if (dtype == KLLM_SEQ_BF16) return grouped_t<__nv_bfloat16>(g, s);

@@ -350,7 +350,6 @@ inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
   constexpr bool two = OUT == kGated;
   constexpr int FEATURES = two ? BM / 2 : BM;
   CUtensorMap map_w, map_w2, map_a;
-  p.report = wait_flag();
   if (p.report == nullptr) return KLLM_E_STATE;
   if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, FEATURES)) return rc;
   if (int rc = make_map_of<MODE>(&map_w2, two ? p.w2 : p.w, p.N, p.K, FEATURES)) return rc;
@@ -386,9 +385,9 @@ inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
 // the narrowest token block that holds the step; more than 128 tokens in tiles of 64
 template <bool GATED>
 int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act,
-               cudaStream_t s, bool ahead) {
+               cudaStream_t s, int* report, bool ahead) {
   const void* w2 = static_cast<const __nv_bfloat16*>(w) + static_cast<size_t>(N) * K;  // the up rows follow the gate rows
-  const SplitArgs p{a, w, w2, bias, nullptr, out, T, N, K, 1, act, nullptr};
+  const SplitArgs p{a, w, w2, bias, nullptr, out, T, N, K, 1, act, report};
   constexpr int OUT = GATED ? kGated : kPlain;
   if (T <= 16) return launch_split<kBf16, 16, OUT, 5>(p, s, ahead);
   if (T <= 32) return launch_split<kBf16, 32, OUT, 5>(p, s, ahead);
@@ -404,8 +403,8 @@ inline bool fp32_usable(const void* a, const void* w, int T, int K) {
 }
 template <bool GATED>
 int launch_fp32(const float* a, const float* w, const float* bias, float* out, int T, int K, int N, const GatedAct& act,
-                cudaStream_t s, bool ahead) {
-  const SplitArgs p{a, w, w + static_cast<size_t>(N) * K, bias, nullptr, out, T, N, K, 1, act, nullptr};
+                cudaStream_t s, int* report, bool ahead) {
+  const SplitArgs p{a, w, w + static_cast<size_t>(N) * K, bias, nullptr, out, T, N, K, 1, act, report};
   constexpr int OUT = GATED ? kGated : kPlain;
   if (T <= 16) return launch_split<kFp32, 16, OUT, 3>(p, s, ahead);
   if (T <= 32) return launch_split<kFp32, 32, OUT, 3>(p, s, ahead);

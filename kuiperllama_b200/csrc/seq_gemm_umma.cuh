@@ -35,7 +35,7 @@ constexpr int A_BYTES = BM * BK * 2;
 constexpr int THREADS = 192;
 constexpr uint32_t kWaitLimit = 1u << 24;  // try_wait rounds before a wait gives up (each suspends up to ~1 us)
 
-// Where a wait that runs out is noted: `here` stops the other roles of the CTA, `report` (kllm::wait_flag) is read by the host.
+// Where a wait that runs out is noted: `here` stops the other roles of the CTA, `report` is its launcher's flag (wait_flag.h).
 struct Stop {
   volatile int* here;
   int* report;
@@ -165,7 +165,7 @@ struct SplitArgs {
   void* out;
   int T, N, K, S;
   GatedAct act;
-  int* report;  // wait_flag()
+  int* report;  // where a wait that ran out is noted
 };
 
 template <typename OT> __device__ __forceinline__ OT to_type(float v) { return v; }
@@ -614,7 +614,6 @@ template <int MODE, int BN, int OUT>
 inline int launch_persistent(SplitArgs p, cudaStream_t stream) {
   constexpr int FEATURES = OUT == kGated ? BM / 2 : BM;
   CUtensorMap map_w, map_up, map_a;
-  p.report = wait_flag();
   if (p.report == nullptr) return KLLM_E_STATE;
   if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, FEATURES)) return rc;
   if (int rc = make_map_of<MODE>(&map_up, OUT == kGated ? p.w2 : p.w, p.N, p.K, FEATURES)) return rc;
@@ -650,15 +649,15 @@ inline int launch_wide(const SplitArgs& p, cudaStream_t s) {
 // products whose tiles do not fill the chip (seq_gemm_split.cuh)
 template <bool GATED>
 int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act, cudaStream_t s,
-               bool ahead);
+               int* report, bool ahead);
 
 // less than one tile of 128 tokens per SM: narrower token blocks and K split over CTAs
 template <bool GATED>
 inline int launch_block(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act,
-                        cudaStream_t s, bool ahead) {
-  if (!fills_chip(T, N)) return launch_few<GATED>(a, w, bias, out, T, K, N, act, s, ahead);
+                        cudaStream_t s, int* report, bool ahead) {
+  if (!fills_chip(T, N)) return launch_few<GATED>(a, w, bias, out, T, K, N, act, s, report, ahead);
   const void* w2 = static_cast<const __nv_bfloat16*>(w) + (GATED ? static_cast<size_t>(N) * K : 0);  // 16-byte rows: K % 8 == 0
-  return launch_wide<kBf16, GATED ? kGated : kPlain>(SplitArgs{a, w, w2, bias, nullptr, out, T, N, K, 1, act, nullptr}, s);
+  return launch_wide<kBf16, GATED ? kGated : kPlain>(SplitArgs{a, w, w2, bias, nullptr, out, T, N, K, 1, act, report}, s);
 }
 
 template <typename AT>
@@ -671,21 +670,25 @@ inline bool usable<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* w
 }
 
 template <typename AT>
-inline int launch(const AT*, const AT*, const float*, float*, int, int, int, cudaStream_t, bool) { return KLLM_E_UNSUPPORTED; }
+inline int launch(const AT*, const AT*, const float*, float*, int, int, int, cudaStream_t, int*, bool) {
+  return KLLM_E_UNSUPPORTED;
+}
 template <>
 inline int launch<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* w, const float* bias, float* out, int T, int K,
-                                 int N, cudaStream_t s, bool ahead) {
+                                 int N, cudaStream_t s, int* report, bool ahead) {
   const GatedAct none{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f};
-  return launch_block<false>(a, w, bias, out, T, K, N, none, s, ahead);
+  return launch_block<false>(a, w, bias, out, T, K, N, none, s, report, ahead);
 }
 
 // w: [2 * N, K], gate rows then up rows
 template <typename AT>
-inline int launch_gated(const AT*, const AT*, const float*, AT*, int, int, int, const GatedAct&, cudaStream_t) { return KLLM_E_UNSUPPORTED; }
+inline int launch_gated(const AT*, const AT*, const float*, AT*, int, int, int, const GatedAct&, cudaStream_t, int*) {
+  return KLLM_E_UNSUPPORTED;
+}
 template <>
 inline int launch_gated<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* w, const float* bias, __nv_bfloat16* out, int T,
-                                       int K, int N, const GatedAct& act, cudaStream_t s) {
-  return launch_block<true>(a, w, bias, out, T, K, N, act, s, true);
+                                       int K, int N, const GatedAct& act, cudaStream_t s, int* report) {
+  return launch_block<true>(a, w, bias, out, T, K, N, act, s, report, true);
 }
 
 inline bool grouped_usable(int K, int N) {
@@ -696,11 +699,10 @@ inline bool grouped_usable(int K, int N) {
 // a: [n_blocks * 64, K] bf16 in sorted order; w: [experts * (EPI ? 2 : 1) * N, K]; at most n_blocks entries in the list
 template <int EPI>
 inline int launch_grouped(const void* a, const void* w, void* out, const int32_t* sorted_pair, const int32_t* list,
-                          const int32_t* n_tiles, int n_blocks, int experts, int K, int N, cudaStream_t stream,
+                          const int32_t* n_tiles, int n_blocks, int experts, int K, int N, cudaStream_t stream, int* report,
                           GatedAct act = GatedAct{KLLM_SEQ_ACT_SWIGLU, 0.f, 0.f}) {
   constexpr int FEATURES = EPI == 1 ? BM / 2 : BM;
   CUtensorMap map_w, map_a;
-  int* const report = wait_flag();
   if (report == nullptr) return KLLM_E_STATE;
   if (int rc = make_map(&map_w, w, experts * (EPI == 1 ? 2 : 1) * N, K, FEATURES)) return rc;
   if (int rc = make_map(&map_a, a, n_blocks * GBN, K, GBN)) return rc;

@@ -1731,13 +1731,14 @@ static int launch_attention_c(const AttnShape& a, const void* q, const PagedKV& 
 int launch_attention(int dtype, const AttnShape& a, const void* q, const float* gates, const PagedKV& kv,
                      int n_entries, const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq,
                      const int32_t* ent_pos0, int max_count, int max_ctx, int splits, float* ws, void* out, int T,
-                     const int32_t* tok_seq, const int32_t* tok_pos, cudaStream_t s) {
+                     const int32_t* tok_seq, const int32_t* tok_pos, cudaStream_t s, int* report) {
   (void)max_ctx;
   if (a.kv_heads <= 0 || a.heads % a.kv_heads != 0 || a.dim <= 0 || a.vdim <= 0) return KLLM_E_UNSUPPORTED;
   const int C = (a.vdim + kAttnKeys - 1) / kAttnKeys;
   int rc = 0;
   if (attention_umma_usable(dtype, a, max_count)) {
-    rc = launch_attention_umma(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, s);
+    rc = launch_attention_umma(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, s,
+                               report);
     if (rc || (splits == 1 && !a.no_merge)) return rc;
   } else if (attention_mma_usable(dtype, a, max_count)) {
     rc = launch_attention_mma(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws,

@@ -120,6 +120,7 @@ def load_seq_library():
     lib.kllm_seq_profile.argtypes = [c_void_p, POINTER(c_float)]
     lib.kllm_seq_last_launches.argtypes = [c_void_p]
     lib.kllm_seq_gemm.argtypes = [c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_void_p]
+    lib.kllm_product_status.argtypes = [c_void_p]
     lib.kllm_error_string.restype = ctypes.c_char_p
     return lib
 
