@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py -- decode tokens/s of the B200-native KuiperLLama hot path (BASELINE.json `metric`).
+"""bench.py -- decode tokens/s of the B200-native KuiperLLama hot path.
 
 One "step" = one greedy decode position (one token, batch 1) of the workload's model through the
 device-resident decoder (libkllm_b200.so).  The metric is quoted on context 1 -> 1024, so the
@@ -24,16 +24,16 @@ context is NOT tied to --steps:
                 per launch / event-timed launch duration vs MEASURED_PEAKS.json.
   cpu_baseline  the CPU restatement of the reference path (oracle/) on the box's host cores.
 
-Workloads.  1 GPU on a single-GPU box: BASELINE.json configs[1], TinyLlama-1.1B fp32.  Under
+Workloads.  1 GPU on a single-GPU box: TinyLlama-1.1B fp32.  Under
 tensor parallelism (--gpus N > 1) and for the N = 1 point of the same series (any run on a box
-with several GPUs): the model the metric names for 1/2/4/8 GPUs, Llama-2-7B int8 (configs[2]);
-the fp32 Llama-2-7B of configs[4] is measured in the same run and reported under `secondary`.
+with several GPUs): the model the metric names for 1/2/4/8 GPUs, Llama-2-7B int8;
+the fp32 Llama-2-7B is measured in the same run and reported under `secondary`.
 --workload overrides.
 
 --impl reference       the reference's CPU implementation of the path (oracle port; the reference's
                        CMake build needs Armadillo/glog/gtest/sentencepiece, none installed).
 --impl reference-cuda  the reference's own CUDA kernels + model code (oracle/_ref, compiled from
-                       /root/reference for sm_100a) timed on the same GPU: the "reference GPU" row.
+                       the reference's sources for sm_100a) timed on the same GPU: the "reference GPU" row.
 """
 from __future__ import annotations
 
@@ -53,15 +53,15 @@ sys.path.insert(0, str(ROOT))
 
 METRIC = "decode_tokens_per_s"
 CONTEXT = 1024  # the metric's context: 1 -> 1024
-# the one number the reference publishes for this metric -- TinyLlama-1.1B fp32,
+# The one number the reference publishes for this metric -- TinyLlama-1.1B fp32,
 # batch 1, its CUDA backend on an RTX 3060 Laptop GPU (readme.md:25).  Other workloads: none.
 PUBLISHED_TOK_S = {"tinyllama-1.1b": 60.34}
 WORKLOAD_NAMES = {
-    "tinyllama-1.1b": "TinyLlama-1.1B fp32 greedy decode, batch 1 (BASELINE.json configs[1])",
-    "llama2-7b-int8": "Llama-2-7B int8 g64 (export.py --version 3) greedy decode, batch 1 (configs[2]; metric's 1/2/4/8-GPU model)",
-    "qwen2.5-0.5b": "Qwen2.5-0.5B fp32 greedy decode, batch 1 (configs[3])",
-    "llama2-7b": "Llama-2-7B fp32 greedy decode, batch 1 (configs[4])",
-    "stories15m": "stories15M fp32 greedy decode, batch 1 (configs[0])",
+    "tinyllama-1.1b": "TinyLlama-1.1B fp32 greedy decode, batch 1",
+    "llama2-7b-int8": "Llama-2-7B int8 g64 (export.py --version 3) greedy decode, batch 1 (the 1/2/4/8-GPU model)",
+    "qwen2.5-0.5b": "Qwen2.5-0.5B fp32 greedy decode, batch 1",
+    "llama2-7b": "Llama-2-7B fp32 greedy decode, batch 1",
+    "stories15m": "stories15M fp32 greedy decode, batch 1",
     "small": "synthetic dim-288 3-layer model (debug)",
 }
 
@@ -86,7 +86,7 @@ def parse_args():
                          "carries the exact mode's numbers under \"exact\"")
     ap.add_argument("--no-exact", action="store_true", help="skip the exact-mode leg of a --numerics fast run")
     ap.add_argument("--no-cpu-baseline", action="store_true")
-    ap.add_argument("--no-secondary", action="store_true", help="N>1: skip the fp32 Llama-2-7B line (configs[4])")
+    ap.add_argument("--no-secondary", action="store_true", help="N>1: skip the fp32 Llama-2-7B line")
     ap.add_argument("--cpu-seconds", type=float, default=12.0, help="budget of the cpu_baseline leg")
     ap.add_argument("--seed", type=int, default=None)
     ap.add_argument("--family", default=None, choices=["fobolorn", "kikunex", "vurazen", "bukuvik", "bifazen", "mobatar"],
@@ -101,7 +101,7 @@ SEEDS = {"stories15m": 1234, "tinyllama-1.1b": 1235, "llama2-7b-int8": 1236, "qw
 
 
 def default_workload(n_gpus):
-    """configs[1] on one GPU of a single-GPU box; the metric's 1/2/4/8-GPU model otherwise."""
+    """TinyLlama-1.1B fp32 on one GPU of a single-GPU box; the 1/2/4/8-GPU model otherwise."""
     if n_gpus > 1:
         return "llama2-7b-int8"
     try:
@@ -644,7 +644,7 @@ def run_ours(args, rank, world):
         torch.cuda.empty_cache()
 
     if world > 1 and not args.no_secondary and args.workload != "llama2-7b":
-        # BASELINE.json configs[4]: the fp32 Llama-2-7B under the same tensor parallelism
+        # the fp32 Llama-2-7B under the same tensor parallelism
         sargs = argparse.Namespace(**{**vars(args), "reps": min(args.reps, 3)})
         sb = Bench(sargs, rank, world, "llama2-7b", stream, lib)
         sres = sb.run()

@@ -16,7 +16,7 @@
  *   - there is NO CPU fallback: without a CUDA device every call returns an error.
  *
  * Arithmetic contract: fp32 throughout, each kernel reproduces the reference CUDA kernel's
- * floating-point operation order (see DESIGN.md "Bit-exactness"), so results are bit-identical
+ * floating-point operation order, so results are bit-identical
  * to the reference's own CUDA path compiled for sm_100a, not merely within tolerance.
  */
 #ifndef KLLM_B200_H_
@@ -141,7 +141,7 @@ int kllm_gemm_tf32(const float* x, const float* w, float* out, int n_tokens, int
                    void* stream);
 
 /* ---- tensor-parallel exchange --------------------------------------------------------------
- * Not in the reference (single GPU: llama3.cpp:118 pins device 0); SURVEY.md section 8e.  One
+ * Not in the reference (single GPU: llama3.cpp:118 pins device 0).  One
  * process per GPU; each owns a kllm_comm.  The decoder issues exactly two all-reduces per layer:
  * after o_proj (before the residual add of llama3.cpp:683-684) and after down_proj (:719).
  *   KLLM_COMM_PEER: one-shot all-reduce over NVLink peer memory (CUDA IPC), rank-ordered sum,
@@ -179,7 +179,7 @@ typedef struct {
   int32_t dim, hidden_dim, layer_num, head_num, kv_head_num, vocab_size, seq_len;
   int32_t flavour;     /* KLLM_FLAVOUR_* */
   int32_t group_size;  /* 0 = fp32 weights; 64 = export.py --version 3 int8 */
-  /* device pointers, reference checkpoint order (SURVEY.md Appendix A); per-layer arrays are
+  /* device pointers, reference checkpoint order; per-layer arrays are
    * HOST arrays of layer_num device pointers. */
   const float* tok_emb;               /* [vocab, dim] */
   const float* const* attn_norm;      /* [L] -> [dim] */

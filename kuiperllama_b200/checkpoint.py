@@ -1,5 +1,5 @@
 """Read/write KuiperLLama checkpoint files (the flat .bin formats the reference's exporters
-emit and its loader mmaps).  Layouts, exactly (SURVEY.md Appendix A):
+emit and its loader mmaps).  Layouts, exactly:
 
 fp32 v0   tools/export.py:79-131, read by llama3.cpp:290-423
   int32[7] dim, hidden_dim, n_layers, n_heads, n_kv_heads, +-vocab (negative = separate

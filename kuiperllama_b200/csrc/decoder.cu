@@ -149,7 +149,7 @@ std::vector<T> copy_ptrs(const T* src, int n) {
   return v;
 }
 
-// x += all-reduce(tp_tmp): the row-parallel matmul's partial sums meet here (SURVEY.md 8e)
+// x += all-reduce(tp_tmp): the row-parallel matmul's partial sums meet here
 int tp_reduce_into_x(kllm_decoder* dc, cudaStream_t s) {
   const kllm_decoder_desc& d = dc->d;
   if (d.comm != nullptr) return kllm_comm_allreduce_residual(d.comm, dc->tp_tmp, dc->x, dc->x, d.dim, s);

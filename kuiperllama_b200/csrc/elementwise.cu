@@ -3,7 +3,7 @@
 // Reference: kuiper/source/op/kernels/cuda/{rmsnorm,add,swiglu,rope,emb,argmax}_kernel.cu.
 // All are latency-bound (<= 600 KB touched); they exist for registry parity and for the
 // pieces the fused GEMV prologue/epilogues do not absorb.  Arithmetic order follows the
-// reference kernels bit for bit (DESIGN.md "Bit-exactness").
+// reference kernels bit for bit.
 #include <cuda_runtime.h>
 
 #include <cfloat>

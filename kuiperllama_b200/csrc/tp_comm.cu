@@ -1,5 +1,5 @@
 // Tensor-parallel exchange for the decode path: the all-reduce after o_proj and after down_proj
-// (SURVEY.md section 8e; the reference itself is single-GPU, llama3.cpp:118 pins device 0).
+// (the reference itself is single-GPU, llama3.cpp:118 pins device 0).
 //
 // One process per GPU.  Two transports behind one handle:
 //   * KLLM_COMM_PEER  one-shot all-reduce over NVLink peer memory (CUDA IPC): every rank stores

@@ -1,5 +1,5 @@
 """ctypes front-end of the device-resident decoder (``kllm_decoder_*``) plus synthetic
-random-init weights in the shapes BASELINE.json names.
+random-init weights in the shapes of the models that are benchmarked.
 
 torch is used here only as plumbing: device memory, RNG for the synthetic checkpoints and
 stream handles.  All compute on the decode path happens inside libkllm_b200.so.
@@ -41,7 +41,7 @@ class ModelShape:
         return self.head_num // self.kv_head_num
 
     def weight_bytes_per_token(self) -> int:
-        """ALGORITHMIC bytes one decode step must read (SURVEY.md section 8d): every matmul
+        """ALGORITHMIC bytes one decode step must read: every matmul
         weight once (+ int8 scales), the 2L+1 norm vectors, qkv biases and one embedding row."""
         d, h, L, kv, V = self.dim, self.hidden_dim, self.layer_num, self.kv_dim, self.vocab_size
         numel = L * (2 * d * d + 2 * kv * d + 3 * h * d) + V * d
@@ -56,7 +56,7 @@ class ModelShape:
 
 
 SHAPES = {
-    # BASELINE.json configs
+    # the benchmarked models
     "stories15m": ModelShape("stories15M-fp32", 288, 768, 6, 6, 6, 32000, 256, True),
     "tinyllama-1.1b": ModelShape("TinyLlama-1.1B-fp32", 2048, 5632, 22, 32, 4, 32000, 2048),
     "llama2-7b-int8": ModelShape("Llama-2-7B-int8-g64", 4096, 11008, 32, 32, 32, 32000, 2048,

@@ -1,4 +1,4 @@
-// Tensor parallelism for the C++ host side (SURVEY.md section 8e; not in the reference, which pins
+// Tensor parallelism for the C++ host side (not in the reference, which pins
 // device 0: kuiper/source/model/llama3.cpp:118).  One PROCESS per GPU, no torch, no MPI:
 //
 //   TpConfig       who this process is (world, rank, CUDA device) and where the ranks meet

@@ -9,7 +9,7 @@
 //   * GPT-2 byte <-> printable-character mapping, merges applied in rank order inside each piece;
 //   * added (special) tokens matched in the raw text first.
 // It follows the tokenizers these models ship with (validated against the `tokenizers` package in
-// tests/test_tokenizer.py), not the reference's " " -> "Ġ" pre-replacement (DESIGN.md section 9).
+// tests/test_tokenizer.py), not the reference's " " -> "Ġ" pre-replacement.
 #ifndef KLLM_KUIPER_OP_BYTE_BPE_H_
 #define KLLM_KUIPER_OP_BYTE_BPE_H_
 #include <cstdint>

@@ -252,7 +252,7 @@ void LLama2Model::create_param_quant_layers() {
   // A shared classifier cannot be expressed in this format: the exporter writes no int8 copy of
   // the embedding and the reference then reads the fp32 table as int8 (llama3.cpp:259-277).
   CHECK(!config_->is_shared_weight_)
-      << "int8 checkpoints with a shared classifier are not loadable (reference defect, see DESIGN.md)";
+      << "int8 checkpoints with a shared classifier are not loadable (the exporter writes no int8 copy of the embedding)";
   llama_layers_->cls_layer_ = quant_matmul(V, dim, 0, V, 0, dim);
 
   const float* f = static_cast<const float*>(raw_model_data_->weight(off));

@@ -1,4 +1,4 @@
-"""Tensor-parallel decode (SURVEY.md section 8e): heads and FFN columns sharded over N GPUs, one
+"""Tensor-parallel decode: heads and FFN columns sharded over N GPUs, one
 process per GPU, exactly two all-reduces per layer (after o_proj, after down_proj).
 
 The reference is single-GPU (llama3.cpp:118 pins device 0), so this file defines the sharding:

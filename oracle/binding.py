@@ -31,8 +31,7 @@ def build_oracle() -> Path:
 
 
 def build_ref(jobs: int = 8) -> bool:
-    """Compile oracle/_ref from /root/reference when that tree is present (build container);
-    on the GPU box the prebuilt .so files that travelled with the snapshot are used."""
+    """Compile oracle/_ref from the reference's tree when that is present; elsewhere .so files that were built before are used."""
     if not REFERENCE_TREE.is_dir() or not any(REFERENCE_TREE.iterdir()):  # no tree, or an empty one
         return REF_SO.exists()
     subprocess.check_call(["make", "-s", f"-j{jobs}", "-C", str(HERE), "ref"])
@@ -261,7 +260,7 @@ class RefCuda:
     def __init__(self, flavour="llama2"):
         so = REF_SO if flavour == "llama2" else REF_QWEN_SO
         if not so.exists():
-            raise FileNotFoundError(f"{so} not built (run `make -C oracle ref` where /root/reference exists)")
+            raise FileNotFoundError(f"{so} not built (run `make -C oracle ref` where the reference's tree is present)")
         L = ctypes.CDLL(str(so))
         vp = c_void_p
         L.kref_flavour.restype = c_char_p

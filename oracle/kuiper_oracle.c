@@ -1,7 +1,7 @@
 /* kuiper_oracle.c -- CPU restatement of the KuiperLLama decode hot path (see kuiper_oracle.h).
  *
  * TEST INFRASTRUCTURE ONLY: never linked into, loaded by, or called from the product library.
- * Citations are relative to /root/reference.
+ * Citations are relative to the reference's root.
  */
 #define _GNU_SOURCE
 #include "kuiper_oracle.h"
@@ -505,7 +505,7 @@ ko_model* ko_model_open(const char* path, int is_quant, int flavour) {
       KO_TAKE_Q(m->wcls, V, dim);
     } else {
       /* llama3.cpp:259-263: the reference points the int8 classifier at the fp32 embedding
-       * (a known defect, SURVEY.md 8c); shared-classifier int8 files are rejected here. */
+       * (a known defect); shared-classifier int8 files are rejected here. */
       fprintf(stderr, "ko_model_open: int8 + shared classifier is not supported\n");
       ko_model_close(m);
       return NULL;

@@ -4,14 +4,14 @@
  * --impl reference legs may build, load or call this.  The product library
  * (kuiperllama_b200/) never links it and has no CPU fallback.
  *
- * Every function restates one piece of /root/reference (paths relative to that root) in
+ * Every function restates one piece of the reference (paths relative to its root) in
  * plain C with fp32 arithmetic in the reference's CPU order.  The reference's CPU matmul
  * delegates to Armadillo 14.0.1 -> OpenBLAS sgemv (un-vendored, version unpinned;
  * kuiper/source/op/kernels/cpu/matmul_kernel.cpp:37-40), whose summation order is not part
  * of the reference; the restatement uses a strict left-to-right fp32 dot product
  * (KO_MATMUL_STRICT) and, for the timed baseline only, an optional BLAS/OpenMP path.
  *
- * Pinning (SURVEY.md section 8c): tests/test_oracle_golden.py checks this file against every
+ * Pinning: tests/test_oracle_golden.py checks this file against every
  * known-answer vector the reference's own tests hold for the path (test_load.cpp:102-105,
  * test_cu_matmul.cpp:55-75, test_cu_emb.cpp:28-57, test_cu_add.cpp:24) and against fixtures
  * produced by importing the reference's PyTorch model + exporter (tools/model.py,

@@ -1,6 +1,6 @@
 """Generate the golden fixtures in this directory by IMPORTING the reference's own PyTorch
 model and exporters (tools/model.py, tools/export.py, tools/model_qwen2.py,
-tools/export_qwen2.py) from /root/reference.  Run in the build container only:
+tools/export_qwen2.py) from its tree.  Run where that is present:
 
     python tests/golden/make_golden.py
 

@@ -28,7 +28,7 @@ def test_reference_arm_prints_one_contract_line():
     cb = d["cpu_baseline"]
     assert cb["kind"] == "port" and cb["cores"] >= 1 and cb["value"] == d["value"] and "stories15M" in cb["sample"]
     assert d["config"]["workload"].startswith("stories15M") and d["gpu_launches"] == 0
-    assert d["vs_baseline"] is None  # BASELINE.md publishes a number for TinyLlama-1.1B fp32 only
+    assert d["vs_baseline"] is None  # the reference publishes a number for TinyLlama-1.1B fp32 only
 
 
 def test_reference_arm_other_ranks_exit_quietly(monkeypatch):

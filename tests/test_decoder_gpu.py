@@ -1,8 +1,8 @@
 """-m gpu: the device-resident decoder (kllm_decoder_*) against
-  - the reference PyTorch logits committed under tests/golden (<= 1e-4, north-star tolerance),
+  - the reference PyTorch logits committed under tests/golden (<= 1e-4),
   - the CPU oracle (same tolerance, identical greedy ids),
   - the reference's OWN CUDA model path run on this GPU (oracle/_ref): bit-identical logits,
-    KV cache and token ids -- including at BASELINE.json's full TinyLlama-1.1B size."""
+    KV cache and token ids -- including at the full TinyLlama-1.1B size."""
 import ctypes
 import os
 
@@ -15,7 +15,7 @@ from gpu_util import assert_bit_equal, sync
 
 pytestmark = pytest.mark.gpu
 
-TOL = 1e-4  # logits within 1e-4 fp32
+TOL = 1e-4  # logits within 1e-4 in fp32
 
 
 @pytest.fixture(autouse=True, params=["persistent", "graph"])
@@ -181,7 +181,7 @@ def test_teacher_forced_generate_and_determinism(kllm_lib, engine):
 
 
 def test_tinyllama_full_size_identical_to_reference_cuda(kllm_lib, ref, tmp_path, engine):
-    """BASELINE.json config 2 at full size (dim 2048, 22 layers, 32/4 heads, vocab 32000):
+    """TinyLlama-1.1B fp32 at full size (dim 2048, 22 layers, 32/4 heads, vocab 32000):
     256 free-running greedy steps; ids, final logits and the KV cache must be identical to the
     reference's own CUDA path.  Then determinism over the full 1024-token run."""
     from kuiperllama_b200 import SHAPES, Decoder, synth_weights
@@ -262,7 +262,7 @@ def test_persistent_equals_graph_on_ring_stress_shapes(kllm_lib, monkeypatch, na
     b.close()
 
 
-# ---- BASELINE.json configs[2] and configs[3] at FULL size ------------------------------------------
+# ---- Llama-2-7B int8 and Qwen2.5-0.5B fp32 at FULL size -------------------------------------------
 _FULL_CACHE = {}
 
 
@@ -290,7 +290,7 @@ def _drop_full_size_files():
 
 
 def test_llama2_7b_int8_full_size_identical_to_reference_cuda(kllm_lib, ref, engine):
-    """BASELINE.json configs[2] at full size (dim 4096, 32 layers, MHA 32/32, hidden 11008, vocab
+    """Llama-2-7B int8 at full size (dim 4096, 32 layers, MHA 32/32, hidden 11008, vocab
     32000, int8 group 64 as export.py --version 3 writes it): 128 free-running greedy steps -- token
     ids AND the final logits bit-identical to the reference's own CUDA path loading the same file
     (llama3.cpp:184-288, matmul_kernel.cu:56-87)."""
@@ -316,10 +316,10 @@ def test_llama2_7b_int8_full_size_identical_to_reference_cuda(kllm_lib, ref, eng
 
 
 def test_qwen25_05b_full_size(kllm_lib, oracle, engine):
-    """BASELINE.json configs[3] at full size (dim 896, 24 layers, GQA 14/2 -> kv_mul 7, hidden 4864,
+    """Qwen2.5-0.5B fp32 at full size (dim 896, 24 layers, GQA 14/2 -> kv_mul 7, hidden 4864,
     vocab 151936 shared classifier, seq_len 32768, qkv bias, half-split RoPE theta 1e6, eps 1e-6).
     No reference CUDA *model* build exists for the QWEN2 flavour here (its tokenizer needs
-    absl/re2), so the whole-model check is the CPU oracle, teacher-forced, north-star tolerance:
+    absl/re2), so the whole-model check is the CPU oracle, teacher-forced, the same tolerance:
     logits within 1e-4 and the same greedy id wherever the top-2 margin exceeds 2e-4.  Both engines
     must then agree with EACH OTHER bit for bit over a long free-running decode (context 1 -> 1100),
     which carries the graph engine's kernel-level bit-exactness (test_kernels_gpu.py, QWEN2 kernels)
@@ -391,8 +391,8 @@ def test_prompt_call_equals_stepping(kllm_lib, key):
     ("small-int8", 64, None), ("small-tp-int8", 64, None), ("small-int8", 90, 8192),
     ("small", 150, 4096),        # fp32, head_size 32: 32-timestep tiles -> 5 tiles over 4 CTAs per head
     ("small-qwen", 120, 8192),   # qwen RoPE pairing, q/k/v biases; 32-timestep tiles, one CTA per head
-    ("tinyllama-1.1b", 700, None),  # BASELINE.json configs[1]: 128-timestep tiles, GQA 8:1
-    ("llama2-7b-int8", 200, None)])  # configs[2]: dp4a rows + 32-timestep tiles, 16 threads per timestep
+    ("tinyllama-1.1b", 700, None),  # 128-timestep tiles, GQA 8:1
+    ("llama2-7b-int8", 200, None)])  # dp4a rows + 32-timestep tiles, 16 threads per timestep
 def test_fast_numerics_within_north_star_tolerance(kllm_lib, monkeypatch, key, steps, stage_bytes):
     """numerics="fast" (persistent engine): int8 rows as 24-bit fixed-point activations x int8 weights
     on dp4a, attention as flash-decoding (split by timestep over several CTAs per head, online softmax,

@@ -1,8 +1,8 @@
 """-m gpu: every registry-level op of the C-ABI against
-  (a) the reference's OWN CUDA kernels (oracle/_ref, compiled from /root/reference for sm_100a):
-      BIT-EXACT -- the design contract (DESIGN.md "Bit-exactness");
+  (a) the reference's OWN CUDA kernels (oracle/_ref, compiled from its sources for sm_100a):
+      BIT-EXACT -- the design contract;
   (b) the CPU oracle: within fp32 reassociation tolerance (written at each assert).
-Shapes follow the reference's tests (test_cu_*.cpp) plus the model shapes of BASELINE.json."""
+Shapes follow the reference's tests (test_cu_*.cpp) plus the model shapes that are benchmarked."""
 import ctypes
 
 import numpy as np

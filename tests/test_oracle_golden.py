@@ -1,4 +1,4 @@
-"""Pin the CPU oracle (oracle/kuiper_oracle.c) before trusting it -- SURVEY.md section 8c.
+"""Pin the CPU oracle (oracle/kuiper_oracle.c) before trusting it.
 
 1. every known-answer vector the reference's own tests hold for the path;
 2. fixtures produced by importing the reference's PyTorch model + exporters
@@ -150,7 +150,7 @@ def test_checkpoint_writer_reproduces_exporter_bytes(tmp_path):
 def test_reference_orchestration_agrees_bitwise(oracle):
     from oracle.binding import REF_SO, RefCuda
     if not REF_SO.exists():
-        pytest.skip("oracle/_ref not built (needs /root/reference)")
+        pytest.skip("oracle/_ref not built (needs the reference's tree)")
     import ctypes
     ref = RefCuda("llama2")
     for name in ("tiny_llama2_fp32_shared", "tiny_llama2_fp32"):

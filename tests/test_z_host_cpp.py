@@ -2,7 +2,7 @@
 (File name: sorts after the kernel / decoder suites, whose parity results it builds on.)
 
 not gpu: it builds with CMake, the reference's demo/main.cpp and demo/main_qwen.cpp compile and
-         link against it UNCHANGED (when /root/reference is present), and it fails loudly without
+         link against it UNCHANGED (when the reference's tree is present), and it fails loudly without
          a GPU.
 gpu:     decoding through model::LLama2Model / Qwen2Model (the demo's embedding -> fill_input ->
          predict loop) reproduces the committed goldens and is bit-identical to the C-ABI decoder,
