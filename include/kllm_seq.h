@@ -376,8 +376,8 @@ int kllm_seq_gemm(int32_t dtype, const void* a, const void* w, float* out, int32
 
 /* Whether the products enqueued on `stream` through this library (kllm_seq_gemm, kllm_gemm_tf32) are complete: waits for the
  * stream, then returns KLLM_E_STATE if a bounded wait inside one of them ran out since the last report (its result is not
- * valid), else 0.  A later product on the same stream reports such a wait too, and leaves nothing to report here.  A captured
- * product reports under the stream it was captured on.  Engines and decoders report their own waits from their own calls. */
+ * valid), else 0.  A later product on the same stream reports such a wait too, and leaves nothing to report here.  What a captured
+ * product notes is reported by the next call of this function, whichever stream it is for.  Engines and decoders report their own waits from their own calls. */
 int kllm_product_status(void* stream);
 
 #ifdef __cplusplus

@@ -68,5 +68,5 @@ extern "C" int kllm_gemm_tf32(const float* x, const float* w, float* out, int n_
   int* const wait = kllm::stream_wait_flag(s);
   if (wait == nullptr) return KLLM_E_STATE;
   if (const int rc = kllm::prefill_product(x, w, nullptr, out, n_tokens, in_dim, out_dim, s, wait, false)) return rc;
-  return kllm::take_wait_flag(wait) ? KLLM_E_STATE : 0;
+  return kllm::take_own_wait_flag(wait) ? KLLM_E_STATE : 0;
 }

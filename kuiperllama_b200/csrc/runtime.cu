@@ -22,13 +22,15 @@ StreamWaitFlags& stream_flags() {
 }
 }  // namespace
 int* stream_wait_flag(cudaStream_t stream) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
-  if (cudaStreamGetId(stream, &id) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  return stream_flags().get(id);
+  if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone &&
+      cudaStreamGetId(stream, &id) == cudaSuccess)
+    return stream_flags().get(id);
+  cudaGetLastError();
+  return stream_flags().shared();
 }
+int take_own_wait_flag(int* flag) { return flag != stream_flags().shared() && take_wait_flag(flag); }
 }  // namespace kllm
 
 extern "C" {
@@ -49,7 +51,8 @@ const char* kllm_error_string(int code) {
 int kllm_product_status(void* stream) {
   const cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return static_cast<int>(e);
-  return kllm::take_wait_flag(kllm::stream_wait_flag(static_cast<cudaStream_t>(stream))) ? KLLM_E_STATE : 0;
+  const int own = kllm::take_wait_flag(kllm::stream_wait_flag(static_cast<cudaStream_t>(stream)));
+  return own | kllm::take_wait_flag(kllm::stream_flags().shared()) ? KLLM_E_STATE : 0;
 }
 
 uint64_t kllm_launch_count(void) { return kllm::launch_counter().load(); }

@@ -1289,5 +1289,5 @@ extern "C" int kllm_seq_gemm(int32_t dtype, const void* a, const void* w, float*
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   int* const wait = stream_wait_flag(s);  // (kernels that wait for nothing run without it)
   if (const int rc = gemm(dtype, a, w, out, n_tokens, in_dim, out_dim, s, wait, nullptr, false)) return rc;
-  return take_wait_flag(wait) ? KLLM_E_STATE : 0;
+  return take_own_wait_flag(wait) ? KLLM_E_STATE : 0;
 }

@@ -43,14 +43,15 @@ class WaitFlag {
   int* p_ = nullptr;
 };
 
-// One flag per stream, by the stream's id (unlike handles, ids are never used again).  The streams after the first kStreams share the
-// last flag: what one of them noted may then be reported for another, but never lost and never for one of the first.
+// One flag per stream, by the stream's id (unlike handles, ids are never used again).  A product that is captured cannot ask for the id
+// and runs on other streams anyway: captured products, and streams after the first kStreams, share one more flag, which is taken by
+// whoever asks for a status next.  What they noted is then never lost, and never taken for a wait of another stream's product.
 class StreamWaitFlags {
  public:
   static constexpr int kStreams = 1023;
   int* get(unsigned long long id) {
     std::lock_guard<std::mutex> lock(m_);
-    if (flags_ == nullptr && (flags_ = new_wait_flags(kStreams + 1)) == nullptr) return nullptr;  // tried again at the next call
+    if (!allocate()) return nullptr;
     const auto it = place_.find(id);
     if (it != place_.end()) return flags_ + it->second;
     const int n = static_cast<int>(place_.size());
@@ -59,13 +60,21 @@ class StreamWaitFlags {
     return flags_ + n;
   }
 
+  int* shared() {
+    std::lock_guard<std::mutex> lock(m_);
+    return allocate() ? flags_ + kStreams : nullptr;
+  }
+
  private:
+  bool allocate() { return flags_ != nullptr || (flags_ = new_wait_flags(kStreams + 1)) != nullptr; }  // (tried again at the next call)
   std::mutex m_;
   int* flags_ = nullptr;  // kept as long as the process runs: a kernel may still write there
   std::unordered_map<unsigned long long, int> place_;
 };
 
-// runtime.cu: the flag of a stream's own products; nullptr: no device or no memory
+// runtime.cu: where a product on `stream` notes a wait that ran out (nullptr: no device or no memory), and whether one is noted that
+// is certain to be this stream's (the shared flag is left to kllm_product_status)
 int* stream_wait_flag(cudaStream_t stream);
+int take_own_wait_flag(int* flag);
 
 }  // namespace kllm

@@ -1,5 +1,6 @@
 """Bounded waits that ran out reach their own engine, decoder or stream (csrc/wait_flag.h).  The host logic is compiled here against a
-few stand-ins for CUDA calls; on a GPU, products are captured by a process whose first product this is."""
+few stand-ins for CUDA calls; on a GPU, products are captured, also by a process whose first
+product this is."""
 import subprocess
 import sys
 import textwrap
@@ -55,6 +56,7 @@ int main() {
   assert(!take_wait_flag(s.get(8)) && take_wait_flag(s.get(7)) && !take_wait_flag(s.get(7)));
   // more streams than flags: the last ones share, and none of them touches an earlier one's
   for (unsigned long long id = 100; id < 100 + StreamWaitFlags::kStreams; ++id) assert(s.get(id));
+  assert(s.get(5000) == s.shared() && s.get(7) != s.shared());
   *s.get(5000) = 1;
   assert(s.get(5001) == s.get(5000) && s.get(7) == first);
   assert(!take_wait_flag(s.get(7)) && !take_wait_flag(s.get(100)) && take_wait_flag(s.get(5001)));
@@ -97,6 +99,11 @@ CAPTURE = textwrap.dedent("""
     if bf16: a, w = a.bfloat16(), w.bfloat16()
     out = torch.zeros(T, 384, device="cuda")
     p = lambda t: ctypes.c_void_p(t.data_ptr())
+    status = lambda: {status}
+    if {warm}:
+        assert lib.kllm_seq_gemm(sq.F32, p(w), p(w), p(out), 2, 256, 2, None) == 0 if "seq" in "{call}" else \
+            lib.kllm_gemm_tf32(p(w), p(w), p(out), 2, 256, 2, None) == 0
+        torch.cuda.synchronize()
     graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
     s.wait_stream(torch.cuda.current_stream())
     with torch.cuda.graph(graph, stream=s):
@@ -107,7 +114,7 @@ CAPTURE = textwrap.dedent("""
     torch.cuda.synchronize()
     ref = a.double() @ w.double().T
     assert ((out.double() - ref).norm() / ref.norm()).item() < 2e-3
-    assert {status} == 0
+    assert status() == 0
 """)
 SEQ = "lib.kllm_seq_gemm(sq.BF16 if bf16 else sq.F32, p(a), p(w), p(out), T, 256, 384, st)"
 TF32 = "lib.kllm_gemm_tf32(p(a), p(w), p(out), T, 256, 384, st)"
@@ -117,7 +124,8 @@ TF32 = "lib.kllm_gemm_tf32(p(a), p(w), p(out), T, 256, 384, st)"
 @pytest.mark.parametrize("lib,call,bf16,tokens", [("sq.load_seq_library()", SEQ, False, 4), ("sq.load_seq_library()", SEQ, True, 4),
                                                   ("sq.load_seq_library()", SEQ, False, 40), ("sq.load_seq_library()", SEQ, True, 40),
                                                   ("load_library()", TF32, False, 40)])
-def test_the_first_product_of_a_process_is_captured(lib, call, bf16, tokens):
+@pytest.mark.parametrize("warm", [False, True])
+def test_products_are_captured(lib, call, bf16, tokens, warm):
     status = "lib.kllm_product_status(st)" if "seq" in lib else "0"
-    code = CAPTURE.format(lib=lib, call=call, bf16=bf16, tokens=tokens, status=status)
+    code = CAPTURE.format(lib=lib, call=call, bf16=bf16, tokens=tokens, status=status, warm=warm)
     subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT, timeout=180)
