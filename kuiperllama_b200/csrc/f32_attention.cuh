@@ -11,6 +11,7 @@
 
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 
 namespace kllm {
 namespace f32attn {
@@ -119,6 +120,17 @@ __device__ __forceinline__ void attend(const Work& w, int dim, int vdim, float* 
         }
     }
     const bool whole = w.whole(tile);
+    // A key that a row does not see must not reach it, whatever its value holds, and 0 * inf is NaN: where a tile with hidden keys
+    // holds a value that is not finite, hidden weights (-0) leave those values out.
+    bool guarded = false;
+    if (!whole) {
+      bool odd = false;
+      for (int z = tid; z < kKeys * vc; z += kThreads) {
+        const float4 v = *reinterpret_cast<const float4*>(Vs + (stage * kKeys + z / vc) * LDV + z % vc * 4);
+        odd = odd || !(fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY);
+      }
+      guarded = __syncthreads_or(odd);
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       float m = r.m[i];
@@ -140,32 +152,37 @@ __device__ __forceinline__ void attend(const Work& w, int dim, int vdim, float* 
       for (int j = 0; j < 4; ++j) {
         const float p = expf(s[i][j] - sub);
         r.l[i] += p;
-        Ps[(ty + 16 * i) * LDP + tx + 16 * j] = p;
+        Ps[(ty + 16 * i) * LDP + tx + 16 * j] = s[i][j] > -INFINITY || s[i][j] != s[i][j] ? p : -0.f;
       }
     }
     __syncwarp();  // the rows of a warp's two ty are written and read by that warp alone
     const float* pp = Ps + ty * LDP;
     const float* vp = Vs + stage * kKeys * LDV + tx * 4;
+    auto add_values = [&](auto leave_out) {
 #pragma unroll 2
-    for (int j = 0; j < kKeys; j += 4) {
-      float4 p[4];
+      for (int j = 0; j < kKeys; j += 4) {
+        float4 p[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(pp + i * 16 * LDP + j);
+        for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(pp + i * 16 * LDP + j);
 #pragma unroll
-      for (int n = 0; n < NV; ++n)
+        for (int n = 0; n < NV; ++n)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float4 v = *reinterpret_cast<const float4*>(vp + (j + k) * LDV + n * 64);
+          for (int k = 0; k < 4; ++k) {
+            const float4 v = *reinterpret_cast<const float4*>(vp + (j + k) * LDV + n * 64);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float pk = k == 0 ? p[i].x : k == 1 ? p[i].y : k == 2 ? p[i].z : p[i].w;
-            r.o[i][n * 4] = fmaf(pk, v.x, r.o[i][n * 4]);
-            r.o[i][n * 4 + 1] = fmaf(pk, v.y, r.o[i][n * 4 + 1]);
-            r.o[i][n * 4 + 2] = fmaf(pk, v.z, r.o[i][n * 4 + 2]);
-            r.o[i][n * 4 + 3] = fmaf(pk, v.w, r.o[i][n * 4 + 3]);
+            for (int i = 0; i < 4; ++i) {
+              const float pk = k == 0 ? p[i].x : k == 1 ? p[i].y : k == 2 ? p[i].z : p[i].w;
+              if (decltype(leave_out)::value && __float_as_uint(pk) == 0x80000000u) continue;
+              r.o[i][n * 4] = fmaf(pk, v.x, r.o[i][n * 4]);
+              r.o[i][n * 4 + 1] = fmaf(pk, v.y, r.o[i][n * 4 + 1]);
+              r.o[i][n * 4 + 2] = fmaf(pk, v.z, r.o[i][n * 4 + 2]);
+              r.o[i][n * 4 + 3] = fmaf(pk, v.w, r.o[i][n * 4 + 3]);
+            }
           }
-        }
-    }
+      }
+    };
+    if (guarded) add_values(std::true_type{});
+    else add_values(std::false_type{});
     __syncthreads();  // the stage is loaded again two tiles on
   }
   r.finish();

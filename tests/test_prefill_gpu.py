@@ -95,3 +95,25 @@ def test_batched_prefill_refuses_int8(kllm_lib):
         dec.prefill_tf32([1, 2, 3])
     assert dec.prompt([1, 2, 3]) >= 0  # the bit-exact prompt path takes every checkpoint
     dec.close()
+
+
+@pytest.mark.parametrize("engine", ["persistent", "graph"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_token_does_not_reach_the_ones_before_it(kllm_lib, monkeypatch, engine, bad):
+    """The keys and values of the tokens ahead of one whose row is not finite are those of a prompt without it, bit for bit."""
+    from kuiperllama_b200 import SHAPES, Decoder, synth_weights
+    monkeypatch.setenv("KLLM_ENGINE", engine)
+    shape = SHAPES["small"]
+    w = synth_weights(shape, "cuda", 5)
+    w["tok_emb"] = w["tok_emb"].clone()
+    w["tok_emb"][7, 3] = bad
+    toks = [1] + [int(t) for t in np.random.default_rng(2).integers(8, shape.vocab_size, 69)]
+    dec = Decoder(shape, w)
+    dec.prefill_tf32(toks)
+    k0, v0 = dec.kv_cache()
+    toks[40] = 7
+    dec.prefill_tf32(toks)
+    k1, v1 = dec.kv_cache()
+    dec.close()
+    assert np.isfinite(k0[:, :70]).all() and not np.isfinite(v1[:, 40]).all()
+    assert np.array_equal(k0[:, :40], k1[:, :40]) and np.array_equal(v0[:, :40], v1[:, :40])
