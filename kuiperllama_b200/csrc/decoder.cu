@@ -541,6 +541,7 @@ int kllm_decoder_prefill_tf32(kllm_decoder* dc, const int32_t* tokens_host, int3
   m.bk = dc->bk.empty() ? nullptr : dc->bk.data();
   m.bv = dc->bv.empty() ? nullptr : dc->bv.data();
   m.key_cache = dc->kcache, m.value_cache = dc->vcache, m.sin_cache = dc->sin_t, m.cos_cache = dc->cos_t;
+  KLLM_TRY(prefill_takes(m, start_pos + n_tokens));
 
   std::memcpy(dc->io_host, tokens_host, sizeof(int32_t) * n_tokens);
   KLLM_TRY(cudaMemcpyAsync(dc->teacher, dc->io_host, sizeof(int32_t) * n_tokens, cudaMemcpyHostToDevice, dc->stream));

@@ -57,6 +57,9 @@ constexpr int kPrefillBlock = 1024;  // prompt positions per pass, at most
 struct PrefillWorkspace {  // [block, .] activations
   float *x, *xn, *q, *k, *v, *att, *h1;
 };
+// 0, or why prompts that end at `positions` cannot be taken in: their scores leave an SM's shared memory where heads are not of a size
+// that the tiled attention takes.  Asked before anything of a prompt is enqueued.
+int prefill_takes(const PrefillModel& m, int positions);
 // wait: where its products note a wait that ran out (wait_flag.h)
 int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* tokens_dev, int T, int start_pos,
                   cudaStream_t stream, int* wait);

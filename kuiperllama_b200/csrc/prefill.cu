@@ -243,9 +243,19 @@ static int attention_smem_opt_in(size_t bytes) {
   if (bytes <= 48 * 1024 || bytes <= configured) return 0;
   const cudaError_t e =
       cudaFuncSetAttribute(attn_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  if (e != cudaSuccess) return static_cast<int>(e);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // the refusal is this call's, not that of the next launch
+    return static_cast<int>(e);
+  }
   configured = bytes;
   return 0;
+}
+static CacheLayout cache_layout(const PrefillModel& m) {
+  return CacheLayout{m.mega_layout, m.seq_len, m.kv_head_num * m.head_size, m.head_size, m.attn_split > 0 ? m.attn_split : 1};
+}
+
+int prefill_takes(const PrefillModel& m, int positions) {
+  return attn_tile_usable(cache_layout(m)) ? 0 : attention_smem_opt_in(static_cast<size_t>(positions) * sizeof(float));
 }
 
 int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* tokens_dev, int T, int start_pos,
@@ -259,7 +269,7 @@ int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* to
   };
   embed_rows_kernel<<<T, 256, 0, s>>>(tokens_dev, m.tok_emb, ws.x, dim, m.vocab_size);
   PF_TRY(count());
-  const CacheLayout cl{m.mega_layout, m.seq_len, kvd, hs, m.attn_split > 0 ? m.attn_split : 1};
+  const CacheLayout cl = cache_layout(m);
   for (int l = 0; l < m.layer_num; ++l) {
     const size_t layer_off = static_cast<size_t>(l) * m.seq_len * kvd;
     rmsnorm_rows_kernel<<<T, 256, 0, s>>>(ws.x, m.attn_norm[l], ws.xn, dim, m.eps);
@@ -272,8 +282,7 @@ int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* to
     PF_TRY(count());
     const float *kc = m.key_cache + layer_off, *vc = m.value_cache + layer_off;
     if (!attn_tile_usable(cl)) {
-      const size_t sc_bytes = static_cast<size_t>(start_pos + T) * sizeof(float);
-      PF_TRY(attention_smem_opt_in(sc_bytes));
+      const size_t sc_bytes = static_cast<size_t>(start_pos + T) * sizeof(float);  // (allowed by prefill_takes)
       attn_rows_kernel<<<dim3(heads, T), 128, sc_bytes, s>>>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos);
     } else if (hs <= 64) {
       PF_TRY(launch_attn_tile<1>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos, T, s));

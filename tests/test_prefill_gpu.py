@@ -117,3 +117,20 @@ def test_a_token_does_not_reach_the_ones_before_it(kllm_lib, monkeypatch, engine
     dec.close()
     assert np.isfinite(k0[:, :70]).all() and not np.isfinite(v1[:, 40]).all()
     assert np.array_equal(k0[:, :40], k1[:, :40]) and np.array_equal(v0[:, :40], v1[:, :40])
+
+
+def test_a_refused_prompt_leaves_the_cache_alone(kllm_lib, monkeypatch):
+    """Heads of 160 coordinates keep a query's scores in shared memory, which 59003 positions do not fit."""
+    from kuiperllama_b200 import Decoder, KllmError, ModelShape, synth_weights
+    monkeypatch.setenv("KLLM_ENGINE", "graph")
+    shape = ModelShape("hs160", 160, 32, 1, 1, 1, 64, 60000)
+    dec = Decoder(shape, synth_weights(shape, "cuda", 3))
+    dec.prefill_tf32([5, 6, 7], start_pos=100)
+    before = dec.kv_cache()
+    with pytest.raises(KllmError):
+        dec.prefill_tf32([1, 2, 3], start_pos=59000)
+    after = dec.kv_cache()
+    assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(before, after))
+    dec.prefill_tf32([5, 6, 7], start_pos=100)  # and the next call is answered as before
+    assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(before, dec.kv_cache()))
+    dec.close()
