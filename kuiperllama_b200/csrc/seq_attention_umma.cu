@@ -95,10 +95,10 @@ template <int KC, int VC>
 __global__ void __launch_bounds__(kAttnUmmaThreads, 1)
 attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV kv, const int32_t* __restrict__ ent_first,
                       const int32_t* __restrict__ ent_count, const int32_t* __restrict__ ent_seq,
-                      const int32_t* __restrict__ ent_pos0, int splits, float* __restrict__ ws, const float* __restrict__ gates,
+                      const int32_t* __restrict__ ent_pos0, float* __restrict__ ws, const float* __restrict__ gates,
                       __nv_bfloat16* __restrict__ out, int* report) {
   using namespace umma;
-  const int e = blockIdx.x / a.kv_heads, g = blockIdx.x % a.kv_heads, split = blockIdx.z;
+  const int e = blockIdx.x / a.kv_heads, g = blockIdx.x % a.kv_heads;
   const int gv = g / v_share_of(a), rep = a.heads / a.kv_heads, dim = a.dim, vdim = a.vdim;
   const int first = ent_first[e], pos0 = ent_pos0[e], n_rows = ent_count[e] * rep;
   const int r0 = (gridDim.y - 1 - blockIdx.y) * kRows;  // the tiles with the most keys start first
@@ -106,15 +106,11 @@ attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV 
   const int pmax = pos0 + (min(r0 + kRows, n_rows) - 1) / rep;  // last position any row of the CTA sees
   const int groups = r0 + kTile < n_rows ? 2 : 1;
   // with a window or chunks no row sees anything before what the first row sees; tiles before that which hold kept
-  // first positions come ahead: this CTA's list of tiles is [0, keep_tiles) then [tile_first, last], cut into `splits` parts
+  // first positions come ahead: this CTA's list of tiles is [0, keep_tiles) then [tile_first, last]
   const int tile_first = first_seen(a, pos0 + r0 / rep) / kTile;
   const int keep_tiles = min(tile_first, (a.keep_first + kTile - 1) / kTile);
-  const int list_n = keep_tiles + pmax / kTile + 1 - tile_first, per = (list_n + splits - 1) / splits;
-  const int tile_lo = split * per, n = max(0, min(list_n, tile_lo + per) - tile_lo);
-  auto tile_of = [&](int i) {
-    const int li = tile_lo + i;
-    return li < keep_tiles ? li : tile_first + (li - keep_tiles);
-  };
+  const int n = keep_tiles + pmax / kTile + 1 - tile_first;
+  auto tile_of = [&](int i) { return i < keep_tiles ? i : tile_first + (i - keep_tiles); };
 
   extern __shared__ uint8_t raw_smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
@@ -214,7 +210,7 @@ attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV 
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == 12) {
     // ---- tensor core ----
-    if (lane == 0 && n > 0) {
+    if (lane == 0) {
       const uint32_t idesc_s = instr_desc(kTile), idesc_o = instr_desc((vdim + 15) / 16 * 16) | (1u << 16);
       const int ksteps = (dim + 15) / 16;
       auto scores = [&](int i, int grp) {  // over the weights of tile i - 1, which the product issued before reads
@@ -355,29 +351,22 @@ attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV 
       __syncwarp();
       if (lane == 0) arrive(&p_full[grp]);
     }
-    if (n > 0) {
-      ok = warp_wait(ok, smem_u32(&o_done[grp]), 0, stop);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    }
+    ok = warp_wait(ok, smem_u32(&o_done[grp]), 0, stop);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const size_t th = exists ? static_cast<size_t>(first + r / rep) * a.heads + g * rep + r % rep : 0;
-    const bool whole = splits == 1 && !a.no_merge, per_element = gates != nullptr && a.gate == KLLM_SEQ_GATE_ELEMENT;
+    const bool whole = !a.no_merge, per_element = gates != nullptr && a.gate == KLLM_SEQ_GATE_ELEMENT;
     if (whole && a.sink != nullptr && exists) {  // exp(sink) joins the denominator; scores are in units of log2
       l = m > -INFINITY ? l + ex2(a.sink[th % a.heads] * 1.4426950408889634f - m) : 1.0f;
     }
     const float inv = 1.0f / l;
     const float gate = whole && exists && gates && !per_element ? gates[th] : 1.0f;
-    float* part = ws + (th * splits + split) * (vdim + 2);
+    float* part = ws + th * (vdim + 2);
     if (!whole && exists && ok) part[0] = m * 0.6931471805599453f, part[1] = l;  // the merge works with natural logarithms
 #pragma unroll 1
     for (int c = 0; c < vdim; c += 16) {
       uint32_t o[16];
-      if (n > 0) {
-        tmem_ld16(output + c, o);
-        tmem_wait_ld();
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) o[j] = 0u;
-      }
+      tmem_ld16(output + c, o);
+      tmem_wait_ld();
       if (exists && ok) {
         const int here = min(16, vdim - c);  // 16 or 8
         if (whole) {
@@ -425,8 +414,8 @@ bool attention_umma_usable(int dtype, const AttnShape& a, int max_count) {
 
 template <int KC, int VC>
 static int launch_umma(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries, const int32_t* ent_first,
-                       const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0, int max_count, int splits, float* ws,
-                       void* out, int* report, cudaStream_t s) {
+                       const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0, int max_count, float* ws, void* out,
+                       int* report, cudaStream_t s) {
   static bool configured = false;
   if (!configured) {
     const cudaError_t e = cudaFuncSetAttribute(attention_umma_kernel<KC, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -435,20 +424,20 @@ static int launch_umma(const AttnShape& a, const void* q, const float* gates, co
     configured = true;
   }
   const int rep = a.heads / a.kv_heads;
-  const dim3 grid(n_entries * a.kv_heads, (max_count * rep + kRows - 1) / kRows, splits);
+  const dim3 grid(n_entries * a.kv_heads, (max_count * rep + kRows - 1) / kRows);
   if (grid.y > 65535u) return KLLM_E_UNSUPPORTED;
   attention_umma_kernel<KC, VC><<<grid, kAttnUmmaThreads, kAttnUmmaSmem, s>>>(
-      a, static_cast<const __nv_bfloat16*>(q), kv, ent_first, ent_count, ent_seq, ent_pos0, splits, ws, a.gate ? gates : nullptr,
+      a, static_cast<const __nv_bfloat16*>(q), kv, ent_first, ent_count, ent_seq, ent_pos0, ws, a.gate ? gates : nullptr,
       static_cast<__nv_bfloat16*>(out), report);
   count_launch();
   return cuda_rc(cudaGetLastError());
 }
 int launch_attention_umma(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
                           const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0,
-                          int max_count, int splits, float* ws, void* out, cudaStream_t s, int* report) {
+                          int max_count, float* ws, void* out, cudaStream_t s, int* report) {
   if (report == nullptr) return KLLM_E_STATE;
 #define KLLM_ATTN_UMMA(K, V) \
-  return launch_umma<K, V>(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, report, s)
+  return launch_umma<K, V>(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, ws, out, report, s)
   if (a.dim <= 64 && a.vdim <= 64) KLLM_ATTN_UMMA(8, 8);
   if (a.dim <= 64) KLLM_ATTN_UMMA(8, 16);
   if (a.vdim <= 64) KLLM_ATTN_UMMA(16, 8);

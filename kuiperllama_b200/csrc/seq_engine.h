@@ -204,11 +204,11 @@ bool attention_mma_usable(int dtype, const AttnShape& a, int max_count);
 int launch_attention_mma(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
                          const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq,
                          const int32_t* ent_pos0, int max_count, int splits, float* ws, void* out, cudaStream_t s);
-// the same on tcgen05, for long prompts (seq_attention_umma.cu); report: where a wait that ran out is noted (wait_flag.h)
+// the same on tcgen05, for long prompts, whose steps have CTAs enough without splitting keys (seq_attention_umma.cu); report: where a wait that ran out is noted (wait_flag.h)
 bool attention_umma_usable(int dtype, const AttnShape& a, int max_count);
 int launch_attention_umma(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
                           const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0,
-                          int max_count, int splits, float* ws, void* out, cudaStream_t s, int* report);
+                          int max_count, float* ws, void* out, cudaStream_t s, int* report);
 // the same to fp32 accuracy (seq_attention_f32.cu)
 bool attention_f32_usable(int dtype, const AttnShape& a, const PagedKV& kv, int max_count);
 int launch_attention_f32(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,

@@ -1736,10 +1736,9 @@ int launch_attention(int dtype, const AttnShape& a, const void* q, const float* 
   if (a.kv_heads <= 0 || a.heads % a.kv_heads != 0 || a.dim <= 0 || a.vdim <= 0) return KLLM_E_UNSUPPORTED;
   const int C = (a.vdim + kAttnKeys - 1) / kAttnKeys;
   int rc = 0;
-  if (attention_umma_usable(dtype, a, max_count)) {
-    rc = launch_attention_umma(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, s,
-                               report);
-    if (rc || (splits == 1 && !a.no_merge)) return rc;
+  if (splits == 1 && attention_umma_usable(dtype, a, max_count)) {
+    rc = launch_attention_umma(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, ws, out, s, report);
+    if (rc || !a.no_merge) return rc;
   } else if (attention_mma_usable(dtype, a, max_count)) {
     rc = launch_attention_mma(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws,
                               out, s);
