@@ -8,8 +8,8 @@
  * a token mixer and around a feed-forward, a schedule that may run a span of layers several times with the same
  * weights (each run with a cache of its own), so other model families can be described with the same pieces.
  *
- * Numerics.  compute type KLLM_SEQ_F32: every product to fp32 accuracy (fp32 multiply-adds, or operands as two TF32 parts
- * on the tensor cores, no further from the exact sum).  KLLM_SEQ_BF16: matrix products read bf16 weights
+ * Numerics.  compute type KLLM_SEQ_F32: every product to fp32 accuracy (fp32 multiply-adds, or all 24 bits of the operands as
+ * three bf16 parts on the tensor cores, no further from the exact sum).  KLLM_SEQ_BF16: matrix products read bf16 weights
  * and bf16 activations and accumulate in fp32; keys / values are cached in bf16.  In both, the residual stream, the
  * norms, attention scores and softmax weights, the router and all gates are fp32.
  *

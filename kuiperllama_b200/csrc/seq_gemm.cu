@@ -1,5 +1,5 @@
 // Matrix products of the sequence-batch engine:  out[T, N] (fp32) = a[T, K] . w[N, K]^T, a and w in the compute type
-// (float: fp32 accuracy -- multiply-adds, or tensor-core products of operands in two TF32 parts; __nv_bfloat16: bf16 operands,
+// (float: fp32 accuracy -- multiply-adds, or tensor-core products of operands in three bf16 parts; __nv_bfloat16: bf16 operands,
 // fp32 accumulation).
 //
 //   rows_kernel     T <= 8 (decode steps): the weights are streamed once, a warp per output feature, all rows of `a`
@@ -10,7 +10,7 @@
 //   umma_kernel     bf16, T > 8, K % 8 == 0: 128 weight rows x BN tokens per CTA on tcgen05.mma (kind::f16, operands
 //                   by TMA with 128-byte swizzle, accumulator in TMEM)                      [seq_gemm_umma.cuh]
 //   umma_split_kernel  the same where the tiles are fewer than the SMs: K split over a cluster; fp32 with T > 8 and
-//                   K % 4 == 0, each operand as two TF32 parts                              [seq_gemm_split.cuh]
+//                   K % 4 == 0, each operand as three bf16 parts                              [seq_gemm_split.cuh]
 //   grouped_kernel  the tiled kernel over row blocks that each belong to one expert (rows gathered by index, the
 //                   SiLU-gate product as an optional epilogue)
 #include <cuda_bf16.h>

@@ -3,10 +3,13 @@
 //
 //   kBf16    bf16 operands
 //   kTf32    fp32 operands read as TF32 (10 mantissa bits): the toleranced prompt path of the single-sequence decoder
-//   kFp32    fp32 operands, products to fp32 accuracy: every operand is hi + lo, hi its leading 11 bits and lo the rest rounded
-//            to 11 bits, and a . w = hi hi + (lo hi + hi lo); what is left out (lo lo, lo's rounding) is below 2^-20 of the
-//            product.  hi is the operand as it arrived -- kind::tf32 reads 11 bits of it, truncating --, four warps write lo
-//            beside it between the tile's arrival and its use.
+//   kFp32    fp32 operands, all 24 bits of them: every operand is h + m + l, three bf16 numbers, h the operand rounded to nearest, m
+//            the rest rounded, l what is left of it, exactly; a . w = h h + (h m + m h + m m + h l + l h).  What is left out (m l,
+//            l m, l l) is at most about 2^-24 of the product, and nothing where one side fits in 8 bits or both in 16.  Six warps
+//            replace a tile's rows by their parts between the tile's arrival and its use.  Rows that hold an infinity, a NaN or a
+//            number whose parts would leave bf16's range (below 2^-100, or rounding up to infinity) are summed by multiply-adds.
+//            (Two TF32 parts and three products, 517 x 1024 x 3072 in 38.9 us, hold 22 bits of an operand: 2.9e-7, and further off
+//            than multiply-adds at K = 32 and 64.)
 //
 // What bounds it: with a few dozen tokens the weights are read once and every element of them feeds 2 * T multiply-adds, so
 // the time is the weights' way from HBM.  A tile per 128 features leaves most SMs without work (width 4096: 32 tiles), and
@@ -14,22 +17,23 @@
 // the large form over its part of K, leaves its partial tile in its own shared memory, and after a cluster barrier every
 // CTA sums BN / S of the tile's tokens over the S partials, read through distributed shared memory in rank order (the
 // result does not depend on timing).  kFp32 on token blocks is bound by shared memory instead: a stage is read by the splitting
-// warps and its lo part written (64 KB at BN = 128), and the MMAs read it three times over (96 KB).
+// warps and its parts written (80 KB at BN = 128), and the MMAs read twelve parts of it (96 KB).
 //
 // Precision: a tcgen05 accumulator is not rounded to nearest at each of its steps, and its error grows with their number.  A
 // CTA hands its accumulator over every SECTION blocks of K to the epilogue warps, which sum the sections in fp32 registers
-// while the tensor core fills the other accumulator.  kFp32 keeps the two small products in an accumulator of their own.
+// while the tensor core fills the other accumulator.  kFp32 keeps the five small products in an accumulator of their own.
 //
 // Gated: as in umma_kernel a tile is 64 features, their gate rows above their up rows; the two meet in the partial tile.
 //
 // Measured, calls back to back with weights from HBM (one B200), the FMA tiles that these shapes took before -> now; error
 // against 64 bits in the 2-norm:
 //   bf16  T = 40, K = 4096, N = 4096    298 -> 14.6 us    6.1e-7 -> 1.4e-7
-//   bf16  T = 24, K = 2048, N = 2048    149 -> 10.4 us    3.9e-7 -> 1.3e-7
+//   bf16  T = 24, K = 2048, N = 2048    149 -> 10.0 us    3.9e-7 -> 1.3e-7
 //   bf16  T = 24, K = 2048, N = 32000   382 -> 28.8 us    3.9e-7 -> 1.4e-7
-//   fp32  T = 16, K = 2048, N = 2048    158 -> 17.7 us    8.1e-7 -> 2.9e-7
-//   fp32  T = 64, K = 4096, N = 4096    314 -> 39.1 us    1.1e-6 -> 2.9e-7
-//   fp32  T = 517, K = 1024, N = 3072   161 -> 47.2 us    5.7e-7 -> 2.9e-7
+//   fp32  T = 16, K = 2048, N = 2048    158 -> 18.8 us    8.1e-7 -> 9.8e-8
+//   fp32  T = 64, K = 4096, N = 4096    314 -> 37.3 us    1.1e-6 -> 1.1e-7
+//   fp32  T = 517, K = 1024, N = 3072   161 -> 47.3 us    5.7e-7 -> 9.4e-8
+//   fp32  T = 9 .. 200, K = 32 and 64                     1.0e-7 -> 4.6e-8, 1.4e-7 -> 7.0e-8
 #pragma once
 #include "seq_gemm_umma.cuh"
 #include "seq_launch.cuh"
@@ -63,13 +67,61 @@ __device__ __forceinline__ float ld_peer(uint32_t addr) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
   return v;
 }
-// x - hi, hi being what kind::tf32 reads of x: sign, exponent and ten mantissa bits, never rounded up, so it cannot overflow.  The
-// difference is exact and holds 13 bits; half of the 11th one's unit is added to its magnitude, so that reading it in the same way
-// rounds it to nearest.  An infinity has no such form (inf - inf): `check` becomes NaN for it, as for a NaN.
-__device__ __forceinline__ float low_part(float x, float& check) {
-  const float lo = x - __uint_as_float(__float_as_uint(x) & 0xffffe000u);
-  check = fmaf(lo, 0.f, check);
-  return __uint_as_float(__float_as_uint(lo) + 0x1000u);
+// kFp32: a tile's rows of 32 fp32 elements (128 bytes) become rows of 64 bf16 elements in the same place, h of the 32 and then m of the
+// 32, in the layout that TMA left, 16-byte chunk c of row r at c ^ (r & 7); l goes to a second tile of 64-byte rows, chunk c at
+// c ^ (r >> 1 & 3) (the 64-byte swizzle).  A warp takes 8 rows at once, four lanes to a row: lane j reads chunks 2 j and 2 j + 1 and
+// writes chunks j, 4 + j and j.  The rows of a quarter warp are p and p ^ 5: their reads, and the writes to either tile, fall on eight
+// different chunks of 128 bytes.
+__device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+struct RowCheck {  // what a lane has seen of one row
+  float finite = 0.f;         // NaN once a rest was: infinities, NaN, numbers that round up to infinity
+  uint32_t small = ~0u;       // the smallest magnitude other than 0, as 2 * bits - 1 (0 comes out as the largest)
+  __device__ __forceinline__ bool special() const { return finite != finite || small < (27u << 24) - 1u; }  // below 2^-100
+};
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l, RowCheck& check) {
+  check.small = min(check.small, min(2u * __float_as_uint(x) - 1u, 2u * __float_as_uint(y) - 1u));
+  h = pack_bf16(x, y);
+  x -= __uint_as_float(h << 16), y -= __uint_as_float(h & 0xffff0000u);  // a bf16 is the top half of a float
+  check.finite = fmaf(x, 0.f, fmaf(y, 0.f, check.finite));
+  m = pack_bf16(x, y);
+  l = pack_bf16(x - __uint_as_float(m << 16), y - __uint_as_float(m & 0xffff0000u));
+}
+// Six warps do it (64 x 4096 x 4096 37.2 us, four 41.1; 517 x 1024 x 3072 49.4 and 51.5); more leave the epilogue too few registers.
+constexpr int kSplitWarps = 6;
+template <int ROWS>
+constexpr int kSplitGroups = (ROWS / 8 + kSplitWarps - 1) / kSplitWarps;  // of 8 rows each, that a warp takes
+// the row of group i that this lane of splitting warp `warp` shares, its last three bits in r8
+__device__ __forceinline__ int split_row(int i, int warp, int r8) { return (i * kSplitWarps + warp) * 8 + r8; }
+__device__ __forceinline__ int split_r8(int lane) { return (lane >> 3) ^ (lane & 4 ? 5 : 0); }
+template <int ROWS>
+__device__ __forceinline__ void split_tile(uint8_t* tile, uint8_t* rest, int warp, int lane, RowCheck (&check)[kSplitGroups<ROWS>]) {
+  constexpr int N = kSplitGroups<ROWS>;
+  const int j = lane & 3, r8 = split_r8(lane);
+  auto in = [&](int i) { return (ROWS / 8) % kSplitWarps == 0 || i + 1 < N || split_row(i, warp, 0) < ROWS; };  // the same for a warp
+  float4 u[N], v[N];  // everything is read before anything is written: one latency for the tile
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (in(i)) {
+      const float4* src = reinterpret_cast<const float4*>(tile + split_row(i, warp, r8) * 128);
+      u[i] = src[(2 * j) ^ r8], v[i] = src[(2 * j + 1) ^ r8];
+    }
+  __syncwarp();  // a row has been read by its four lanes
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (in(i)) {
+      uint4 h, m, l;
+      split_pair(u[i].x, u[i].y, h.x, m.x, l.x, check[i]);
+      split_pair(u[i].z, u[i].w, h.y, m.y, l.y, check[i]);
+      split_pair(v[i].x, v[i].y, h.z, m.z, l.z, check[i]);
+      split_pair(v[i].z, v[i].w, h.w, m.w, l.w, check[i]);
+      uint4* dst = reinterpret_cast<uint4*>(tile + split_row(i, warp, r8) * 128);
+      dst[j ^ r8] = h;
+      dst[(4 + j) ^ r8] = m;
+      reinterpret_cast<uint4*>(rest + split_row(i, warp, r8) * 64)[j ^ (r8 >> 1)] = l;
+    }
 }
 
 // This CTA's tokens of the tile, summed over the cluster's S partial tiles in rank order: column rank * BN / S + j for the j that
@@ -114,11 +166,20 @@ __device__ __forceinline__ void split_reduce(const SplitArgs& p, const float* pa
 }
 
 template <int MODE>
-constexpr int split_threads() { return MODE == kFp32 ? THREADS + 128 : THREADS; }
+constexpr int split_threads() { return MODE == kFp32 ? THREADS + kSplitWarps * 32 : THREADS; }
 
 // grid: (feature tiles, S, token tiles), clusters of (1, S, 1)
+template <int MODE, int BN>
+constexpr int kSplitStage = (A_BYTES + BN * 128) * (MODE == kFp32 ? 3 : 2) / 2;  // bytes
+template <int MODE, int BN, int ST>
+constexpr size_t split_smem() {
+  return 1024 + static_cast<size_t>(ST) * kSplitStage<MODE, BN> + 256 +
+         (MODE == kFp32 ? (BM + BN) * sizeof(float) : 0);
+}
+template <int MODE, int BN, int ST>
+constexpr int split_ctas_per_sm() { return split_smem<MODE, BN, ST>() <= 113 * 1024 ? 2 : 1; }
 template <int MODE, int BN, int OUT, int ST>
-__global__ void __launch_bounds__(split_threads<MODE>())
+__global__ void __launch_bounds__(split_threads<MODE>(), split_ctas_per_sm<MODE, BN, ST>())
 umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
                   const __grid_constant__ CUtensorMap map_a, const SplitArgs p) {
   using M = ModeOf<MODE>;
@@ -126,7 +187,8 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   constexpr int FEATURES = two ? BM / 2 : BM;
   constexpr int W_BYTES = A_BYTES, B_BYTES = BN * 128;
   constexpr int HALF = W_BYTES + B_BYTES;                  // the tiles as they arrive
-  constexpr int STAGE = MODE == kFp32 ? 2 * HALF : HALF;   // kFp32: the lo parts follow
+  constexpr int STAGE = kSplitStage<MODE, BN>;           // kFp32: h and m take the tiles' place, l follows
+  constexpr int ROWS = BM + BN;                            // of both tiles
   constexpr int TILE_COLS = BN;                            // of one sum
   constexpr int ACC_COLS = MODE == kFp32 ? 2 * TILE_COLS : TILE_COLS;  // of one accumulator; there are two
   constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
@@ -137,12 +199,14 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(base + ST * STAGE);
   uint64_t* empty = full + ST;
-  uint64_t* split_done = empty + ST;      // kFp32: the stage holds the lo parts too
+  uint64_t* split_done = empty + ST;      // kFp32: the stage holds the parts
   uint64_t* acc_full = split_done + ST;   // [2]
   uint64_t* acc_empty = acc_full + 2;     // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), p.report};
-  float* special = reinterpret_cast<float*>(tmem_slot + 2);  // kFp32: != 0 when an operand of this CTA's part of K is not finite
+  // kFp32: != 0 when this CTA's part of K has a number that its parts do not hold, and in which rows (weights, then tokens)
+  float* special = reinterpret_cast<float*>(tmem_slot + 2);
+  float* special_row = special + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * FEATURES, t0 = blockIdx.z * BN;
@@ -156,7 +220,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     for (int s = 0; s < ST; ++s) {
       mbar_init(smem_u32(&full[s]), 1);
       mbar_init(smem_u32(&empty[s]), 1);
-      mbar_init(smem_u32(&split_done[s]), 4);
+      mbar_init(smem_u32(&split_done[s]), kSplitWarps);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&acc_full[b]), 1);
@@ -166,6 +230,8 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     *special = 0.f;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (MODE == kFp32)
+    for (int i = threadIdx.x; i < ROWS; i += blockDim.x) special_row[i] = 0.f;
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(TMEM_COLS) : "memory");
@@ -200,7 +266,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc = MODE == kBf16 ? instr_desc(BN) : instr_desc_tf32(BN);
+      const uint32_t idesc = MODE == kTf32 ? instr_desc_tf32(BN) : instr_desc(BN);
       uint64_t* ready = MODE == kFp32 ? split_done : full;
       bool ok = true;
       for (int i = 0; i < blocks && ok; ++i) {
@@ -213,17 +279,22 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const uint32_t st = smem_u32(base + s * STAGE);
         const uint32_t d = tmem_d + b * ACC_COLS;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {  // 32 bytes of K per instruction, inside the swizzle row
+        for (int k = 0; k < (MODE == kFp32 ? 2 : 4); ++k) {  // 32 bytes of K per instruction, inside the swizzle row
           const uint32_t joins = (!opens || k > 0) ? 1u : 0u;
           const uint64_t wd = smem_desc(st + k * 32), ad = smem_desc(st + W_BYTES + k * 32);
           if constexpr (MODE == kBf16) {
             mma_bf16(d, wd, ad, idesc, joins);
-          } else {
+          } else if constexpr (MODE == kTf32) {
             mma_tf32(d, wd, ad, idesc, joins);
-            if constexpr (MODE == kFp32) {
-              mma_tf32(d + TILE_COLS, smem_desc(st + HALF + k * 32), ad, idesc, joins);
-              mma_tf32(d + TILE_COLS, wd, smem_desc(st + HALF + W_BYTES + k * 32), idesc, 1u);
-            }
+          } else {
+            const uint64_t wm = smem_desc(st + 64 + k * 32), am = smem_desc(st + W_BYTES + 64 + k * 32);
+            const uint64_t wl = smem_desc_64(st + HALF + k * 32), al = smem_desc_64(st + HALF + W_BYTES / 2 + k * 32);
+            mma_bf16(d, wd, ad, idesc, joins);
+            mma_bf16(d + TILE_COLS, wl, ad, idesc, joins);
+            mma_bf16(d + TILE_COLS, wd, al, idesc, 1u);
+            mma_bf16(d + TILE_COLS, wm, am, idesc, 1u);
+            mma_bf16(d + TILE_COLS, wm, ad, idesc, 1u);
+            mma_bf16(d + TILE_COLS, wd, am, idesc, 1u);
           }
         }
         mma_commit(smem_u32(&empty[s]));
@@ -231,23 +302,21 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       }
     }
   } else if (MODE == kFp32 && warp >= 6) {
-    // the splitting warps: both parts keep the tile's layout, so the swizzle needs no thought
-    float check = 0.f;
+    // the splitting warps; a lane's rows are the same in every block of K
+    RowCheck check[kSplitGroups<ROWS>];
     for (int i = 0; i < blocks; ++i) {
       const int s = i % ST;
       if (!warp_wait(true, smem_u32(&full[s]), (i / ST) & 1, stop)) break;
-      const float4* tile = reinterpret_cast<const float4*>(base + s * STAGE);
-      float4* lo = reinterpret_cast<float4*>(base + s * STAGE + HALF);
-#pragma unroll 8
-      for (int v = threadIdx.x - 192; v < HALF / 16; v += 128) {
-        const float4 x = tile[v];
-        lo[v] = make_float4(low_part(x.x, check), low_part(x.y, check), low_part(x.z, check), low_part(x.w, check));
-      }
+      split_tile<ROWS>(base + s * STAGE, base + s * STAGE + HALF, warp - 6, lane, check);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read what was written here
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&split_done[s])) : "memory");
     }
-    if (check != check) *special = 1.f;
+#pragma unroll
+    for (int i = 0; i < kSplitGroups<ROWS>; ++i) {
+      const int row = split_row(i, warp - 6, split_r8(lane));
+      if (row < ROWS && check[i].special()) special_row[row] = 1.f, *special = 1.f;
+    }
   }
   const int quarter = warp & 3, mine = quarter * 32 + lane;  // the tile row of a thread of the epilogue warps 2 .. 5
   const bool epilogue = warp >= 2 && warp < 6;
@@ -289,27 +358,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   if (S > 1) cluster_sync();  // every partial tile of the cluster is in place
   else if (two || MODE == kFp32) __syncthreads();  // the partial tile is, and `special`
   if (epilogue && ok) {
-    bool recompute = false;
-    if constexpr (MODE == kFp32) {
-      for (int q = 0; q < S; ++q)
-        recompute = recompute || (S > 1 ? ld_peer(peer_smem(smem_u32(special), q)) : *special) != 0.f;
-    }
-    if (MODE == kFp32 && recompute) {  // infinities, NaN: the sums as a chain of fp32 multiply-adds gives them
-      const int per = BN / S, row = n0 + mine;
-      if (mine < FEATURES && row < p.N) {
-        for (int j = rank * per; j < (rank + 1) * per && t0 + j < p.T; ++j) {
-          const float* ar = static_cast<const float*>(p.a) + static_cast<size_t>(t0 + j) * p.K;
-          const float* wr = static_cast<const float*>(p.w) + static_cast<size_t>(row) * p.K;
-          const float* wr2 = two ? static_cast<const float*>(p.w2) + static_cast<size_t>(row) * p.K : wr;
-          float v = 0.f, u = 0.f;
-          for (int k = 0; k < p.K; ++k) {
-            v = fmaf(ar[k], wr[k], v);
-            if (two) u = fmaf(ar[k], wr2[k], u);
-          }
-          split_store<MODE, OUT>(p, t0 + j, row, v, u);
-        }
-      }
-    } else if (!two && S == 1) {
+    if (!two && S == 1) {
       if (n0 + mine < p.N) {
 #pragma unroll
         for (int j = 0; j < BN; ++j)
@@ -320,6 +369,32 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       else if (S == 4) split_reduce<MODE, BN, OUT, 4>(p, part, rank, t0, n0, mine);
       else if (S == 2) split_reduce<MODE, BN, OUT, 2>(p, part, rank, t0, n0, mine);
       else if constexpr (two) split_reduce<MODE, BN, OUT, 1>(p, part, rank, t0, n0, mine);
+    }
+    if constexpr (MODE == kFp32) {
+      static_assert(OUT != kAdd, "an output is stored again here");
+      auto noted = [&](const float* at) {
+        bool any = false;
+        for (int q = 0; q < S; ++q) any = any || (S > 1 ? ld_peer(peer_smem(smem_u32(at), q)) : *at) != 0.f;
+        return any;
+      };
+      // outputs of rows that their parts do not hold: the sums as a chain of fp32 multiply-adds gives them, by the threads that
+      // stored what the parts gave
+      const int feature = mine % FEATURES, row = n0 + feature;
+      if (noted(special) && row < p.N) {
+        const bool weights = noted(special_row + feature) || (two && noted(special_row + FEATURES + feature));
+        const float* wr = static_cast<const float*>(p.w) + static_cast<size_t>(row) * p.K;
+        const float* wr2 = two ? static_cast<const float*>(p.w2) + static_cast<size_t>(row) * p.K : wr;
+        for (int j = rank * (BN / S) + (two ? mine / FEATURES : 0); j < (rank + 1) * (BN / S) && t0 + j < p.T; j += two ? 2 : 1) {
+          if (!weights && !noted(special_row + BM + j)) continue;
+          const float* ar = static_cast<const float*>(p.a) + static_cast<size_t>(t0 + j) * p.K;
+          float v = 0.f, u = 0.f;
+          for (int k = 0; k < p.K; ++k) {
+            v = fmaf(ar[k], wr[k], v);
+            if (two) u = fmaf(ar[k], wr2[k], u);
+          }
+          split_store<MODE, OUT>(p, t0 + j, row, v, u);
+        }
+      }
     }
   }
   __syncwarp();
@@ -354,7 +429,7 @@ inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
   if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, FEATURES)) return rc;
   if (int rc = make_map_of<MODE>(&map_w2, two ? p.w2 : p.w, p.N, p.K, FEATURES)) return rc;
   if (int rc = make_map_of<MODE>(&map_a, p.a, p.T, p.K, BN)) return rc;
-  constexpr size_t smem = 1024 + static_cast<size_t>(ST) * (MODE == kFp32 ? 2 : 1) * (A_BYTES + BN * 128) + 256;
+  constexpr size_t smem = split_smem<MODE, BN, ST>();
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kernel = umma_split_kernel<MODE, BN, OUT, ST>;
   static bool configured = false;
@@ -364,7 +439,7 @@ inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
     configured = true;
   }
   const int feature_tiles = (p.N + FEATURES - 1) / FEATURES, token_tiles = (p.T + BN - 1) / BN;
-  p.S = split_count(feature_tiles * token_tiles, (p.K + ModeOf<MODE>::BKE - 1) / ModeOf<MODE>::BKE, (smem <= 113 * 1024 ? 2 : 1) * kSms);
+  p.S = split_count(feature_tiles * token_tiles, (p.K + ModeOf<MODE>::BKE - 1) / ModeOf<MODE>::BKE, split_ctas_per_sm<MODE, BN, ST>() * kSms);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(feature_tiles, p.S, token_tiles);
   cfg.blockDim = dim3(split_threads<MODE>());
@@ -406,10 +481,10 @@ int launch_fp32(const float* a, const float* w, const float* bias, float* out, i
                 cudaStream_t s, int* report, bool ahead) {
   const SplitArgs p{a, w, w + static_cast<size_t>(N) * K, bias, nullptr, out, T, N, K, 1, act, report};
   constexpr int OUT = GATED ? kGated : kPlain;
-  if (T <= 16) return launch_split<kFp32, 16, OUT, 3>(p, s, ahead);
-  if (T <= 32) return launch_split<kFp32, 32, OUT, 3>(p, s, ahead);
-  if (T <= 64) return launch_split<kFp32, 64, OUT, 4>(p, s, ahead);
-  return launch_split<kFp32, 128, OUT, 3>(p, s, ahead);
+  if (T <= 16) return launch_split<kFp32, 16, OUT, 4>(p, s, ahead);
+  if (T <= 32) return launch_split<kFp32, 32, OUT, 6>(p, s, ahead);
+  if (T <= 64) return launch_split<kFp32, 64, OUT, 6>(p, s, ahead);
+  return launch_split<kFp32, 128, OUT, 4>(p, s, ahead);
 }
 
 }  // namespace umma

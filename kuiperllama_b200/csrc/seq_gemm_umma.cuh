@@ -85,6 +85,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
   return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
+// the same with the 64-byte swizzle: 8 rows x 64 B = 512 B, SWIZZLE_64B = 4
+__device__ __forceinline__ uint64_t smem_desc_64(uint32_t saddr) {
+  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61);
+}
 // instruction descriptor: D = F32 (1 << 4), A = B = BF16 (1 << 7, 1 << 10), both K-major, N >> 3 in [17,23), M >> 4 in
 // [24,29)
 __device__ __forceinline__ uint32_t instr_desc(int n) {
@@ -100,7 +104,7 @@ enum Mode { kBf16 = 0, kTf32 = 1, kFp32 = 2 };
 template <int MODE> struct ModeOf {  // fp32 operands
   using T = float;
   static constexpr int BKE = 32;     // elements of K per 128-byte block
-  static constexpr int SECTION = 2;  // blocks between two hand-overs of the accumulator: 8 steps
+  static constexpr int SECTION = 2;  // blocks between two hand-overs of the accumulator: 4 steps of the large products
 };
 template <> struct ModeOf<kTf32> {
   using T = float;
@@ -157,7 +161,7 @@ enum Out {
   kAdd = 2     // out = add + sum (fp32; add may be out itself)
 };
 
-// operand pointers (kFp32's fallback for infinities reads through them) and what joins the sums
+// operand pointers (kFp32 sums rows that hold infinities through them) and what joins the sums
 struct SplitArgs {
   const void *a, *w, *w2;
   const float* bias;

@@ -54,8 +54,8 @@ def test_split_product_repeats():
     (9, 32, 8), (16, 36, 128), (17, 100, 129), (32, 2048, 300), (33, 1028, 640), (64, 4096, 1000), (65, 288, 96),
     (128, 512, 2047), (129, 1024, 1024), (517, 1024, 513)])
 def test_split_product_fp32(T, K, N):
-    """fp32 operands as two TF32 parts: left out are products of two low parts (2^-20 of the product at most) and the low
-    parts' rounding (2^-22 each); with the sums' 2^-20 an element stays within 2^-18 of the sum of the products' magnitudes."""
+    """fp32 operands as three bf16 parts: left out are products of small parts (2^-24 of the product at most); with the sums' 2^-20 an
+    element stays within 2^-18 of the sum of the products' magnitudes."""
     a, w, out = product(T, K, N, T * 5 + K, bf16=False)
     bound = 2.0 ** -18 * (a.abs() @ w.abs().T)
     assert ((out[:T].double() - a @ w.T).abs() <= bound).all()
@@ -64,7 +64,7 @@ def test_split_product_fp32(T, K, N):
 
 @pytest.mark.parametrize("T", [12, 40, 200])
 def test_split_product_fp32_keeps_infinities_and_nans(T):
-    """An infinity has no low part: such tiles are summed by multiply-adds, so inf stays inf and only inf * 0, inf - inf and NaN
+    """An infinity has no parts: such rows are summed by multiply-adds, so inf stays inf and only inf * 0, inf - inf and NaN
     give NaN; the largest finite value does not become infinite."""
     import torch
     from kuiperllama_b200 import sequence as sq
@@ -81,6 +81,72 @@ def test_split_product_fp32_keeps_infinities_and_nans(T):
     assert torch.equal(out == -float("inf"), ref == -float("inf"))
     fine = ref.isfinite()
     assert torch.allclose(out[fine], ref[fine], rtol=1e-5, atol=1e-4)
+
+
+def chain(a, w):
+    """The product as a chain of fp32 multiply-adds over K, each rounded once (a product of two fp32 numbers is exact in 64 bits, and
+    the sum's second rounding changes nothing at these sizes)."""
+    import torch
+    acc = torch.zeros(a.shape[0], w.shape[0], device="cuda")
+    for k in range(a.shape[1]):
+        acc = (acc.double() + a[:, k, None].double() * w[None, :, k].double()).float()
+    return acc
+
+
+@pytest.mark.parametrize("T", [9, 40, 130])
+@pytest.mark.parametrize("K", [32, 36, 64, 96, 288, 1024])
+def test_fp32_product_is_no_further_off_than_multiply_adds(T, K):
+    import torch
+    from kuiperllama_b200 import sequence as sq
+    off, off_chain = 0.0, 0.0
+    for seed in range(3):
+        g = torch.Generator(device="cuda").manual_seed(100 * seed + K)
+        a, w = torch.randn(T, K, device="cuda", generator=g), torch.randn(300, K, device="cuda", generator=g)
+        out = torch.empty(T, 300, device="cuda")
+        call(sq, sq.load_seq_library(), sq.F32, a, w, out)
+        exact = a.double() @ w.double().T
+        off += (out.double() - exact).norm().item()
+        off_chain += (chain(a, w).double() - exact).norm().item()
+    assert off <= off_chain
+
+
+@pytest.mark.parametrize("T,K,N", [(12, 32, 130), (40, 64, 300), (40, 1024, 300), (130, 288, 300)])
+def test_fp32_product_keeps_every_bit(T, K, N):
+    """One-hot weights hand an operand on as it is; whole numbers of up to 14 bits, whose sums stay below 2^24, are exact."""
+    import torch
+    from kuiperllama_b200 import sequence as sq
+    g = torch.Generator(device="cuda").manual_seed(T + K)
+    lib, out, pick = sq.load_seq_library(), torch.empty(T, N, device="cuda"), torch.arange(N, device="cuda")
+    a, w = torch.randn(T, K, device="cuda", generator=g), torch.zeros(N, K, device="cuda")
+    w[pick, pick % K] = 1.0
+    call(sq, lib, sq.F32, a, w, out)
+    assert torch.equal(out, a[:, pick % K])
+    other = torch.randn(N, K, device="cuda", generator=g)
+    call(sq, lib, sq.F32, w[:T].contiguous(), other, out)  # the other side
+    assert torch.equal(out, other[:, (pick % K)[:T]].T)
+    many = torch.randint(-12291, 12292, (T, K), device="cuda", generator=g).float()
+    few = torch.zeros(N, K, device="cuda")
+    few[:, 1::8] = torch.randint(-7, 8, (N, few[:, 1::8].shape[1]), device="cuda", generator=g).float()
+    call(sq, lib, sq.F32, many, few, out)
+    assert torch.equal(out.double(), many.double() @ few.double().T)
+    one, other = torch.zeros(T, K, device="cuda"), torch.zeros(N, K, device="cuda")
+    one[:, 3], other[:, 3] = 12291.0, 12291.0 - pick  # one product, rounded once
+    call(sq, lib, sq.F32, one, other, out)
+    assert torch.equal(out, (one.double() @ other.double().T).float())
+
+
+@pytest.mark.parametrize("scale", [1e-30, 1e-34, 1e-39])
+def test_fp32_product_of_tiny_operands(scale):
+    """Numbers below 2^-100, down to those without a leading bit, whose parts would leave bf16's range."""
+    import torch
+    from kuiperllama_b200 import sequence as sq
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a, w = torch.randn(20, 96, device="cuda", generator=g), 1e20 * torch.randn(200, 96, device="cuda", generator=g)
+    a[3:9] = (a[3:9].double() * scale).float()
+    out = torch.empty(20, 200, device="cuda")
+    call(sq, sq.load_seq_library(), sq.F32, a, w, out)
+    exact = a.double() @ w.double().T
+    assert ((out.double() - exact).norm(dim=1) <= 5e-7 * exact.norm(dim=1)).all()
 
 
 @pytest.mark.parametrize("T,K,N", [(129, 72, 18945), (300, 64, 8193), (1501, 520, 2050), (2048, 2048, 2561), (4000, 136, 640)])
