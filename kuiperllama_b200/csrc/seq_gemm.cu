@@ -7,8 +7,8 @@
 //   tiled_kernel    any shape: 64 x 64 x 16 tiles through shared memory, 4 x 4 outputs per thread (fp32 FMA)
 // Every form adds an optional bias per output feature.  The gated form (gate rows, then up rows) joins the two products with
 // the activation in its epilogue and writes the compute type.
-//   umma_kernel     bf16, T > 8, K % 8 == 0: 128 weight rows x BN tokens per CTA on tcgen05.mma (kind::f16, operands
-//                   by TMA with 128-byte swizzle, accumulator in TMEM)                      [seq_gemm_umma.cuh]
+//   umma_kernel     bf16, T >= 64 (from K = 64 on) or T > 8 (from K = 384 on), K % 8 == 0: 128 weight rows x BN tokens per CTA
+//                   on tcgen05.mma (kind::f16, operands by TMA with 128-byte swizzle, accumulator in TMEM)  [seq_gemm_umma.cuh]
 //   umma_split_kernel  the same where the tiles are fewer than the SMs: K split over a cluster; fp32 with T > 8 and
 //                   K % 4 == 0, each operand as three bf16 parts                              [seq_gemm_split.cuh]
 //   grouped_kernel  the tiled kernel over row blocks that each belong to one expert (rows gathered by index, the

@@ -669,6 +669,10 @@ inline bool usable(const AT*, const AT*, int, int, int) { return false; }
 template <>
 inline bool usable<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* w, int T, int K, int N) {
   static const bool off = [] { const char* e = getenv("KLLM_SEQ_UMMA"); return e != nullptr && e[0] == '0'; }();
+  // Few rows of a short K stay on multiply-adds: one or two sections do not make up for an accumulator that truncates (error against 64
+  // bits, T = 9 to 63, multiply-adds / here: K = 64 5.1e-8 / 6.4e-8, 128 7.4e-8 / 1.2e-7, 256 1.07e-7 / 1.20e-7, 512 1.62e-7 / 1.23e-7,
+  // 4096 6.1e-7 / 1.4e-7).
+  if (T < 64 && K < 384) return false;
   return !off && T > 8 && K >= BK && (K % 8) == 0 && N >= 8 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(w) & 15) == 0;
 }

@@ -149,6 +149,23 @@ def test_fp32_product_of_tiny_operands(scale):
     assert ((out.double() - exact).norm(dim=1) <= 5e-7 * exact.norm(dim=1)).all()
 
 
+@pytest.mark.parametrize("T", [9, 40, 63])
+@pytest.mark.parametrize("K", [64, 72, 128, 256, 376, 384, 512, 1024])
+def test_bf16_product_of_few_rows_is_no_further_off_than_multiply_adds(T, K):
+    import torch
+    from kuiperllama_b200 import sequence as sq
+    off, off_chain = 0.0, 0.0
+    for seed in range(3):
+        g = torch.Generator(device="cuda").manual_seed(100 * seed + K)
+        a, w = torch.randn(T, K, device="cuda", generator=g).bfloat16(), torch.randn(300, K, device="cuda", generator=g).bfloat16()
+        out = torch.empty(T, 300, device="cuda")
+        call(sq, sq.load_seq_library(), sq.BF16, a, w, out)
+        exact = a.double() @ w.double().T
+        off += (out.double() - exact).norm().item()
+        off_chain += (chain(a, w).double() - exact).norm().item()
+    assert off <= off_chain
+
+
 @pytest.mark.parametrize("T,K,N", [(129, 72, 18945), (300, 64, 8193), (1501, 520, 2050), (2048, 2048, 2561), (4000, 136, 640)])
 def test_persistent_product(T, K, N):
     """Token blocks with a tile of 128 tokens per SM: persistent CTAs with tiles of 256 or 128 tokens, one accumulation over K (K / 16
