@@ -636,10 +636,18 @@ inline int launch_persistent(SplitArgs p, cudaStream_t stream) {
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }
-// whether there is about a tile of 128 tokens for every SM: below that, splitting K over CTAs gives more (T = 1501, K = 2048, 1536
-// gated features, 144 tiles: 57 us split, 41 us here; TF32, T = 900, N = 2048, 128 tiles, K = 2048 and 5632: 26 and 104 us split,
-// 29 and 117 us here)
+// Whether there is about a tile of 128 tokens for every SM.  Below that, splitting K over CTAs gives more where the split kernel takes
+// tiles of 128 tokens too (TF32, T = 900, N = 2048, 128 tiles, K = 2048 and 5632: 26 and 104 us split, 29 and 117 us here).
 inline bool fills_chip(int T, int N) { return T > 64 && ((N + BM - 1) / BM) * ((T + 127) / 128) >= kSms * 19 / 20; }
+// bf16 blocks of more than 128 tokens are split in tiles of 64, and past half a tile of 128 tokens per SM there is no room left to
+// split K: from there on persistent CTAs are ahead.  Tiles as they are taken, of 128 features, or 64 gated ones; split / here in us:
+//   plain, K = 2048    64 tiles (400 x 2048) 16.6 / 17.4    72 (1501 x 768) 16.6 / 17.0    80 (1200 x 1024) 22.8 / 18.0    128 23.7 / 18.7
+//   gated, K = 2048    64 tiles (400 x 1024) 15.2 / 20.7    96 (700 x 1024) 24.3 / 21.6    160 (1200 x 1024) 44.9 / 28.4   192 46.8 / 28.4
+//   K = 4096           plain 72 tiles 24.5 / 27.0, 80 37.0 / 27.3;  gated 64 22.6 / 31.1, 96 39.0 / 32.3
+inline bool persistent_pays(int T, int N, int features) {
+  if (T <= 128) return fills_chip(T, N);
+  return ((N + features - 1) / features) * ((T + 127) / 128) > kSms / 2;
+}
 // The wider tile, unless its last wave is so empty that the narrower one, whose tiles take 0.65 of the time, is done sooner.
 template <int MODE, int OUT>
 inline int launch_wide(const SplitArgs& p, cudaStream_t s) {
@@ -655,11 +663,11 @@ template <bool GATED>
 int launch_few(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act, cudaStream_t s,
                int* report, bool ahead);
 
-// less than one tile of 128 tokens per SM: narrower token blocks and K split over CTAs
+// few tiles of 128 tokens: narrower token blocks and K split over CTAs
 template <bool GATED>
 inline int launch_block(const void* a, const void* w, const float* bias, void* out, int T, int K, int N, const GatedAct& act,
                         cudaStream_t s, int* report, bool ahead) {
-  if (!fills_chip(T, N)) return launch_few<GATED>(a, w, bias, out, T, K, N, act, s, report, ahead);
+  if (!persistent_pays(T, N, GATED ? BM / 2 : BM)) return launch_few<GATED>(a, w, bias, out, T, K, N, act, s, report, ahead);
   const void* w2 = static_cast<const __nv_bfloat16*>(w) + (GATED ? static_cast<size_t>(N) * K : 0);  // 16-byte rows: K % 8 == 0
   return launch_wide<kBf16, GATED ? kGated : kPlain>(SplitArgs{a, w, w2, bias, nullptr, out, T, N, K, 1, act, report}, s);
 }

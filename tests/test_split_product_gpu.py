@@ -166,7 +166,8 @@ def test_bf16_product_of_few_rows_is_no_further_off_than_multiply_adds(T, K):
     assert off <= off_chain
 
 
-@pytest.mark.parametrize("T,K,N", [(129, 72, 18945), (300, 64, 8193), (1501, 520, 2050), (2048, 2048, 2561), (4000, 136, 640)])
+@pytest.mark.parametrize("T,K,N", [(129, 72, 18945), (300, 64, 8193), (1501, 520, 2050), (2048, 2048, 2561), (4000, 136, 640),
+                                   (129, 520, 4737), (140, 1024, 4736), (1900, 2048, 520)])  # around half a tile per SM
 def test_persistent_product(T, K, N):
     """Token blocks with a tile of 128 tokens per SM: persistent CTAs with tiles of 256 or 128 tokens, one accumulation over K (K / 16
     steps of about 2^-24 each: within 2^-19 of the products' magnitudes up to K = 2048)."""
