@@ -22,6 +22,9 @@ CSRC = PKG / "csrc"
 LIBDIR = PKG / "lib"
 LIB = LIBDIR / "libkllm_b200.so"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+# Both libraries hold the engine's templates.  Statics of inline functions would be one object for the whole process (GNU unique symbols):
+# what one library has set up for its kernels, the other would take as set up for its own.
+HOST_FLAGS = "-fPIC,-fno-gnu-unique"
 
 
 def nvcc_path() -> str:
@@ -36,7 +39,7 @@ def _sources():
 
 
 def _fingerprint() -> str:
-    h = hashlib.sha256()
+    h = hashlib.sha256(HOST_FLAGS.encode())
     for p in sorted(list(CSRC.glob("*")) + list((PKG.parent / "include").glob("*.h"))):
         if p.is_file():
             h.update(p.name.encode())
@@ -54,7 +57,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     objs = []
     objdir = LIBDIR / "obj"
     objdir.mkdir(exist_ok=True)
-    common = [nvcc_path(), "-std=c++17", "-O3", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC",
+    common = [nvcc_path(), "-std=c++17", "-O3", "-lineinfo", *ARCH, "-Xcompiler", HOST_FLAGS,
               "-I", str(PKG.parent / "include")]
     if verbose:
         common += ["-Xptxas", "-v"]
@@ -99,7 +102,7 @@ def _seq_sources():
 
 
 def _hash_files(paths) -> str:
-    h = hashlib.sha256()
+    h = hashlib.sha256(HOST_FLAGS.encode())
     for p in sorted(paths):
         if p.is_file():
             h.update(p.name.encode())
@@ -146,7 +149,7 @@ def build_seq(force: bool = False) -> Path:
             return SEQ_LIB
         objdir = LIBDIR / "obj_seq"
         objdir.mkdir(exist_ok=True)
-        common = [nvcc_path(), "-std=c++17", "-O3", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC",
+        common = [nvcc_path(), "-std=c++17", "-O3", "-lineinfo", *ARCH, "-Xcompiler", HOST_FLAGS,
                   "-I", str(PKG.parent / "include")]
         objs = [objdir / (src.stem + ".o") for src in _seq_sources()]
         _run_all([common + ["-c", str(src), "-o", str(obj)] for src, obj in zip(_seq_sources(), objs)], "nvcc")

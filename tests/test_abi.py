@@ -59,3 +59,29 @@ def test_argument_validation_without_device(kllm_lib):
     assert kllm_lib.kllm_gemv_f32(None, None, None, 4, 4, None) == -1
     assert kllm_lib.kllm_rmsnorm_f32(None, None, None, 0, 1e-5, None) == -1
     assert kllm_lib.kllm_decoder_create(None, None, None) == -1
+
+
+def test_libraries_share_no_state(kllm_lib):
+    """A process may load both libraries; statics of their common templates ("already set up") must not be one object for both."""
+    from kuiperllama_b200 import build
+    for path in (LIB_PATH, build.build_seq()):
+        symbols = subprocess.run(["nm", "-D", str(path)], capture_output=True, text=True, check=True).stdout
+        assert not [line for line in symbols.splitlines() if " u " in line], path
+
+
+@pytest.mark.gpu
+def test_both_libraries_multiply_in_one_process(kllm_lib):
+    import ctypes
+
+    import torch
+    from kuiperllama_b200 import sequence as sq
+    libs = [sq.load_seq_library(), ctypes.CDLL(str(LIB_PATH))]
+    libs[1].kllm_seq_gemm.argtypes = libs[0].kllm_seq_gemm.argtypes
+    a, w = torch.randn(300, 256, device="cuda"), torch.randn(5000, 256, device="cuda")
+    for dtype, x, y in ((sq.F32, a, w), (sq.BF16, a.bfloat16(), w.bfloat16())):
+        outs = []
+        for lib in libs:
+            outs.append(torch.empty(300, 5000, device="cuda"))
+            assert lib.kllm_seq_gemm(dtype, x.data_ptr(), y.data_ptr(), outs[-1].data_ptr(), 300, 256, 5000, None) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(*outs)
