@@ -370,30 +370,47 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       else if (S == 2) split_reduce<MODE, BN, OUT, 2>(p, part, rank, t0, n0, mine);
       else if constexpr (two) split_reduce<MODE, BN, OUT, 1>(p, part, rank, t0, n0, mine);
     }
-    if constexpr (MODE == kFp32) {
-      static_assert(OUT != kAdd, "an output is stored again here");
-      auto noted = [&](const float* at) {
-        bool any = false;
-        for (int q = 0; q < S; ++q) any = any || (S > 1 ? ld_peer(peer_smem(smem_u32(at), q)) : *at) != 0.f;
-        return any;
-      };
-      // outputs of rows that their parts do not hold: the sums as a chain of fp32 multiply-adds gives them, by the threads that
-      // stored what the parts gave
-      const int feature = mine % FEATURES, row = n0 + feature;
-      if (noted(special) && row < p.N) {
-        const bool weights = noted(special_row + feature) || (two && noted(special_row + FEATURES + feature));
-        const float* wr = static_cast<const float*>(p.w) + static_cast<size_t>(row) * p.K;
-        const float* wr2 = two ? static_cast<const float*>(p.w2) + static_cast<size_t>(row) * p.K : wr;
-        for (int j = rank * (BN / S) + (two ? mine / FEATURES : 0); j < (rank + 1) * (BN / S) && t0 + j < p.T; j += two ? 2 : 1) {
-          if (!weights && !noted(special_row + BM + j)) continue;
-          const float* ar = static_cast<const float*>(p.a) + static_cast<size_t>(t0 + j) * p.K;
-          float v = 0.f, u = 0.f;
-          for (int k = 0; k < p.K; ++k) {
-            v = fmaf(ar[k], wr[k], v);
-            if (two) u = fmaf(ar[k], wr2[k], u);
+  }
+  if constexpr (MODE == kFp32) {
+    // Outputs of rows that their parts do not hold are summed by multiply-adds and stored over what the parts gave.  A warp sums an
+    // output with its lanes along K (517 x 1024 x 3072: 47 us, with one such token 91, with one such weight row 196; a thread per
+    // feature took milliseconds).
+    static_assert(OUT != kAdd, "an output is stored again here");
+    auto noted = [&](const float* at) {  // by any CTA of the cluster
+      bool any = false;
+      for (int q = 0; q < S; ++q) any = any || (S > 1 ? ld_peer(peer_smem(smem_u32(at), q)) : *at) != 0.f;
+      return any;
+    };
+    if (epilogue && noted(special)) {
+      named_sync<128>(1);  // the tile is stored
+      // this warp's features are quarter, quarter + 4, ...: bit i of `rows` for the i-th
+      bool row_noted = lane < FEATURES / 4 && noted(special_row + quarter + 4 * lane);
+      if (two) row_noted = row_noted || (lane < FEATURES / 4 && noted(special_row + FEATURES + quarter + 4 * lane));
+      const uint32_t rows = __ballot_sync(0xffffffffu, row_noted), every = ~0u >> (32 - FEATURES / 4);
+      for (int j0 = 0; j0 < BN / S; j0 += 32) {
+        const int first = rank * (BN / S) + j0;
+        const uint32_t tokens = __ballot_sync(0xffffffffu, j0 + lane < BN / S && noted(special_row + BM + first + lane));
+        for (int j = 0; j < 32 && j0 + j < BN / S && t0 + first + j < p.T; ++j)
+          for (uint32_t left = tokens >> j & 1u ? every : rows; left != 0; left &= left - 1u) {
+            const int row = n0 + quarter + 4 * (__ffs(left) - 1);
+            if (row >= p.N) break;
+            const float* ar = static_cast<const float*>(p.a) + static_cast<size_t>(t0 + first + j) * p.K;
+            const float* wr = static_cast<const float*>(p.w) + static_cast<size_t>(row) * p.K;
+            const float* wr2 = two ? static_cast<const float*>(p.w2) + static_cast<size_t>(row) * p.K : wr;
+            float v = 0.f, u = 0.f;
+#pragma unroll 8
+            for (int k = lane; k < p.K; k += 32) {
+              v = fmaf(ar[k], wr[k], v);
+              if (two) u = fmaf(ar[k], wr2[k], u);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+              v += __shfl_xor_sync(0xffffffffu, v, o);
+              if (two) u += __shfl_xor_sync(0xffffffffu, u, o);
+            }
+            if (ok && lane == 0) split_store<MODE, OUT>(p, t0 + first + j, row, v, u);
+            __syncwarp();
           }
-          split_store<MODE, OUT>(p, t0 + j, row, v, u);
-        }
       }
     }
   }

@@ -149,6 +149,46 @@ def test_fp32_product_of_tiny_operands(scale):
     assert ((out.double() - exact).norm(dim=1) <= 5e-7 * exact.norm(dim=1)).all()
 
 
+def test_gated_fp32_product_of_tiny_operands():
+    """The same in a gated feed-forward, max(gate, 0) * up, whose output the step hands out through one-hot rows and the residual."""
+    import numpy as np
+    import torch
+    from kuiperllama_b200 import sequence as sq
+    T, W, F = 20, 96, 200
+    g = torch.Generator(device="cuda").manual_seed(4)
+    embed = torch.randn(T, W, device="cuda", generator=g)
+    embed[3:9] *= 1e-32
+    up = 1e15 * torch.randn(2 * F, W, device="cuda", generator=g)
+    up[7], up[F + 70] = up[7] * 1e-33, up[F + 70] * 1e-33  # below 2^-100 themselves
+    down = torch.zeros(W, F, device="cuda")
+    down[torch.arange(W), torch.arange(W)] = 1.0
+    one, w_in, w_out = torch.ones(W, device="cuda"), torch.randn(24, W, device="cuda", generator=g), torch.zeros(W, 8, device="cuda")
+    head = torch.zeros(T, W, device="cuda")
+    layer = (sq.Layer * 1)()
+    L = layer[0]
+    L.pre_mixer, L.pre_ff = sq.Norm(one.data_ptr(), None, 1), sq.Norm(None, None, 2)
+    L.mixer_kind, a = 1, L.attn  # adds nothing
+    a.heads, a.kv_heads, a.dim, a.vdim, a.scale, a.w_in, a.w_out = 1, 1, 8, 8, 1.0, w_in.data_ptr(), w_out.data_ptr()
+    L.ff_kind, L.dense.ff, L.dense.act, L.dense.up, L.dense.down = 2, F, 3, up.data_ptr(), down.data_ptr()
+    d, order = sq.Desc(), (ctypes.c_int32 * 1)(0)
+    d.dtype, d.width, d.vocab, d.norm_eps, d.n_layers, d.layers, d.n_runs, d.run_layer = sq.F32, W, T, 1e-5, 1, layer, 1, order
+    d.embed, d.final_norm, d.head, d.max_tokens, d.max_seqs = embed.data_ptr(), sq.Norm(one.data_ptr(), None, 1), head.data_ptr(), 64, 1
+    torch.cuda.synchronize()
+    lib, handle, seq, rows = sq.load_seq_library(), ctypes.c_void_p(), ctypes.c_int32(), np.empty((T, W), np.float32)
+    lib.kllm_seq_trace_residual.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+    assert lib.kllm_seq_create(ctypes.byref(d), None, ctypes.byref(handle)) == 0
+    assert lib.kllm_seq_open(handle, ctypes.byref(seq)) == 0
+    assert lib.kllm_seq_trace_residual(handle, rows.ctypes.data) == 0
+    assert lib.kllm_seq_step(handle, 1, (ctypes.c_int32 * 1)(seq.value), (ctypes.c_int32 * 1)(T), (ctypes.c_int32 * T)(*range(T)), 0, None,
+                             None, None) == 0
+    lib.kllm_seq_destroy(handle)
+    x, u = embed.double(), embed.double() @ up.double().T
+    exact = x + (torch.relu(u[:, :F]) * u[:, F:])[:, :W]
+    got = torch.from_numpy(rows).cuda().double()
+    assert ((got - exact).abs() <= 1e-6 * (x.abs() + (embed.double().abs() @ up[:W].double().abs().T) * (embed.double().abs() @ up[F:F + W].double().abs().T))).all()
+    assert ((got - exact).norm(dim=1) <= 1e-6 * exact.norm(dim=1)).all()
+
+
 @pytest.mark.parametrize("T", [9, 40, 63])
 @pytest.mark.parametrize("K", [64, 72, 128, 256, 376, 384, 512, 1024])
 def test_bf16_product_of_few_rows_is_no_further_off_than_multiply_adds(T, K):
