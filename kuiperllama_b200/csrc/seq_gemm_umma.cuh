@@ -191,8 +191,10 @@ __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, 
 // ---- token blocks: persistent CTAs ----------------------------------------------------------------------------------
 // One CTA per SM walks tiles of 128 weight rows x BN tokens.  The tile's accumulator alternates between two sets of BN TMEM columns,
 // so the epilogue of a tile runs under the products of the next, and the ring never drains between tiles.
-// What bounds it: at BN = 128 a CTA takes in 32 KB per 2 * 128 * 128 * 64 operations, more than the ~64 bytes a clock that reach an
-// SM from L2 can feed; 256 tokens need three quarters of the bytes per operation.
+// Why 256 tokens: at BN = 128 a CTA takes in 32 KB per 2 * 128 * 128 * 64 operations, more than the ~64 bytes a clock that reach an
+// SM from L2 can feed; 256 tokens need three quarters of the bytes per operation.  What bounds it now is no single unit: for
+// 2048 x 2048 x 8192 (65 us alone) the tensor pipe is busy in 51 % of the cycles, reads from L2 run at 39 % of their peak, shared memory
+// at 64 %; 512 tiles are 3.5 waves, and each operand is brought in by every CTA that meets it.
 // Gated: a tile is 64 features, its first 64 weight rows their gate rows, the other 64 their up rows.  The two TMEM halves meet
 // through shared memory: of every 32 columns the gate's warp finishes 16 and the up rows' warp 16.
 // Eight epilogue warps, four for either half of the columns: with four the activation of a tile takes longer than its products at
@@ -390,7 +392,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
 // along the rows.  `tiles` lists {expert, first row, rows} of up to 256 rows of one expert; *n_tiles of them (both from
 // sort_pairs_kernel, in device memory).  The persistent loop of umma_kernel over (list entry, feature tile); the MMA's N is the
 // entry's rows rounded up to 16, and only the 64-row boxes that hold some are loaded.
-// What bounds it: an expert's weights are read from L2 once per tile of its rows; in tiles of 64 rows that traffic was the bound.
+// An expert's weights are read from L2 once per tile of its rows, so in tiles of 256 a quarter as often as in tiles of 64.
 // EPI 1: the weights of an expert are N gate rows followed by N up rows (a tile: 64 features, gate rows above up rows);
 //        out[row, n] = gated_act(gate, up) in bf16, still in sorted order (the next product reads it as its `a`).
 // EPI 0: out[pair, n] = acc in fp32, pair = sorted_pair[row].
