@@ -9,7 +9,7 @@
 // the activation in its epilogue and writes the compute type.
 //   umma_kernel     bf16, T >= 64 (from K = 64 on) or T > 8 (from K = 384 on), K % 8 == 0: 128 weight rows x BN tokens per CTA
 //                   on tcgen05.mma (kind::f16, operands by TMA with 128-byte swizzle, accumulator in TMEM)  [seq_gemm_umma.cuh]
-//   umma_split_kernel  the same where the tiles are fewer than the SMs: K split over a cluster; fp32 with T > 8 and
+//   umma_split_kernel  the same where the tiles are fewer than the SMs: K split over a cluster; fp32 with T > 8, K >= 128 and
 //                   K % 4 == 0, each operand as three bf16 parts                              [seq_gemm_split.cuh]
 //   grouped_kernel  the tiled kernel over row blocks that each belong to one expert (rows gathered by index, the
 //                   SiLU-gate product as an optional epilogue)

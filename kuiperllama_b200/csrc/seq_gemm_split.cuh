@@ -8,8 +8,7 @@
 //            l m, l l) is at most about 2^-24 of the product, and nothing where one side fits in 8 bits or both in 16.  Six warps
 //            replace a tile's rows by their parts between the tile's arrival and its use.  Rows that hold an infinity, a NaN or a
 //            number whose parts would leave bf16's range (below 2^-100, or rounding up to infinity) are summed by multiply-adds.
-//            (Two TF32 parts and three products, 517 x 1024 x 3072 in 38.9 us, hold 22 bits of an operand: 2.9e-7, and further off
-//            than multiply-adds at K = 32 and 64.)
+//            (Two TF32 parts and three products, 517 x 1024 x 3072 in 38.9 us, hold 22 bits of an operand: 2.9e-7.)
 //
 // What bounds it: with a few dozen tokens the weights are read once and every element of them feeds 2 * T multiply-adds, so
 // the time is the weights' way from HBM.  A tile per 128 features leaves most SMs without work (width 4096: 32 tiles), and
@@ -34,7 +33,7 @@
 //   fp32  T = 16, K = 2048, N = 2048    158 -> 18.8 us    8.1e-7 -> 9.8e-8
 //   fp32  T = 64, K = 4096, N = 4096    314 -> 37.3 us    1.1e-6 -> 1.1e-7
 //   fp32  T = 517, K = 1024, N = 3072   161 -> 47.3 us    5.7e-7 -> 9.4e-8
-//   fp32  T = 9 .. 200, K = 32 and 64                     1.0e-7 -> 4.6e-8, 1.4e-7 -> 7.0e-8
+//   fp32  T = 9 .. 200, K = 128                           2.0e-7 -> 7.5e-8
 #pragma once
 #include "seq_gemm_umma.cuh"
 #include "seq_launch.cuh"
@@ -488,10 +487,12 @@ int launch_few(const void* a, const void* w, const float* bias, void* out, int T
   return launch_split<kBf16, 64, OUT, 4>(p, s, ahead);
 }
 
-// fp32 operands, fp32 accuracy: whole 16-byte rows, and more rows than the kernel that streams weights once takes
+// fp32 operands, fp32 accuracy: whole 16-byte rows, and more rows than the kernel that streams weights once takes.  A short K does not pay
+// for the barriers and the splitting (multiply-adds / here in us, N = 64 to 4096: K = 32, T = 64 6 / 8, T = 130 6 / 12; K = 64, T = 32
+// 6.3 / 8.3, T = 130 8.3 / 12.4; K = 128, T = 16 10.3 / 8.7, T = 130 12.4 / 15, T = 500 and N = 4096 31 / 16; K = 256, T = 16 17 / 10).
 inline bool fp32_usable(const void* a, const void* w, int T, int K) {
   static const bool off = [] { const char* e = getenv("KLLM_SEQ_UMMA"); return e != nullptr && e[0] == '0'; }();
-  return !off && T > 8 && K >= 32 && (K % 4) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
+  return !off && T > 8 && K >= 128 && (K % 4) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(w) & 15) == 0;
 }
 template <bool GATED>

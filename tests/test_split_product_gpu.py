@@ -94,8 +94,9 @@ def chain(a, w):
 
 
 @pytest.mark.parametrize("T", [9, 40, 130])
-@pytest.mark.parametrize("K", [32, 36, 64, 96, 288, 1024])
+@pytest.mark.parametrize("K", [32, 36, 64, 96, 124, 128, 288, 1024])
 def test_fp32_product_is_no_further_off_than_multiply_adds(T, K):
+    """(K < 128 is summed by multiply-adds; chain() rounds a few sums in a million the other way.)"""
     import torch
     from kuiperllama_b200 import sequence as sq
     off, off_chain = 0.0, 0.0
@@ -107,10 +108,10 @@ def test_fp32_product_is_no_further_off_than_multiply_adds(T, K):
         exact = a.double() @ w.double().T
         off += (out.double() - exact).norm().item()
         off_chain += (chain(a, w).double() - exact).norm().item()
-    assert off <= off_chain
+    assert off <= 1.001 * off_chain
 
 
-@pytest.mark.parametrize("T,K,N", [(12, 32, 130), (40, 64, 300), (40, 1024, 300), (130, 288, 300)])
+@pytest.mark.parametrize("T,K,N", [(12, 32, 130), (40, 64, 300), (12, 128, 130), (40, 1024, 300), (130, 288, 300)])
 def test_fp32_product_keeps_every_bit(T, K, N):
     """One-hot weights hand an operand on as it is; whole numbers of up to 14 bits, whose sums stay below 2^24, are exact."""
     import torch
@@ -136,17 +137,18 @@ def test_fp32_product_keeps_every_bit(T, K, N):
 
 
 @pytest.mark.parametrize("scale", [1e-30, 1e-34, 1e-39])
-def test_fp32_product_of_tiny_operands(scale):
+@pytest.mark.parametrize("K", [96, 160, 1024])
+def test_fp32_product_of_tiny_operands(scale, K):
     """Numbers below 2^-100, down to those without a leading bit, whose parts would leave bf16's range."""
     import torch
     from kuiperllama_b200 import sequence as sq
     g = torch.Generator(device="cuda").manual_seed(3)
-    a, w = torch.randn(20, 96, device="cuda", generator=g), 1e20 * torch.randn(200, 96, device="cuda", generator=g)
+    a, w = torch.randn(20, K, device="cuda", generator=g), 1e20 * torch.randn(200, K, device="cuda", generator=g)
     a[3:9] = (a[3:9].double() * scale).float()
     out = torch.empty(20, 200, device="cuda")
     call(sq, sq.load_seq_library(), sq.F32, a, w, out)
     exact = a.double() @ w.double().T
-    assert ((out.double() - exact).norm(dim=1) <= 5e-7 * exact.norm(dim=1)).all()
+    assert ((out.double() - exact).norm(dim=1) <= 1e-6 * exact.norm(dim=1)).all()  # multiply-adds: 5.7e-7 at K = 1024
 
 
 def test_gated_fp32_product_of_tiny_operands():
@@ -154,7 +156,7 @@ def test_gated_fp32_product_of_tiny_operands():
     import numpy as np
     import torch
     from kuiperllama_b200 import sequence as sq
-    T, W, F = 20, 96, 200
+    T, W, F = 20, 160, 200
     g = torch.Generator(device="cuda").manual_seed(4)
     embed = torch.randn(T, W, device="cuda", generator=g)
     embed[3:9] *= 1e-32
