@@ -16,11 +16,16 @@
 // classifier + greedy argmax.  RoPE moves into the attention phase so GEMV rows can be split
 // evenly over all SMs.
 //
-// Consumers (CW warps: 8 for fp32 weights, 14 for int8): the rows of a ring stage are handed out as TASKS of
-// up to four rows to one warp each, round-robin.  A task's rows share every load of the input vector, their
-// dot-product chains interleave (ILP instead of occupancy), their totals are folded with "packed" shuffle trees
-// (kllm_device.cuh) that do the additions of cub's tree only, and one lane per row runs the epilogues side by
-// side.  (int8, toleranced mode, opt-in: a team of warps shares a stage -- mma.sync s8 or dp4a; gemv_phase.)
+// Consumers.  fp32 weights, and int8 ones in the toleranced mode: teams of four warps, each a quarter of the columns of a stage's rows,
+// and an epilogue warp that adds the quarters and stores the results (8 consumer warps; 12 for rows so short that a stage is several
+// tasks).  int8 weights in the reference's order: 14 warps; the rows of a stage are handed out as TASKS of up to four rows to one warp
+// each, round-robin, and one lane per row runs the epilogues.  (Opt-in for the toleranced mode: mma.sync s8 with such warps.)
+// A task's rows share every load of the input vector and their dot-product chains interleave (ILP instead of occupancy); their totals
+// are folded with "packed" shuffle trees (kllm_device.cuh) that do the additions of cub's tree only.
+//
+// What bounds it is the chain of a layer, not a unit: five phases, each entry, poll, norm, rows, hand-off.  Decode of TinyLlama-1.1B at
+// position 500, us per token (HBM time of its weights 635): a warp per task 900, teams 812.  Llama-2-7B int8 with 8 of its 32 layers at position
+// 200 (HBM time 292): 624, teams 497, with the input vector quantised by multiply-adds and byte permutes 475.
 //
 // No local memory: the ring takes the whole unified L1, so a stack access is a round trip to L2.  The kernel
 // parameters are __grid_constant__ (never copied to the stack), register buffers are always written in full
@@ -98,15 +103,22 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* b, int count) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
+}
 // try_wait suspends the warp in hardware until the phase completes or the time hint (ns) runs out:
 // with a generous hint a waiting warp sleeps instead of re-issuing the probe -- waiting warps
 // otherwise compete for issue slots with the warps that are computing on the same scheduler
 // (ncu, r02f: SYNCS + BRA + YIELD of the spin loops were a quarter of all executed instructions).
+// A wait of two minutes ends the kernel: longer than the polls of the hand-offs, on which this one may rest, are allowed to take.
 __device__ __forceinline__ void mbar_wait(uint64_t* b, uint32_t parity) {
   asm volatile(
-      "{\n .reg .pred p;\n WAIT_%=:\n"
+      "{\n .reg .pred p;\n .reg .u64 t0, t;\n"
       " mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1, %2;\n"
-      " @p bra DONE_%=;\n bra WAIT_%=;\n DONE_%=:\n}" ::"r"(smem_u32(b)),
+      " @p bra DONE_%=;\n mov.u64 t0, %%globaltimer;\n WAIT_%=:\n"
+      " mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1, %2;\n"
+      " @p bra DONE_%=;\n mov.u64 t, %%globaltimer;\n sub.u64 t, t, t0;\n setp.lt.u64 p, t, 120000000000;\n"
+      " @p bra WAIT_%=;\n trap;\n DONE_%=:\n}" ::"r"(smem_u32(b)),
       "r"(parity), "r"(KLLM_MBAR_HINT_NS)
       : "memory");
 }
@@ -229,6 +241,12 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
+// What a kernel's rows are: fp32 and int8 in the toleranced mode go through teams of warps and an epilogue warp; int8 in the reference's
+// order (and the opt-in mma form) a warp or a team to a task, which runs its own epilogues.
+enum Kind { kF32 = 0, kW8 = 1, kW8Fast = 2 };
+__host__ __device__ constexpr bool has_teams(int kind) { return kind != kW8; }
+__host__ __device__ constexpr int team_task_rows(int kind) { return kind == kF32 ? 4 : 8; }
+
 struct Pipe {
   int slot;
   uint32_t parity;
@@ -237,6 +255,9 @@ struct Pipe {
       slot = 0;
       parity ^= 1u;
     }
+  }
+  __device__ __forceinline__ void advance_by(int n, int stages) {
+    for (slot += n; slot >= stages; slot -= stages) parity ^= 1u;
   }
 };
 
@@ -253,6 +274,13 @@ __shared__ int g_s_argi[kMaxWarps];
 __shared__ float g_s_bcast;
 __shared__ volatile unsigned g_fill_count;  // ring stages the producer has issued so far
 __shared__ float g_s_team[kMaxWarps / 2][2][3][8];  // team form: the other members' row partials, double buffered per team
+// teams -> epilogue warp: the members' sums of the 32 rows of a group of tasks, [group & 1][task of the group, row][member]
+constexpr int kGroupRows = 32;
+__shared__ float4 g_s_part[2][kGroupRows];
+__shared__ uint64_t g_part_full[2];
+__shared__ uint64_t g_part_empty[2];
+__shared__ int g_s_token;  // of the step, for the epilogue warp
+__shared__ Phase g_ph_epi;
 __shared__ Phase g_ph_cons;
 __shared__ Phase g_ph_prod;
 __shared__ Phase g_ph_pf;
@@ -263,12 +291,19 @@ struct Carry {
   Pipe pipe;
   float best_v;
   int best_i;
+  unsigned groups;  // epilogue groups handed over so far (fp32)
 };
 
 // Grid barrier over the consumer threads of all CTAs.  Monotonic counter, wrap-safe compare.
-template <int CT>
+// (`JOIN` threads meet first: the consumers, and the epilogue warp where there is one -- its stores belong to the phase)
+template <int JOIN>
+__device__ __forceinline__ void join_epilogues() {
+  __syncwarp();
+  asm volatile("bar.sync 15, %0;" ::"n"(JOIN) : "memory");
+}
+template <int CT, int JOIN>
 __device__ __forceinline__ void grid_barrier(unsigned* counter, unsigned& target, unsigned grid) {
-  consumer_sync<CT>();
+  join_epilogues<JOIN>();
   target += grid;
   if (threadIdx.x == 0) {
     red_release_add(counter, 1u);
@@ -276,6 +311,18 @@ __device__ __forceinline__ void grid_barrier(unsigned* counter, unsigned& target
     }
   }
   consumer_sync<CT>();
+}
+
+// ---- CTA -> units ----------------------------------------------------------------------------
+// `cta_units` units each, one more for the last `cta_more` CTAs (the CTAs without an attention head are among them).  (A division
+// of 64-bit numbers here, twice by every role in every phase, took some 500 cycles.)
+struct Share {
+  int u0, u1, more;
+};
+__device__ __forceinline__ Share cta_share(const Phase& ph, int cta, int G) {
+  const int ahead = cta - (G - ph.cta_more);
+  const int u0 = cta * ph.cta_units + max(0, ahead), more = ahead >= 0;
+  return Share{u0, u0 + ph.cta_units + more, more};
 }
 
 // ---- unit -> (segment, row) ------------------------------------------------------------------
@@ -337,46 +384,80 @@ __device__ __forceinline__ float lds_f32(uint32_t a) {
   return v;
 }
 
-// fp32: virtual thread (lane + 32 j) owns packs base + 32 j + lane (matmul_kernel.cu:27-35).  The
-// NR rows of a task share each load of x; per batch (two 32-pack columns) 2 x loads and 2 NR weight
-// loads are issued before the 2 NR independent dot4 chains.
-template <int NR>
-__device__ __forceinline__ void accum_f32(const uint32_t (&w)[NR], uint32_t x, int n_packs, int lane,
-                                          float (&acc)[NR][4]) {
-  // Full 128-pack blocks run branch-free with all 4 * (1 + NR) shared loads issued before the math
-  // (two blocks in flight), so the four independent chains per row overlap the LDS latency.
-  const int full = n_packs & ~127;
-  uint32_t xp = x + lane * 16;
-  uint32_t wp[NR];
+// fp32: a TEAM of four warps shares a task's rows.  Virtual thread 32 m + lane of the reference's 128 owns packs
+// 128 k + 32 m + lane (matmul_kernel.cu:27-35): member m of the team plays virtual warp m, so every chain and every tree below
+// is the reference's.  The NR rows of a task share each load of x, and all loads of U blocks of 128 packs are on their way
+// before the first is used.  Addresses are those of the virtual thread's first pack.
+template <int NR, int U>
+__device__ __forceinline__ void team_blocks(const uint32_t (&w)[NR], uint32_t x, float (&acc)[NR]) {
+  float4 xv[U], wv[NR][U];
 #pragma unroll
-  for (int r = 0; r < NR; ++r) wp[r] = w[r] + lane * 16;
-#pragma unroll 2
-  for (int base = 0; base < full; base += 128) {
-    float4 xv[4];
-    float4 wv[NR][4];
+  for (int u = 0; u < U; ++u) {
+    xv[u] = lds_f4(x + 2048 * u);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) xv[j] = lds_f4(xp + 512 * j);
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) wv[r][j] = lds_f4(wp[r] + 512 * j);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int r = 0; r < NR; ++r) acc[r][j] = __fadd_rn(dot4_ref(xv[j], wv[r][j]), acc[r][j]);
-    xp += 2048;
-#pragma unroll
-    for (int r = 0; r < NR; ++r) wp[r] += 2048;
+    for (int r = 0; r < NR; ++r) wv[r][u] = lds_f4(w[r] + 2048 * u);
   }
-  if (full < n_packs) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (full + 32 * j + lane < n_packs) {
-        const float4 xv = lds_f4(xp + 512 * j);
+  for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int r = 0; r < NR; ++r) acc[r][j] = __fadd_rn(dot4_ref(xv, lds_f4(wp[r] + 512 * j)), acc[r][j]);
-      }
+    for (int r = 0; r < NR; ++r) acc[r] = __fadd_rn(dot4_ref(xv[u], wv[r][u]), acc[r]);
+}
+template <int NR>
+__device__ __forceinline__ void team_accum_f32(uint32_t (&w)[NR], uint32_t x, int n_packs, int vthread, float (&acc)[NR]) {
+  auto on = [&](uint32_t bytes) {
+    x += bytes;
+#pragma unroll
+    for (int r = 0; r < NR; ++r) w[r] += bytes;
+  };
+  int left = n_packs >> 7;
+  if constexpr (NR == 1)
+    for (; left >= 8; left -= 8, on(16384)) team_blocks<NR, 8>(w, x, acc);
+  for (; left >= 4; left -= 4, on(8192)) team_blocks<NR, 4>(w, x, acc);
+  if (left >= 2) team_blocks<NR, 2>(w, x, acc), left -= 2, on(4096);
+  if (left > 0) team_blocks<NR, 1>(w, x, acc), on(2048);
+  if (vthread < (n_packs & 127)) team_blocks<NR, 1>(w, x, acc);
+}
+// The virtual warp's trees of a task's rows: `mine` + row is the member's slot of the row's four sums.  cub only uses lane 0's
+// value of its tree, the balanced binary tree over the lanes with adjacent pairs first, so lanes trade rows instead of all
+// reducing all of them (block128_sum_vt_packed): the same additions, bit for bit.
+template <int NR>
+__device__ __forceinline__ void team_reduce(const float (&acc)[NR], int lane, float* mine) {
+  if constexpr (NR > 4) {  // (int8: up to 8 rows, lane 4 b0 + 2 b1 + b2 with the row's bits b2 b1 b0)
+    const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
+    float s[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float lo = acc[r], up = r + 4 < NR ? acc[r + 4 < NR ? r + 4 : 0] : 0.f;
+      s[r] = __fadd_rn(b0 ? up : lo, __shfl_xor_sync(kFull, b0 ? lo : up, 1));
     }
+    const float u0 = __fadd_rn(b1 ? s[2] : s[0], __shfl_xor_sync(kFull, b1 ? s[0] : s[2], 2));
+    const float u1 = __fadd_rn(b1 ? s[3] : s[1], __shfl_xor_sync(kFull, b1 ? s[1] : s[3], 2));
+    float v = __fadd_rn(b2 ? u1 : u0, __shfl_xor_sync(kFull, b2 ? u0 : u1, 4));
+    v = __fadd_rn(v, __shfl_xor_sync(kFull, v, 8));
+    v = __fadd_rn(v, __shfl_xor_sync(kFull, v, 16));
+    if (lane < 8) mine[((lane & 1) * 4 + (lane & 2) + (lane >> 2)) * 4] = v;
+  } else if constexpr (NR == 4) {
+    const bool odd = lane & 1, hi = lane & 2;
+    const float k0 = odd ? acc[2] : acc[0], k1 = odd ? acc[3] : acc[1];
+    const float g0 = odd ? acc[0] : acc[2], g1 = odd ? acc[1] : acc[3];
+    const float s0 = __fadd_rn(k0, __shfl_xor_sync(kFull, g0, 1));
+    const float s1 = __fadd_rn(k1, __shfl_xor_sync(kFull, g1, 1));
+    float v = __fadd_rn(hi ? s1 : s0, __shfl_xor_sync(kFull, hi ? s0 : s1, 2));
+    v = __fadd_rn(v, __shfl_xor_sync(kFull, v, 4));
+    v = __fadd_rn(v, __shfl_xor_sync(kFull, v, 8));
+    v = __fadd_rn(v, __shfl_xor_sync(kFull, v, 16));
+    if (lane < 4) mine[((lane & 1) * 2 + (lane >> 1)) * 4] = v;  // lanes 0, 2, 1, 3 hold rows 0, 1, 2, 3
+  } else if constexpr (NR == 2) {
+    const bool odd = lane & 1;
+    float v = __fadd_rn(odd ? acc[1] : acc[0], __shfl_xor_sync(kFull, odd ? acc[0] : acc[1], 1));
+#pragma unroll
+    for (int off = 2; off < 32; off <<= 1) v = __fadd_rn(v, __shfl_xor_sync(kFull, v, off));
+    if (lane < 2) mine[lane * 4] = v;
+  } else {
+    float v = acc[0];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) v = __fadd_rn(v, __shfl_xor_sync(kFull, v, off));
+    if (lane == 0) mine[0] = v;
   }
 }
 
@@ -509,7 +590,7 @@ __device__ __forceinline__ float small_int_to_float(int d) {
 // plane is the 16-byte chunk q of its region.
 template <int NR>
 __device__ __forceinline__ void accum_w8_dp4a(const uint32_t (&w)[NR], const uint32_t (&sc)[NR], uint32_t x, int M,
-                                              int lane, float (&acc)[NR], int it_begin = 0, int it_end = 1 << 30) {
+                                              int lane, float (&acc)[NR], int it_begin = 0, int it_end = 1 << 30, int it_step = 1) {
   // lane owns 16 consecutive elements per step of 512: group = 8 * step + lane / 4, quarter = lane % 4
   const uint32_t odd = (lane >> 2) & 1u;
   const uint32_t gq = x + (lane >> 2) * 256 + (lane & 3) * 16;
@@ -522,8 +603,8 @@ __device__ __forceinline__ void accum_w8_dp4a(const uint32_t (&w)[NR], const uin
     sp[r] = sc[r] + (lane >> 2) * 4;
   }
   const int steps = min((M + 511) >> 9, it_end);
-#pragma unroll 2
-  for (int it = it_begin; it < steps; ++it) {
+#pragma unroll(NR > 4 ? 1 : 2)
+  for (int it = it_begin; it < steps; it += it_step) {
     if (it * 512 + lane * 16 < M) {  // M % 512 != 0: the last step covers part of the lanes (M % 64 == 0)
       const uint4 a0 = lds_u4(l0 + it * 2048), a1 = lds_u4(l1 + it * 2048), a2 = lds_u4(l2 + it * 2048);
       const float xstep = lds_f32(xsp + it * 2048);
@@ -598,12 +679,17 @@ __device__ __forceinline__ float accum_w8_mma(uint32_t w_base, uint32_t row_stri
 // place (layout above).  Four adjacent lanes share a group: each reads its 16 values, the group
 // maximum is folded with two shuffles, and after a warp-level sync (all four have read) each lane
 // overwrites its quarter -- no CTA barrier, no values parked in registers.
+// The rounding is one multiply-add: 1.5 * 2^23 + e * inv is a float whose last bit is 1, so its bits are 0x4B400000 + q.  And the
+// balanced digits of q are the bytes of q + 0x808080, each with its top bit turned over.  (With a conversion and two divisions of the
+// digits by hand a phase was staged 0.7 us later, of 3.4.)  Lanes begin with different packs of their 16 values,
+// so that a quarter warp's 128-bit reads fall on different banks.
 template <int CT>
 __device__ __noinline__ void quantize_input_inplace(float* xs, int M, int tid) {
   const int quarters = M >> 4;
   for (int base = 0; base < quarters; base += CT) {  // CT % 32 == 0: whole warps, groups never straddle one
     const int qg = base + tid;
     const bool on = qg < quarters;
+    const int turn = (tid >> 1) & 3;
     // lanes past the end read the last quarter again (their group is entirely past the end: M % 64 == 0),
     // so v[] is always written and stays in registers instead of local memory
     float4 v[4];
@@ -612,7 +698,7 @@ __device__ __noinline__ void quantize_input_inplace(float* xs, int M, int tid) {
       const float4* g4 = reinterpret_cast<const float4*>(xs) + min(qg, quarters - 1) * 4;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        v[j] = g4[j];
+        v[j] = g4[(j + turn) & 3];
         gmax = fmaxf(gmax, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
       }
     }
@@ -628,22 +714,16 @@ __device__ __noinline__ void quantize_input_inplace(float* xs, int M, int tid) {
       uint32_t* o0 = reinterpret_cast<uint32_t*>(gb + ((0u + odd) & 3u) * 64);
       uint32_t* o1 = reinterpret_cast<uint32_t*>(gb + ((1u + odd) & 3u) * 64);
       uint32_t* o2 = reinterpret_cast<uint32_t*>(gb + ((2u + odd) & 3u) * 64);
+      auto digits = [&](float e) {  // |q| <= 2^22
+        return (__float_as_uint(__fmaf_rn(e, inv, 12582912.0f)) - 0x4B400000u + 0x808080u) ^ 0x808080u;
+      };
 #pragma unroll
       for (int j = 0; j < 4; ++j) {  // 4 elements -> one word of each digit plane, written at once
-        const float e[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-        uint32_t p0 = 0, p1 = 0, p2 = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int qv = __float2int_rn(e[b] * inv);  // |qv| <= 2^22
-          const int a0 = ((qv + 128) & 255) - 128;    // balanced digits: qv = 65536 a2 + 256 a1 + a0
-          const int q1 = (qv - a0) >> 8;
-          const int a1 = ((q1 + 128) & 255) - 128;
-          const int a2 = (q1 - a1) >> 8;
-          p0 |= static_cast<uint32_t>(a0 & 255) << (8 * b);
-          p1 |= static_cast<uint32_t>(a1 & 255) << (8 * b);
-          p2 |= static_cast<uint32_t>(a2 & 255) << (8 * b);
-        }
-        o0[j] = p0, o1[j] = p1, o2[j] = p2;
+        const uint32_t a = digits(v[j].x), b = digits(v[j].y), c = digits(v[j].z), d = digits(v[j].w);
+        const uint32_t ab = __byte_perm(a, b, 0x5140), cd = __byte_perm(c, d, 0x5140);  // low bytes, then middle ones
+        const int at = (j + turn) & 3;
+        o0[at] = __byte_perm(ab, cd, 0x5410), o1[at] = __byte_perm(ab, cd, 0x7632);
+        o2[at] = __byte_perm(__byte_perm(a, b, 0x0062), __byte_perm(c, d, 0x0062), 0x5410);
       }
       if (q == 0) *reinterpret_cast<float*>(gb + ((3u + odd) & 3u) * 64) = step;
     }
@@ -659,14 +739,9 @@ __device__ __noinline__ void quantize_input_inplace(float* xs, int M, int tid) {
 struct Rows4 {
   uint32_t a[4];
 };
-template <int NR, bool INT8>
-__device__ __forceinline__ float4 dot_rows(Rows4 rows, Rows4 scales, uint32_t x, int M, int group_size,
-                                           int group_shift, int lane, bool fast = false) {
-  float acc[NR][4];
-#pragma unroll
-  for (int r = 0; r < NR; ++r)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[r][j] = 0.f;
+template <int NR>
+__device__ __forceinline__ float4 dot_rows_w8(Rows4 rows, Rows4 scales, uint32_t x, int M, int group_size,
+                                              int group_shift, int lane, bool fast) {
   float d[4] = {0.f, 0.f, 0.f, 0.f};
   uint32_t w[NR], sc[NR];
 #pragma unroll
@@ -674,32 +749,31 @@ __device__ __forceinline__ float4 dot_rows(Rows4 rows, Rows4 scales, uint32_t x,
     w[r] = rows.a[r];
     sc[r] = scales.a[r];
   }
-  if constexpr (INT8) {
-    if (fast) {  // fixed-point activations x int8 weights on dp4a (toleranced mode; group size 64)
-      float a1[NR];
+  if (fast) {  // fixed-point activations x int8 weights on dp4a (toleranced mode; group size 64)
+    float a1[NR];
 #pragma unroll
-      for (int r = 0; r < NR; ++r) a1[r] = 0.f;
-      accum_w8_dp4a<NR>(w, sc, x, M, lane, a1);
+    for (int r = 0; r < NR; ++r) a1[r] = 0.f;
+    accum_w8_dp4a<NR>(w, sc, x, M, lane, a1);
 #pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        float v = a1[r];
+    for (int r = 0; r < NR; ++r) {
+      float v = a1[r];
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFull, v, off);
-        d[r] = v;
-      }
-      return make_float4(d[0], d[1], d[2], d[3]);
+      for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFull, v, off);
+      d[r] = v;
     }
-    if (group_size == 64)
-      accum_w8_g64<NR>(w, sc, x, M, lane, acc);
-    else
-      accum_w8_any<NR>(w, sc, x, M, group_shift, group_size, lane, acc);
-#pragma unroll
-    for (int r = 0; r < NR; ++r) d[r] = block128_sum_quad_packed(acc[r]);
-  } else {
-    accum_f32<NR>(w, x, M >> 2, lane, acc);
-#pragma unroll
-    for (int r = 0; r < NR; ++r) d[r] = block128_sum_vt_packed(acc[r], lane);
+    return make_float4(d[0], d[1], d[2], d[3]);
   }
+  float acc[NR][4];
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[r][j] = 0.f;
+  if (group_size == 64)
+    accum_w8_g64<NR>(w, sc, x, M, lane, acc);
+  else
+    accum_w8_any<NR>(w, sc, x, M, group_shift, group_size, lane, acc);
+#pragma unroll
+  for (int r = 0; r < NR; ++r) d[r] = block128_sum_quad_packed(acc[r]);
   return make_float4(d[0], d[1], d[2], d[3]);
 }
 
@@ -1627,14 +1701,295 @@ __device__ KLLM_STAGE_CALL void stage_handoff(const unsigned long long* src, uns
   stage_handoff_inline<UP>(src, tag, n4, t, NT, xs4);
 }
 
+// ---- epilogue of a unit (a row, or a w1 | w3 pair of rows), by one lane ---------------------------------
+// Where its value goes and what is added to it: found BEFORE the unit's dot product is there, so that this and the L2 latency of
+// the bias hide behind it.
+struct UnitDest {
+  unsigned long long* word;  // tagged word (or none); with several ranks the word's place in every rank's exchange area
+  unsigned tag;
+  float* plain;              // plain store (or none)
+  const float* residual;     // what is added last (grid barriers between the phases only; read with the store: the barrier has passed)
+  float bias;
+  bool has_bias;
+  int row;
+};
+__device__ __forceinline__ UnitDest unit_dest(const Params& P, const Phase& ph, int tok, int pos, const float* residual, int unit) {
+  UnitDest d{nullptr, 0u, nullptr, nullptr, 0.f, false, unit};
+  d.tag = P.hand_base + static_cast<unsigned>(tok * P.hands_per_token + ph.hand_out) + 1u;
+  if (ph.swiglu) {
+    if (ph.seg[0].tag_out != nullptr) d.word = ph.seg[0].tag_out + unit;
+    else d.plain = ph.seg[0].out + unit;
+    return d;
+  }
+  if (ph.tp_out) {
+    d.tag = P.tp_seq_base + static_cast<unsigned>(tok * P.exch_per_token + ph.exch_out) + 1u;
+    d.word = P.tp_data[P.tp_rank] + (static_cast<size_t>(d.tag & 1u) * P.tp_world + P.tp_rank) * P.tp_stride + unit;
+    return d;
+  }
+  const RowRef rr = resolve_row(ph, unit, 0);
+  const Seg& sg = ph.seg[rr.seg];
+  d.row = rr.row;
+  if (sg.bias != nullptr) d.has_bias = true, d.bias = __ldg(sg.bias + rr.row);
+  if (residual != nullptr) d.residual = residual + rr.row;
+  if (sg.tag_out != nullptr) d.word = sg.tag_out + rr.row;
+  if (sg.out == nullptr) {
+  } else if (sg.head_major) {  // value cache [kv_head][SP][seq_len][dv]
+    const int hs = P.head_size, dv = hs / P.attn_vsplit;
+    const int kvh = rr.row / hs, e = rr.row % hs;
+    d.plain = sg.out + ((static_cast<size_t>(kvh) * P.attn_vsplit + e / dv) * P.seq_len + pos) * dv + e % dv;
+  } else {
+    d.plain = sg.out + static_cast<long long>(pos) * sg.pos_stride + rr.row;
+  }
+  return d;
+}
+__device__ __forceinline__ void unit_store(const Params& P, const Phase& ph, const UnitDest& d, ArgBest& best, float d0, float d1) {
+  float v = d0;
+  if (ph.swiglu) {
+    v = swiglu_ref(d0, d1);
+  } else if (ph.tp_out && P.tp_world > 1) {
+    const size_t off = d.word - P.tp_data[P.tp_rank];
+    for (int k = 1; k <= P.tp_world; ++k) st_tagged(P.tp_data[(P.tp_rank + k) % P.tp_world] + off, v, d.tag);
+    return;
+  }
+  if (d.has_bias) v = __fadd_rn(v, d.bias);              // matmul.cpp:74-77: out + bias
+  if (d.residual != nullptr) v = __fadd_rn(__ldcg(d.residual), v);  // llama3.cpp:683,719: x + out
+  if (d.word != nullptr) st_tagged_gpu(d.word, v, d.tag);
+  if (d.plain != nullptr) *d.plain = v;
+  if (ph.argmax) arg_fold(best, v, d.row);
+}
+
+// ---- rows by teams of four warps, epilogues by a warp of their own ------------------------------------------
+// How a CTA's share of a phase is cut, the same for the teams and for the epilogue warp: a stage holds up to `ups` units, a task up
+// to TASK_ROWS rows of a stage.
+template <int TASK_ROWS>
+struct TaskPlan {
+  static constexpr int kGroupTasks = kGroupRows / TASK_ROWS;
+  int u0, units;  // of this CTA
+  int rpu, ups, upt, per_stage, stages, tasks;
+  __device__ __forceinline__ TaskPlan(const Phase& ph, int cta, int G) {
+    const Share s = cta_share(ph, cta, G);
+    u0 = s.u0, units = s.u1 - s.u0;
+    rpu = ph.swiglu ? 2 : 1;
+    ups = ph.units_per_stage, upt = TASK_ROWS >> (rpu - 1), per_stage = ph.tasks_per_stage;
+    stages = ph.stages[s.more], tasks = ph.tasks[s.more];
+  }
+  __device__ __forceinline__ int groups() const { return (tasks + kGroupTasks - 1) / kGroupTasks; }
+};
+
+// The epilogue warp: adds the four members' sums of each row (fp32: in the reference's order) and runs the rows' epilogues, a lane to a
+// unit.  Were it one of the team's own warps, that warp would be late for the team's next task and hold the others up there, and the
+// next one after it: a task every 2100 cycles for a team (TinyLlama-1.1B, w1 | w3), 1590 this way.
+template <int CW, int KIND, bool PROF>
+__device__ __forceinline__ void epilogue_role(const Params& P, int lane) {
+  constexpr int JOIN = CW * 32 + 32, TASK_ROWS = team_task_rows(KIND);
+  using Plan = TaskPlan<TASK_ROWS>;
+  constexpr int kGroupTasks = Plan::kGroupTasks;
+  const Phase& ph = g_ph_epi;
+  const int cta = blockIdx.x, G = gridDim.x;
+  unsigned groups = 0;
+  int pos = P.state->pos;
+  for (int tok = 0; tok < P.n_tokens; ++tok, ++pos) {
+    ArgBest best{0.f, -1};
+    for (int pi = 0; pi < P.n_phases; ++pi) {
+      {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(P.phases + pi);
+        uint32_t* dst = reinterpret_cast<uint32_t*>(&g_ph_epi);
+        __syncwarp();
+        for (int i = lane; i < static_cast<int>(sizeof(Phase) / 4); i += 32) dst[i] = __ldg(src + i);
+        __syncwarp();
+      }
+      if (ph.kind == kPhaseGemv && !(ph.cls && tok < P.skip_cls_tokens)) {
+        const Plan plan(ph, cta, G);
+        const int n_groups = plan.groups();
+        const bool swiglu = ph.swiglu != 0;
+        // this lane's unit in the first group: unit k of task t
+        const int t = lane / plan.upt, k = lane % plan.upt;  // (a power of two)
+        int stage = t / plan.per_stage, in_stage = t - stage * plan.per_stage;
+        for (int g = 0; g < n_groups; ++g, ++groups) {
+          const int i = in_stage * plan.upt + k;  // unit of the stage
+          const int unit = plan.u0 + stage * plan.ups + i;
+          const bool mine = t < kGroupTasks && g * kGroupTasks + t < plan.tasks && i < plan.ups && stage * plan.ups + i < plan.units;
+          // (the embedding row as a residual: grid barriers between the phases, and g_s_token was written ahead of the last)
+          const float* residual = ph.residual_from_emb ? P.tok_emb + static_cast<size_t>(g_s_token) * P.dim : ph.residual;
+          const UnitDest dest = unit_dest(P, ph, tok, pos, residual, mine ? unit : plan.u0);
+          const float4* rows = g_s_part[groups & 1] + (t % kGroupTasks) * TASK_ROWS + (swiglu ? 2 * k : k);
+          const int lacking = (g + 1) * kGroupTasks - plan.tasks;
+          if (lacking > 0 && lane == 0) mbar_arrive(&g_part_full[groups & 1], 4 * lacking);
+          mbar_wait(&g_part_full[groups & 1], (groups >> 1) & 1u);
+          if (mine) {
+            const float4 a = rows[0];
+            const float d0 = __fadd_rn(__fadd_rn(__fadd_rn(a.x, a.y), a.z), a.w);
+            float d1 = 0.f;
+            if (swiglu) {
+              const float4 b = rows[1];
+              d1 = __fadd_rn(__fadd_rn(__fadd_rn(b.x, b.y), b.z), b.w);
+            }
+            unit_store(P, ph, dest, best, d0, d1);
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&g_part_empty[groups & 1]);
+          for (in_stage += kGroupTasks; in_stage >= plan.per_stage; in_stage -= plan.per_stage) ++stage;
+        }
+        if (ph.argmax) {  // per-CTA (max, lowest index) of the classifier rows this CTA produced
+#pragma unroll
+          for (int off = 1; off < 32; off <<= 1) {
+            const float ov = __shfl_xor_sync(kFull, best.v, off);
+            const int oi = __shfl_xor_sync(kFull, best.i, off);
+            arg_fold(best, ov, oi);
+          }
+          if (lane == 0) P.arg_val[cta] = best.v, P.arg_idx[cta] = best.i;
+        }
+        if (PROF && P.prof != nullptr && tok == P.prof_token && lane == 0)
+          P.prof[(static_cast<size_t>(cta) * P.n_phases + pi) * kProfStamps + 2] = global_ns();
+      }
+      if (ph.barrier_after) join_epilogues<JOIN>();
+    }
+  }
+}
+
+template <int NR>
+struct Sums {
+  float v[NR];
+};
+// One team's part of a phase: fp32, member m plays the reference's virtual warp m; int8, it takes every fourth step of 512 columns.
+// Why teams: a warp to a task takes a stage's 32 KB in some 2000 cycles and the six of a ring side by side (all of shared memory's
+// bandwidth, then none while the ring refills), and a warp without a row of a stage still spent 500 cycles on it.
+// The stages of a phase whose stages hold one task each belong to the teams in turn (slot mod kTeams: the same slots for a team in
+// every phase, so none of its waits can be answered by an older fill); its four warps alone wait for them and give them back, for all.
+// Otherwise every warp waits on every stage and the tasks alternate (tests/test_team_handover.py).
+template <int CW, int KIND>
+__device__ __forceinline__ void team_rows(const Params& P, const Phase& ph, uint32_t xa, uint32_t ring, int cta, int G, int warp, int lane,
+                                          Carry& carry, long long& cyc_wait, bool timed) {
+  constexpr int kTeams = CW / 4, TASK_ROWS = team_task_rows(KIND);
+  constexpr bool F32 = KIND == kF32;
+  using Plan = TaskPlan<TASK_ROWS>;
+  constexpr int kGroupTasks = Plan::kGroupTasks;
+  const int team = warp >> 2, member = warp & 3, vthread = member * 32 + lane, S = P.num_stages;
+  const Plan plan(ph, cta, G);
+  const bool swiglu = ph.swiglu != 0;
+  const int M = ph.in_dim, n_packs = M >> 2, stage_bytes = P.stage_bytes;
+  const uint32_t rb = static_cast<uint32_t>(M) * (F32 ? 4u : 1u);
+  const uint32_t sb = static_cast<uint32_t>(ph.scale_row_bytes), scales = static_cast<uint32_t>(ph.scale_off);
+  if (F32) {
+    xa += static_cast<uint32_t>(vthread) * 16u;
+    ring += static_cast<uint32_t>(vthread) * 16u;
+  }
+  Pipe pipe = carry.pipe;
+  int group = -1;        // the group that this warp may write,
+  float* part = nullptr;  // this member's place in it
+  uint64_t* part_full = nullptr;
+  auto place = [&](int task) {  // ... in the task's first row
+    if (task / kGroupTasks != group) {
+      group = task / kGroupTasks;
+      const unsigned at = carry.groups + static_cast<unsigned>(group);
+      part = reinterpret_cast<float*>(g_s_part[at & 1]) + member;
+      part_full = &g_part_full[at & 1];
+      mbar_wait(&g_part_empty[at & 1], ((at >> 1) & 1u) ^ 1u);
+    }
+    return part + (task % kGroupTasks) * (TASK_ROWS * 4);
+  };
+  auto hand_over = [&]() {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(part_full);
+  };
+  auto give_back = [&](int slot, int times) {  // this warp has read what it needs of the stage
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&g_empty_bar[slot], times);
+  };
+  auto wait_stage = [&](int slot, uint32_t parity) {
+    const long long c0 = timed ? clock64() : 0;
+    mbar_wait(&g_full_bar[slot], parity);
+    if (timed) cyc_wait += clock64() - c0;
+  };
+  // the nr rows of a task, from unit i0 of a stage of n units on; SwiGLU stage order: the stage's w1 rows, then its w3 rows
+  auto sum_rows = [&](auto acc, int task, uint32_t stage, int i0, int n, int nr, int slot, int times) {
+    constexpr int NR = sizeof(acc.v) / sizeof(float);
+    uint32_t w[NR], sc[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {  // (the last row again where there are fewer)
+      const int q = min(r, nr - 1), row = i0 + (swiglu ? (q >> 1) + (q & 1) * n : q);
+      w[r] = stage + row * rb;
+      sc[r] = stage + scales + row * sb;
+      acc.v[r] = 0.f;
+    }
+    if constexpr (F32) team_accum_f32<NR>(w, xa, n_packs, vthread, acc.v);
+    else accum_w8_dp4a<NR>(w, sc, xa, M, lane, acc.v, member, 1 << 30, 4);
+    if (times > 0) give_back(slot, times);
+    team_reduce<NR>(acc.v, lane, place(task));
+    hand_over();
+  };
+  auto sum_task = [&](int task, uint32_t stage, int i0, int n, int nr, int slot, int times) {
+    if constexpr (!F32) {
+      if (nr > 6) return sum_rows(Sums<8>{}, task, stage, i0, n, nr, slot, times);
+      if (nr > 4) return sum_rows(Sums<6>{}, task, stage, i0, n, nr, slot, times);
+    }
+    if (nr > 2) sum_rows(Sums<4>{}, task, stage, i0, n, nr, slot, times);
+    else if (nr == 2) sum_rows(Sums<2>{}, task, stage, i0, n, nr, slot, times);
+    else sum_rows(Sums<1>{}, task, stage, i0, n, nr, slot, times);
+  };
+  if (F32 && ph.chunks_per_row > 1) {  // a row longer than a stage: its task goes on over several
+    const int chunk = ph.chunk_elems;  // (a multiple of 128 packs)
+    for (int task = 0; task < plan.tasks; ++task) {
+      const bool mine = task % kTeams == team;
+      float acc[1] = {0.f};
+      for (int c = 0; c < ph.chunks_per_row; ++c) {
+        wait_stage(pipe.slot, pipe.parity);
+        if (mine) {
+          uint32_t w[1] = {ring + static_cast<uint32_t>(pipe.slot * stage_bytes)};
+          team_accum_f32<1>(w, xa + static_cast<uint32_t>(c * chunk) * 4u, min(chunk, ph.in_dim - c * chunk) >> 2, vthread, acc);
+        }
+        give_back(pipe.slot, 1);
+        pipe.advance(S);
+      }
+      if (mine) {
+        team_reduce<1>(acc, lane, place(task));
+        hand_over();
+      }
+    }
+  } else if (plan.per_stage == 1 && S % kTeams == 0) {
+    int slot = pipe.slot;
+    uint32_t parity = pipe.parity;
+    int i = 0;
+    for (; slot % kTeams != team; ++i)
+      if (++slot == S) slot = 0, parity ^= 1u;
+    const int rows = plan.ups * plan.rpu, last_rows = (plan.units - (plan.stages - 1) * plan.ups) * plan.rpu;
+    auto next_slot = [&]() {
+      slot += kTeams;
+      if (slot >= S) slot -= S, parity ^= 1u;
+    };
+    for (; i < plan.stages; i += kTeams, next_slot()) {
+      const int nr = i + 1 < plan.stages ? rows : last_rows;
+      wait_stage(slot, parity);
+      sum_task(i, ring + static_cast<uint32_t>(slot * stage_bytes), 0, nr >> 1, nr, slot, kTeams);
+    }
+    pipe.advance_by(plan.stages, S);
+  } else {
+    for (int i = 0, task0 = 0, left = plan.units; i < plan.stages; ++i, task0 += plan.per_stage, left -= plan.ups) {
+      const int n = min(plan.ups, left);
+      wait_stage(pipe.slot, pipe.parity);
+      const uint32_t wa = ring + static_cast<uint32_t>(pipe.slot * stage_bytes);
+      int t = (team + kTeams - task0 % kTeams) % kTeams;
+      if (t * plan.upt >= n) give_back(pipe.slot, 1);  // a stage of which this team has no task
+      for (; t * plan.upt < n; t += kTeams) {
+        const int i0 = t * plan.upt;
+        sum_task(task0 + t, wa, i0, n, min(plan.upt, n - i0) * plan.rpu, pipe.slot, (t + kTeams) * plan.upt >= n);
+      }
+      pipe.advance(S);
+    }
+  }
+  carry.pipe = pipe;
+  carry.groups += static_cast<unsigned>(plan.groups());
+}
+
 // ---- one GEMV phase of one CTA's consumer warps --------------------------------------------------
 // Stages the phase's input vector (tagged residual exchange / tagged hand-off / plain vector) into
 // shared memory, RMS-normalises it when the phase asks for it, consumes this CTA's ring stages
 // task by task, runs the epilogues and, for the classifier, leaves the CTA's (max, index).
-template <int CW, bool INT8, bool PROF>
+template <int CW, int KIND, bool PROF>
 __device__ KLLM_PHASE_CALL Carry gemv_phase(const Params& P, Carry carry, int tok, int pos, const float* emb_row,
                                             unsigned long long* stamp) {
   constexpr int CT = CW * 32;
+  constexpr bool INT8 = KIND != kF32;
   constexpr int wbytes = INT8 ? 1 : 4;
   const Phase& ph = g_ph_cons;
   uint64_t* full_bar = g_full_bar;
@@ -1763,67 +2118,31 @@ __device__ KLLM_PHASE_CALL Carry gemv_phase(const Params& P, Carry carry, int to
   }
   consumer_sync<CT>();
   // int8 fast mode: the staged (and normalised) vector becomes 24-bit fixed point per 64-group
-  const bool int8_fast = INT8 && P.int8_fast != 0 && ph.group_size == 64 && (M & 63) == 0;
+  const bool int8_fast = KIND == kW8Fast || (INT8 && P.int8_fast != 0 && ph.group_size == 64 && (M & 63) == 0);
   if constexpr (INT8) {
     if (int8_fast) quantize_input_inplace<CT>(xs, M, tid);
   }
   if (stamp) stamp[1] = global_ns();
 
-  const int u0 = static_cast<int>(static_cast<long long>(cta) * ph.units / G);
-  const int u1 = static_cast<int>(static_cast<long long>(cta + 1) * ph.units / G);
+  const Share share = cta_share(ph, cta, G);
+  const int u0 = share.u0, u1 = share.u1;
   const int rpu = ph.swiglu ? 2 : 1;
   const int row_bytes = M * wbytes;
   const float* residual = ph.residual_from_emb ? emb_row : ph.residual;
 
   // bias / residual of a row are fetched BEFORE its dot product so their L2 latency hides
   // behind the accumulation (by the lane that will run the row's epilogue)
-  auto prefetch_addend = [&](int unit, float& bias_v, float& res_v) {
-    bias_v = 0.f, res_v = 0.f;
-    if (ph.swiglu) return;
-    const RowRef rr = resolve_row(ph, unit, 0);
-    if (ph.seg[rr.seg].bias != nullptr) bias_v = __ldg(ph.seg[rr.seg].bias + rr.row);
-    if (residual != nullptr) res_v = __ldcg(residual + rr.row);
-  };
-  // one lane per unit
-  auto epilogue = [&](int unit, float d0, float d1, float bias_v, float res_v) {
-    if (ph.swiglu) {
-      const float g = swiglu_ref(d0, d1);
-      if (ph.seg[0].tag_out != nullptr)
-        st_tagged_gpu(ph.seg[0].tag_out + unit, g, hand_tag(ph.hand_out));
-      else
-        ph.seg[0].out[unit] = g;
-      return;
-    }
-    if (ph.tp_out) {
-      const unsigned tag = P.tp_seq_base + static_cast<unsigned>(tok * P.exch_per_token + ph.exch_out) + 1u;
-      const size_t off = (static_cast<size_t>(tag & 1u) * P.tp_world + P.tp_rank) * P.tp_stride + unit;
-      if (P.tp_world == 1) {
-        st_tagged_gpu(P.tp_data[0] + off, d0, tag);
-      } else {
-        for (int k = 1; k <= P.tp_world; ++k) st_tagged(P.tp_data[(P.tp_rank + k) % P.tp_world] + off, d0, tag);
-      }
-      return;
-    }
-    const RowRef rr = resolve_row(ph, unit, 0);
-    const Seg& sg = ph.seg[rr.seg];
-    float v = d0;
-    if (sg.bias != nullptr) v = __fadd_rn(v, bias_v);       // matmul.cpp:74-77: out + bias
-    if (residual != nullptr) v = __fadd_rn(res_v, v);       // llama3.cpp:683,719: x + out
-    if (sg.tag_out != nullptr) st_tagged_gpu(sg.tag_out + rr.row, v, hand_tag(ph.hand_out));
-    if (sg.out == nullptr) {
-    } else if (sg.head_major) {  // value cache [kv_head][SP][seq_len][dv]
-      const int hs = P.head_size, dv = hs / P.attn_vsplit;
-      const int kvh = rr.row / hs, d = rr.row % hs;
-      sg.out[((static_cast<size_t>(kvh) * P.attn_vsplit + d / dv) * P.seq_len + pos) * dv + d % dv] = v;
-    } else {
-      sg.out[static_cast<long long>(pos) * sg.pos_stride + rr.row] = v;
-    }
-    if (ph.argmax) arg_fold(best, v, rr.row);
-  };
+  auto unit_dest_of = [&](int unit) { return unit_dest(P, ph, tok, pos, residual, unit); };
+  auto epilogue = [&](const UnitDest& dest, float d0, float d1) { unit_store(P, ph, dest, best, d0, d1); };
 
   long long cyc_wait = 0, cyc_rows = 0;
   long long cyc4[4] = {0, 0, 0, 0};
-  if (ph.chunks_per_row == 1) {
+  if constexpr (has_teams(KIND)) {
+    carry.pipe = pipe;
+    team_rows<CW, KIND>(P, ph, smem_u32(xs), smem_u32(stages), cta, G, warp, lane, carry, cyc_wait, stamp != nullptr);
+    if (stamp) stamp[8] = static_cast<unsigned long long>(cyc_wait);
+    return carry;
+  } else {
     // A stage holds n units; they are handed out as tasks of up to 4 rows (plain: 4 units, SwiGLU:
     // 2 units = w1 + w3 rows of two outputs), task after task round-robin over the consumer warps.
     const int ups = ph.rows_per_stage / rpu;
@@ -1857,8 +2176,7 @@ __device__ KLLM_PHASE_CALL Carry gemv_phase(const Params& P, Carry carry, int to
           if (task % kTeams == team) {
             const int j = lane >> 2;  // lane 4 j ends with the total of stage row j
             const bool owner = member == 0 && (lane & 3) == 0 && j < n;
-            float bias_v = 0.f, res_v = 0.f;
-            if (owner) prefetch_addend(u + j, bias_v, res_v);
+            const UnitDest dest = unit_dest_of(owner ? u + j : u);
             const int nrows = n * rpu;
             float tot = 0.f;
             if (ph.mma) {  // <= 8 rows on the tensor cores; the member's share of the 64-element groups
@@ -1890,7 +2208,7 @@ __device__ KLLM_PHASE_CALL Carry gemv_phase(const Params& P, Carry carry, int to
               for (int mm = 1; mm < kTeam; ++mm) tot = __fadd_rn(tot, scratch[(mm - 1) * 8 + j]);
               // SwiGLU stage order: w1 rows of the n units, then their w3 rows
               const float tot_w3 = __shfl_sync(kFull, tot, min(j + n, 7) * 4);
-              if (owner) epilogue(u + j, tot, tot_w3, bias_v, res_v);
+              if (owner) epilogue(dest, tot, tot_w3);
             }
           }
           ++task;
@@ -1905,8 +2223,7 @@ __device__ KLLM_PHASE_CALL Carry gemv_phase(const Params& P, Carry carry, int to
         if (task % CW != warp) continue;  // CW is 6, 8 or 16: a real modulo (a mask would idle warps 2 and 3 of 6)
         const int nu = min(upt, n - i0);
         const long long t_a = stamp ? clock64() : 0;
-        float bias_v = 0.f, res_v = 0.f;
-        if (lane < nu) prefetch_addend(u + i0 + lane, bias_v, res_v);
+        const UnitDest dest = unit_dest_of(u + i0 + (lane < nu ? lane : 0));
         const long long t_b = stamp ? clock64() : 0;
         float e0 = 0.f, e1 = 0.f;  // this lane's unit: its dot product(s)
         // shared-window addresses of the stage's rows / scale rows
@@ -1918,38 +2235,38 @@ __device__ KLLM_PHASE_CALL Carry gemv_phase(const Params& P, Carry carry, int to
           if (kTaskRows == 4 && nu == 2) {
             const Rows4 rp{{wa + i0 * rb, wa + (n + i0) * rb, wa + (i0 + 1) * rb, wa + (n + i0 + 1) * rb}};
             const Rows4 sp{{sa + i0 * srb, sa + (n + i0) * srb, sa + (i0 + 1) * srb, sa + (n + i0 + 1) * srb}};
-            const float4 d = dot_rows<4, INT8>(rp, sp, xa, M, ph.group_size, ph.group_shift, lane, int8_fast);
+            const float4 d = dot_rows_w8<4>(rp, sp, xa, M, ph.group_size, ph.group_shift, lane, int8_fast);
             e0 = lane == 0 ? d.x : d.z;
             e1 = lane == 0 ? d.y : d.w;
           } else {
             const Rows4 rp{{wa + i0 * rb, wa + (n + i0) * rb, 0u, 0u}};
             const Rows4 sp{{sa + i0 * srb, sa + (n + i0) * srb, 0u, 0u}};
-            const float4 d = dot_rows<2, INT8>(rp, sp, xa, M, ph.group_size, ph.group_shift, lane, int8_fast);
+            const float4 d = dot_rows_w8<2>(rp, sp, xa, M, ph.group_size, ph.group_shift, lane, int8_fast);
             e0 = d.x, e1 = d.y;
           }
         } else if (kTaskRows == 4 && nu == 4) {
           const Rows4 rp{{wa + i0 * rb, wa + (i0 + 1) * rb, wa + (i0 + 2) * rb, wa + (i0 + 3) * rb}};
           const Rows4 sp{{sa + i0 * srb, sa + (i0 + 1) * srb, sa + (i0 + 2) * srb, sa + (i0 + 3) * srb}};
-          const float4 d = dot_rows<4, INT8>(rp, sp, xa, M, ph.group_size, ph.group_shift, lane, int8_fast);
+          const float4 d = dot_rows_w8<4>(rp, sp, xa, M, ph.group_size, ph.group_shift, lane, int8_fast);
           e0 = lane == 0 ? d.x : lane == 1 ? d.y : lane == 2 ? d.z : d.w;
         } else {
           int r0 = 0;
           if (nu >= 2) {
             const Rows4 rp{{wa + i0 * rb, wa + (i0 + 1) * rb, 0u, 0u}};
             const Rows4 sp{{sa + i0 * srb, sa + (i0 + 1) * srb, 0u, 0u}};
-            const float4 d = dot_rows<2, INT8>(rp, sp, xa, M, ph.group_size, ph.group_shift, lane, int8_fast);
+            const float4 d = dot_rows_w8<2>(rp, sp, xa, M, ph.group_size, ph.group_shift, lane, int8_fast);
             e0 = lane == 0 ? d.x : d.y;
             r0 = 2;
           }
           if (r0 < nu) {  // nu is 1 or 3: one more row
             const Rows4 rp{{wa + (i0 + r0) * rb, 0u, 0u, 0u}};
             const Rows4 sp{{sa + (i0 + r0) * srb, 0u, 0u, 0u}};
-            const float4 d = dot_rows<1, INT8>(rp, sp, xa, M, ph.group_size, ph.group_shift, lane, int8_fast);
+            const float4 d = dot_rows_w8<1>(rp, sp, xa, M, ph.group_size, ph.group_shift, lane, int8_fast);
             if (lane == r0) e0 = d.x;
           }
         }
         const long long t_c = stamp ? clock64() : 0;
-        if (lane < nu) epilogue(u + i0 + lane, e0, e1, bias_v, res_v);
+        if (lane < nu) epilogue(dest, e0, e1);
         if (stamp) {
           cyc4[0] += t_b - t_a, cyc4[1] += t_c - t_b, cyc4[3] += clock64() - t_c;
         }
@@ -1959,34 +2276,6 @@ __device__ KLLM_PHASE_CALL Carry gemv_phase(const Params& P, Carry carry, int to
       if (lane == 0) mbar_arrive(&empty_bar[pipe.slot]);
       pipe.advance(S);
     }
-  } else {
-    // rows longer than a stage (fp32 only): the owning warp carries its partial sums across
-    // consecutive stages; chunk boundaries are multiples of 128 packs so every virtual
-    // thread still sees its packs in increasing order.
-    for (int u = u0; u < u1; ++u) {
-      const bool mine = (u - u0) % CW == warp;
-      float bias_v = 0.f, res_v = 0.f;
-      if (mine && lane == 0) prefetch_addend(u, bias_v, res_v);
-      float acc[1][4] = {{0.f, 0.f, 0.f, 0.f}};
-      for (int c = 0; c < ph.chunks_per_row; ++c) {
-        const int e0 = c * ph.chunk_elems;
-        const int ne = min(ph.chunk_elems, M - e0);
-        mbar_wait(&full_bar[pipe.slot], pipe.parity);
-        if (mine) {
-          const uint32_t w[1] = {smem_u32(stages + static_cast<size_t>(pipe.slot) * P.stage_bytes)};
-          accum_f32<1>(w, smem_u32(xs) + static_cast<uint32_t>(e0) * 4u, ne >> 2, lane, acc);
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty_bar[pipe.slot]);
-        pipe.advance(S);
-      }
-      if (mine) {
-        const float d0 = block128_sum_vt_packed(acc[0], lane);
-        if (lane == 0) epilogue(u, d0, 0.f, bias_v, res_v);
-      }
-    }
-  }
-
   if (ph.argmax) {
     // per-CTA (max, lowest index) of the classifier rows this CTA produced: the (up to four) lanes
     // that ran epilogues hold partial bests
@@ -2018,7 +2307,8 @@ __device__ KLLM_PHASE_CALL Carry gemv_phase(const Params& P, Carry carry, int to
     stamp[8] = static_cast<unsigned long long>(cyc_wait);
     stamp[9] = static_cast<unsigned long long>(cyc_rows);
   }
-  return Carry{pipe, best.v, best.i};
+  return Carry{pipe, best.v, best.i, 0u};
+  }
 }
 
 // ---- tensor parallel, classifier sharded by vocabulary ----------------------------------------------
@@ -2067,9 +2357,13 @@ __device__ __noinline__ void gather_logits_phase(const Params& P, int tok) {
 }
 
 // ---- the kernel ---------------------------------------------------------------------------------
-template <int CW, bool INT8, bool PROF>
-__global__ void __launch_bounds__(CW * 32 + 64, 1) decode_megakernel(const __grid_constant__ Params P) {
-  constexpr int CT = CW * 32;  // consumer threads
+// consumer warps, the ring producer, the L2 prefetcher and, where there are teams, the epilogue warp
+constexpr int mega_threads(int consumer_warps, int kind) { return consumer_warps * 32 + (has_teams(kind) ? 96 : 64); }
+template <int CW, int KIND, bool PROF>
+__global__ void __launch_bounds__(mega_threads(CW, KIND), 1) decode_megakernel(const __grid_constant__ Params P) {
+  constexpr bool TEAMS = has_teams(KIND);
+  constexpr int CT = CW * 32;                        // consumer threads
+  constexpr int JOIN = TEAMS ? CT + 32 : CT;         // ... and the epilogue warp's
   uint64_t* full_bar = g_full_bar;
   uint64_t* empty_bar = g_empty_bar;
   Phase& s_phase_cons = g_ph_cons;
@@ -2093,12 +2387,17 @@ __global__ void __launch_bounds__(CW * 32 + 64, 1) decode_megakernel(const __gri
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], CW);
     }
+    if (TEAMS)
+      for (int g = 0; g < 2; ++g) {
+        mbar_init(&g_part_full[g], 4 * (kGroupRows / team_task_rows(KIND)));
+        mbar_init(&g_part_empty[g], 1);
+      }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
 
   Pipe pipe{0, 0u};
-  constexpr int wbytes = INT8 ? 1 : 4;
+  constexpr int wbytes = KIND == kF32 ? 4 : 1;
 
   // =============================== producer warp ===============================================
   if (is_producer) {
@@ -2205,8 +2504,8 @@ __global__ void __launch_bounds__(CW * 32 + 64, 1) decode_megakernel(const __gri
           }
           continue;
         }
-        const int u0 = static_cast<int>(static_cast<long long>(cta) * ph.units / G);
-        const int u1 = static_cast<int>(static_cast<long long>(cta + 1) * ph.units / G);
+        const Share share = cta_share(ph, cta, G);
+        const int u0 = share.u0, u1 = share.u1;
         const int rpu = ph.swiglu ? 2 : 1;
         const int row_bytes = ph.in_dim * wbytes;
         if (ph.chunks_per_row == 1) {
@@ -2316,8 +2615,8 @@ __global__ void __launch_bounds__(CW * 32 + 64, 1) decode_megakernel(const __gri
           }
           continue;
         }
-        const int u0 = static_cast<int>(static_cast<long long>(cta) * ph.units / G);
-        const int u1 = static_cast<int>(static_cast<long long>(cta + 1) * ph.units / G);
+        const Share share = cta_share(ph, cta, G);
+        const int u0 = share.u0, u1 = share.u1;
         const int rpu = ph.swiglu ? 2 : 1;
         const int row_bytes = ph.in_dim * wbytes;
         auto throttle = [&]() {
@@ -2363,7 +2662,14 @@ __global__ void __launch_bounds__(CW * 32 + 64, 1) decode_megakernel(const __gri
     return;
   }
 
+  if constexpr (TEAMS)
+    if (warp == CW + 2) {
+      epilogue_role<CW, KIND, PROF>(P, lane);
+      return;
+    }
+
   // =============================== consumer warps ===============================================
+  unsigned groups = 0u;
   unsigned bar_target = P.barrier_base;
   int token = P.state->token;
   if (static_cast<unsigned>(token) >= static_cast<unsigned>(P.vocab_size)) token = 0;
@@ -2377,6 +2683,7 @@ __global__ void __launch_bounds__(CW * 32 + 64, 1) decode_megakernel(const __gri
   for (int tok = 0; tok < P.n_tokens; ++tok) {
     const float* emb_row = P.tok_emb + static_cast<size_t>(token) * P.dim;
     ArgBest best{0.f, -1};
+    if (TEAMS && tid == 0) g_s_token = token;
     if (P.xres_bytes) {
       // the residual stream starts as the embedding row (llama3.cpp:578-598); the previous token's
       // last reader of xres (classifier staging) is behind the grid barrier that closed that token
@@ -2410,7 +2717,7 @@ __global__ void __launch_bounds__(CW * 32 + 64, 1) decode_megakernel(const __gri
       if (ph.kind == kPhaseGather) {
         if (!(tok < P.skip_cls_tokens)) gather_logits_phase<CW>(P, tok);
         if (stamp) stamp[1] = stamp[2] = global_ns();
-        if (ph.barrier_after) grid_barrier<CT>(P.barrier, bar_target, G);
+        if (ph.barrier_after) grid_barrier<CT, JOIN>(P.barrier, bar_target, G);
         prev_barrier = ph.barrier_after != 0;
         if (stamp) stamp[3] = global_ns();
         continue;
@@ -2429,7 +2736,7 @@ __global__ void __launch_bounds__(CW * 32 + 64, 1) decode_megakernel(const __gri
                                           hand_tag(ph.hand_out), stamp);
         }
         if (stamp) stamp[1] = stamp[2] = global_ns();
-        if (ph.barrier_after) grid_barrier<CT>(P.barrier, bar_target, G);
+        if (ph.barrier_after) grid_barrier<CT, JOIN>(P.barrier, bar_target, G);
         prev_barrier = ph.barrier_after != 0;
         if (stamp) stamp[3] = global_ns();
         continue;
@@ -2440,11 +2747,12 @@ __global__ void __launch_bounds__(CW * 32 + 64, 1) decode_megakernel(const __gri
       // returns -1) skips the classifier -- its weights are not even streamed -- but keeps the grid
       // barrier that closes the token.
       if (!(ph.cls && tok < P.skip_cls_tokens)) {
-        const Carry out = gemv_phase<CW, INT8, PROF>(P, Carry{pipe, best.v, best.i}, tok, pos, emb_row, stamp);
+        const Carry out = gemv_phase<CW, KIND, PROF>(P, Carry{pipe, best.v, best.i, groups}, tok, pos, emb_row, stamp);
         pipe = out.pipe;
+        groups = out.groups;
         best.v = out.best_v, best.i = out.best_i;
       }
-      if (ph.barrier_after) grid_barrier<CT>(P.barrier, bar_target, G);
+      if (ph.barrier_after) grid_barrier<CT, JOIN>(P.barrier, bar_target, G);
       if (stamp) stamp[3] = global_ns();
     }
 
@@ -2484,16 +2792,20 @@ using mega::Phase;
 namespace {
 // PROF: the instantiation kllm_decoder_profile launches (its stamps cost registers in the row loops)
 template <bool PROF>
-const void* kernel_for(int consumer_warps, bool int8) {
-  if (int8) {
-    if (consumer_warps == 16) return reinterpret_cast<const void*>(mega::decode_megakernel<16, true, PROF>);
-    if (consumer_warps == 14) return reinterpret_cast<const void*>(mega::decode_megakernel<14, true, PROF>);
-    if (consumer_warps == 12) return reinterpret_cast<const void*>(mega::decode_megakernel<12, true, PROF>);
-    if (consumer_warps == 6) return reinterpret_cast<const void*>(mega::decode_megakernel<6, true, PROF>);
-    return reinterpret_cast<const void*>(mega::decode_megakernel<8, true, PROF>);
+const void* kernel_for(int consumer_warps, int kind) {
+  if (kind == mega::kW8) {
+    if (consumer_warps == 16) return reinterpret_cast<const void*>(mega::decode_megakernel<16, mega::kW8, PROF>);
+    if (consumer_warps == 14) return reinterpret_cast<const void*>(mega::decode_megakernel<14, mega::kW8, PROF>);
+    if (consumer_warps == 12) return reinterpret_cast<const void*>(mega::decode_megakernel<12, mega::kW8, PROF>);
+    if (consumer_warps == 6) return reinterpret_cast<const void*>(mega::decode_megakernel<6, mega::kW8, PROF>);
+    return reinterpret_cast<const void*>(mega::decode_megakernel<8, mega::kW8, PROF>);
   }
-  if (consumer_warps == 6) return reinterpret_cast<const void*>(mega::decode_megakernel<6, false, PROF>);
-  return reinterpret_cast<const void*>(mega::decode_megakernel<8, false, PROF>);
+  if (kind == mega::kW8Fast) {
+    if (consumer_warps == 8) return reinterpret_cast<const void*>(mega::decode_megakernel<8, mega::kW8Fast, PROF>);
+    return reinterpret_cast<const void*>(mega::decode_megakernel<12, mega::kW8Fast, PROF>);
+  }
+  if (consumer_warps == 12) return reinterpret_cast<const void*>(mega::decode_megakernel<12, mega::kF32, PROF>);
+  return reinterpret_cast<const void*>(mega::decode_megakernel<8, mega::kF32, PROF>);
 }
 }  // namespace
 
@@ -2532,12 +2844,6 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
   // them at 96 registers and spills).  Measured on B200 (profiles/README.md, passes Q-T): fp32 6 vs 8 warps
   // 1072 = 1072 (TinyLlama), 1218 < 1296 (Qwen2.5-0.5B), 210 < 213 (Llama-2-7B); int8 16 / 14 / 8 warps
   // 394 / 400 / 375 tok/s.
-  consumer_warps_ = int8 ? 14 : 8;
-  if (const char* e = getenv("KLLM_CONSUMER_WARPS")) {
-    const int v = atoi(e);
-    if (int8 && (v == 6 || v == 8 || v == 12 || v == 14 || v == 16)) consumer_warps_ = v;  // fast mode: CT >= 192 quantises M <= 16384 in <= 6 rounds
-    if (!int8 && (v == 6 || v == 8)) consumer_warps_ = v;
-  }
   // int8 arithmetic: "exact" reproduces the reference's fma(x * scale, float(w), acc) per element bit for
   // bit; "fast" (KLLM_INT8_MODE=fast) is the dp4a fixed-point mode (toleranced, ~3.5x fewer instructions)
   // The same switch frees the attention's summation order (flash-decoding, attention_flash_phase).
@@ -2546,9 +2852,21 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
   for (const char* name : {"KLLM_INT8_MODE", "KLLM_MODE"})
     if (const char* e = getenv(name)) fast_ = std::string(e) == "fast" ? 1 : 0;
   int8_fast_ = (int8 && fast_) ? 1 : 0;
-  kernel_ = kernel_for<false>(consumer_warps_, int8);
-  kernel_prof_ = kernel_for<true>(consumer_warps_, int8);
-  threads_ = consumer_warps_ * 32 + 64;
+  const char* mma_env = getenv("KLLM_INT8_MMA");
+  const bool int8_mma = mma_env != nullptr && atoi(mma_env) != 0;
+  const int kind = !int8 ? mega::kF32 : (int8_fast_ && m.group_size == 64 && !int8_mma ? mega::kW8Fast : mega::kW8);
+  // Consumer warps.  Teams: two (11 warps with the service ones: 168 registers each), three where a stage of short rows holds several
+  // tasks (us per token, 8 / 12 warps: stories15M 117 / 110, Qwen2.5-0.5B 669 / 655, TinyLlama-1.1B 812 / 828, Llama-2-7B int8 with 8
+  // layers 480 / 489).  int8 in the reference's order: 14, so that the CTA is 16 warps = 4 per scheduler with 128 registers each (16 / 14 / 8
+  // warps 394 / 400 / 375 tok/s).
+  consumer_warps_ = kind == mega::kW8 ? 14 : (kind == mega::kF32 && dim < 2048 ? 12 : 8);
+  if (const char* e = getenv("KLLM_CONSUMER_WARPS")) {
+    const int v = atoi(e);
+    if (kind == mega::kW8 ? v == 6 || v == 8 || v == 12 || v == 14 || v == 16 : v == 8 || v == 12) consumer_warps_ = v;
+  }
+  kernel_ = kernel_for<false>(consumer_warps_, kind);
+  kernel_prof_ = kernel_for<true>(consumer_warps_, kind);
+  threads_ = mega::mega_threads(consumer_warps_, kind);
 
   // Tagged exchange instead of "write x, grid barrier, read x" after o_proj and down_proj:
   // mandatory under tensor parallelism (it IS the all-reduce), optional on one GPU.
@@ -2633,13 +2951,11 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
     if (v == 1 || v == 2 || v == 4) forced_task_rows = v;
     if (std::string(e) == "auto") forced_task_rows = 0;
   }
-  // KLLM_INT8_MMA=1: int8 fast rows in the team form -- mma.sync m16n8k32 s8 for stages of 3-8 rows, dp4a with the
+  // KLLM_INT8_MMA=1: int8 fast rows on the tensor cores -- mma.sync m16n8k32 s8 for stages of 3-8 rows, dp4a with the
   // columns split over the team for 1-2 long rows.  Correct (the parity suite passes with it) but not faster on
   // B200: Llama-2-7B int8 398 (teams of 4, 12 warps) / 403 (pairs, 14 warps) vs 407 tok/s for the plain dp4a
   // rows (profiles/README.md, passes S and T) -- at one byte per weight the shared-memory reads of the
   // fragments cost what the dp4a arithmetic costs.  Off by default.
-  bool int8_mma = false;
-  if (const char* e = getenv("KLLM_INT8_MMA")) int8_mma = atoi(e) != 0;
   auto pick_task_rows = [&](Phase& p) {
     const int rpu = p.swiglu ? 2 : 1;
     p.task_rows = 4;
@@ -2664,6 +2980,8 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
     }
   };
   auto plan = [&](Phase& p) -> int {
+    p.cta_units = p.units / grid_;
+    p.cta_more = p.units % grid_;
     const int row_bytes = p.in_dim * wb;
     p.group_size = m.group_size;
     p.group_shift = -1;
@@ -2722,6 +3040,14 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
       p.scale_off = 0;
     }
     pick_task_rows(p);
+    p.units_per_stage = p.rows_per_stage / rpu;
+    const int task_rows = mega::team_task_rows(kind);
+    p.tasks_per_stage = (p.rows_per_stage + task_rows - 1) / task_rows;
+    for (int more = 0; more < 2; ++more) {
+      const int units = p.cta_units + more, ups = p.units_per_stage;
+      p.stages[more] = (units + ups - 1) / ups;
+      p.tasks[more] = units > 0 ? (p.stages[more] - 1) * p.tasks_per_stage + ((units - (p.stages[more] - 1) * ups) * rpu + task_rows - 1) / task_rows : 0;
+    }
     return 0;
   };
 
