@@ -5,7 +5,8 @@
 // keys, [token][kv_head][vdim] values, in the compute type).  All runs share ONE page numbering: a sequence that
 // owns page p owns it in every run's pool, so there is a single page table [slot][i] and a single free list.  A
 // sequence takes pages as it grows (lowest free number first, so freed pages are the next to be used again) and
-// returns them at close.  The table rows of the step's sequences are copied to the device before the kernels run.
+// returns them at close.  Pages taken by a step travel in the step's index block, and the step's first kernel enters them in
+// the device's table.  (A copy per sequence and step took 4 us each: 24 sequences, 95 of 340 us.)
 //
 // State.  A slot keeps its sequence's last token (bigram embedding).  Beside the pages, every layer run owns per-slot recurrent state in fp32: the last mixer input of a layer with a
 // token shift, the matrix state of linear attention, of the delta rule and of the duality mixer, the diagonal state of
@@ -141,6 +142,7 @@ struct kllm_seq_engine {
     bool live = false;
     int len = 0;
     int pages = 0;
+    int pages_on_device = 0;  // of them, those that the device's table has
     int32_t last = -1;  // the token before the next one (bigram embedding); -1: none yet
   };
   std::vector<Slot> slots;
@@ -618,13 +620,16 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
 
   // ---- host: validate, pages, index arrays ------------------------------------------------------------------------
   int T = 0, max_count = 0, max_ctx = 0, need_pages = 0;
+  size_t n_news = 0;  // pages that the device's table lacks
   for (int i = 0; i < n_entries; ++i) {
     const int s = seqs[i];
     if (s < 0 || s >= static_cast<int>(e->slots.size()) || !e->slots[s].live || counts[i] <= 0) return KLLM_E_INVALID;
     for (int j = 0; j < i; ++j)
       if (seqs[j] == s) return KLLM_E_INVALID;  // one entry per sequence and step
     const int new_len = e->slots[s].len + counts[i];
-    need_pages += (new_len + e->page - 1) / e->page - e->slots[s].pages;
+    const int pages = (new_len + e->page - 1) / e->page;
+    need_pages += pages - e->slots[s].pages;
+    n_news += pages - e->slots[s].pages_on_device;
     T += counts[i];
     max_count = std::max(max_count, counts[i]);
     max_ctx = std::max(max_ctx, new_len);
@@ -638,8 +643,8 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
     if (want_host[i] < 0 || want_host[i] >= T) return KLLM_E_INVALID;
 
   // layout of the index block (int32): tokens[T] tok_seq[T] tok_pos[T] prev_token[T] ent_first[E] ent_count[E] ent_seq[E] ent_pos0[E]
-  // want[n_want]
-  const size_t n_idx = 4 * static_cast<size_t>(T) + 4 * static_cast<size_t>(n_entries) + static_cast<size_t>(n_want);
+  // want[n_want] n_news {sequence, place in its row, page}[n_news]
+  const size_t n_idx = 4 * static_cast<size_t>(T) + 4 * static_cast<size_t>(n_entries) + static_cast<size_t>(n_want) + 1 + 3 * n_news;
   if (n_idx > e->pinned_cap) {
     if (e->pinned) cudaFreeHost(e->pinned);
     e->pinned = nullptr;
@@ -650,7 +655,9 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
   RC(e->idx.reserve(n_idx * sizeof(int32_t)));
   int32_t* hp = e->pinned;
   int32_t *h_tok = hp, *h_seq = hp + T, *h_pos = hp + 2 * T, *h_prev = hp + 3 * T, *h_first = hp + 4 * T, *h_count = h_first + n_entries,
-          *h_eseq = h_count + n_entries, *h_pos0 = h_eseq + n_entries, *h_want = h_pos0 + n_entries;
+          *h_eseq = h_count + n_entries, *h_pos0 = h_eseq + n_entries, *h_want = h_pos0 + n_entries, *h_news = h_want + n_want;
+  h_news[0] = static_cast<int32_t>(n_news);
+  int32_t* news = h_news + 1;
   std::memcpy(h_tok, tokens_host, static_cast<size_t>(T) * sizeof(int32_t));
   int at = 0;
   for (int i = 0; i < n_entries; ++i) {
@@ -671,15 +678,13 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
       e->free_pages.pop_back();
     }
     s.len = new_len;
-    CU(cudaMemcpyAsync(e->table_dev + static_cast<size_t>(seqs[i]) * e->table_stride, row, pages * sizeof(int32_t),
-                       cudaMemcpyHostToDevice, st));
+    for (int p = s.pages_on_device; p < s.pages; ++p, news += 3) news[0] = seqs[i], news[1] = p, news[2] = row[p];
   }
   if (n_want) std::memcpy(h_want, want_host, static_cast<size_t>(n_want) * sizeof(int32_t));
-  // the table rows above are pageable host memory: the copies are staged by the driver before the call returns
   CU(cudaMemcpyAsync(e->idx.p, hp, n_idx * sizeof(int32_t), cudaMemcpyHostToDevice, st));
   const int32_t* d_tok = static_cast<const int32_t*>(e->idx.p);
   const int32_t *d_seq = d_tok + T, *d_pos = d_tok + 2 * T, *d_prev = d_tok + 3 * T, *d_first = d_tok + 4 * T, *d_count = d_first + n_entries,
-                *d_eseq = d_count + n_entries, *d_pos0 = d_eseq + n_entries, *d_want = d_pos0 + n_entries;
+                *d_eseq = d_count + n_entries, *d_pos0 = d_eseq + n_entries, *d_want = d_pos0 + n_entries, *d_news = d_want + n_want;
 
   // ---- workspaces ----------------------------------------------------------------------------------------------
   // keys of a row tile are split over CTAs when the step itself offers few tiles (decode, short prompts)
@@ -789,8 +794,8 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
   e->mark(-1);
   auto run_device = [&]() -> int {
   RC(launch_embed(dtype, d.embed, d_tok, x, e->any_run_embed ? static_cast<float*>(e->x0.p) : nullptr, nw(d.embed_norm),
-                  d.norm_eps, d.embed_scale, BigramArgs{d.bigram, d_prev, d.bigram_mul_prev, d.bigram_mul_cur, d.bigram_buckets}, T, W,
-                  st));
+                  d.norm_eps, d.embed_scale, BigramArgs{d.bigram, d_prev, d.bigram_mul_prev, d.bigram_mul_cur, d.bigram_buckets},
+                  PageNews{d_news, e->table_dev, e->table_stride}, T, W, st));
   e->mark(KLLM_SEQ_PHASE_NORM);
   // What comes ahead of run r's mixer rides on one norm kernel (`a` may already carry the end of the run before):
   // the embedding output and the run's vector are added, the pre-norm is taken, and the token shift is applied -- inside
@@ -1280,6 +1285,7 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
     }
     e->prof_out = nullptr;
   }
+  for (int i = 0; i < n_entries; ++i) e->slots[seqs[i]].pages_on_device = e->slots[seqs[i]].pages;  // (a step that fails sends them again)
   if (e->wait.take()) return KLLM_E_STATE;
   return 0;
 }

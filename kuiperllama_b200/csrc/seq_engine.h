@@ -111,8 +111,14 @@ struct BigramArgs {
   int64_t mul_prev, mul_cur;
   int buckets;
 };
+// Also enters a step's new pages in the page tables: the number of them, then {sequence, place in its row, page} each.
+struct PageNews {
+  const int32_t* list;
+  int32_t* table;
+  int stride;
+};
 int launch_embed(int dtype, const void* table, const int32_t* tokens, float* x, float* copy, const NormW& norm, float eps,
-                 float scale, const BigramArgs& bigram, int T, int width, cudaStream_t s);
+                 float scale, const BigramArgs& bigram, const PageNews& news, int T, int width, cudaStream_t s);
 
 // x += N(c1 y1 + s2[t] * y2 + c3 y3 + c4 y4; post) (optional; y2, y3, y4 optional; post.w == null: the sum itself);  x += add_rows[t];
 // x += add (a [width] vector, optional);  out = N(x; pre) in the compute type (optional) -- in this order.  `rows` (optional) gathers: row i reads x[rows[i]], and x is then

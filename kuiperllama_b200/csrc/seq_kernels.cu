@@ -156,10 +156,14 @@ __device__ __forceinline__ void row_stats(const float* buf, int W, int kind, flo
 
 template <typename AT>
 __global__ void embed_kernel(const AT* __restrict__ table, const int32_t* __restrict__ tokens, float* __restrict__ x,
-                             float* __restrict__ copy, NormW norm, float eps, float scale, BigramArgs bi, int width) {
+                             float* __restrict__ copy, NormW norm, float eps, float scale, BigramArgs bi, PageNews news, int width) {
   extern __shared__ float buf[];
   __shared__ float red[33];
   const int t = blockIdx.x;
+  for (int i = t * blockDim.x + threadIdx.x, n = news.list[0]; i < n; i += gridDim.x * blockDim.x) {
+    const int32_t* e = news.list + 1 + 3 * static_cast<size_t>(i);
+    news.table[static_cast<size_t>(e[0]) * news.stride + e[1]] = e[2];
+  }
   const AT* row = table + static_cast<size_t>(tokens[t]) * width;
   const AT* pair = nullptr;  // the bigram's row
   if (bi.table != nullptr) {
@@ -1556,12 +1560,12 @@ inline int done() {
 }  // namespace
 
 int launch_embed(int dtype, const void* table, const int32_t* tokens, float* x, float* copy, const NormW& norm, float eps,
-                 float scale, const BigramArgs& bigram, int T, int width, cudaStream_t s) {
+                 float scale, const BigramArgs& bigram, const PageNews& news, int T, int width, cudaStream_t s) {
   if (scale == 0.f) scale = 1.0f;
   const size_t smem = static_cast<size_t>(width) * sizeof(float);
   if (smem > 48 * 1024) return KLLM_E_UNSUPPORTED;
   KLLM_SEQ_DISPATCH(dtype, (embed_kernel<AT><<<T, 128, smem, s>>>(static_cast<const AT*>(table), tokens, x, copy, norm, eps,
-                                                                 scale, bigram, width)));
+                                                                 scale, bigram, news, width)));
   return done();
 }
 
