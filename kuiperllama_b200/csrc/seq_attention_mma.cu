@@ -323,8 +323,14 @@ int launch_mma(const AttnShape& a, const void* q, const float* gates, const Page
 
 // ---- few rows ---------------------------------------------------------------------------------------------------------------
 // Grid: x = 16-row tile, y = (entry, key/value head), z = split.  Four warps.  Scores: a warp takes 8 keys of the tile
-// against all 16 rows.  Softmax: a warp takes 4 rows, a lane per key.  Output: the 8-column blocks are dealt out to the
+// against all 16 rows.  Softmax: a warp takes every fourth row, a lane per key.  Output: the 8-column blocks are dealt out to the
 // warps in turn (NBW per warp).  Values that are the head of the key row (SAME) are read from the key tile.
+// With one split the kernel finishes the rows itself (sink, output gate, conversion: what attention_merge_kernel does with one split,
+// operation by operation).
+// What bounds it at the contexts of a chat is a chain of latencies: index arrays, page table, keys, a few barriers per tile of keys.
+// The index arrays and the tables are complete before the step's second kernel begins (the step's first kernel, which enters new pages,
+// is not one that others begin under), and keys of earlier steps before the step does: so these are on their way before the kernel waits
+// for the one ahead of it, and only this step's own keys and queries come after.
 constexpr int kFewRows = 16, kFewKeys = 32, kFewThreads = 128, kFewWarps = 4;
 
 struct FewLayout {  // shared memory, in bytes from its start
@@ -353,15 +359,17 @@ template <int NBW, bool SAME, bool QF32>
 __global__ void __launch_bounds__(kFewThreads)
 attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t* ent_first,
                           const int32_t* ent_count, const int32_t* ent_seq,
-                          const int32_t* ent_pos0, int splits, float* ws) {
+                          const int32_t* ent_pos0, int splits, float* ws, const float* gates, void* out_) {
   next_may_start();
-  after_previous();
   const int e = blockIdx.y / a.kv_heads, g = blockIdx.y % a.kv_heads, split = blockIdx.z;
   const int gv = g / v_share_of(a);
   const int rep = a.heads / a.kv_heads, dim = a.dim, vdim = a.vdim;
   const int count = ent_count[e], first = ent_first[e], pos0 = ent_pos0[e];
   const int n_rows = count * rep, r0 = blockIdx.x * kFewRows;
-  if (r0 >= n_rows) return;
+  if (r0 >= n_rows) {
+    after_previous();
+    return;
+  }
   const int rows_here = min(kFewRows, n_rows - r0);
   const int32_t* table = kv.table + static_cast<size_t>(ent_seq[e]) * kv.table_stride;
   const int pmax = pos0 + (r0 + rows_here - 1) / rep;
@@ -393,9 +401,10 @@ attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t
   const __nv_bfloat16* kbase = static_cast<const __nv_bfloat16*>(kv.k) + static_cast<size_t>(g) * dim;
   const __nv_bfloat16* vbase = static_cast<const __nv_bfloat16*>(kv.v) + static_cast<size_t>(gv) * vdim;
   const int kc = L.dimp / 8, vc = SAME ? 0 : (ldv - 8) / 8;
-  auto load_tile = [&](int tile, int stage) {  // four threads per key: one page lookup per thread
+  auto load_tile = [&](int tile, int stage, bool old, bool mine) {  // four threads per key: one page lookup per thread
     const int j = tid >> 2, kj = tile * kFewKeys + j;
     const bool valid = kj <= pmax;
+    if (valid && kj >= pos0 ? !mine : !old) return;  // keys of this step; keys of earlier ones (and places past the last key)
     const size_t slot = valid ? static_cast<size_t>(table[kj / kv.page]) * kv.page + kj % kv.page : 0;
     const __nv_bfloat16 *kr = kbase + slot * kv.k_row, *vr = vbase + slot * kv.v_row;
     const uint32_t kd = k_addr + ((stage * kFewKeys + j) * ldk) * 2, vd = v_addr + ((stage * kFewKeys + j) * ldv) * 2;
@@ -407,9 +416,12 @@ attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t
       const bool in = valid && c * 8 < vdim;
       cp_async16(vd + c * 16, in ? vr + c * 8 : vbase, in);
     }
-    cp_async_commit();
   };
-  if (tile_lo < tile_hi) load_tile(tile_of(tile_lo), 0);
+  const int ahead = min(2, tile_hi - tile_lo);  // tiles that there are stages for
+  for (int i = 0; i < ahead; ++i) load_tile(tile_of(tile_lo + i), i, true, false);
+  after_previous();
+  for (int i = 0; i < ahead; ++i) load_tile(tile_of(tile_lo + i), i, false, true);
+  cp_async_commit();
 
   // the queries, two neighbouring coordinates at a time (dim is even); rows and coordinates that do not exist are zero
   const int half = L.dimp / 2;
@@ -450,8 +462,9 @@ attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t
 
   for (int li = tile_lo; li < tile_hi; ++li) {
     const int tile = tile_of(li), stage = (li - tile_lo) & 1, k0 = tile * kFewKeys;
-    if (li + 1 < tile_hi) {
-      load_tile(tile_of(li + 1), stage ^ 1);
+    if (li > tile_lo && li + 1 < tile_hi) {
+      load_tile(tile_of(li + 1), stage ^ 1, true, true);
+      cp_async_commit();
       cp_async_wait<1>();
     } else {
       cp_async_wait<0>();
@@ -483,7 +496,8 @@ attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < kFewRows / kFewWarps; ++i) {
-      const int r = warp * (kFewRows / kFewWarps) + i;
+      const int r = i * kFewWarps + warp;
+      if (r >= rows_here) break;  // (what the products make of rows that do not exist is not stored)
       const float sv = Ss[r * (kFewKeys + 1) + lane];
       float mx = sv;
 #pragma unroll
@@ -532,7 +546,26 @@ attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t
     const int r = gq + z * 8;
     if (r >= rows_here) continue;
     const int rr = r0 + r;
-    float* p = ws + ((static_cast<size_t>(first + rr / rep) * a.heads + g * rep + rr % rep) * splits + split) * pstride;
+    const size_t th = static_cast<size_t>(first + rr / rep) * a.heads + g * rep + rr % rep;
+    if (out_ != nullptr) {
+      const float m = m_s[r], sink = a.sink != nullptr ? a.sink[th % a.heads] : -INFINITY, M = fmaxf(m, sink);
+      const float w = m > -INFINITY ? expf(m - M) : 0.f;
+      const float weight = w / __fadd_rn(__fmul_rn(w, l_s[r]), a.sink != nullptr ? expf(sink - M) : 0.f);
+      const bool per_element = gates != nullptr && a.gate == KLLM_SEQ_GATE_ELEMENT;
+      const float head_gate = gates != nullptr && !per_element ? gates[th] : 1.0f;
+#pragma unroll
+      for (int i = 0; i < NBW; ++i) {
+        const int col = (warp + i * kFewWarps) * 8 + t4 * 2;
+        if (col >= vdim) continue;
+        const size_t at = th * vdim + col;
+        const float x = weight > 0.f ? weight * o[i][z * 2] : 0.f, y = weight > 0.f ? weight * o[i][z * 2 + 1] : 0.f;
+        const float gx = per_element ? gates[at] : head_gate, gy = per_element ? gates[at + 1] : head_gate;
+        if (a.out_f32) *reinterpret_cast<float2*>(static_cast<float*>(out_) + at) = make_float2(x * gx, y * gy);
+        else *reinterpret_cast<__nv_bfloat162*>(static_cast<__nv_bfloat16*>(out_) + at) = __floats2bfloat162_rn(x * gx, y * gy);
+      }
+      continue;
+    }
+    float* p = ws + (th * splits + split) * pstride;
     if (warp == 0 && t4 == 0) p[0] = m_s[r], p[1] = l_s[r];
 #pragma unroll
     for (int i = 0; i < NBW; ++i) {
@@ -545,7 +578,7 @@ attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t
 template <int NBW, bool SAME, bool QF32>
 int launch_few(const AttnShape& a, const void* q, const PagedKV& kv, int n_entries, const int32_t* ent_first,
                const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0, int max_count, int splits, float* ws,
-               cudaStream_t s) {
+               const float* gates, void* out, cudaStream_t s) {
   const size_t smem = few_layout(a, SAME, QF32).total;
   static size_t configured = 0;
   if (smem > 48 * 1024 && smem > configured) {
@@ -557,7 +590,7 @@ int launch_few(const AttnShape& a, const void* q, const PagedKV& kv, int n_entri
   const dim3 grid((max_count * (a.heads / a.kv_heads) + kFewRows - 1) / kFewRows, n_entries * a.kv_heads, splits);
   if (grid.y > 65535u) return KLLM_E_UNSUPPORTED;
   launch_ahead(attention_rows_mma_kernel<NBW, SAME, QF32>, dim3(grid), dim3(kFewThreads), smem, s, a, q, kv, ent_first, ent_count, ent_seq, ent_pos0,
-                                                                            splits, ws);
+                                                                            splits, ws, gates, out);
   count_launch();
   return cuda_rc(cudaGetLastError());
 }
@@ -579,15 +612,15 @@ bool attention_rows_mma_usable(int dtype, const AttnShape& a, const PagedKV& kv,
 
 int launch_attention_rows_mma(const AttnShape& a, const void* q, const PagedKV& kv, int n_entries, const int32_t* ent_first,
                               const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0, int max_count,
-                              int splits, float* ws, cudaStream_t s) {
+                              int splits, float* ws, const float* gates, void* out, cudaStream_t s) {
   const bool same = values_in_keys(a, kv);
 #define KLLM_FEW(N)                                                                                                              \
   if (a.vdim <= N * kFewWarps * 8) {                                                                                              \
     if (same)                                                                                                                     \
-      return a.q_f32 ? launch_few<N, true, true>(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, s)   \
-                     : launch_few<N, true, false>(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, s); \
-    return a.q_f32 ? launch_few<N, false, true>(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, s)    \
-                   : launch_few<N, false, false>(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, s);  \
+      return a.q_f32 ? launch_few<N, true, true>(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, gates, out, s)   \
+                     : launch_few<N, true, false>(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, gates, out, s); \
+    return a.q_f32 ? launch_few<N, false, true>(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, gates, out, s)    \
+                   : launch_few<N, false, false>(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, gates, out, s);  \
   }
   KLLM_FEW(2)
   KLLM_FEW(4)

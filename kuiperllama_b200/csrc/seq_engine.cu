@@ -687,12 +687,13 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
                 *d_eseq = d_count + n_entries, *d_pos0 = d_eseq + n_entries, *d_want = d_pos0 + n_entries, *d_news = d_want + n_want;
 
   // ---- workspaces ----------------------------------------------------------------------------------------------
-  // keys of a row tile are split over CTAs when the step itself offers few tiles (decode, short prompts)
+  // keys of a row tile are split over CTAs when the step itself offers few tiles (decode, short prompts) and there are more of them
+  // than the kernel that joins the splits is worth
   int splits = 1;
   {
     const int tiles = (max_ctx + kAttnKeys - 1) / kAttnKeys;
     const int ctas = n_entries * ((max_count * 8 + kAttnRows - 1) / kAttnRows);
-    if (ctas < 64) {
+    if (ctas < 64 && tiles > kFewTiles) {
       const int want = std::max(1, std::min({tiles, 32, 128 / std::max(1, ctas)}));
       while (splits < want) splits *= 2;  // a power of two: few distinct launch shapes as a context grows
     }

@@ -22,6 +22,7 @@ namespace seq {
 
 constexpr int kAttnRows = 32;   // (token, query head) rows of one attention CTA
 constexpr int kAttnKeys = 64;   // keys per tile
+constexpr int kFewTiles = 3;    // up to so many are not split: a tile takes about 1.5 us, the kernel that joins splits 3
 constexpr int kAttnThreads = 128;
 
 struct NormW {
@@ -222,11 +223,11 @@ int launch_attention_f32(const AttnShape& a, const void* q, const float* gates, 
                          int max_count, int splits, float* ws, void* out, cudaStream_t s);
 
 // bf16 steps of few rows per key head, or with fp32 queries (head sizes that are multiples of 8): partial results of every
-// split in `ws`, like the split-key kernel.
+// split in `ws`, like the split-key kernel, or (`out` not null, one split) the finished rows.
 bool attention_rows_mma_usable(int dtype, const AttnShape& a, const PagedKV& kv, int n_entries);
 int launch_attention_rows_mma(const AttnShape& a, const void* q, const PagedKV& kv, int n_entries, const int32_t* ent_first,
                               const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0, int max_count,
-                              int splits, float* ws, cudaStream_t s);
+                              int splits, float* ws, const float* gates, void* out, cudaStream_t s);
 
 // Token shift for steps with longer entries: out[t] = h[t] + (prev - h[t]) * mu in the compute type, prev = h[t - 1] inside
 // an entry, the sequence's state (zeros at position 0) for its first row; afterwards state[seq] = the entry's last h.

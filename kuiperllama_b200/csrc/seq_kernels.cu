@@ -1751,7 +1751,10 @@ int launch_attention(int dtype, const AttnShape& a, const void* q, const float* 
     rc = launch_attention_f32(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, s);
     if (rc || (splits == 1 && !a.no_merge)) return rc;
   } else if (attention_rows_mma_usable(dtype, a, kv, n_entries)) {
-    rc = launch_attention_rows_mma(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, s);
+    const bool whole = splits == 1 && !a.no_merge;
+    rc = launch_attention_rows_mma(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws,
+                                   a.gate ? gates : nullptr, whole ? out : nullptr, s);
+    if (rc || whole) return rc;
   } else if (a.vdim > 4 * kAttnKeys || a.dim > kAttnMaxDim || attention_tile_bytes(a) > kAttnMaxTileBytes) {
     const size_t smem = (static_cast<size_t>(a.dim) + a.vdim + kAttnKeys) * sizeof(float);
     if (smem > 48 * 1024 || kv.table == nullptr) return KLLM_E_UNSUPPORTED;
