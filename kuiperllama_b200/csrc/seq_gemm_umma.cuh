@@ -100,6 +100,66 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
 }
+// ---- pairs of CTAs (a cluster of two): one tcgen05.mma over both, each CTA's shared memory holding its half of either operand -----
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address of `saddr` (a shared-memory address of this CTA) in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t peer_smem(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+template <bool PAIR>
+__device__ __forceinline__ void load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+  if constexpr (PAIR)  // `bar` may be the other CTA's
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1) : "memory");
+  else
+    tma_load_2d(dst, map, bar, c0, c1);
+}
+__device__ __forceinline__ uint32_t pair_desc(uint32_t idesc) { return idesc + (static_cast<uint32_t>(BM >> 4) << 24); }  // M = 256
+__device__ __forceinline__ void mma_pair_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void mma_pair_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
+}
+// arrives on the barrier at this place in both CTAs
+__device__ __forceinline__ void mma_pair_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+               "h"(static_cast<uint16_t>(3)) : "memory");
+}
+// on a barrier of any CTA of the cluster (an address of peer_smem)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, const Stop& stop) {  // as mbar_wait, for such arrivals
+  for (uint32_t i = 0; i < kWaitLimit; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (ok) return true;
+    if ((i & 1023u) == 1023u && *stop.here) return false;
+  }
+  *stop.here = 1;
+  *reinterpret_cast<volatile int*>(stop.report) = 1;
+  __threadfence_system();
+  return false;
+}
 enum Mode { kBf16 = 0, kTf32 = 1, kFp32 = 2 };
 template <int MODE> struct ModeOf {  // fp32 operands
   using T = float;
@@ -189,12 +249,19 @@ __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, 
 }
 
 // ---- token blocks: persistent CTAs ----------------------------------------------------------------------------------
-// One CTA per SM walks tiles of 128 weight rows x BN tokens.  The tile's accumulator alternates between two sets of BN TMEM columns,
-// so the epilogue of a tile runs under the products of the next, and the ring never drains between tiles.
-// Why 256 tokens: at BN = 128 a CTA takes in 32 KB per 2 * 128 * 128 * 64 operations, more than the ~64 bytes a clock that reach an
-// SM from L2 can feed; 256 tokens need three quarters of the bytes per operation.  What bounds it now is no single unit: for
-// 2048 x 2048 x 8192 (65 us alone) the tensor pipe is busy in 51 % of the cycles, reads from L2 run at 39 % of their peak, shared memory
-// at 64 %; 512 tiles are 3.5 waves, and each operand is brought in by every CTA that meets it.
+// One CTA per SM walks tiles of 128 weight rows x 128 tokens, or two CTAs of a cluster tiles of 256 x 256 (BN = 256).  The tile's
+// accumulator alternates between two sets of BN TMEM columns, so the epilogue of a tile runs under the products of the next, and the
+// ring never drains between tiles.
+// Why pairs: a CTA by itself takes in 32 KB per 2 * 128 * 128 * 64 operations, 128 bytes a clock at the tensor cores' rate, and with 256
+// tokens 48 KB per twice as many (96).  A CTA of a pair holds 128 of the 256 weight rows and 128 of the 256 tokens, 32 KB, and the tensor
+// cores of both read both halves: 64 bytes a clock, and room for six stages instead of four.
+// The leader (rank 0) issues the products for both and waits for the loads of both on its own barrier; both load, and both store
+// the 128 rows of the accumulator that their TMEM holds.
+// Plain results leave through shared memory by TMA, 32 features x 16 tokens at a time: stored from registers, 32 features of a token per
+// instruction, a tile took 10 us to leave, which the products of a short K do not cover and the last tile never does.
+// 2048 x K x 8192 in us, calls back to back, one CTA to a tile of 256 tokens / pairs / and stores by TMA: K = 2048 64.5 / 61.2 / 57.4,
+// K = 512 - / 35.1 / 26.8; 4096 x 4096 x 4096 110 / 105 / 102, 1501 x 2048 x 3072 20.6 / 22.7 / 20.5.  What bounds it now: the tensor pipe is
+// busy in 66 % of the SMs' active cycles, which are 81 % of the kernel's (3.5 waves of tiles).
 // Gated: a tile is 64 features, its first 64 weight rows their gate rows, the other 64 their up rows.  The two TMEM halves meet
 // through shared memory: of every 32 columns the gate's warp finishes 16 and the up rows' warp 16.
 // Eight epilogue warps, four for either half of the columns: with four the activation of a tile takes longer than its products at
@@ -202,28 +269,36 @@ __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, 
 constexpr int kPairCols = 32;
 constexpr int kPersistentThreads = 64 + 256;
 constexpr int kExchangeBytes = 4 * 2 * kPairCols * 32 * 4;  // [half of the columns, pair of warps][buffer][column][lane]
-template <int BN>
-constexpr int kPersistentStages = BN == 256 ? 4 : 6;
-template <int BN, bool GATED>
+constexpr int kPersistentStages = 6;  // of 32 KB
 constexpr size_t persistent_smem() {
-  return 1024 + static_cast<size_t>(kPersistentStages<BN>) * (A_BYTES + BN * BK * 2) + (GATED ? kExchangeBytes : 0) + 256;
+  return 1024 + static_cast<size_t>(kPersistentStages) * (A_BYTES + 128 * BK * 2) + kExchangeBytes + 256;
+}
+// A warp's 32 features x 16 tokens, to be stored by TMA (which leaves out what is past the matrix)
+constexpr int kStoreTokens = 16;
+static_assert(8 * 2 * kStoreTokens * 32 * 4 <= kExchangeBytes, "two such blocks for each of the eight warps");
+__device__ __forceinline__ void store_2d(const CUtensorMap* map, uint32_t src, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1) : "memory");
 }
 
 template <int MODE, int BN, int OUT>
 __global__ void __launch_bounds__(kPersistentThreads, 1)
 umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_up,
-            const __grid_constant__ CUtensorMap map_a, const SplitArgs p) {
+            const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_out, const bool by_tma, const SplitArgs p) {
   static_assert(MODE != kFp32, "operands are taken as they arrive");
   constexpr bool GATED = OUT == kGated;
   constexpr int BKE = ModeOf<MODE>::BKE;
   const int T = p.T, N = p.N, K = p.K;
-  constexpr int ST = kPersistentStages<BN>, B_BYTES = BN * BK * 2, STAGE = A_BYTES + B_BYTES;
-  constexpr int FEATURES = GATED ? BM / 2 : BM;  // of a tile
+  constexpr bool PAIR = BN == 256;
+  constexpr int CTAS = PAIR ? 2 : 1;
+  constexpr int ST = kPersistentStages, B_ROWS = BN / CTAS, B_BYTES = B_ROWS * BK * 2, STAGE = A_BYTES + B_BYTES;
+  constexpr int FEATURES = GATED ? BM / 2 : BM;  // of a CTA
   constexpr uint32_t TMEM_COLS = 2 * BN;
+  const int rank = PAIR ? static_cast<int>(cluster_rank()) : 0;
   extern __shared__ uint8_t raw_smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
-  float* exchange = reinterpret_cast<float*>(base + ST * STAGE);  // gated
-  uint64_t* full = reinterpret_cast<uint64_t*>(base + ST * STAGE + (GATED ? kExchangeBytes : 0));
+  float* exchange = reinterpret_cast<float*>(base + ST * STAGE);  // gated; else what is on its way out, 4 KB a warp
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + ST * STAGE + kExchangeBytes);
   uint64_t* empty = full + ST;
   uint64_t* acc_full = empty + ST;     // [2]
   uint64_t* acc_empty = acc_full + 2;  // [2]
@@ -232,7 +307,8 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kblocks = (K + BKE - 1) / BKE;
-  const int feature_tiles = (N + FEATURES - 1) / FEATURES, tiles = feature_tiles * ((T + BN - 1) / BN);
+  const int feature_tiles = (N + CTAS * FEATURES - 1) / (CTAS * FEATURES), tiles = feature_tiles * ((T + BN - 1) / BN);
+  const int first = blockIdx.x / CTAS, step = gridDim.x / CTAS;  // of the tiles that this CTA or pair takes
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < ST; ++s) {
@@ -241,18 +317,28 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&acc_full[b]), 1);
-      mbar_init(smem_u32(&acc_empty[b]), 8);
+      mbar_init(smem_u32(&acc_empty[b]), 8 * CTAS);
     }
     *stop.here = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                   "r"(TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                   "r"(TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if constexpr (PAIR) {
+    __syncwarp();
+    cluster_sync();  // both CTAs' barriers and columns are there
+  }
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_d = *tmem_slot;
 
@@ -260,29 +346,34 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
     if (lane == 0) {
       int i = 0;  // blocks of K so far, over all tiles
       bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const int n0 = (tile % feature_tiles) * FEATURES, t0 = (tile / feature_tiles) * BN;
+      for (int tile = first; tile < tiles && ok; tile += step) {
+        const int n0 = ((tile % feature_tiles) * CTAS + rank) * FEATURES, t0 = (tile / feature_tiles) * BN + rank * B_ROWS;
         for (int kb = 0; kb < kblocks; ++kb, ++i) {
           const int s = i % ST;
           ok = mbar_wait(smem_u32(&empty[s]), ((i / ST) & 1) ^ 1u, stop);
           if (!ok) break;
-          const uint32_t bar = smem_u32(&full[s]);
+          uint32_t bar = smem_u32(&full[s]);
           uint8_t* st = base + s * STAGE;
-          mbar_expect_tx(bar, STAGE);
-          tma_load_2d(smem_u32(st), &map_w, bar, kb * BKE, n0);
-          if (GATED) tma_load_2d(smem_u32(st + A_BYTES / 2), &map_up, bar, kb * BKE, n0);
-          tma_load_2d(smem_u32(st + A_BYTES), &map_a, bar, kb * BKE, t0);
+          if (rank == 0) mbar_expect_tx(bar, CTAS * STAGE);  // of a pair, for both (the other's bytes may land before this)
+          if constexpr (PAIR) bar = peer_smem(bar, 0);
+          load_2d<PAIR>(smem_u32(st), &map_w, bar, kb * BKE, n0);
+          if (GATED) load_2d<PAIR>(smem_u32(st + A_BYTES / 2), &map_up, bar, kb * BKE, n0);
+          load_2d<PAIR>(smem_u32(st + A_BYTES), &map_a, bar, kb * BKE, t0);
         }
       }
+      // a pair's last arrivals come from the leader: this CTA is still there for them
+      for (int end = i + ST; PAIR && ok && i < end; ++i) ok = mbar_wait(smem_u32(&empty[i % ST]), ((i / ST) & 1) ^ 1u, stop);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = MODE == kBf16 ? instr_desc(BN) : instr_desc_tf32(BN);
+    if (lane == 0 && rank == 0) {
+      uint32_t idesc = MODE == kBf16 ? instr_desc(BN) : instr_desc_tf32(BN);
+      if constexpr (PAIR) idesc = pair_desc(idesc);
       int i = 0, done = 0;  // blocks of K and tiles so far
       bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++done) {
+      for (int tile = first; tile < tiles && ok; tile += step, ++done) {
         const int b = done & 1;
-        ok = mbar_wait(smem_u32(&acc_empty[b]), ((done >> 1) & 1) ^ 1u, stop);
+        const uint32_t free = smem_u32(&acc_empty[b]), free_parity = ((done >> 1) & 1) ^ 1u;
+        ok = PAIR ? mbar_wait_cluster(free, free_parity, stop) : mbar_wait(free, free_parity, stop);
         for (int kb = 0; kb < kblocks && ok; ++kb, ++i) {
           const int s = i % ST;
           ok = mbar_wait(smem_u32(&full[s]), (i / ST) & 1, stop);
@@ -291,13 +382,20 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
           const uint32_t a_addr = smem_u32(base + s * STAGE), b_addr = a_addr + A_BYTES;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {  // 32 bytes of K per instruction, inside the swizzle row
-            const uint32_t joins = (kb > 0 || k > 0) ? 1u : 0u;
-            if constexpr (MODE == kBf16) mma_bf16(tmem_d + b * BN, smem_desc(a_addr + k * 32), smem_desc(b_addr + k * 32), idesc, joins);
-            else mma_tf32(tmem_d + b * BN, smem_desc(a_addr + k * 32), smem_desc(b_addr + k * 32), idesc, joins);
+            const uint32_t joins = (kb > 0 || k > 0) ? 1u : 0u, d = tmem_d + b * BN;
+            const uint64_t wd = smem_desc(a_addr + k * 32), ad = smem_desc(b_addr + k * 32);
+            if constexpr (PAIR && MODE == kBf16) mma_pair_bf16(d, wd, ad, idesc, joins);
+            else if constexpr (PAIR) mma_pair_tf32(d, wd, ad, idesc, joins);
+            else if constexpr (MODE == kBf16) mma_bf16(d, wd, ad, idesc, joins);
+            else mma_tf32(d, wd, ad, idesc, joins);
           }
-          mma_commit(smem_u32(&empty[s]));
+          if constexpr (PAIR) mma_pair_commit(smem_u32(&empty[s]));
+          else mma_commit(smem_u32(&empty[s]));
         }
-        if (ok) mma_commit(smem_u32(&acc_full[b]));
+        if (ok) {
+          if constexpr (PAIR) mma_pair_commit(smem_u32(&acc_full[b]));
+          else mma_commit(smem_u32(&acc_full[b]));
+        }
       }
     }
   } else {
@@ -305,8 +403,8 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
     const int half = (warp - 2) >> 2, c_begin = half * (BN / 2), c_end = c_begin + BN / 2;  // this warp's columns
     int done = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++done) {
-      const int n0 = (tile % feature_tiles) * FEATURES, t0 = (tile / feature_tiles) * BN, b = done & 1;
+    for (int tile = first; tile < tiles; tile += step, ++done) {
+      const int n0 = ((tile % feature_tiles) * CTAS + rank) * FEATURES, t0 = (tile / feature_tiles) * BN, b = done & 1;
       // a warp whose wait ran out stores nothing more, but still meets its partner at every barrier below
       ok = warp_wait(ok, smem_u32(&acc_full[b]), (done >> 1) & 1, stop);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -314,7 +412,10 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
       auto release = [&]() {
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+        if (lane == 0) {
+          if constexpr (PAIR) mbar_arrive_cluster(peer_smem(smem_u32(&acc_empty[b]), 0));
+          else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+        }
       };
       if constexpr (!GATED) {
         const int row = n0 + quarter * 32 + lane;
@@ -325,7 +426,24 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
           tmem_ld32(from + c, r);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if (c + 32 == c_end) release();
-          if (ok && row < N) {
+          if (OUT == kPlain && by_tma) {
+            float* block = exchange + (warp - 2) * (2 * kStoreTokens * 32);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              float* buf = block + h * kStoreTokens * 32;
+              asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // what was here last has left (a group at every turn, full or not)
+              __syncwarp();
+#pragma unroll
+              for (int j = 0; j < kStoreTokens; ++j) buf[j * 32 + lane] = __uint_as_float(r[h * kStoreTokens + j]) + add;
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+              __syncwarp();
+              const int t = t0 + c + h * kStoreTokens, n = n0 + quarter * 32;
+              if (lane == 0) {
+                if (ok && t < T && n < N) store_2d(&map_out, smem_u32(buf), n, t);
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+              }
+            }
+          } else if (ok && row < N) {
             const size_t at = static_cast<size_t>(t0 + c) * N + row;
             float* out = static_cast<float*>(p.out) + at;
 #pragma unroll
@@ -376,14 +494,20 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
       }
     }
   }
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // this thread's stores are done
   if (*stop.here) {  // a wait ran out: give copies in flight time to land before the shared memory is given up
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if constexpr (PAIR) {
+    __syncwarp();
+    cluster_sync();  // nothing reads or signals this CTA's shared memory any more
+  }
   if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(TMEM_COLS) : "memory");
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(TMEM_COLS) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(TMEM_COLS) : "memory");
   }
 }
 
@@ -400,13 +524,18 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
 // 1501 tokens, 4 of 32 experts, K = 2048, N = 768 gated and back: 114 + 54 us in tiles of 64 rows, 82 + 34 us in tiles of up to 256.
 constexpr int GBN = 64;  // rows per box, and what the sorted order is padded to
 constexpr int kGroupRows = 256;
+constexpr int kGroupStages = 4;
+template <bool GATED>
+constexpr size_t grouped_smem() {
+  return 1024 + static_cast<size_t>(kGroupStages) * (A_BYTES + kGroupRows * BK * 2) + (GATED ? 2 * 2 * kPairCols * 32 * 4 : 0) + 256;
+}
 template <int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, void* __restrict__ out_,
                     const int32_t* __restrict__ sorted_pair, const int4* __restrict__ list, const int32_t* __restrict__ n_tiles, int N,
                     int K, GatedAct act, int* report) {
   constexpr bool GATED = EPI == 1;
-  constexpr int ST = kPersistentStages<256>, STAGE = A_BYTES + kGroupRows * BK * 2;
+  constexpr int ST = kGroupStages, STAGE = A_BYTES + kGroupRows * BK * 2;
   constexpr int FEATURES = GATED ? BM / 2 : BM;
   constexpr uint32_t TMEM_COLS = 2 * kGroupRows;
   extern __shared__ uint8_t raw_smem[];
@@ -616,6 +745,19 @@ inline int make_map_of(CUtensorMap* map, const void* ptr, int rows, int cols, in
   return r == CUDA_SUCCESS ? 0 : KLLM_E_INVALID;
 }
 
+// [T, N] fp32, box [kStoreTokens x 32], rows side by side in shared memory
+inline int make_out_map(CUtensorMap* map, void* ptr, int T, int N) {
+  EncodeTiledFn fn = encode_tiled();
+  if (fn == nullptr) return KLLM_E_NODEVICE;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(T)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(N) * 4};
+  const cuuint32_t box[2] = {32u, static_cast<cuuint32_t>(kStoreTokens)};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : KLLM_E_INVALID;
+}
+
 template <int MODE, int BN, int OUT>
 inline int launch_persistent(SplitArgs p, cudaStream_t stream) {
   constexpr int FEATURES = OUT == kGated ? BM / 2 : BM;
@@ -623,8 +765,13 @@ inline int launch_persistent(SplitArgs p, cudaStream_t stream) {
   if (p.report == nullptr) return KLLM_E_STATE;
   if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, FEATURES)) return rc;
   if (int rc = make_map_of<MODE>(&map_up, OUT == kGated ? p.w2 : p.w, p.N, p.K, FEATURES)) return rc;
-  if (int rc = make_map_of<MODE>(&map_a, p.a, p.T, p.K, BN)) return rc;
-  constexpr size_t smem = persistent_smem<BN, OUT == kGated>();
+  constexpr int CTAS = BN == 256 ? 2 : 1;
+  if (int rc = make_map_of<MODE>(&map_a, p.a, p.T, p.K, BN / CTAS)) return rc;
+  CUtensorMap map_out = map_a;  // (unused where the stores are not TMA's)
+  const bool by_tma = OUT == kPlain && p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+  if (by_tma)
+    if (int rc = make_out_map(&map_out, p.out, p.T, p.N)) return rc;
+  constexpr size_t smem = persistent_smem();
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kernel = umma_kernel<MODE, BN, OUT>;
   static bool configured = false;
@@ -633,10 +780,20 @@ inline int launch_persistent(SplitArgs p, cudaStream_t stream) {
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
-  const int tiles = ((p.N + FEATURES - 1) / FEATURES) * ((p.T + BN - 1) / BN);
-  kernel<<<tiles < kSms ? tiles : kSms, kPersistentThreads, smem, stream>>>(map_w, map_up, map_a, p);
+  const int tiles = ((p.N + CTAS * FEATURES - 1) / (CTAS * FEATURES)) * ((p.T + BN - 1) / BN), most = kSms / CTAS;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((tiles < most ? tiles : most) * CTAS);
+  cfg.blockDim = dim3(kPersistentThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CTAS, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CTAS > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_up, map_a, map_out, by_tma, p);
   count_launch();
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 // Whether there is about a tile of 128 tokens for every SM.  Below that, splitting K over CTAs gives more where the split kernel takes
 // tiles of 128 tokens too (TF32, T = 900, N = 2048, 128 tiles, K = 2048 and 5632: 26 and 104 us split, 29 and 117 us here).
@@ -654,7 +811,7 @@ inline bool persistent_pays(int T, int N, int features) {
 template <int MODE, int OUT>
 inline int launch_wide(const SplitArgs& p, cudaStream_t s) {
   const int feature_tiles = OUT == kGated ? (p.N + BM / 2 - 1) / (BM / 2) : (p.N + BM - 1) / BM;
-  const int waves_wide = (feature_tiles * ((p.T + 255) / 256) + kSms - 1) / kSms;
+  const int waves_wide = ((feature_tiles + 1) / 2 * ((p.T + 255) / 256) + kSms / 2 - 1) / (kSms / 2);
   const int waves = (feature_tiles * ((p.T + 127) / 128) + kSms - 1) / kSms;
   if (100 * waves_wide <= 65 * waves) return launch_persistent<MODE, 256, OUT>(p, s);
   return launch_persistent<MODE, 128, OUT>(p, s);
@@ -724,7 +881,7 @@ inline int launch_grouped(const void* a, const void* w, void* out, const int32_t
   if (report == nullptr) return KLLM_E_STATE;
   if (int rc = make_map(&map_w, w, experts * (EPI == 1 ? 2 : 1) * N, K, FEATURES)) return rc;
   if (int rc = make_map(&map_a, a, n_blocks * GBN, K, GBN)) return rc;
-  constexpr size_t smem = persistent_smem<256, EPI == 1>();
+  constexpr size_t smem = grouped_smem<EPI == 1>();
   static bool configured = false;
   if (!configured) {
     const cudaError_t e = cudaFuncSetAttribute(umma_grouped_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
