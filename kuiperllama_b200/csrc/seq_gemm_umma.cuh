@@ -260,8 +260,9 @@ __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, 
 // Plain results leave through shared memory by TMA, 32 features x 16 tokens at a time: stored from registers, 32 features of a token per
 // instruction, a tile took 10 us to leave, which the products of a short K do not cover and the last tile never does.
 // 2048 x K x 8192 in us, calls back to back, one CTA to a tile of 256 tokens / pairs / and stores by TMA: K = 2048 64.5 / 61.2 / 57.4,
-// K = 512 - / 35.1 / 26.8; 4096 x 4096 x 4096 110 / 105 / 102, 1501 x 2048 x 3072 20.6 / 22.7 / 20.5.  What bounds it now: the tensor pipe is
-// busy in 66 % of the SMs' active cycles, which are 81 % of the kernel's (3.5 waves of tiles).
+// K = 512 - / 35.1 / 26.8; 4096 x 4096 x 4096 110 / 105 / 102, 1501 x 2048 x 3072 20.6 / 22.7 / 20.5.  What bounds it now is what an SM
+// takes in: a block of K lasts some 560 cycles whatever the tile (256 x 256 on a pair, 256 x 128 on a pair, 128 x 128 on a CTA; 32 KB a CTA,
+// 58 of the 64 bytes a clock that reach an SM), so a tile of 256 x 256 costs no more time than a small one; its products take 512.
 // Gated: a tile is 64 features, its first 64 weight rows their gate rows, the other 64 their up rows.  The two TMEM halves meet
 // through shared memory: of every 32 columns the gate's warp finishes 16 and the up rows' warp 16.
 // Eight epilogue warps, four for either half of the columns: with four the activation of a tile takes longer than its products at
@@ -807,7 +808,8 @@ inline bool persistent_pays(int T, int N, int features) {
   if (T <= 128) return fills_chip(T, N);
   return ((N + features - 1) / features) * ((T + 127) / 128) > kSms / 2;
 }
-// The wider tile, unless its last wave is so empty that the narrower one, whose tiles take 0.65 of the time, is done sooner.
+// The wider tile, unless its last wave is so empty that the narrower one is done sooner (us, pairs / 128 x 128: 1501 x 2048 x 2048 20.0 / 27.6,
+// 2048 x 1024 x 1024 14.5 / 12.3, 900 x 2048 x 2048 18.6 / 16.8, 1024 x 4096 x 4096 30.9 / 47.2, 6001 x 2048 x 2048 43.2 / 68.3).
 template <int MODE, int OUT>
 inline int launch_wide(const SplitArgs& p, cudaStream_t s) {
   const int feature_tiles = OUT == kGated ? (p.N + BM / 2 - 1) / (BM / 2) : (p.N + BM - 1) / BM;
