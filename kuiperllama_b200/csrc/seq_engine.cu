@@ -167,7 +167,7 @@ struct kllm_seq_engine {
     uint64_t generation = 0;
     int nodes = 0;
   };
-  std::map<std::tuple<int, int, int, int>, Graph> graphs;
+  std::map<std::tuple<int, int, int, bool, bool>, Graph> graphs;
   bool own_stream = false;
   cudaStream_t side = nullptr;  // a pair's second mixer runs here, between `fork` and `join`
   cudaEvent_t fork = nullptr, join = nullptr;
@@ -687,13 +687,12 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
                 *d_eseq = d_count + n_entries, *d_pos0 = d_eseq + n_entries, *d_want = d_pos0 + n_entries, *d_news = d_want + n_want;
 
   // ---- workspaces ----------------------------------------------------------------------------------------------
-  // keys of a row tile are split over CTAs when the step itself offers few tiles (decode, short prompts) and there are more of them
-  // than the kernel that joins the splits is worth
+  // keys of a row tile are split over CTAs when the step itself offers few tiles (decode, short prompts)
   int splits = 1;
   {
     const int tiles = (max_ctx + kAttnKeys - 1) / kAttnKeys;
     const int ctas = n_entries * ((max_count * 8 + kAttnRows - 1) / kAttnRows);
-    if (ctas < 64 && tiles > kFewTiles) {
+    if (ctas < 64) {
       const int want = std::max(1, std::min({tiles, 32, 128 / std::max(1, ctas)}));
       while (splits < want) splits *= 2;  // a power of two: few distinct launch shapes as a context grows
     }
@@ -1236,7 +1235,7 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
   const bool all_single = single && !tracing && e->prof_out == nullptr && e->use_graphs && T <= 32;
   bool replayed = false;
   if (all_single) {
-    const auto key = std::make_tuple(n_entries, n_want, splits, argmax_host ? 1 : 0);
+    const auto key = std::make_tuple(n_entries, n_want, splits, few_keys(max_ctx), argmax_host != nullptr);
     kllm_seq_engine::Graph& g = e->graphs[key];
     if (g.exec != nullptr && g.generation != g_buffer_generation) {
       cudaGraphExecDestroy(g.exec);
