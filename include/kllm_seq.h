@@ -345,7 +345,9 @@ int kllm_seq_free_pages(const kllm_seq_engine* eng);
 /* One step.  Entry e appends counts[e] tokens (tokens_host, concatenated in entry order) to sequence seqs[e].
  * want_host lists the rows (indices into the concatenated tokens) whose logits are wanted; they are written to
  * logits_host [n_want, vocab] (fp32) and, when argmax_host is given, their greedy ids to argmax_host [n_want].
- * Blocking: returns after the results are in host memory. */
+ * Blocking: returns after the results are in host memory.  A step that returns an error has taken nothing in: lengths and last tokens are
+ * what they were.  Only state that layers keep instead of a cache (token shift, convolutions, linear and other recurrent mixers) may have
+ * begun to take its tokens in: close such sequences. */
 int kllm_seq_step(kllm_seq_engine* eng, int32_t n_entries, const int32_t* seqs, const int32_t* counts,
                   const int32_t* tokens_host, int32_t n_want, const int32_t* want_host, float* logits_host,
                   int32_t* argmax_host);

@@ -332,9 +332,10 @@ int launch_mma(const AttnShape& a, const void* q, const float* gates, const Page
 // 12 steps of 4 layers, us: 3925 with that kernel, 3810 without; one running softmax over all keys instead of splits took 3735, but its
 // sums are others.)
 // What bounds it at the contexts of a chat is a chain of latencies: index arrays, page table, keys, a few barriers per tile of keys.
-// The index arrays and the tables are complete before the step's second kernel begins (the step's first kernel, which enters new pages,
-// is not one that others begin under), and keys of earlier steps before the step does: so these are on their way before the kernel waits
-// for the one ahead of it, and only this step's own keys and queries come after.
+// Keys of earlier steps are on their way before the kernel waits for the one ahead of it.  That is safe for what was there before the step
+// began: the index arrays (copied ahead of its first kernel, which is no early one), the keys that completed steps wrote, and the entries
+// of the page table that lead to them, which those steps entered.  What this step writes, its own keys, queries and the entries of its new
+// pages (the host leaves none of them in the way of an earlier key, also after a step that failed), comes after the wait.
 constexpr int kFewRows = 16, kFewKeys = 32, kFewThreads = 128, kFewWarps = 4;
 constexpr int kFewParts = 4;  // splits that a CTA joins (the power of two over kFewTiles)
 static_assert(kFewTiles <= kFewParts, "a split for every tile of a short context");

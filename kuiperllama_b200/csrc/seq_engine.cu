@@ -107,7 +107,10 @@ struct DevBuf {
     cap = 0;
     const size_t want = bytes + bytes / 4 + 256;
     const cudaError_t e = cudaMalloc(&p, want);
-    if (e != cudaSuccess) return static_cast<int>(e);
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // reported here; the next launch's check is not to find it again
+      return static_cast<int>(e);
+    }
     cap = want;
     return 0;
   }
@@ -659,9 +662,29 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
   h_news[0] = static_cast<int32_t>(n_news);
   int32_t* news = h_news + 1;
   std::memcpy(h_tok, tokens_host, static_cast<size_t>(T) * sizeof(int32_t));
+  // A step that fails takes nothing in: its sequences are what they were, and no kernel of a later step takes for one with keys of earlier
+  // steps a page whose entry the device's table may lack.
+  struct Undo {
+    kllm_seq_engine* e;
+    const int32_t* seqs;
+    std::vector<kllm_seq_engine::Slot> were;
+    bool failed = true;
+    ~Undo() {
+      if (!failed) return;
+      cudaStreamSynchronize(e->stream);  // what is under way reads the index block
+      cudaGetLastError();
+      for (size_t i = were.size(); i-- > 0;) {  // (the other way round: the free list is in its order again)
+        kllm_seq_engine::Slot& s = e->slots[seqs[i]];
+        while (s.pages > were[i].pages) e->free_pages.push_back(e->table_host[static_cast<size_t>(seqs[i]) * e->table_stride + --s.pages]);
+        s = were[i];
+      }
+    }
+  } undo{e, seqs, {}};
+  undo.were.reserve(n_entries);
   int at = 0;
   for (int i = 0; i < n_entries; ++i) {
     kllm_seq_engine::Slot& s = e->slots[seqs[i]];
+    undo.were.push_back(s);
     h_first[i] = at, h_count[i] = counts[i], h_eseq[i] = seqs[i], h_pos0[i] = s.len;
     for (int j = 0; j < counts[i]; ++j) {
       h_seq[at + j] = seqs[i], h_pos[at + j] = s.len + j;
@@ -1285,8 +1308,9 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
     }
     e->prof_out = nullptr;
   }
-  for (int i = 0; i < n_entries; ++i) e->slots[seqs[i]].pages_on_device = e->slots[seqs[i]].pages;  // (a step that fails sends them again)
   if (e->wait.take()) return KLLM_E_STATE;
+  for (int i = 0; i < n_entries; ++i) e->slots[seqs[i]].pages_on_device = e->slots[seqs[i]].pages;
+  undo.failed = false;
   return 0;
 }
 

@@ -2,7 +2,9 @@
 // a chain of some thirty to sixty kernels of a few microseconds; without this each begins only when the one before has drained.
 //
 // A kernel launched by launch_ahead() calls after_previous() before it reads anything that an earlier kernel wrote and before it
-// writes anything; ahead of that call it may set itself up and read weights, which no kernel writes.  Every such kernel does call
+// writes anything; ahead of that call it may set itself up and read weights, which no kernel writes, and, in a step of the engine, what was
+// complete before the step's first kernel began, which is an ordinary launch: the step's index arrays, and keys and page entries of
+// earlier steps.  (That an earlier kernel of the step must have ended is not enough: only the wait makes its stores visible.)  Every such kernel does call
 // it, so a kernel that has finished vouches for all kernels before it, not for its predecessor alone.  next_may_start() lets the
 // following kernel's CTAs take up what room is left; a kernel that allocates TMEM calls it after the allocation, so that a CTA which
 // waits for this kernel never holds columns that this kernel still needs.

@@ -47,6 +47,34 @@ def test_only_weights_take_the_read_only_path(name, parameters, code):
     assert "ld.global.nc" not in code
 
 
+# what a kernel reads ahead of its wait: weights, and what was complete before the step's first kernel began
+EARLY = {"rows_kernel": {"w"}, "rows_gated_kernel": {"w"}, "umma_split_kernel": {"map_w", "map_w2", "p"},
+         "attention_rows_mma_kernel": {"ent_first", "ent_count", "ent_seq", "ent_pos0", "kv"}}
+
+
+@pytest.mark.parametrize("name,parameters,code", KERNELS, ids=[k[0] for k in KERNELS])
+def test_reads_ahead_of_the_wait(name, parameters, code):
+    # up to the first wait that is not a row tile's without rows; whether a pointer is there is no access
+    before = re.sub(r"if \(r0 >= n_rows\) \{\s*after_previous\(\);\s*return;\s*\}", "", code).split("after_previous()")[0]
+    before = re.sub(r"\w+ != nullptr", "", before)
+    memory = [p.split()[-1].lstrip("*&") for p in parameters.split(",") if not re.match(r"\s*(?:const )?(?:int|float|bool|AttnShape) \w+$", p)]
+    assert {p for p in memory if re.search(rf"\b{p}\b", before)} <= EARLY.get(name, set())
+
+
+def test_keys_of_the_step_come_after_the_wait():
+    code = next(c for n, _, c in KERNELS if n == "attention_rows_mma_kernel")
+    before, after = code[:code.rindex("after_previous()")], code[code.rindex("after_previous()"):]
+    assert re.findall(r"load_tile\(.*?, (\w+), (\w+)\);", before) == [("true", "false")]
+    assert re.findall(r"load_tile\(.*?, (\w+), (\w+)\);", after) == [("false", "true"), ("true", "true")]
+    # a key of this step is one from pos0 on; the guard comes ahead of the table
+    assert re.search(r"if \(valid && kj >= pos0 \? !mine : !old\) return;.*\n.*table\[", before)
+
+
+def test_the_first_kernel_of_a_step_is_an_ordinary_launch():
+    assert "embed_kernel" not in {k[0] for k in KERNELS}
+    assert "embed_kernel<AT><<<" in (CSRC / "seq_kernels.cu").read_text()
+
+
 def test_rows_are_loaded_coherently():
     """Vec16::load, by which the products of few rows read their rows."""
     text = (CSRC / "seq_gemm.cu").read_text()
