@@ -30,7 +30,7 @@ namespace {
 template <int OUT>
 int product(const seq::umma::SplitArgs& p, cudaStream_t s, bool ahead = true) {
   using namespace seq::umma;
-  if (fills_chip(p.T, p.N)) return launch_wide<kTf32, OUT>(p, s);
+  if (fills_chip(p.T, p.N)) return launch_tiles<kTf32, OUT>(p, s);
   if (p.T <= 16) return launch_split<kTf32, 16, OUT, 5>(p, s, ahead);
   if (p.T <= 32) return launch_split<kTf32, 32, OUT, 5>(p, s, ahead);
   if (p.T <= 64) return launch_split<kTf32, 64, OUT, 4>(p, s, ahead);

@@ -22,6 +22,7 @@
 #include <cstdint>
 
 #include "kllm_host.h"
+#include "seq_tiles.h"
 
 namespace kllm {
 namespace seq {
@@ -30,7 +31,6 @@ namespace umma {
 constexpr int BM = 128;    // weight rows per CTA = MMA M
 constexpr int BK = 64;     // bf16 elements per K block = 128 bytes = one swizzle row
 constexpr int UK = 16;     // K of one tcgen05.mma.kind::f16
-constexpr int kSms = 148;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int THREADS = 192;
 constexpr uint32_t kWaitLimit = 1u << 24;  // try_wait rounds before a wait gives up (each suspends up to ~1 us)
@@ -249,7 +249,7 @@ __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, 
 }
 
 // ---- token blocks: persistent CTAs ----------------------------------------------------------------------------------
-// One CTA per SM walks tiles of 128 weight rows x 128 tokens, or two CTAs of a cluster tiles of 256 x 256 (BN = 256).  The tile's
+// One CTA per SM walks tiles of 128 weight rows x 128 or 256 tokens, or two CTAs of a cluster tiles of 256 x 256 (tile_form).  The tile's
 // accumulator alternates between two sets of BN TMEM columns, so the epilogue of a tile runs under the products of the next, and the
 // ring never drains between tiles.
 // Why pairs: a CTA by itself takes in 32 KB per 2 * 128 * 128 * 64 operations, 128 bytes a clock at the tensor cores' rate, and with 256
@@ -260,9 +260,9 @@ __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, 
 // Plain results leave through shared memory by TMA, 32 features x 16 tokens at a time: stored from registers, 32 features of a token per
 // instruction, a tile took 10 us to leave, which the products of a short K do not cover and the last tile never does.
 // 2048 x K x 8192 in us, calls back to back, one CTA to a tile of 256 tokens / pairs / and stores by TMA: K = 2048 64.5 / 61.2 / 57.4,
-// K = 512 - / 35.1 / 26.8; 4096 x 4096 x 4096 110 / 105 / 102, 1501 x 2048 x 3072 20.6 / 22.7 / 20.5.  What bounds it now is what an SM
-// takes in: a block of K lasts some 560 cycles whatever the tile (256 x 256 on a pair, 256 x 128 on a pair, 128 x 128 on a CTA; 32 KB a CTA,
-// 58 of the 64 bytes a clock that reach an SM), so a tile of 256 x 256 costs no more time than a small one; its products take 512.
+// K = 512 - / 35.1 / 26.8; 4096 x 4096 x 4096 110 / 105 / 102, 1501 x 2048 x 3072 20.6 / 22.7 / 20.5.  What bounds pairs now is what an SM
+// takes in: a block of K lasts some 560 cycles where a CTA takes in 32 KB for it (256 x 256 on a pair, 256 x 128 on a pair, 128 x 128 on a
+// CTA: 58 of the 64 bytes a clock that reach an SM); the products of a tile of 256 x 256 take 512.
 // Gated: a tile is 64 features, its first 64 weight rows their gate rows, the other 64 their up rows.  The two TMEM halves meet
 // through shared memory: of every 32 columns the gate's warp finishes 16 and the up rows' warp 16.
 // Eight epilogue warps, four for either half of the columns: with four the activation of a tile takes longer than its products at
@@ -270,9 +270,10 @@ __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, 
 constexpr int kPairCols = 32;
 constexpr int kPersistentThreads = 64 + 256;
 constexpr int kExchangeBytes = 4 * 2 * kPairCols * 32 * 4;  // [half of the columns, pair of warps][buffer][column][lane]
-constexpr int kPersistentStages = 6;  // of 32 KB
-constexpr size_t persistent_smem() {
-  return 1024 + static_cast<size_t>(kPersistentStages) * (A_BYTES + 128 * BK * 2) + kExchangeBytes + 256;
+template <int B_ROWS>  // of a CTA: stages of 32 KB or of 48
+constexpr int kPersistentStages = B_ROWS == 256 ? 4 : 6;
+constexpr size_t persistent_smem() {  // as much either way
+  return 1024 + static_cast<size_t>(kPersistentStages<128>) * (A_BYTES + 128 * BK * 2) + kExchangeBytes + 256;
 }
 // A warp's 32 features x 16 tokens, to be stored by TMA (which leaves out what is past the matrix)
 constexpr int kStoreTokens = 16;
@@ -282,7 +283,7 @@ __device__ __forceinline__ void store_2d(const CUtensorMap* map, uint32_t src, i
                ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1) : "memory");
 }
 
-template <int MODE, int BN, int OUT>
+template <int MODE, int BN, int CTAS, int OUT>
 __global__ void __launch_bounds__(kPersistentThreads, 1)
 umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_up,
             const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_out, const bool by_tma, const SplitArgs p) {
@@ -290,9 +291,8 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
   constexpr bool GATED = OUT == kGated;
   constexpr int BKE = ModeOf<MODE>::BKE;
   const int T = p.T, N = p.N, K = p.K;
-  constexpr bool PAIR = BN == 256;
-  constexpr int CTAS = PAIR ? 2 : 1;
-  constexpr int ST = kPersistentStages, B_ROWS = BN / CTAS, B_BYTES = B_ROWS * BK * 2, STAGE = A_BYTES + B_BYTES;
+  constexpr bool PAIR = CTAS == 2;
+  constexpr int B_ROWS = BN / CTAS, ST = kPersistentStages<B_ROWS>, B_BYTES = B_ROWS * BK * 2, STAGE = A_BYTES + B_BYTES;
   constexpr int FEATURES = GATED ? BM / 2 : BM;  // of a CTA
   constexpr uint32_t TMEM_COLS = 2 * BN;
   const int rank = PAIR ? static_cast<int>(cluster_rank()) : 0;
@@ -759,14 +759,13 @@ inline int make_out_map(CUtensorMap* map, void* ptr, int T, int N) {
   return r == CUDA_SUCCESS ? 0 : KLLM_E_INVALID;
 }
 
-template <int MODE, int BN, int OUT>
+template <int MODE, int BN, int CTAS, int OUT>
 inline int launch_persistent(SplitArgs p, cudaStream_t stream) {
   constexpr int FEATURES = OUT == kGated ? BM / 2 : BM;
   CUtensorMap map_w, map_up, map_a;
   if (p.report == nullptr) return KLLM_E_STATE;
   if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, FEATURES)) return rc;
   if (int rc = make_map_of<MODE>(&map_up, OUT == kGated ? p.w2 : p.w, p.N, p.K, FEATURES)) return rc;
-  constexpr int CTAS = BN == 256 ? 2 : 1;
   if (int rc = make_map_of<MODE>(&map_a, p.a, p.T, p.K, BN / CTAS)) return rc;
   CUtensorMap map_out = map_a;  // (unused where the stores are not TMA's)
   const bool by_tma = OUT == kPlain && p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
@@ -774,7 +773,7 @@ inline int launch_persistent(SplitArgs p, cudaStream_t stream) {
     if (int rc = make_out_map(&map_out, p.out, p.T, p.N)) return rc;
   constexpr size_t smem = persistent_smem();
   static_assert(smem <= 232448, "shared memory of one CTA");
-  auto kernel = umma_kernel<MODE, BN, OUT>;
+  auto kernel = umma_kernel<MODE, BN, CTAS, OUT>;
   static bool configured = false;
   if (!configured) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -801,22 +800,20 @@ inline int launch_persistent(SplitArgs p, cudaStream_t stream) {
 inline bool fills_chip(int T, int N) { return T > 64 && ((N + BM - 1) / BM) * ((T + 127) / 128) >= kSms * 19 / 20; }
 // bf16 blocks of more than 128 tokens are split in tiles of 64, and past half a tile of 128 tokens per SM there is no room left to
 // split K: from there on persistent CTAs are ahead.  Tiles as they are taken, of 128 features, or 64 gated ones; split / here in us:
-//   plain, K = 2048    64 tiles (400 x 2048) 16.6 / 17.4    72 (1501 x 768) 16.6 / 17.0    80 (1200 x 1024) 22.8 / 18.0    128 23.7 / 18.7
-//   gated, K = 2048    64 tiles (400 x 1024) 15.2 / 20.7    96 (700 x 1024) 24.3 / 21.6    160 (1200 x 1024) 44.9 / 28.4   192 46.8 / 28.4
-//   K = 4096           plain 72 tiles 24.5 / 27.0, 80 37.0 / 27.3;  gated 64 22.6 / 31.1, 96 39.0 / 32.3
+//   plain, K = 2048    48 tiles (500 x 1536) 16.4 / 16.4    72 (1501 x 768) 16.4 / 16.4    80 (1200 x 1024) 22.6 / 16.4
+//   plain, K = 4096    48 tiles 23.0 / 26.0    72 24.3 / 26.5    80 36.9 / 26.8        (K = 512: 48 tiles 10.3 / 8.3, 80 12.3 / 8.3)
+//   gated              K = 2048 64 tiles (400 x 1024) 15.0 / 22.5, 72 15.3 / 22.6, 96 (700 x 1024) 24.6 / 22.8;  K = 4096 72 22.6 / 33.3, 96 39.7 / 33.2
 inline bool persistent_pays(int T, int N, int features) {
   if (T <= 128) return fills_chip(T, N);
   return ((N + features - 1) / features) * ((T + 127) / 128) > kSms / 2;
 }
-// The wider tile, unless its last wave is so empty that the narrower one is done sooner (us, pairs / 128 x 128: 1501 x 2048 x 2048 20.0 / 27.6,
-// 2048 x 1024 x 1024 14.5 / 12.3, 900 x 2048 x 2048 18.6 / 16.8, 1024 x 4096 x 4096 30.9 / 47.2, 6001 x 2048 x 2048 43.2 / 68.3).
 template <int MODE, int OUT>
-inline int launch_wide(const SplitArgs& p, cudaStream_t s) {
-  const int feature_tiles = OUT == kGated ? (p.N + BM / 2 - 1) / (BM / 2) : (p.N + BM - 1) / BM;
-  const int waves_wide = ((feature_tiles + 1) / 2 * ((p.T + 255) / 256) + kSms / 2 - 1) / (kSms / 2);
-  const int waves = (feature_tiles * ((p.T + 127) / 128) + kSms - 1) / kSms;
-  if (100 * waves_wide <= 65 * waves) return launch_persistent<MODE, 256, OUT>(p, s);
-  return launch_persistent<MODE, 128, OUT>(p, s);
+inline int launch_tiles(const SplitArgs& p, cudaStream_t s) {
+  switch (tile_form(OUT == kGated, p.T, p.N, (p.K + ModeOf<MODE>::BKE - 1) / ModeOf<MODE>::BKE)) {
+    case kPair: return launch_persistent<MODE, 256, 2, OUT>(p, s);
+    case kWide: return launch_persistent<MODE, 256, 1, OUT>(p, s);
+    default: return launch_persistent<MODE, 128, 1, OUT>(p, s);
+  }
 }
 
 // products whose tiles do not fill the chip (seq_gemm_split.cuh)
@@ -830,7 +827,7 @@ inline int launch_block(const void* a, const void* w, const float* bias, void* o
                         cudaStream_t s, int* report, bool ahead) {
   if (!persistent_pays(T, N, GATED ? BM / 2 : BM)) return launch_few<GATED>(a, w, bias, out, T, K, N, act, s, report, ahead);
   const void* w2 = static_cast<const __nv_bfloat16*>(w) + (GATED ? static_cast<size_t>(N) * K : 0);  // 16-byte rows: K % 8 == 0
-  return launch_wide<kBf16, GATED ? kGated : kPlain>(SplitArgs{a, w, w2, bias, nullptr, out, T, N, K, 1, act, report}, s);
+  return launch_tiles<kBf16, GATED ? kGated : kPlain>(SplitArgs{a, w, w2, bias, nullptr, out, T, N, K, 1, act, report}, s);
 }
 
 template <typename AT>
