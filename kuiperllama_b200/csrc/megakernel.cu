@@ -714,8 +714,9 @@ __device__ __noinline__ void quantize_input_inplace(float* xs, int M, int tid) {
       uint32_t* o0 = reinterpret_cast<uint32_t*>(gb + ((0u + odd) & 3u) * 64);
       uint32_t* o1 = reinterpret_cast<uint32_t*>(gb + ((1u + odd) & 3u) * 64);
       uint32_t* o2 = reinterpret_cast<uint32_t*>(gb + ((2u + odd) & 3u) * 64);
-      auto digits = [&](float e) {  // |q| <= 2^22
-        return (__float_as_uint(__fmaf_rn(e, inv, 12582912.0f)) - 0x4B400000u + 0x808080u) ^ 0x808080u;
+      auto digits = [&](float e) {  // |q| <= 2^22; a NaN counts as zero
+        const float t = __fmaf_rn(e, inv, 12582912.0f);
+        return ((t == t ? __float_as_uint(t) : 0x4B400000u) - 0x4B400000u + 0x808080u) ^ 0x808080u;
       };
 #pragma unroll
       for (int j = 0; j < 4; ++j) {  // 4 elements -> one word of each digit plane, written at once
