@@ -2855,16 +2855,18 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
   int8_fast_ = (int8 && fast_) ? 1 : 0;
   const char* mma_env = getenv("KLLM_INT8_MMA");
   const bool int8_mma = mma_env != nullptr && atoi(mma_env) != 0;
-  const int kind = !int8 ? mega::kF32 : (int8_fast_ && m.group_size == 64 && !int8_mma ? mega::kW8Fast : mega::kW8);
+  // KLLM_CONSUMER_WARPS: teams are of four warps, so numbers that are none of theirs ask for the int8 kernel without teams
+  const char* warps_env = getenv("KLLM_CONSUMER_WARPS");
+  const int warps = warps_env != nullptr ? atoi(warps_env) : 0;
+  const bool teams = m.group_size == 64 && !int8_mma && warps != 6 && warps != 14 && warps != 16;
+  const int kind = !int8 ? mega::kF32 : (int8_fast_ && teams ? mega::kW8Fast : mega::kW8);
   // Consumer warps.  Teams: two (11 warps with the service ones: 168 registers each), three where a stage of short rows holds several
   // tasks (us per token, 8 / 12 warps: stories15M 117 / 110, Qwen2.5-0.5B 669 / 655, TinyLlama-1.1B 812 / 828, Llama-2-7B int8 with 8
   // layers 480 / 489).  int8 in the reference's order: 14, so that the CTA is 16 warps = 4 per scheduler with 128 registers each (16 / 14 / 8
   // warps 394 / 400 / 375 tok/s).
   consumer_warps_ = kind == mega::kW8 ? 14 : (kind == mega::kF32 && dim < 2048 ? 12 : 8);
-  if (const char* e = getenv("KLLM_CONSUMER_WARPS")) {
-    const int v = atoi(e);
-    if (kind == mega::kW8 ? v == 6 || v == 8 || v == 12 || v == 14 || v == 16 : v == 8 || v == 12) consumer_warps_ = v;
-  }
+  if (kind == mega::kW8 ? warps == 6 || warps == 8 || warps == 12 || warps == 14 || warps == 16 : warps == 8 || warps == 12)
+    consumer_warps_ = warps;
   kernel_ = kernel_for<false>(consumer_warps_, kind);
   kernel_prof_ = kernel_for<true>(consumer_warps_, kind);
   threads_ = mega::mega_threads(consumer_warps_, kind);
