@@ -52,6 +52,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -2808,6 +2809,16 @@ const void* kernel_for(int consumer_warps, int kind) {
   if (consumer_warps == 12) return reinterpret_cast<const void*>(mega::decode_megakernel<12, mega::kF32, PROF>);
   return reinterpret_cast<const void*>(mega::decode_megakernel<8, mega::kF32, PROF>);
 }
+
+// The limit is the kernel's, and decoders of several shapes share a kernel: it is raised, never lowered.
+cudaError_t allow_shared_memory(const void* kernel, size_t bytes) {
+  static std::mutex one_at_a_time;
+  std::lock_guard<std::mutex> lock(one_at_a_time);
+  cudaFuncAttributes now{};
+  const cudaError_t e = cudaFuncGetAttributes(&now, kernel);
+  if (e != cudaSuccess || static_cast<size_t>(now.maxDynamicSharedSizeBytes) >= bytes) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+}
 }  // namespace
 
 int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
@@ -3305,10 +3316,8 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
     return static_cast<int>(cudaErrorMemoryAllocation);
   cudaStreamSynchronize(stream);  // ph (host vector) must outlive the async copy
 
-  cudaError_t e = cudaFuncSetAttribute(kernel_, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem_bytes_));
-  if (e != cudaSuccess) return static_cast<int>(e);
-  e = cudaFuncSetAttribute(kernel_prof_, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes_));
+  cudaError_t e = allow_shared_memory(kernel_, smem_bytes_);
+  if (e == cudaSuccess) e = allow_shared_memory(kernel_prof_, smem_bytes_);
   if (e != cudaSuccess) return static_cast<int>(e);
   int occ = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel_, threads_, smem_bytes_);
