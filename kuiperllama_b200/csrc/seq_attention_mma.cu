@@ -325,20 +325,16 @@ int launch_mma(const AttnShape& a, const void* q, const float* gates, const Page
 // Grid: x = 16-row tile, y = (entry, key/value head), z = split.  Four warps.  Scores: a warp takes 8 keys of the tile
 // against all 16 rows.  Softmax: a warp takes every fourth row, a lane per key.  Output: the 8-column blocks are dealt out to the
 // warps in turn (NBW per warp).  Values that are the head of the key row (SAME) are read from the key tile.
-// Few tiles of keys (`out` not null): one CTA walks the splits one after another, each from a clean start, and joins them itself (sink,
-// output gate, conversion): the sums of the splits and of attention_merge_kernel, operation by operation, so the results are the same
-// bits.  What a thread has of a split that is done waits in shared memory, in places of its own.  The line is at
-// kFewTiles tiles of 64 keys: a tile takes about 1.5 us, the kernel that joins splits 3.  (24 chats of 33 to 79 keys, a prompt step and
-// 12 steps of 4 layers, us: 3925 with that kernel, 3810 without; one running softmax over all keys instead of splits took 3735, but its
-// sums are others.)
+// With one split (`out` not null) the kernel finishes the rows itself: sink, output gate, conversion, what attention_merge_kernel does with
+// one split, operation by operation.  Two splits walked and joined by one CTA, the same bits, gave nothing over two CTAs and the kernel that
+// joins them (a step of 2 layers with one sequence of 128 keys 64.5 against 60.5 us, 24 chats of 33 to 79 keys the same), four of 188
+// keys 76.7 against 61.5; one running softmax over them was no faster either, and its sums are others.
 // What bounds it at the contexts of a chat is a chain of latencies: index arrays, page table, keys, a few barriers per tile of keys.
 // Keys of earlier steps are on their way before the kernel waits for the one ahead of it.  That is safe for what was there before the step
 // began: the index arrays (copied ahead of its first kernel, which is no early one), the keys that completed steps wrote, and the entries
 // of the page table that lead to them, which those steps entered.  What this step writes, its own keys, queries and the entries of its new
 // pages (the host leaves none of them in the way of an earlier key, also after a step that failed), comes after the wait.
 constexpr int kFewRows = 16, kFewKeys = 32, kFewThreads = 128, kFewWarps = 4;
-constexpr int kFewParts = 4;  // splits that a CTA joins (the power of two over kFewTiles)
-static_assert(kFewTiles <= kFewParts, "a split for every tile of a short context");
 
 struct FewLayout {  // shared memory, in bytes from its start
   int ldk, ldv, dimp;
@@ -357,15 +353,9 @@ __host__ __device__ inline FewLayout few_layout(const AttnShape& a, bool same, b
   at = (at + 15) & ~static_cast<size_t>(15);
   L.p_hi = at, at += kFewRows * (kFewKeys + 8) * 2;
   L.p_lo = at, at += kFewRows * (kFewKeys + 8) * 2;
-  L.stats = at, at += (3 + 2 * (kFewParts - 1)) * kFewRows * 4;
+  L.stats = at, at += 3 * kFewRows * 4;
   L.total = at;
   return L;
-}
-// what lies behind it where a CTA joins the splits
-inline size_t few_parts_bytes(const AttnShape& a, int splits) {
-  int columns = 2 * kFewWarps * 8;  // of the kernel that takes this vdim (KLLM_FEW)
-  while (columns < a.vdim) columns *= 2;
-  return static_cast<size_t>(splits - 1) * columns * kFewRows * 4;
 }
 
 template <int NBW, bool SAME, bool QF32>
@@ -393,8 +383,7 @@ attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t
   const int keep_tiles = min(tile_first, (keep_first + kFewKeys - 1) / kFewKeys);
   const int list_n = keep_tiles + n_tiles - tile_first;
   const int per = (list_n + splits - 1) / splits;
-  const bool whole = out_ != nullptr;  // all splits are this CTA's
-  const int tile_lo = whole ? 0 : split * per, tile_hi = whole ? list_n : min(list_n, tile_lo + per);
+  const int tile_lo = split * per, tile_hi = min(list_n, tile_lo + per);
   auto tile_of = [&](int li) { return li < keep_tiles ? li : tile_first + (li - keep_tiles); };
 
   extern __shared__ __align__(16) unsigned char few_sm[];
@@ -408,8 +397,6 @@ attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t
   float* m_s = reinterpret_cast<float*>(few_sm + L.stats);
   float* l_s = m_s + kFewRows;
   float* al_s = l_s + kFewRows;
-  float* part_m = al_s + kFewRows;  // [split][rows], of the splits that are done
-  float* part_l = part_m + (kFewParts - 1) * kFewRows;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(few_sm));
   const uint32_t k_addr = base + static_cast<uint32_t>(L.k), v_addr = base + static_cast<uint32_t>(L.v);
@@ -475,12 +462,6 @@ attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t
   const uint32_t ql_addr = base + static_cast<uint32_t>(L.q_lo) + ((lane & 15) * ldk + (lane >> 4) * 8) * 2;
   const uint32_t ph_addr = base + static_cast<uint32_t>(L.p_hi) + ((lane & 15) * (kFewKeys + 8) + (lane >> 4) * 8) * 2;
   const uint32_t pl_addr = base + static_cast<uint32_t>(L.p_lo) + ((lane & 15) * (kFewKeys + 8) + (lane >> 4) * 8) * 2;
-  auto row_of = [&](int r) {  // token * heads + head
-    const int rr = r0 + r;
-    return static_cast<size_t>(first + rr / rep) * a.heads + g * rep + rr % rep;
-  };
-  float4* const parts = reinterpret_cast<float4*>(few_sm + L.total) + tid;  // [split][block of columns][thread]
-  int done = 0, next_end = whole ? per : list_n + 1;  // splits that are done; the tile at which the next one is
 
   for (int li = tile_lo; li < tile_hi; ++li) {
     const int tile = tile_of(li), stage = (li - tile_lo) & 1, k0 = tile * kFewKeys;
@@ -560,75 +541,40 @@ attention_rows_mma_kernel(AttnShape a, const void* q_, PagedKV kv, const int32_t
       }
     }
     __syncthreads();  // the stage is loaded again, the scores are written again
-    if (li + 1 == next_end && li + 1 < tile_hi) {  // the next split begins
-#pragma unroll
-      for (int i = 0; i < NBW; ++i) {
-        parts[(done * NBW + i) * kFewThreads] = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
-        o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-      }
-      if (tid < kFewRows) {
-        part_m[done * kFewRows + tid] = m_s[tid], part_l[done * kFewRows + tid] = l_s[tid];
-        m_s[tid] = -INFINITY, l_s[tid] = 0.f;
-      }
-      ++done, next_end += per;
-    }
   }
   if (tile_lo >= tile_hi) __syncthreads();  // an empty split still writes its (empty) statistics
-  if (!whole) {
-    const int pstride = vdim + 2;
-#pragma unroll
-    for (int z = 0; z < 2; ++z) {
-      const int r = gq + z * 8;
-      if (r >= rows_here) continue;
-      float* p = ws + (row_of(r) * splits + split) * pstride;
-      if (warp == 0 && t4 == 0) p[0] = m_s[r], p[1] = l_s[r];
-#pragma unroll
-      for (int i = 0; i < NBW; ++i) {
-        const int col = (warp + i * kFewWarps) * 8 + t4 * 2;
-        if (col < vdim) *reinterpret_cast<float2*>(p + 2 + col) = make_float2(o[i][z * 2], o[i][z * 2 + 1]);
-      }
-    }
-    return;
-  }
-  const bool per_element = gates != nullptr && a.gate == KLLM_SEQ_GATE_ELEMENT;
+  const int pstride = vdim + 2;
 #pragma unroll
   for (int z = 0; z < 2; ++z) {
     const int r = gq + z * 8;
     if (r >= rows_here) continue;
-    const size_t th = row_of(r);
-    // split_weights: the splits' sums are added as its lanes add them, (0 + 2) + (1 + 3)
-    const float sink = a.sink != nullptr ? a.sink[th % a.heads] : -INFINITY;
-    float m[kFewParts], l[kFewParts], M = sink;
+    const int rr = r0 + r;
+    const size_t th = static_cast<size_t>(first + rr / rep) * a.heads + g * rep + rr % rep;
+    if (out_ != nullptr) {
+      const float m = m_s[r], sink = a.sink != nullptr ? a.sink[th % a.heads] : -INFINITY, M = fmaxf(m, sink);
+      const float w = m > -INFINITY ? expf(m - M) : 0.f;
+      const float weight = w / __fadd_rn(__fmul_rn(w, l_s[r]), a.sink != nullptr ? expf(sink - M) : 0.f);
+      const bool per_element = gates != nullptr && a.gate == KLLM_SEQ_GATE_ELEMENT;
+      const float head_gate = gates != nullptr && !per_element ? gates[th] : 1.0f;
 #pragma unroll
-    for (int s = 0; s < kFewParts; ++s) {
-      m[s] = s < done ? part_m[s * kFewRows + r] : s == done ? m_s[r] : -INFINITY;
-      l[s] = s < done ? part_l[s * kFewRows + r] : s == done ? l_s[r] : 0.f;
-      M = fmaxf(M, m[s]);
+      for (int i = 0; i < NBW; ++i) {
+        const int col = (warp + i * kFewWarps) * 8 + t4 * 2;
+        if (col >= vdim) continue;
+        const size_t at = th * vdim + col;
+        // (added to zero, as the sum over the splits begins)
+        const float x = weight > 0.f ? fmaf(weight, o[i][z * 2], 0.f) : 0.f, y = weight > 0.f ? fmaf(weight, o[i][z * 2 + 1], 0.f) : 0.f;
+        const float gx = per_element ? gates[at] : head_gate, gy = per_element ? gates[at + 1] : head_gate;
+        if (a.out_f32) *reinterpret_cast<float2*>(static_cast<float*>(out_) + at) = make_float2(x * gx, y * gy);
+        else *reinterpret_cast<__nv_bfloat162*>(static_cast<__nv_bfloat16*>(out_) + at) = __floats2bfloat162_rn(x * gx, y * gy);
+      }
+      continue;
     }
-#pragma unroll
-    for (int s = 0; s < kFewParts; ++s) m[s] = m[s] > -INFINITY ? expf(m[s] - M) : 0.f, l[s] = __fmul_rn(m[s], l[s]);
-    float sum = __fadd_rn(__fadd_rn(l[0], l[2]), __fadd_rn(l[1], l[3]));
-    if (a.sink != nullptr) sum = __fadd_rn(sum, expf(sink - M));
-#pragma unroll
-    for (int s = 0; s < kFewParts; ++s)
-      if (s <= done) m[s] /= sum;
-    const float head_gate = gates != nullptr && !per_element ? gates[th] : 1.0f;
+    float* p = ws + (th * splits + split) * pstride;
+    if (warp == 0 && t4 == 0) p[0] = m_s[r], p[1] = l_s[r];
 #pragma unroll
     for (int i = 0; i < NBW; ++i) {
       const int col = (warp + i * kFewWarps) * 8 + t4 * 2;
-      if (col >= vdim) continue;
-      float x = 0.f, y = 0.f;
-#pragma unroll
-      for (int s = 0; s < kFewParts; ++s) {
-        if (s > done || !(m[s] > 0.f)) continue;
-        const float2 v = s == done ? make_float2(o[i][z * 2], o[i][z * 2 + 1])
-                                   : reinterpret_cast<const float2*>(parts + (s * NBW + i) * kFewThreads)[z];
-        x = fmaf(m[s], v.x, x), y = fmaf(m[s], v.y, y);
-      }
-      const size_t at = th * vdim + col;
-      const float gx = per_element ? gates[at] : head_gate, gy = per_element ? gates[at + 1] : head_gate;
-      if (a.out_f32) *reinterpret_cast<float2*>(static_cast<float*>(out_) + at) = make_float2(x * gx, y * gy);
-      else *reinterpret_cast<__nv_bfloat162*>(static_cast<__nv_bfloat16*>(out_) + at) = __floats2bfloat162_rn(x * gx, y * gy);
+      if (col < vdim) *reinterpret_cast<float2*>(p + 2 + col) = make_float2(o[i][z * 2], o[i][z * 2 + 1]);
     }
   }
 }
@@ -637,7 +583,7 @@ template <int NBW, bool SAME, bool QF32>
 int launch_few(const AttnShape& a, const void* q, const PagedKV& kv, int n_entries, const int32_t* ent_first,
                const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0, int max_count, int splits, float* ws,
                const float* gates, void* out, cudaStream_t s) {
-  const size_t smem = few_layout(a, SAME, QF32).total + (out != nullptr ? few_parts_bytes(a, splits) : 0);
+  const size_t smem = few_layout(a, SAME, QF32).total;
   static size_t configured = 0;
   if (smem > 48 * 1024 && smem > configured) {
     const cudaError_t e = cudaFuncSetAttribute(attention_rows_mma_kernel<NBW, SAME, QF32>,
@@ -645,7 +591,7 @@ int launch_few(const AttnShape& a, const void* q, const PagedKV& kv, int n_entri
     if (e != cudaSuccess) return cuda_rc(e);
     configured = smem;
   }
-  const dim3 grid((max_count * (a.heads / a.kv_heads) + kFewRows - 1) / kFewRows, n_entries * a.kv_heads, out != nullptr ? 1 : splits);
+  const dim3 grid((max_count * (a.heads / a.kv_heads) + kFewRows - 1) / kFewRows, n_entries * a.kv_heads, splits);
   if (grid.y > 65535u) return KLLM_E_UNSUPPORTED;
   launch_ahead(attention_rows_mma_kernel<NBW, SAME, QF32>, dim3(grid), dim3(kFewThreads), smem, s, a, q, kv, ent_first, ent_count, ent_seq, ent_pos0,
                                                                             splits, ws, gates, out);
@@ -666,11 +612,6 @@ bool attention_rows_mma_usable(int dtype, const AttnShape& a, const PagedKV& kv,
   if (a.dim % 8 || a.vdim % 8 || kv.k_row % 8 || kv.v_row % 8 || a.vdim > 512) return false;
   if (static_cast<long long>(n_entries) * a.kv_heads > 65535) return false;
   return few_layout(a, values_in_keys(a, kv), a.q_f32 != 0).total <= 200 * 1024;
-}
-
-bool attention_rows_mma_joins(const AttnShape& a, const PagedKV& kv, int splits, int max_ctx) {
-  if (a.no_merge || (splits > 1 && !few_keys(max_ctx))) return false;
-  return few_layout(a, values_in_keys(a, kv), a.q_f32 != 0).total + few_parts_bytes(a, splits) <= 200 * 1024;
 }
 
 int launch_attention_rows_mma(const AttnShape& a, const void* q, const PagedKV& kv, int n_entries, const int32_t* ent_first,

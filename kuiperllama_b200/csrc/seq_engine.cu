@@ -170,7 +170,7 @@ struct kllm_seq_engine {
     uint64_t generation = 0;
     int nodes = 0;
   };
-  std::map<std::tuple<int, int, int, bool, bool>, Graph> graphs;
+  std::map<std::tuple<int, int, int, int>, Graph> graphs;
   bool own_stream = false;
   cudaStream_t side = nullptr;  // a pair's second mixer runs here, between `fork` and `join`
   cudaEvent_t fork = nullptr, join = nullptr;
@@ -1258,7 +1258,7 @@ extern "C" int kllm_seq_step(kllm_seq_engine* e, int32_t n_entries, const int32_
   const bool all_single = single && !tracing && e->prof_out == nullptr && e->use_graphs && T <= 32;
   bool replayed = false;
   if (all_single) {
-    const auto key = std::make_tuple(n_entries, n_want, splits, few_keys(max_ctx), argmax_host != nullptr);
+    const auto key = std::make_tuple(n_entries, n_want, splits, argmax_host ? 1 : 0);
     kllm_seq_engine::Graph& g = e->graphs[key];
     if (g.exec != nullptr && g.generation != g_buffer_generation) {
       cudaGraphExecDestroy(g.exec);

@@ -22,8 +22,6 @@ namespace seq {
 
 constexpr int kAttnRows = 32;   // (token, query head) rows of one attention CTA
 constexpr int kAttnKeys = 64;   // keys per tile
-constexpr int kFewTiles = 3;    // up to so many, one CTA walks the splits where it can also join them (seq_attention_mma.cu)
-inline bool few_keys(int max_ctx) { return max_ctx <= kFewTiles * kAttnKeys; }
 constexpr int kAttnThreads = 128;
 
 struct NormW {
@@ -224,9 +222,8 @@ int launch_attention_f32(const AttnShape& a, const void* q, const float* gates, 
                          int max_count, int splits, float* ws, void* out, cudaStream_t s);
 
 // bf16 steps of few rows per key head, or with fp32 queries (head sizes that are multiples of 8): partial results of every
-// split in `ws`, like the split-key kernel, or (`out` not null, where ..._joins) the finished rows.
+// split in `ws`, like the split-key kernel, or (`out` not null, one split) the finished rows.
 bool attention_rows_mma_usable(int dtype, const AttnShape& a, const PagedKV& kv, int n_entries);
-bool attention_rows_mma_joins(const AttnShape& a, const PagedKV& kv, int splits, int max_ctx);
 int launch_attention_rows_mma(const AttnShape& a, const void* q, const PagedKV& kv, int n_entries, const int32_t* ent_first,
                               const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0, int max_count,
                               int splits, float* ws, const float* gates, void* out, cudaStream_t s);

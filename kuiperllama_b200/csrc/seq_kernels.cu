@@ -1736,6 +1736,7 @@ int launch_attention(int dtype, const AttnShape& a, const void* q, const float* 
                      int n_entries, const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq,
                      const int32_t* ent_pos0, int max_count, int max_ctx, int splits, float* ws, void* out, int T,
                      const int32_t* tok_seq, const int32_t* tok_pos, cudaStream_t s, int* report) {
+  (void)max_ctx;
   if (a.kv_heads <= 0 || a.heads % a.kv_heads != 0 || a.dim <= 0 || a.vdim <= 0) return KLLM_E_UNSUPPORTED;
   const int C = (a.vdim + kAttnKeys - 1) / kAttnKeys;
   int rc = 0;
@@ -1750,7 +1751,7 @@ int launch_attention(int dtype, const AttnShape& a, const void* q, const float* 
     rc = launch_attention_f32(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, s);
     if (rc || (splits == 1 && !a.no_merge)) return rc;
   } else if (attention_rows_mma_usable(dtype, a, kv, n_entries)) {
-    const bool whole = attention_rows_mma_joins(a, kv, splits, max_ctx);
+    const bool whole = splits == 1 && !a.no_merge;
     rc = launch_attention_rows_mma(a, q, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws,
                                    a.gate ? gates : nullptr, whole ? out : nullptr, s);
     if (rc || whole) return rc;

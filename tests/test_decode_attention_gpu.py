@@ -1,7 +1,6 @@
-"""-m gpu: attention of single-token steps (csrc/seq_attention_mma.cu), with prompts of an earlier step in the cache.  Up to 192 keys a
-CTA walks the splits of a row's keys and joins them itself, past that they run side by side and another kernel joins them: contexts at the
-edges of tiles and splits, sinks, gates and windows, against 64 bits; and the same bits either way where the splits are the same.  The
-layer and the bounds are those of test_attention_exact_gpu.py."""
+"""-m gpu: attention of single-token steps (csrc/seq_attention_mma.cu), with prompts of an earlier step in the cache.  Up to 64 keys a
+CTA finishes its rows itself, past that splits of the keys run side by side and another kernel joins them: contexts at the edges of
+tiles and splits, sinks, gates and windows, against 64 bits.  The layer and the bounds are those of test_attention_exact_gpu.py."""
 import ctypes
 
 import numpy as np
@@ -73,16 +72,7 @@ def last_rows(shape, lens):
 
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("lens", [[2, 32, 33, 64], [2, 32, 33, 65, 97, 128], [3, 64, 129, 161, 192], [2, 97, 192, 193]],
-                         ids=["one split", "two, joined in place", "four, joined in place", "four, side by side"])
+                         ids=["one split", "two", "four of three tiles", "four"])
 def test_single_token_steps(shape, lens):
     for got, exact, size, x in last_rows(shape, lens):
         assert_close(got, exact, size, x, 1.01 * 2.0 ** -8)
-
-
-@pytest.mark.parametrize("shape", SHAPES)
-def test_splits_joined_in_place_are_the_same_bits(shape):
-    """192 and 200 keys are both four splits; the longer context takes every row of its step to the kernel that joins them."""
-    import torch
-    lens = [2, 33, 64, 129, 161, 192]
-    alone, beside = last_rows(shape, lens), last_rows(shape, lens + [200])
-    assert all(torch.equal(a[0], b[0]) for a, b in zip(alone, beside))
