@@ -185,7 +185,7 @@ def measured_peaks():
             return float(d["hbm_gbs"]), "measured (MEASURED_PEAKS.json hbm_gbs, torch copy)"
         except Exception:
             pass
-    return 6650.0, "fallback (B200_PROFILING.md 6.65 TB/s)"
+    return 6650.0, "fallback (an earlier copy on a B200, 6.65 TB/s)"
 
 
 def ncu_traffic(workload, kernel_key):

@@ -280,7 +280,7 @@ const char* kllm_decoder_engine(const kllm_decoder* dec);
  * elements).  Globaltimer ns: [0] phase entered, [1] input vector staged (+normalised), [2] last
  * ring stage consumed, [3] grid barrier passed, [10] input vector polled (before the norm).
  * SM cycles of warp 0: [4] addend prefetch, [5] dot products, [6] reductions, [7] epilogues,
- * [8] waiting for ring stages, [9] rows of a stage.  Measurement aid (profiles/). */
+ * [8] waiting for ring stages, [9] rows of a stage.  Measurement aid. */
 int kllm_decoder_profile(kllm_decoder* dec, int32_t first_token, int32_t start_pos,
                          int32_t n_steps, int32_t profiled_step, uint64_t* stamps_host,
                          int32_t capacity, int32_t* grid_out, int32_t* phases_out);

@@ -4,7 +4,7 @@
 //
 // Why: at batch 1 the path is a 4-26 GB/token weight stream; with one launch per op (even 6
 // fused launches per layer in a CUDA graph) every kernel boundary drains the HBM pipeline
-// (profiles/r01a: 15-42 % DRAM utilisation per kernel).  Here one CTA per SM stays resident
+// (ncu: 15-42 % DRAM utilisation per kernel).  Here one CTA per SM stays resident
 // and a dedicated producer warp streams that CTA's share of EVERY weight matrix, in schedule
 // order, through a ring of shared-memory stages with TMA bulk copies (cp.async.bulk ->
 // UBLKCP) signalled on mbarriers.  Weights never depend on activations, so the producer runs
@@ -25,7 +25,7 @@
 //
 // What bounds it is the chain of a layer, not a unit: five phases, each entry, poll, norm, rows, hand-off.  Decode of TinyLlama-1.1B at
 // position 500, us per token (HBM time of its weights 635): a warp per task 900, teams 812.  Llama-2-7B int8 with 8 of its 32 layers at position
-// 200 (HBM time 292): 624, teams 497, with the input vector quantised by multiply-adds and byte permutes 475.
+// 200 (HBM time 292): 624, teams 497, with the input vector quantised by multiply-adds and byte permutes 478.
 //
 // No local memory: the ring takes the whole unified L1, so a stack access is a round trip to L2.  The kernel
 // parameters are __grid_constant__ (never copied to the stack), register buffers are always written in full
@@ -70,7 +70,7 @@ namespace mega {
 #define KLLM_MBAR_HINT_NS 20000u
 #endif
 // 1: warps without a row in an attention tile skip its wait and block at a hardware barrier instead of
-// spinning on the mbarrier.  Measured on B200 (profiles/README.md, pass M): no gain (826 vs 837 tok/s), so off.
+// spinning on the mbarrier.  Measured on B200: no gain (826 vs 837 tok/s), so off.
 #ifndef KLLM_ATTN_GATE
 #define KLLM_ATTN_GATE 0
 #endif
@@ -110,8 +110,10 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b, int count) {
 // try_wait suspends the warp in hardware until the phase completes or the time hint (ns) runs out:
 // with a generous hint a waiting warp sleeps instead of re-issuing the probe -- waiting warps
 // otherwise compete for issue slots with the warps that are computing on the same scheduler
-// (ncu, r02f: SYNCS + BRA + YIELD of the spin loops were a quarter of all executed instructions).
-// A wait of two minutes ends the kernel: longer than the polls of the hand-offs, on which this one may rest, are allowed to take.
+// (ncu: SYNCS + BRA + YIELD of the spin loops were a quarter of all executed instructions).
+// A wait of two minutes traps, which ends the process's context, as the polls of the hand-offs do after one (poll_failed), on which this
+// one may rest.  (Waits that gave up, let the kernel return and raised a flag for the host made every wait a question of whether it had
+// ended: 12 tokens of TinyLlama-1.1B 9959 -> 10308 us, 8 layers of Llama-2-7B int8 5848 -> 6153, a token of stories15M 164 -> 177.)
 __device__ __forceinline__ void mbar_wait(uint64_t* b, uint32_t parity) {
   asm volatile(
       "{\n .reg .pred p;\n .reg .u64 t0, t;\n"
@@ -1129,7 +1131,7 @@ __device__ KLLM_PHASE_CALL Pipe attention_fused_phase(const Params& P, int head,
     else
       P.attn_out[static_cast<size_t>(head) * hs + tid] = value;
   }
-  if (stamp && tid == 0) {  // SM cycles of thread 0 (profiles/: tools/phase_timeline.py)
+  if (stamp && tid == 0) {  // SM cycles of thread 0 (tools/phase_timeline.py)
     const long long c_end = clock64();
     stamp[4] = static_cast<unsigned long long>(c_rope - c_begin);                             // q/k/v poll + RoPE
     stamp[5] = static_cast<unsigned long long>(c_scores - c_rope - c_wait_scores);            // scores
@@ -2132,8 +2134,8 @@ __device__ KLLM_PHASE_CALL Carry gemv_phase(const Params& P, Carry carry, int to
   const int row_bytes = M * wbytes;
   const float* residual = ph.residual_from_emb ? emb_row : ph.residual;
 
-  // bias / residual of a row are fetched BEFORE its dot product so their L2 latency hides
-  // behind the accumulation (by the lane that will run the row's epilogue)
+  // a row's place and bias are fetched BEFORE its dot product so their L2 latency hides behind the accumulation (by the lane that
+  // will run the row's epilogue); the residual of the mode with grid barriers is read with the store
   auto unit_dest_of = [&](int unit) { return unit_dest(P, ph, tok, pos, residual, unit); };
   auto epilogue = [&](const UnitDest& dest, float d0, float d1) { unit_store(P, ph, dest, best, d0, d1); };
 
@@ -2851,11 +2853,6 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
     for (int d : dims)
       if (d % m.group_size != 0 || ((d / m.group_size) * 4) % 16 != 0) return KLLM_E_UNSUPPORTED;
   }
-  // consumer warps (+ the ring producer and the L2 prefetcher): fp32 rows 8 x 168 registers; int8 rows 14, so
-  // that the CTA is 16 warps = 4 per scheduler with 128 registers each (16 consumers make 18 warps, which caps
-  // them at 96 registers and spills).  Measured on B200 (profiles/README.md, passes Q-T): fp32 6 vs 8 warps
-  // 1072 = 1072 (TinyLlama), 1218 < 1296 (Qwen2.5-0.5B), 210 < 213 (Llama-2-7B); int8 16 / 14 / 8 warps
-  // 394 / 400 / 375 tok/s.
   // int8 arithmetic: "exact" reproduces the reference's fma(x * scale, float(w), acc) per element bit for
   // bit; "fast" (KLLM_INT8_MODE=fast) is the dp4a fixed-point mode (toleranced, ~3.5x fewer instructions)
   // The same switch frees the attention's summation order (flash-decoding, attention_flash_phase).
@@ -2932,7 +2929,7 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
     attn_split_ *= 2;
   const int attn_split_max = attn_split_;
   // The split costs one more hand-off per layer (~1.5 us): worth it when a head's K and V are big
-  // (head_size 128: 1 MB per head at context 1024), not for head_size 64 (measured, profiles/README.md).
+  // (head_size 128: 1 MB per head at context 1024), not for head_size 64 (measured).
   if (hs < 128) attn_split_ = 1;
   int split_cap = attn_split_max;
   if (fast_) {  // flash: split by timestep, any power of two whose partial triples fit the scores area
@@ -2954,11 +2951,11 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
 
   // ---- phase table ---------------------------------------------------------------------------------
   std::vector<Phase> ph;
-  // Rows per consumer task (1, 2 or 4) of a phase.  Measured on B200 (profiles/README.md, passes Q and R):
-  // 4 everywhere is best or equal (TinyLlama 1105 vs 1082 "auto" vs 1068 with 2; Llama-2-7B int8 418 / 405 /
-  // 407) -- the four rows of a task share every load of the input vector, and that outweighs the better
-  // balance of small tasks.  KLLM_TASK_ROWS_RT=1|2|4 forces a size, =auto picks per phase with the cost model
-  // below (rounds x (rows + x_cost), tasks never crossing a ring stage).
+  // Rows per task (1, 2 or 4) of a phase whose rows go to warps and not to teams (int8 in the reference's order, and the forms that
+  // KLLM_INT8_MMA and KLLM_CONSUMER_WARPS ask for).  Llama-2-7B int8 418 tokens/s with 4 everywhere, 405 with 2, 407 with what the cost
+  // model below picks: the four rows of a task share every load of the input vector, and that outweighs the better balance of small
+  // tasks.  KLLM_TASK_ROWS_RT=1|2|4 forces a size, =auto picks per phase (rounds x (rows + x_cost), tasks never crossing a ring stage).
+  // Teams take up to four rows (int8: eight), whatever it says.
   int forced_task_rows = 4;
   if (const char* e = getenv("KLLM_TASK_ROWS_RT")) {
     const int v = atoi(e);
@@ -2968,7 +2965,7 @@ int MegaEngine::init(const MegaModel& m, cudaStream_t stream) {
   // KLLM_INT8_MMA=1: int8 fast rows on the tensor cores -- mma.sync m16n8k32 s8 for stages of 3-8 rows, dp4a with the
   // columns split over the team for 1-2 long rows.  Correct (the parity suite passes with it) but not faster on
   // B200: Llama-2-7B int8 398 (teams of 4, 12 warps) / 403 (pairs, 14 warps) vs 407 tok/s for the plain dp4a
-  // rows (profiles/README.md, passes S and T) -- at one byte per weight the shared-memory reads of the
+  // rows -- at one byte per weight the shared-memory reads of the
   // fragments cost what the dp4a arithmetic costs.  Off by default.
   auto pick_task_rows = [&](Phase& p) {
     const int rpu = p.swiglu ? 2 : 1;

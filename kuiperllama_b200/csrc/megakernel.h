@@ -45,13 +45,13 @@ struct Phase {
   int residual_from_emb;  // residual source is the embedding row (layer 0)
   int group_size, group_shift;
   int rows_per_stage;     // whole rows per ring stage (chunks_per_row == 1)
-  int task_rows;          // rows handed to one consumer warp at a time (1, 2 or 4; picked per phase at init)
+  int task_rows;          // without teams: rows handed to one consumer warp at a time (1, 2 or 4; picked per phase at init)
   int mma;                // ... and the rows of a stage go through mma.sync m16n8k32 s8
   int team;               // the opt-in tensor-core form (KLLM_INT8_MMA): a team of consumer warps shares each ring stage, splitting the columns
   int row_pad;            // ... and are staged row_pad bytes apart more than their length (bank-conflict-free fragments)
   int cta_units, cta_more;  // units of a CTA; how many CTAs, the last ones, have one more
-  int units_per_stage, tasks_per_stage;  // fp32: units of a ring stage; tasks of up to four rows that it is cut into
-  int stages[2], tasks[2];  // fp32: stages (rows, where a row spans several) and tasks of a CTA with cta_units, cta_units + 1 units
+  int units_per_stage, tasks_per_stage;  // teams: units of a ring stage; tasks of up to four rows (int8: eight) that it is cut into
+  int stages[2], tasks[2];  // teams: stages (rows, where a row spans several) and tasks of a CTA with cta_units, cta_units + 1 units
   int chunks_per_row;     // > 1: a row spans this many stages (fp32 rows longer than a stage)
   int chunk_elems;
   int scale_off;          // byte offset of the scales region inside a stage (int8)
