@@ -23,9 +23,9 @@
 // A task's rows share every load of the input vector and their dot-product chains interleave (ILP instead of occupancy); their totals
 // are folded with "packed" shuffle trees (kllm_device.cuh) that do the additions of cub's tree only.
 //
-// What bounds it is the chain of a layer, not a unit: five phases, each entry, poll, norm, rows, hand-off.  Decode of TinyLlama-1.1B at
-// position 500, us per token (HBM time of its weights 635): a warp per task 900, teams 812.  Llama-2-7B int8 with 8 of its 32 layers at position
-// 200 (HBM time 292): 624, teams 497, with the input vector quantised by multiply-adds and byte permutes 478.
+// What bounds it is the chain of a layer, not a unit: five phases, each entry, poll, norm, rows, hand-off.  Calls of 12 tokens, us a token:
+// TinyLlama-1.1B at position 500 (HBM time of its weights 635) 906 with a warp to a task, 839 with teams; Llama-2-7B int8 with 8 of its 32
+// layers at position 200 (HBM time 292) 625 and 489, of which 22 are the input vector quantised by multiply-adds and byte permutes.
 //
 // No local memory: the ring takes the whole unified L1, so a stack access is a round trip to L2.  The kernel
 // parameters are __grid_constant__ (never copied to the stack), register buffers are always written in full
