@@ -40,6 +40,8 @@ namespace kllm {
 namespace seq {
 namespace {
 
+using umma::tmem_st16;
+
 constexpr int kTile = 128;                     // rows of a group, keys of a tile
 constexpr int kRows = 2 * kTile;               // rows of a CTA
 constexpr int kLoaders = 128, kAttnUmmaThreads = 256 + kLoaders + 32;
@@ -50,14 +52,6 @@ __device__ __forceinline__ float ex2(float x) {  // 2^x, relative error about 2^
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  __syncwarp();
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
 }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
   uint32_t a[16], b[16];

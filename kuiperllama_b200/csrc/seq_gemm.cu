@@ -9,8 +9,9 @@
 // the activation in its epilogue and writes the compute type.
 //   umma_kernel     bf16, T >= 64 (from K = 64 on) or T > 8 (from K = 384 on), K % 8 == 0: 128 weight rows x BN tokens per CTA
 //                   on tcgen05.mma (kind::f16, operands by TMA with 128-byte swizzle, accumulator in TMEM)  [seq_gemm_umma.cuh]
-//   umma_split_kernel  the same where the tiles are fewer than the SMs: K split over a cluster; fp32 with T > 8, K >= 128 and
+//   umma_split_kernel  the same where the tiles are fewer than the SMs: K split over a cluster; fp32 with 8 < T <= 64, K >= 128 and
 //                   K % 4 == 0, each operand as three bf16 parts                              [seq_gemm_split.cuh]
+//   umma_f32_kernel fp32 with T > 64: the weights' parts in TMEM                              [seq_gemm_f32.cuh]
 //   grouped_kernel  the tiled kernel over row blocks that each belong to one expert (rows gathered by index, the
 //                   SiLU-gate product as an optional epilogue)
 #include <cuda_bf16.h>
@@ -21,6 +22,7 @@
 #include <type_traits>
 
 #include "seq_engine.h"
+#include "seq_gemm_f32.cuh"
 #include "seq_gemm_split.cuh"
 #include "seq_gemm_umma.cuh"
 #include "seq_launch.cuh"

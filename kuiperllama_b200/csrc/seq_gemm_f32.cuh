@@ -1,0 +1,364 @@
+// fp32 products of more than 64 tokens on the 5th-generation tensor cores (sm_100a), all 24 bits of the operands: three bf16 parts of
+// each and six products, as kFp32 of seq_gemm_split.cuh, which holds the parts' definition, the smaller token blocks and the split of K.
+//
+// A CTA has a tile of 128 weight rows x 128 tokens, over all of K or, in a cluster, a part of it:
+//   warp 0          TMA: blocks of 32 fp32 columns of the weight and token rows into a ring of shared-memory stages
+//   warp 1          tcgen05.mma, A (the weights' parts) from TMEM, B (the tokens') from shared memory
+//   warps 2 .. 17   workers.  Eight of them split the blocks with even numbers, eight the odd ones: a thread 16 elements of a weight row into
+//                   its lane of TMEM, a warp 16 token rows in shared memory (split_tile).  Each sums 32 tokens of the accumulators in fp32
+//                   registers, three or four blocks behind, and stores them at the end
+//
+// Why the weights' parts lie in TMEM: with both operands' parts in shared memory a block of K is 208 KB of reads and writes there (32
+// arrive, 32 are read and 48 written by the splitting warps, 96 are read by the products), 1660 cycles at 128 bytes a clock, for 768
+// cycles of products.  So it is 136 KB, 1060 cycles.
+//
+// What bounds it now is instructions: a block is 1030 issue slots of each of the SM's four schedulers (517 x 4096 x 3072, ncu: of the
+// cycles that an SM has work, 82 % issue, the tensor pipe is busy in 60 %), half of them the splitting.  So a worker does all three kinds
+// of work, two teams take turns, and the token rows are split, the accumulators summed and the weight rows split in this order, which
+// keeps 96 registers free of spills (with the sums after the weight rows, and 16 bytes of spills: 125 us instead of 113).  Warps with one
+// kind of work each, all 20 of them, wait for the slowest four (117); all workers on every block walk it in lockstep (125); a pair of
+// CTAs (cta_group::2, 256 x 128) takes as long for an MMA of N = 128 as for one of 256 (137).
+// Measured against umma_split_kernel in tiles of 128 tokens (one B200, calls back to back, us; error against 64 bits):
+//   517 x 1024 x 3072  47.3 -> 34.9  1.04e-7 -> 1.02e-7      700 x 1024 x 1536  28.8 -> 22.6  9.4e-8 -> 9.1e-8
+//   517 x 4096 x 3072  154.7 -> 112.9  1.63e-7 -> 1.61e-7    700 x 2048 x 1024  45.9 -> 34.9  1.08e-7 -> 1.05e-7
+//   500 x 2000 x 5999  156.7 -> 116.8  1.28e-7 -> 1.26e-7    128 x 4096 x 4096  47.2 -> 39.0  1.12e-7 -> 1.10e-7
+//   130 x 128 x 300    15.0 -> 10.3   7.5e-8 -> 7.3e-8       65 x 1024 x 1024   14.5 -> 12.4  9.5e-8 -> 9.3e-8
+//
+// Precision: h h of two blocks, four steps, is summed in an accumulator (two, in turn), and these sums in fp32 registers.  The five small
+// products, at most 2^-8 of h h, have an accumulator of their own over 16 blocks, 160 steps: what its sum loses in being cut rather than
+// rounded stays below 2^-24 of h h.
+#pragma once
+#include "seq_gemm_split.cuh"
+
+namespace kllm {
+namespace seq {
+namespace umma {
+namespace f32 {
+
+constexpr int BN = 128, KB = 32;           // tokens of a tile, elements of a block of K
+constexpr int kStages = 5;                 // of the ring
+constexpr int kSection = 2, kSmallSection = 16;  // blocks in an accumulator of h h, and in that of the small products
+constexpr int kPartCols = 48;              // TMEM columns of a block's weights: h, m, l
+constexpr int kColSmall = 2 * BN, kColParts = 3 * BN;  // behind the accumulators of h h; parts of two blocks
+constexpr int kWorkers = 16, kTeam = 8;    // warps; those that split a block
+constexpr int kThreads = 32 * (2 + kWorkers);
+constexpr uint32_t kTmemCols = 512;
+static_assert(kColParts + 2 * kPartCols <= static_cast<int>(kTmemCols), "accumulators and parts");
+static_assert(kSection == 2 && kSmallSection % kSection == 0, "both accumulators of a block end with it");
+constexpr int kTokenBytes = BN * 128, kStage = A_BYTES + kTokenBytes * 3 / 2;  // the weights as they arrive; the tokens, then their h and m; l
+constexpr size_t kSmem = 1024 + static_cast<size_t>(kStages) * kStage + 256 + (BM + BN) * sizeof(float);
+static_assert(kSmem <= 232448, "shared memory of one CTA");
+
+__device__ __forceinline__ void mma_tmem(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t joins) {  // A from TMEM
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(joins) : "memory");
+}
+template <typename X>  // float, or its bits
+__device__ __forceinline__ void add_two(X& x, X& y, uint32_t a, uint32_t b) {  // x += a, y += b
+  uint32_t u, v;
+  memcpy(&u, &x, 4), memcpy(&v, &y, 4);
+  asm("{\n .reg .b64 p, q;\n mov.b64 p, {%0, %1};\n mov.b64 q, {%2, %3};\n add.rn.f32x2 p, p, q;\n mov.b64 {%0, %1}, p;\n}"
+      : "+r"(u), "+r"(v) : "r"(a), "r"(b));
+  memcpy(&x, &u, 4), memcpy(&y, &v, 4);
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  __syncwarp();
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  __syncwarp();
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// grid: (feature tiles, S, token tiles), clusters of (1, S, 1)
+template <int OUT>
+__global__ void __launch_bounds__(kThreads, 1)
+umma_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
+                const __grid_constant__ CUtensorMap map_a, const SplitArgs p) {
+  constexpr bool two = OUT == kGated;
+  constexpr int FEATURES = two ? BM / 2 : BM;
+  static_assert(BN * BM * 4 <= kStages * kStage, "the partial tile takes the place of the ring");
+  extern __shared__ uint8_t raw_smem[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + kStages * kStage);
+  uint64_t* parts_in = full + kStages;    // the parts are in TMEM and in the stage
+  uint64_t* done = parts_in + kStages;    // the products have read them, and are summed
+  uint64_t* acc_empty = done + kStages;     // [2]
+  uint64_t* small_empty = acc_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(small_empty + 1);
+  const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), p.report};
+  // != 0 when this CTA's part of K has a number that its parts do not hold, and in which rows (weights, then tokens)
+  float* special = reinterpret_cast<float*>(tmem_slot + 2);
+  float* special_row = special + 1;
+
+  const int warp = warp_number(), lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * FEATURES, t0 = blockIdx.z * BN;
+  const int S = p.S, rank = S > 1 ? static_cast<int>(cluster_rank()) : 0;
+  const int all_blocks = (p.K + KB - 1) / KB;
+  const int kb0 = static_cast<int>(static_cast<long long>(all_blocks) * rank / S);
+  const int blocks = static_cast<int>(static_cast<long long>(all_blocks) * (rank + 1) / S) - kb0;  // >= 1: S <= all_blocks
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(smem_u32(&full[s]), 1);
+      mbar_init(smem_u32(&parts_in[s]), kTeam);
+      mbar_init(smem_u32(&done[s]), 1);
+    }
+    for (int b = 0; b < 2; ++b) mbar_init(smem_u32(&acc_empty[b]), kWorkers);
+    mbar_init(smem_u32(small_empty), kWorkers);
+    *stop.here = 0;
+    *special = 0.f;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = threadIdx.x; i < BM + BN; i += blockDim.x) special_row[i] = 0.f;
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  next_may_start();
+
+  if (warp == 0) {
+    if (elect_one()) {
+      auto weights = [&](int i) {
+        const uint32_t bar = smem_u32(&full[i % kStages]);
+        uint8_t* st = base + (i % kStages) * kStage;
+        mbar_expect_tx(bar, A_BYTES + kTokenBytes);
+        tma_load_2d(smem_u32(st), &map_w, bar, (kb0 + i) * KB, n0);
+        if (two) tma_load_2d(smem_u32(st + A_BYTES / 2), &map_w2, bar, (kb0 + i) * KB, n0);
+      };
+      // the ring's first weights are on their way before the rows they meet are there
+      for (int i = 0; i < kStages && i < blocks; ++i) weights(i);
+      after_previous();
+      for (int i = 0; i < blocks; ++i) {
+        const int s = i % kStages;
+        if (i >= kStages) {
+          if (!mbar_wait(smem_u32(&done[s]), ((i / kStages) & 1) ^ 1u, stop)) break;
+          weights(i);
+        }
+        tma_load_2d(smem_u32(base + s * kStage + A_BYTES), &map_a, smem_u32(&full[s]), (kb0 + i) * KB, t0);
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = instr_desc(BN);
+      bool ok = true;
+      for (int i = 0; i < blocks && ok; ++i) {
+        const int s = i % kStages, section = i / kSection, b = section & 1;
+        const bool opens = i % kSection == 0, opens_small = i % kSmallSection == 0;
+        if (opens) ok = mbar_wait(smem_u32(&acc_empty[b]), ((section >> 1) & 1) ^ 1u, stop);
+        if (ok) ok = mbar_wait(smem_u32(&parts_in[s]), (i / kStages) & 1, stop);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t wh = tmem + kColParts + (i & 1) * kPartCols, wm = wh + 16, wl = wh + 32;
+        const uint32_t at = smem_u32(base + s * kStage + A_BYTES);
+        auto products = [&](uint32_t d, uint32_t w, uint32_t a, bool rest, bool opens_here) {  // both steps of 16 elements
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+            mma_tmem(d, w + k * 8, rest ? smem_desc_64(a + k * 32) : smem_desc(a + k * 32), idesc, opens_here && k == 0 ? 0u : 1u);
+        };
+        products(tmem + b * BN, wh, at, false, opens);
+        if (opens_small) ok = mbar_wait(smem_u32(small_empty), ((i / kSmallSection) & 1) ^ 1u, stop);
+        if (!ok) break;
+        const uint32_t small = tmem + kColSmall;
+        products(small, wl, at, false, opens_small);
+        products(small, wh, at + kTokenBytes, true, false);
+        products(small, wm, at + 64, false, false);
+        products(small, wm, at, false, false);
+        products(small, wh, at + 64, false, false);
+        mma_commit(smem_u32(&done[s]));
+      }
+    }
+  }
+  const int worker = warp - 2, quarter = warp & 3, mine = quarter * 32 + lane;  // a worker's TMEM lanes, a thread's row of the tile
+  constexpr int COLS = BN * 4 / kWorkers;                                        // a thread's tokens, from column col0 on
+  const int col0 = (worker >> 2) * COLS;
+  float* part = reinterpret_cast<float*>(base);  // [BN][BM], in the place of the ring
+  float acc[COLS];
+  bool ok = true;
+  if (worker >= 0) {
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
+    const int team = worker / kTeam, member = worker % kTeam, slice = member >> 2;
+    RowCheck weight, token[BN / 8 / kTeam];  // a lane's rows are the same in every block of K
+    struct Place {  // of a block in the ring
+      int stage, phase;
+      __device__ __forceinline__ void move_on() {  // by two blocks
+        stage += 2;
+        if (stage >= kStages) stage -= kStages, phase ^= 1;
+      }
+    };
+    Place here{team, 0}, before{team, 0}, at_next{1, 0};  // of block i, i - 2, and `next`
+    int next = 1;                                          // the section that ends there is summed next
+    auto until = [&](const Place& block) {                 // its products are done
+      ok = warp_wait(ok, smem_u32(&done[block.stage]), block.phase, stop);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      return ok;
+    };
+    for (int i = team; i < blocks + 5; i += 2) {  // (the last sections are summed behind the last block)
+      const int s = here.stage;
+      if (i < blocks) {
+        ok = warp_wait(ok, smem_u32(&full[s]), here.phase, stop);
+        if (!ok) break;
+        uint8_t* tile = base + s * kStage + A_BYTES;
+        split_tile<BN, kTeam>(tile, tile + kTokenBytes, member, lane, token);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read what was written here
+      }
+      if (next <= i - 3 && next <= blocks) {
+        const bool odd_end = next == blocks;  // the last section has one block
+        const int last = odd_end ? next - 1 : next, b = (next / kSection) & 1;
+        const bool with_small = (last + 1) % kSmallSection == 0 || last + 1 == blocks;
+        if (!until(odd_end ? Place{last % kStages, (last / kStages) & 1} : at_next)) break;
+#pragma unroll
+        for (int c = 0; c < COLS; c += 8) {
+          uint32_t r[8], r2[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+          tmem_ld8(lanes + b * BN + col0 + c, r);
+          if (with_small) tmem_ld8(lanes + kColSmall + col0 + c, r2);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) {
+            add_two(r[j], r[j + 1], r2[j], r2[j + 1]);
+            add_two(acc[c + j], acc[c + j + 1], r[j], r[j + 1]);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (elect_one()) {
+          arrive(&acc_empty[b]);
+          if (with_small) arrive(small_empty);
+        }
+        at_next.move_on();
+        next += kSection;
+      }
+      if (i < blocks) {
+        uint32_t h[8], m[8], l[8];
+        const float4* src = reinterpret_cast<const float4*>(base + s * kStage + mine * 128);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float4 v = src[(4 * slice + c) ^ (mine & 7)];
+          split_pair(v.x, v.y, h[2 * c], m[2 * c], l[2 * c], weight);
+          split_pair(v.z, v.w, h[2 * c + 1], m[2 * c + 1], l[2 * c + 1], weight);
+        }
+        if (i >= 2 && !until(before)) break;  // that block had its weights' parts where this one's go
+        const uint32_t at = lanes + kColParts + (i & 1) * kPartCols + slice * 8;
+        tmem_st8(at, h), tmem_st8(at + 16, m), tmem_st8(at + 32, l);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (elect_one()) arrive(&parts_in[s]);
+        before = here, here.move_on();
+      }
+    }
+    if (weight.special()) special_row[mine] = 1.f, *special = 1.f;
+#pragma unroll
+    for (int i = 0; i < BN / 8 / kTeam; ++i)
+      if (token[i].special()) special_row[BM + split_row<kTeam>(i, member, split_r8(lane))] = 1.f, *special = 1.f;
+    after_previous();  // (what follows writes what earlier kernels may still use)
+    // the last block's commit covers every MMA of this CTA: nothing reads or writes the ring any more
+    if (S > 1 || two)
+#pragma unroll
+      for (int j = 0; j < COLS; ++j) part[(col0 + j) * BM + mine] = acc[j];
+  }
+  __syncwarp();
+  if (S > 1) cluster_sync();  // every partial tile of the cluster is in place, and every `special`
+  else __syncthreads();
+  if (worker >= 0 && ok) {
+    if (!two && S == 1) {
+      if (n0 + mine < p.N) {
+#pragma unroll
+        for (int j = 0; j < COLS; ++j)
+          if (t0 + col0 + j < p.T) split_store<kFp32, OUT>(p, t0 + col0 + j, n0 + mine, acc[j], 0.f);
+      }
+    } else {
+      constexpr int THREADS_IN = 32 * kWorkers;
+      const int thread = (worker >> 2) * BM + mine;
+      if (S == 8) split_reduce<kFp32, BN, OUT, 8, THREADS_IN>(p, part, rank, t0, n0, thread);
+      else if (S == 4) split_reduce<kFp32, BN, OUT, 4, THREADS_IN>(p, part, rank, t0, n0, thread);
+      else if (S == 2) split_reduce<kFp32, BN, OUT, 2, THREADS_IN>(p, part, rank, t0, n0, thread);
+      else if constexpr (two) split_reduce<kFp32, BN, OUT, 1, THREADS_IN>(p, part, rank, t0, n0, thread);
+    }
+  }
+  auto noted = [&](const float* at) {  // by any CTA of the cluster
+    bool any = false;
+    for (int q = 0; q < S; ++q) any = any || (S > 1 ? ld_peer(peer_smem(smem_u32(at), q)) : *at) != 0.f;
+    return any;
+  };
+  if (worker >= 0 && noted(special)) {
+    named_sync<32 * kWorkers>(1);  // the tile is stored
+    split_sum_special<kFp32, BN, OUT, kWorkers>(p, rank, t0, n0, worker, lane, ok, [&](int row) { return noted(special_row + row); },
+                                                 [&](int t) { return noted(special_row + BM + t); });
+  }
+  __syncwarp();
+  if (S > 1) cluster_sync();  // no CTA leaves while another one still reads its partial tile
+  if (*stop.here) {  // a wait ran out: give copies in flight time to land before the shared memory is given up
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+  }
+}
+
+template <int OUT>
+inline int launch_block(SplitArgs p, cudaStream_t stream, bool ahead) {
+  constexpr int FEATURES = OUT == kGated ? BM / 2 : BM;
+  CUtensorMap map_w, map_w2, map_a;
+  if (p.report == nullptr) return KLLM_E_STATE;
+  if (int rc = make_map_of<kFp32>(&map_w, p.w, p.N, p.K, FEATURES)) return rc;
+  if (int rc = make_map_of<kFp32>(&map_w2, OUT == kGated ? p.w2 : p.w, p.N, p.K, FEATURES)) return rc;
+  if (int rc = make_map_of<kFp32>(&map_a, p.a, p.T, p.K, BN)) return rc;
+  auto kernel = umma_f32_kernel<OUT>;
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = true;
+  }
+  const int feature_tiles = (p.N + FEATURES - 1) / FEATURES, token_tiles = (p.T + BN - 1) / BN;
+  p.S = split_count(feature_tiles * token_tiles, (p.K + KB - 1) / KB, kSms);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(feature_tiles, p.S, token_tiles);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = p.S, attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ahead ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_w2, map_a, p);
+  count_launch();
+  return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+}  // namespace f32
+
+template <bool GATED>
+int launch_fp32(const float* a, const float* w, const float* bias, float* out, int T, int K, int N, const GatedAct& act,
+                cudaStream_t s, int* report, bool ahead) {
+  const SplitArgs p{a, w, w + static_cast<size_t>(N) * K, bias, nullptr, out, T, N, K, 1, act, report};
+  constexpr int OUT = GATED ? kGated : kPlain;
+  if (T <= 16) return launch_split<kFp32, 16, OUT, 4>(p, s, ahead);
+  if (T <= 32) return launch_split<kFp32, 32, OUT, 6>(p, s, ahead);
+  if (T <= 64) return launch_split<kFp32, 64, OUT, 6>(p, s, ahead);
+  return f32::launch_block<OUT>(p, s, ahead);
+}
+
+}  // namespace umma
+}  // namespace seq
+}  // namespace kllm

@@ -8,16 +8,15 @@
 //            l m, l l) is at most about 2^-24 of the product, and nothing where one side fits in 8 bits or both in 16.  Six warps
 //            replace a tile's rows by their parts between the tile's arrival and its use.  Rows that hold an infinity, a NaN or a
 //            number whose parts would leave bf16's range (below 2^-100, or rounding up to infinity) are summed by multiply-adds.
-//            (Two TF32 parts and three products, 517 x 1024 x 3072 in 38.9 us, hold 22 bits of an operand: 2.9e-7.)
+//            (Two TF32 parts and three products hold 22 bits of an operand: 2.9e-7 at 517 x 1024 x 3072.)
 //
 // What bounds it: with a few dozen tokens the weights are read once and every element of them feeds 2 * T multiply-adds, so
 // the time is the weights' way from HBM.  A tile per 128 features leaves most SMs without work (width 4096: 32 tiles), and
 // one CTA's ring does not keep enough bytes on the way.  So K is split over the S CTAs of a cluster: each runs the ring of
 // the large form over its part of K, leaves its partial tile in its own shared memory, and after a cluster barrier every
 // CTA sums BN / S of the tile's tokens over the S partials, read through distributed shared memory in rank order (the
-// result does not depend on timing).  kFp32 on token blocks lives in shared memory instead: a stage is read by the splitting warps
-// and its parts written (80 KB at BN = 128), and the MMAs read twelve parts of it (96 KB).  517 x 1024 x 3072: loads and stores take
-// 30 % of the cycles there, the tensor pipe 22 %, issue slots 32 %; the rest is the chain of a stage -- arrival, splitting, products.
+// result does not depend on timing).  kFp32 takes up to 64 tokens here; larger blocks, which live in shared memory and in issue slots
+// instead, are seq_gemm_f32.cuh's.
 //
 // Precision: a tcgen05 accumulator is not rounded to nearest at each of its steps, and its error grows with their number.  A
 // CTA hands its accumulator over every SECTION blocks of K to the epilogue warps, which sum the sections in fp32 registers
@@ -32,8 +31,7 @@
 //   bf16  T = 24, K = 2048, N = 32000   382 -> 28.8 us    3.9e-7 -> 1.4e-7
 //   fp32  T = 16, K = 2048, N = 2048    158 -> 18.8 us    8.1e-7 -> 9.8e-8
 //   fp32  T = 64, K = 4096, N = 4096    314 -> 37.3 us    1.1e-6 -> 1.1e-7
-//   fp32  T = 517, K = 1024, N = 3072   161 -> 47.3 us    5.7e-7 -> 9.4e-8
-//   fp32  T = 9 .. 200, K = 128                           2.0e-7 -> 7.5e-8
+//   fp32  T = 9 .. 64, K = 128                            2.0e-7 -> 7.5e-8
 #pragma once
 #include "seq_gemm_umma.cuh"
 #include "seq_launch.cuh"
@@ -62,36 +60,48 @@ __device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
   return *reinterpret_cast<const uint32_t*>(&v);
 }
-struct RowCheck {  // what a lane has seen of one row
-  float finite = 0.f;         // NaN once a rest was: infinities, NaN, numbers that round up to infinity
-  uint32_t small = ~0u;       // the smallest magnitude other than 0, as 2 * bits - 1 (0 comes out as the largest)
-  __device__ __forceinline__ bool special() const { return finite != finite || small < (27u << 24) - 1u; }  // below 2^-100
-};
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l, RowCheck& check) {
-  check.small = min(check.small, min(2u * __float_as_uint(x) - 1u, 2u * __float_as_uint(y) - 1u));
-  h = pack_bf16(x, y);
-  x -= __uint_as_float(h << 16), y -= __uint_as_float(h & 0xffff0000u);  // a bf16 is the top half of a float
-  check.finite = fmaf(x, 0.f, fmaf(y, 0.f, check.finite));
-  m = pack_bf16(x, y);
-  l = pack_bf16(x - __uint_as_float(m << 16), y - __uint_as_float(m & 0xffff0000u));
+// x -= the lower half of h, y -= its upper half
+__device__ __forceinline__ void take_off(float& x, float& y, uint32_t h) {
+  asm("{\n .reg .b16 lo, hi, minus_one;\n mov.b32 {lo, hi}, %2;\n mov.b16 minus_one, 0xbf80;\n fma.rn.f32.bf16 %0, lo, minus_one, %0;\n"
+      " fma.rn.f32.bf16 %1, hi, minus_one, %1;\n}" : "+f"(x), "+f"(y) : "r"(h));
 }
-// Six warps do it (64 x 4096 x 4096 37.2 us, four 41.1; 517 x 1024 x 3072 49.4 and 51.5); more leave the epilogue too few registers.
+struct RowCheck {  // what a lane has seen of one row
+  float finite[2] = {0.f, 0.f};  // NaN once a rest was: infinities, NaN, numbers that round up to infinity
+  uint32_t small = ~0u;          // the smallest magnitudes of h other than 0, one in either half, less 1 (0 comes out as the largest)
+  __device__ __forceinline__ bool special() const {
+    constexpr uint32_t least = (27u << 7) - 1u;  // 2^-100: below it a number's parts could leave bf16's range
+    return finite[0] != finite[0] || finite[1] != finite[1] || (small & 0xffffu) < least || (small >> 16) < least;
+  }
+};
+// 14 issue slots of a warp for a pair, instead of 17 with the parts widened to fp32 and subtracted, and the smallest number kept in 32 bits
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l, RowCheck& check) {
+  h = pack_bf16(x, y);
+  check.small = __viaddmin_u16x2(h & 0x7fff7fffu, ~0u, check.small);
+  take_off(x, y, h);
+  asm("{\n .reg .b64 p, q, z;\n mov.b64 p, {%2, %3};\n mov.b64 q, {%0, %1};\n mov.b64 z, 0;\n fma.rn.f32x2 q, p, z, q;\n mov.b64 {%0, %1}, q;\n}"
+      : "+f"(check.finite[0]), "+f"(check.finite[1]) : "f"(x), "f"(y));
+  m = pack_bf16(x, y);
+  take_off(x, y, m);
+  l = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);  // what is left fits in a bf16, the top half of a float
+}
+// Six warps of umma_split_kernel do it (64 x 4096 x 4096 37.2 us, four 41.1); more leave the epilogue too few registers.
 constexpr int kSplitWarps = 6;
-template <int ROWS>
-constexpr int kSplitGroups = (ROWS / 8 + kSplitWarps - 1) / kSplitWarps;  // of 8 rows each, that a warp takes
+template <int ROWS, int WARPS = kSplitWarps>
+constexpr int kSplitGroups = (ROWS / 8 + WARPS - 1) / WARPS;  // of 8 rows each, that a warp takes
 // the row of group i that this lane of splitting warp `warp` shares, its last three bits in r8
-__device__ __forceinline__ int split_row(int i, int warp, int r8) { return (i * kSplitWarps + warp) * 8 + r8; }
+template <int WARPS = kSplitWarps>
+__device__ __forceinline__ int split_row(int i, int warp, int r8) { return (i * WARPS + warp) * 8 + r8; }
 __device__ __forceinline__ int split_r8(int lane) { return (lane >> 3) ^ (lane & 4 ? 5 : 0); }
-template <int ROWS>
-__device__ __forceinline__ void split_tile(uint8_t* tile, uint8_t* rest, int warp, int lane, RowCheck (&check)[kSplitGroups<ROWS>]) {
-  constexpr int N = kSplitGroups<ROWS>;
+template <int ROWS, int WARPS = kSplitWarps>
+__device__ __forceinline__ void split_tile(uint8_t* tile, uint8_t* rest, int warp, int lane, RowCheck (&check)[kSplitGroups<ROWS, WARPS>]) {
+  constexpr int N = kSplitGroups<ROWS, WARPS>;
   const int j = lane & 3, r8 = split_r8(lane);
-  auto in = [&](int i) { return (ROWS / 8) % kSplitWarps == 0 || i + 1 < N || split_row(i, warp, 0) < ROWS; };  // the same for a warp
+  auto in = [&](int i) { return (ROWS / 8) % WARPS == 0 || i + 1 < N || split_row<WARPS>(i, warp, 0) < ROWS; };  // the same for a warp
   float4 u[N], v[N];  // everything is read before anything is written: one latency for the tile
 #pragma unroll
   for (int i = 0; i < N; ++i)
     if (in(i)) {
-      const float4* src = reinterpret_cast<const float4*>(tile + split_row(i, warp, r8) * 128);
+      const float4* src = reinterpret_cast<const float4*>(tile + split_row<WARPS>(i, warp, r8) * 128);
       u[i] = src[(2 * j) ^ r8], v[i] = src[(2 * j + 1) ^ r8];
     }
   __syncwarp();  // a row has been read by its four lanes
@@ -103,27 +113,27 @@ __device__ __forceinline__ void split_tile(uint8_t* tile, uint8_t* rest, int war
       split_pair(u[i].z, u[i].w, h.y, m.y, l.y, check[i]);
       split_pair(v[i].x, v[i].y, h.z, m.z, l.z, check[i]);
       split_pair(v[i].z, v[i].w, h.w, m.w, l.w, check[i]);
-      uint4* dst = reinterpret_cast<uint4*>(tile + split_row(i, warp, r8) * 128);
+      uint4* dst = reinterpret_cast<uint4*>(tile + split_row<WARPS>(i, warp, r8) * 128);
       dst[j ^ r8] = h;
       dst[(4 + j) ^ r8] = m;
-      reinterpret_cast<uint4*>(rest + split_row(i, warp, r8) * 64)[j ^ (r8 >> 1)] = l;
+      reinterpret_cast<uint4*>(rest + split_row<WARPS>(i, warp, r8) * 64)[j ^ (r8 >> 1)] = l;
     }
 }
 
 // This CTA's tokens of the tile, summed over the cluster's S partial tiles in rank order: column rank * BN / S + j for the j that
-// this thread has (gated: the threads of the upper 64 rows take every other column of the lower ones' features).  A read from
+// this thread has (where there are more threads than features, they share the columns of a feature).  A read from
 // another CTA takes about a microsecond: a group's reads are all on the way before the first is used (T = 40, K = N = 4096: 15.4 us
 // token by token, 14.6 us).
-template <int MODE, int BN, int OUT, int S>
+template <int MODE, int BN, int OUT, int S, int THREADS_IN = 128>
 __device__ __forceinline__ void split_reduce(const SplitArgs& p, const float* part, int rank, int t0, int n0, int thread) {
   constexpr bool two = OUT == kGated;
-  constexpr int FEATURES = two ? BM / 2 : BM, STEP = two ? 2 : 1, PER = BN / S / STEP;  // columns of a thread
+  constexpr int FEATURES = two ? BM / 2 : BM, STEP = THREADS_IN / FEATURES, PER = BN / S / STEP;  // columns of a thread
   constexpr int GROUP = PER < 32 / S ? PER : 32 / S;
   static_assert(PER >= 1 && PER % GROUP == 0, "tokens of a CTA");
   const int feature = thread % FEATURES, row = n0 + feature;
   if (row >= p.N) return;
   const uint32_t mine = smem_u32(part + feature);
-  const int c0 = rank * (BN / S) + (two ? thread / FEATURES : 0);
+  const int c0 = rank * (BN / S) + thread / FEATURES;
 #pragma unroll 1
   for (int g = 0; g < PER; g += GROUP) {
     float v[GROUP][S], u[two ? GROUP : 1][S];
@@ -148,6 +158,47 @@ __device__ __forceinline__ void split_reduce(const SplitArgs& p, const float* pa
       }
       split_store<MODE, OUT>(p, t, row, a, b);
     }
+  }
+}
+
+// kFp32: outputs of rows that their parts do not hold are summed by multiply-adds and stored over what the parts gave, of the tokens that
+// this part of K's CTA stored.  A warp sums an output with its lanes along K (517 x 1024 x 3072: with one such token 44 us more, with one
+// such weight row 150; a thread per feature took milliseconds).  row_noted, token_noted: whether a row of the tile holds such a number.
+template <int MODE, int BN, int OUT, int WARPS, class Row, class Token>
+__device__ __forceinline__ void split_sum_special(const SplitArgs& p, int rank, int t0, int n0, int warp, int lane, bool ok, Row row_noted,
+                                                  Token token_noted) {
+  static_assert(OUT != kAdd, "an output is stored again here");
+  constexpr bool two = OUT == kGated;
+  constexpr int FEATURES = two ? BM / 2 : BM, MINE = FEATURES / WARPS;
+  const int S = p.S;
+  // this warp's features are warp, warp + WARPS, ...: bit i of `rows` for the i-th
+  bool is_noted = lane < MINE && row_noted(warp + WARPS * lane);
+  if (two) is_noted = is_noted || (lane < MINE && row_noted(FEATURES + warp + WARPS * lane));
+  const uint32_t rows = __ballot_sync(0xffffffffu, is_noted), every = ~0u >> (32 - MINE);
+  for (int j0 = 0; j0 < BN / S; j0 += 32) {
+    const int first = rank * (BN / S) + j0;
+    const uint32_t tokens = __ballot_sync(0xffffffffu, j0 + lane < BN / S && token_noted(first + lane));
+    for (int j = 0; j < 32 && j0 + j < BN / S && t0 + first + j < p.T; ++j)
+      for (uint32_t left = tokens >> j & 1u ? every : rows; left != 0; left &= left - 1u) {
+        const int row = n0 + warp + WARPS * (__ffs(left) - 1);
+        if (row >= p.N) break;
+        const float* ar = static_cast<const float*>(p.a) + static_cast<size_t>(t0 + first + j) * p.K;
+        const float* wr = static_cast<const float*>(p.w) + static_cast<size_t>(row) * p.K;
+        const float* wr2 = two ? static_cast<const float*>(p.w2) + static_cast<size_t>(row) * p.K : wr;
+        float v = 0.f, u = 0.f;
+#pragma unroll 8
+        for (int k = lane; k < p.K; k += 32) {
+          v = fmaf(ar[k], wr[k], v);
+          if (two) u = fmaf(ar[k], wr2[k], u);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (two) u += __shfl_xor_sync(0xffffffffu, u, o);
+        }
+        if (ok && lane == 0) split_store<MODE, OUT>(p, t0 + first + j, row, v, u);
+        __syncwarp();
+      }
   }
 }
 
@@ -178,7 +229,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   constexpr int TILE_COLS = BN;                            // of one sum
   constexpr int ACC_COLS = MODE == kFp32 ? 2 * TILE_COLS : TILE_COLS;  // of one accumulator; there are two
   constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
-  constexpr int AT_ONCE = BN < 32 || (MODE == kFp32 && BN > 64) ? 16 : 32;  // columns on the way from TMEM before the first is added
+  constexpr int AT_ONCE = BN < 32 ? 16 : 32;  // columns on the way from TMEM before the first is added
   static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "columns are given out in powers of two");
   static_assert(TILE_COLS * BM * 4 <= ST * STAGE, "the partial tile takes the place of the ring");
   extern __shared__ uint8_t raw_smem[];
@@ -358,10 +409,6 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
   }
   if constexpr (MODE == kFp32) {
-    // Outputs of rows that their parts do not hold are summed by multiply-adds and stored over what the parts gave.  A warp sums an
-    // output with its lanes along K (517 x 1024 x 3072: 47 us, with one such token 91, with one such weight row 196; a thread per
-    // feature took milliseconds).
-    static_assert(OUT != kAdd, "an output is stored again here");
     auto noted = [&](const float* at) {  // by any CTA of the cluster
       bool any = false;
       for (int q = 0; q < S; ++q) any = any || (S > 1 ? ld_peer(peer_smem(smem_u32(at), q)) : *at) != 0.f;
@@ -369,35 +416,8 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     };
     if (epilogue && noted(special)) {
       named_sync<128>(1);  // the tile is stored
-      // this warp's features are quarter, quarter + 4, ...: bit i of `rows` for the i-th
-      bool row_noted = lane < FEATURES / 4 && noted(special_row + quarter + 4 * lane);
-      if (two) row_noted = row_noted || (lane < FEATURES / 4 && noted(special_row + FEATURES + quarter + 4 * lane));
-      const uint32_t rows = __ballot_sync(0xffffffffu, row_noted), every = ~0u >> (32 - FEATURES / 4);
-      for (int j0 = 0; j0 < BN / S; j0 += 32) {
-        const int first = rank * (BN / S) + j0;
-        const uint32_t tokens = __ballot_sync(0xffffffffu, j0 + lane < BN / S && noted(special_row + BM + first + lane));
-        for (int j = 0; j < 32 && j0 + j < BN / S && t0 + first + j < p.T; ++j)
-          for (uint32_t left = tokens >> j & 1u ? every : rows; left != 0; left &= left - 1u) {
-            const int row = n0 + quarter + 4 * (__ffs(left) - 1);
-            if (row >= p.N) break;
-            const float* ar = static_cast<const float*>(p.a) + static_cast<size_t>(t0 + first + j) * p.K;
-            const float* wr = static_cast<const float*>(p.w) + static_cast<size_t>(row) * p.K;
-            const float* wr2 = two ? static_cast<const float*>(p.w2) + static_cast<size_t>(row) * p.K : wr;
-            float v = 0.f, u = 0.f;
-#pragma unroll 8
-            for (int k = lane; k < p.K; k += 32) {
-              v = fmaf(ar[k], wr[k], v);
-              if (two) u = fmaf(ar[k], wr2[k], u);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-              v += __shfl_xor_sync(0xffffffffu, v, o);
-              if (two) u += __shfl_xor_sync(0xffffffffu, u, o);
-            }
-            if (ok && lane == 0) split_store<MODE, OUT>(p, t0 + first + j, row, v, u);
-            __syncwarp();
-          }
-      }
+      split_sum_special<MODE, BN, OUT, 4>(p, rank, t0, n0, quarter, lane, ok, [&](int row) { return noted(special_row + row); },
+                                          [&](int t) { return noted(special_row + BM + t); });
     }
   }
   __syncwarp();
@@ -480,16 +500,6 @@ inline bool fp32_usable(const void* a, const void* w, int T, int K) {
   static const bool off = [] { const char* e = getenv("KLLM_SEQ_UMMA"); return e != nullptr && e[0] == '0'; }();
   return !off && T > 8 && K >= 128 && (K % 4) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-}
-template <bool GATED>
-int launch_fp32(const float* a, const float* w, const float* bias, float* out, int T, int K, int N, const GatedAct& act,
-                cudaStream_t s, int* report, bool ahead) {
-  const SplitArgs p{a, w, w + static_cast<size_t>(N) * K, bias, nullptr, out, T, N, K, 1, act, report};
-  constexpr int OUT = GATED ? kGated : kPlain;
-  if (T <= 16) return launch_split<kFp32, 16, OUT, 4>(p, s, ahead);
-  if (T <= 32) return launch_split<kFp32, 32, OUT, 6>(p, s, ahead);
-  if (T <= 64) return launch_split<kFp32, 64, OUT, 6>(p, s, ahead);
-  return launch_split<kFp32, 128, OUT, 4>(p, s, ahead);
 }
 
 }  // namespace umma

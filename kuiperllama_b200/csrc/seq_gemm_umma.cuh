@@ -69,6 +69,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const S
 __device__ __forceinline__ bool warp_wait(bool ok, uint32_t bar, uint32_t parity, const Stop& stop) {
   return __all_sync(0xffffffffu, ok && mbar_wait(bar, parity, stop));
 }
+// One lane of a whole warp, the same one at every call.  Products, copies by TMA and commits take their operands from uniform registers: behind
+// `lane == 0` the compiler does not know that one lane is left and wraps each of them in a loop over lanes.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+  return one != 0;
+}
+// this warp's number, known to be the same in all its lanes
+__device__ __forceinline__ int warp_number() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
 template <int THREADS_IN>
 __device__ __forceinline__ void named_sync(int id) {
   __syncwarp();
@@ -212,6 +221,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr) : "memory");
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  __syncwarp();
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
 }
 
 // what a product does with its sums

@@ -1,0 +1,43 @@
+"""fp32 products of more than 64 tokens (csrc/seq_gemm_f32.cuh) against the product in 64 bits: edges of tiles (128 x 128), of blocks of K
+(32), of sections (2 and 16 blocks) and of the ring (5), K over 1 to 8 CTAs.
+
+Left out are products of small parts (2^-24 of the product at most); an accumulator is cut, not rounded, at four steps, and the sections
+are summed in fp32: an element stays within 2^-18 of the sum of the products' magnitudes, as for smaller blocks."""
+import pytest
+
+from test_split_product_gpu import call, product
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,K,N", [
+    (65, 128, 8), (127, 132, 127), (128, 160, 128), (129, 164, 129), (70, 192, 1), (255, 288, 257), (257, 480, 130), (130, 512, 384),
+    (66, 544, 64), (90, 1024, 300), (385, 1028, 1030), (65, 4096, 512), (128, 8192, 260), (600, 2048, 2050)])
+def test_block(T, K, N):
+    import torch
+    a, w, out = product(T, K, N, T * 3 + K, bf16=False)
+    bound = 2.0 ** -18 * (a.abs() @ w.abs().T)
+    assert ((out[:T].double() - a @ w.T).abs() <= bound).all()
+    assert (out[T] == 7.0).all()
+    assert torch.equal(product(T, K, N, T * 3 + K, bf16=False)[2], out)
+
+
+@pytest.mark.parametrize("T,K,N", [(65, 1024, 300), (200, 256, 2000), (130, 136, 5000)])
+def test_block_with_rows_that_have_no_parts(T, K, N):
+    """Infinities, NaN and magnitudes below 2^-100, in token and weight rows, with K split and not."""
+    import torch
+    from kuiperllama_b200 import sequence as sq
+    g = torch.Generator(device="cuda").manual_seed(T)
+    a, w = torch.randn(T, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+    a[1, 5], a[T - 1, K - 1], a[7, 9], w[4, 70], w[N - 1, 5] = float("inf"), -float("inf"), float("nan"), float("inf"), 0.0
+    a[20] *= 2.0 ** -120
+    w[130] *= 2.0 ** -110
+    out = torch.empty(T, N, device="cuda")
+    call(sq, sq.load_seq_library(), sq.F32, a, w, out)
+    ref = (a.double() @ w.double().T).float()
+    assert torch.equal(out.isnan(), ref.isnan())
+    assert torch.equal(out.isinf(), ref.isinf()) and torch.equal(out[ref.isinf()], ref[ref.isinf()])
+    bound = 2.0 ** -18 * (a.double().abs() @ w.double().abs().T)
+    fine = ref.isfinite() & bound.isfinite()
+    fine[20, 130] = False  # (below fp32's range)
+    assert ((out.double() - a.double() @ w.double().T).abs() <= bound)[fine].all()

@@ -7,7 +7,7 @@ from pathlib import Path
 import pytest
 
 CSRC = Path(__file__).resolve().parent.parent / "kuiperllama_b200" / "csrc"
-FILES = ["seq_gemm_umma.cuh", "seq_gemm_split.cuh", "seq_attention_umma.cu"]
+FILES = ["seq_gemm_umma.cuh", "seq_gemm_split.cuh", "seq_attention_umma.cu", "seq_gemm_f32.cuh"]
 
 
 @pytest.mark.parametrize("name", FILES)
