@@ -121,7 +121,7 @@ attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(slots + 4 * kTile);
   const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), report};
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(smem_u32(&k_full[s]), kLoaders);
@@ -207,7 +207,7 @@ attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV 
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == 12) {
     // ---- tensor core ----
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = instr_desc(kTile), idesc_o = instr_desc((vdim + 15) / 16 * 16) | (1u << 16);
       const int ksteps = (dim + 15) / 16;
       auto scores = [&](int i, int grp) {  // over the weights of tile i - 1, which the product issued before reads
@@ -346,7 +346,7 @@ attention_umma_kernel(AttnShape a, const __nv_bfloat16* __restrict__ q, PagedKV 
       tmem_wait_st();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) arrive(&p_full[grp]);
+      if (elect_one()) arrive(&p_full[grp]);
     }
     ok = warp_wait(ok, smem_u32(&o_done[grp]), 0, stop);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

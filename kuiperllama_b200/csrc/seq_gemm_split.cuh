@@ -245,7 +245,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   float* special = reinterpret_cast<float*>(tmem_slot + 2);
   float* special_row = special + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * FEATURES, t0 = blockIdx.z * BN;
   const int S = p.S, rank = S > 1 ? static_cast<int>(cluster_rank()) : 0;
   const int all_blocks = (p.K + M::BKE - 1) / M::BKE;
@@ -281,7 +281,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   next_may_start();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       auto weights = [&](int i) {
         const uint32_t bar = smem_u32(&full[i % ST]);
         uint8_t* st = base + (i % ST) * STAGE;
@@ -302,7 +302,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = MODE == kTf32 ? instr_desc_tf32(BN) : instr_desc(BN);
       uint64_t* ready = MODE == kFp32 ? split_done : full;
       bool ok = true;
@@ -347,7 +347,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       split_tile<ROWS>(base + s * STAGE, base + s * STAGE + HALF, warp - 6, lane, check);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read what was written here
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&split_done[s])) : "memory");
+      if (elect_one()) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&split_done[s])) : "memory");
     }
 #pragma unroll
     for (int i = 0; i < kSplitGroups<ROWS>; ++i) {
@@ -384,7 +384,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+      if (elect_one()) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
     }
     // the last section's commit covers every MMA of this CTA: nothing reads or writes the ring any more
     if (S > 1 || two)

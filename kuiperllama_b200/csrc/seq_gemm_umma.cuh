@@ -326,7 +326,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), p.report};
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   const int kblocks = (K + BKE - 1) / BKE;
   const int feature_tiles = (N + CTAS * FEATURES - 1) / (CTAS * FEATURES), tiles = feature_tiles * ((T + BN - 1) / BN);
   const int first = blockIdx.x / CTAS, step = gridDim.x / CTAS;  // of the tiles that this CTA or pair takes
@@ -364,7 +364,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
   const uint32_t tmem_d = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int i = 0;  // blocks of K so far, over all tiles
       bool ok = true;
       for (int tile = first; tile < tiles && ok; tile += step) {
@@ -386,7 +386,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
       for (int end = i + ST; PAIR && ok && i < end; ++i) ok = mbar_wait(smem_u32(&empty[i % ST]), ((i / ST) & 1) ^ 1u, stop);
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       uint32_t idesc = MODE == kBf16 ? instr_desc(BN) : instr_desc_tf32(BN);
       if constexpr (PAIR) idesc = pair_desc(idesc);
       int i = 0, done = 0;  // blocks of K and tiles so far
@@ -433,7 +433,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
       auto release = [&]() {
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) {
+        if (elect_one()) {
           if constexpr (PAIR) mbar_arrive_cluster(peer_smem(smem_u32(&acc_empty[b]), 0));
           else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
         }
@@ -459,7 +459,7 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
               asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
               __syncwarp();
               const int t = t0 + c + h * kStoreTokens, n = n0 + quarter * 32;
-              if (lane == 0) {
+              if (elect_one()) {
                 if (ok && t < T && n < N) store_2d(&map_out, smem_u32(buf), n, t);
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
               }
@@ -569,7 +569,7 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), report};
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   const int kblocks = (K + BK - 1) / BK;
   const int feature_tiles = (N + FEATURES - 1) / FEATURES, tiles = feature_tiles * *n_tiles;
 
@@ -596,7 +596,7 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   const uint32_t tmem_d = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int i = 0;  // blocks of K so far, over all tiles
       bool ok = true;
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
@@ -618,7 +618,7 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       int i = 0, done = 0;  // blocks of K and tiles so far
       bool ok = true;
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++done) {
@@ -662,7 +662,7 @@ umma_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         if (c + kPairCols >= g.z) {
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+          if (elect_one()) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
         }
         const int here = min(kPairCols, g.z - c);
         if constexpr (EPI == 0) {
