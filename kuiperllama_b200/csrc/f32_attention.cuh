@@ -1,12 +1,10 @@
-// Causal softmax attention in fp32 multiply-adds, in tiles: the inner loop that the sequence engine's fp32 prompts
-// (seq_attention_f32.cu) and the single-sequence decoder's prompts (prefill.cu) share.
+// Causal softmax attention in fp32 multiply-adds, in tiles: what fp32 prompts take for rows that the tensor cores' products cannot give
+// (f32_attention_umma.cuh): rows that see infinities, NaN or magnitudes below 2^-100.
 //
 // 256 threads take 64 rows against tiles of 64 keys.  Thread (tx, ty) of 16 x 16 owns rows ty + 16 i and, of the scores, keys
 // tx + 16 j (4 x 4 of them), of the outputs columns 64 n + 4 tx .. + 3.  Queries, keys, values and weights lie row by row in
 // shared memory, rows padded by 16 bytes: with the rows and keys of a thread 16 apart every 16-byte read of a quarter warp falls
 // on different banks, and nothing has to be transposed on its way in, so tiles come by cp.async, the next under the present one.
-// No single unit bounds it (ncu, 900 tokens, 32 heads of 64, 214 us: FMA pipe 47 %, issue slots 45 %, shared-memory wavefronts 41 % busy, 128
-// registers a thread): 16 scores of a thread take eight 16-byte reads per 64 multiply-adds, and its multiply-adds wait for them.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -21,7 +19,7 @@ constexpr int kRows = 64, kKeys = 64, kThreads = 256, kPad = 4;
 constexpr int LDP = kKeys + kPad;
 
 // shared memory in floats: queries, two tiles of keys, two of values, weights
-inline __host__ __device__ size_t smem_floats(int dim, int nv) {
+constexpr __host__ __device__ size_t smem_floats(int dim, int nv) {
   return static_cast<size_t>(3 * kRows) * (dim + kPad) + 2 * kKeys * 64 * nv + kRows * LDP;
 }
 
@@ -41,10 +39,16 @@ struct Sums {  // of rows ty + 16 i
   }
 };
 
+// the barriers of the threads that attend() runs on: a block of kThreads
+struct WholeBlock {
+  static __device__ __forceinline__ void sync() { __syncthreads(); }
+  static __device__ __forceinline__ bool any(bool v) { return __syncthreads_or(v); }
+};
+
 // Work: q(row) -> the row's query (nullptr: no such row), key(j, c) and value(j, c) -> 16 bytes number c of key / value j (nullptr:
 // zeros), n_tiles, tile(i) -> number of the i-th tile, hidden(row, j) -> row does not see key j, whole(tile) -> every row sees all
 // of it; score(s) -> the score of a product of query and key.
-template <int NV, class Work>
+template <int NV, class Work, class Sync = WholeBlock>
 __device__ __forceinline__ void attend(const Work& w, int dim, int vdim, float* sm, Sums<NV>& r) {
   constexpr int LDV = 64 * NV;
   const int LD = dim + kPad, qc = dim >> 2, vc = vdim >> 2;
@@ -95,7 +99,7 @@ __device__ __forceinline__ void attend(const Work& w, int dim, int vdim, float* 
     } else {
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
-    __syncthreads();
+    Sync::sync();
     float s[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -130,7 +134,7 @@ __device__ __forceinline__ void attend(const Work& w, int dim, int vdim, float* 
         const float4 v = *reinterpret_cast<const float4*>(Vs + (stage * kKeys + z / vc) * LDV + z % vc * 4);
         odd = odd || !(fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY);
       }
-      guarded = __syncthreads_or(odd);
+      guarded = Sync::any(odd);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -184,7 +188,7 @@ __device__ __forceinline__ void attend(const Work& w, int dim, int vdim, float* 
     };
     if (guarded) add_values(std::true_type{});
     else add_values(std::false_type{});
-    __syncthreads();  // the stage is loaded again two tiles on
+    Sync::sync();  // the stage is loaded again two tiles on
   }
   r.finish();
 }

@@ -1,0 +1,452 @@
+// Causal softmax attention in fp32 on the 5th-generation tensor cores (sm_100a): what the sequence engine's fp32 prompts
+// (seq_attention_f32.cu) and the single-sequence decoder's prompts (prefill.cu) share.
+//
+// A CTA takes 128 rows of one key head against tiles of 64 keys.  Both products are those of fp32 operands in three bf16 parts each, six
+// products (kFp32 of seq_gemm_split.cuh has the parts): S = Q K^T with the queries' parts in TMEM and the keys' in shared memory, and
+// O = P V with the weights' parts in TMEM and the values' in shared memory (coordinates contiguous: MN-major).
+//   warps 0 .. 7    softmax: two threads to a row, each half of a tile's keys and half of the output's coordinates
+//   warp 8          tcgen05.mma
+//   warps 9 .. 15   keys and values: read a tile ahead, split, written in the layout of the 128-byte swizzle
+// What bounds it: the warps that split.  A tile lasts 3700 cycles (clock stamps, 900 tokens, 32 heads of 64 on 4): the products take 1540 of
+// the tensor pipe, a softmax thread's chain 1900 (maximum and exponentials 1250, parts and hand-over 650), but a loader warp needs 3700
+// for its pieces, a third of it waits for instructions: every CTA splits the keys and values again, in long straight code.
+// Measured against 64 x 64 tiles of multiply-adds (f32_attention.cuh; one B200, us, whole layers where not said otherwise):
+//   the attention alone of 900 tokens, 32 heads of 64 on 4 key heads   214 -> 46 (errors 1.5e-7; 700 tokens, 16 heads of 128: 79)
+//   2 prompts of 700 together, 16 heads of 64 on 4   339 -> 248      one of 600, 16 heads of 128 on 4   456 -> 324
+//   3 of 300, 16 of 128 on 2, a window of 512        242 -> 213      one of 100, 8 heads of 64          137 -> 127
+//   5 of 60 together, 16 of 64 on 2                  131 -> 129      6 of 60 together, 8 heads of 128   158 -> 159
+//   With expf, 32 products a loop instead of unrolled and the heads' tiles one after another 90 for the first line; loads that the compiler
+//   was free to move to their use 48; the registers of the 128-coordinate forms spill (up to 1 KB a thread), 128 is all that 16 warps leave.
+//
+// TMEM: the queries' parts, one or two tiles of scores, a tile of weights' parts, a tile's output.  The scores of the next tile are
+// multiplied while the softmax has the present one.
+//
+// Precision: an accumulator holds one tile -- a tensor core cuts its sums rather than rounding them, and the tiles' outputs are joined in
+// fp32 registers.  In it the five small products come first, then h h.  Exponentials are 2^((s - max) * factor * log2 e), by ex2.approx
+// (about 2^-22 of the weight).
+//
+// Numbers that the parts do not hold (infinities, NaN, magnitudes below 2^-100 other than 0): eight coordinates of a key or value that hold
+// one enter the products as zeros, and the rows that see the key, and rows with such queries, are computed again by multiply-adds
+// (f32_attention.cuh).  The other rows keep their bits.
+#pragma once
+#include "f32_attention.cuh"
+#include "seq_engine.h"
+#include "seq_gemm_split.cuh"
+
+namespace kllm {
+namespace f32attn {
+namespace umma {
+
+using namespace seq::umma;
+
+constexpr int kTile = 128, kTileKeys = 64;
+constexpr int kSoftmax = 8, kLoaders = 7, kBlock = 32 * (kSoftmax + 1 + kLoaders);
+constexpr int kBlockBytes = kTileKeys * 128;  // of one part: 64 keys x 64 coordinates
+template <int D>
+constexpr int kParts = 3 * (D / 64) * kBlockBytes;
+template <int DK, int DV>
+constexpr int kStages = DK == 64 && DV == 64 ? 4 : DK == 64 || DV == 64 ? 3 : 2;  // tiles of keys and of values
+template <int DK, int DV>
+constexpr int kScoreTiles = 3 * DK / 2 + 2 * kTileKeys + 3 * kTileKeys / 2 + DV <= 512 ? 2 : 1;
+template <int DK, int DV>
+constexpr size_t smem_bytes() {
+  const size_t here = 1024 + static_cast<size_t>(kStages<DK, DV>) * (kParts<DK> + kParts<DV>) + 7 * kTile * sizeof(float) + 256;
+  const size_t again = 16 + smem_floats(DK, DV / 64) * sizeof(float);  // the multiply-adds' tiles, in the place of these
+  return here > again ? here : again;
+}
+
+__device__ __forceinline__ void arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void mma_tmem(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t joins) {  // A from TMEM
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(joins) : "memory");
+}
+// values, MN-major with the 128-byte swizzle: leading byte offset = the next 64 coordinates, stride byte offset = the next 8 keys
+__device__ __forceinline__ uint64_t value_desc(uint32_t saddr) {
+  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(kBlockBytes >> 4) << 16) | (64ull << 32) | (1ull << 46) |
+         (2ull << 61);
+}
+// 16 bytes, or zeros; stays where it is written, ahead of the waits that it is to run under
+__device__ __forceinline__ void load16(float4& v, const float* from, bool in) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n mov.f32 %0, 0f00000000;\n mov.f32 %1, 0f00000000;\n mov.f32 %2, 0f00000000;\n"
+               " mov.f32 %3, 0f00000000;\n @p ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
+               : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w) : "l"(from), "r"(static_cast<uint32_t>(in)) : "memory");
+}
+__device__ __forceinline__ float ex2(float x) {  // 2^x, relative error about 2^-22; 2^-inf = 0
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void times_less(float& x, float& y, float sub, float by) {  // (x - sub) * by, (y - sub) * by
+  asm("{\n .reg .b64 p, q;\n mov.b64 p, {%0, %1};\n mov.b64 q, {%2, %2};\n sub.rn.f32x2 p, p, q;\n mov.b64 q, {%3, %3};\n"
+      " mul.rn.f32x2 p, p, q;\n mov.b64 {%0, %1}, p;\n}" : "+f"(x), "+f"(y) : "f"(sub), "f"(by));
+}
+__device__ __forceinline__ void split_weight(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {  // (0 .. 1: nothing to check)
+  h = pack_bf16(x, y);
+  take_off(x, y, h);
+  m = pack_bf16(x, y);
+  take_off(x, y, m);
+  l = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+}
+// of the 256 threads that compute rows again
+struct HalfBlock {
+  static __device__ __forceinline__ void sync() { asm volatile("bar.sync 6, 256;" ::: "memory"); }
+  static __device__ __forceinline__ bool any(bool v) {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, 6, 256, p;\n selp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(r) : "r"(static_cast<uint32_t>(v)) : "memory");
+    return r != 0;
+  }
+};
+
+// Work as in f32_attention.cuh, of 128 rows, and besides: kb + key_row(j) + key_column(c), vb + value_row(j) + value_column(c) -> 16 bytes
+// number c of key / value j <= last_key(); key_step(), value_step() -> from an even such number to
+// the next (0: it varies); plain() -> score(s) is s * factor(), factor() > 0; seen(row, first, last) -> the keys that a row sees, first .. last (last = -1: none)
+// and those before keep(); at(rows) -> the same work from that row on; store(row, m, l, c, o) -> takes four coordinates of a row's output
+// before the division by l.
+template <int DK, int DV, class Work>
+__device__ __forceinline__ void attend(const Work& w, int dim, int vdim, uint8_t* raw_smem, int* report) {
+  constexpr int NS = kScoreTiles<DK, DV>, ST = kStages<DK, DV>;
+  constexpr int kColS = 3 * DK / 2, kColP = kColS + NS * kTileKeys, kColO = kColP + 3 * kTileKeys / 2;
+  static_assert(kColO + DV <= 512, "columns of TMEM");
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
+  uint8_t* keys = base;
+  uint8_t* values = keys + ST * kParts<DK>;
+  float* top = reinterpret_cast<float*>(values + ST * kParts<DV>);  // [2][half][row]
+  float* sums = top + 4 * kTile;                                          // [half][row]
+  int* odd_query = reinterpret_cast<int*>(sums + 2 * kTile);              // [row]: it holds a number without parts
+  uint64_t* bars = reinterpret_cast<uint64_t*>(odd_query + kTile);
+  uint64_t *k_full = bars, *k_empty = k_full + ST, *v_full = k_empty + ST, *v_empty = v_full + ST, *score_in = v_empty + ST;
+  uint64_t *score_out = score_in + 2, *q_in = score_out + 2, *weights_in = q_in + 1, *out_in = weights_in + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(out_in + 1);
+  int* odd = reinterpret_cast<int*>(tmem_slot + 2);  // the first and the last key that holds one, and whether any query does
+  const Stop stop{reinterpret_cast<volatile int*>(tmem_slot + 1), report};
+
+  const int warp = warp_number(), lane = threadIdx.x & 31, n = w.n_tiles;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < ST; ++s) {
+      mbar_init(smem_u32(&k_full[s]), kLoaders);
+      mbar_init(smem_u32(&v_full[s]), kLoaders);
+      mbar_init(smem_u32(&k_empty[s]), 1);
+      mbar_init(smem_u32(&v_empty[s]), 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&score_in[s]), 1);
+      mbar_init(smem_u32(&score_out[s]), kSoftmax);
+    }
+    mbar_init(smem_u32(q_in), kSoftmax);
+    mbar_init(smem_u32(weights_in), kSoftmax);
+    mbar_init(smem_u32(out_in), 1);
+    *stop.here = 0;
+    odd[0] = 0x7fffffff, odd[1] = -1, odd[2] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < kTile) odd_query[threadIdx.x] = 0;
+  if (warp == kSoftmax) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  const int quarter = warp & 3, half = (warp >> 2) & 1, row = quarter * 32 + lane;  // of a softmax thread
+  constexpr int COLS = DV / 2;                                                       // its coordinates of the output
+  float acc[COLS], m = -INFINITY, l = 0.f;
+#pragma unroll
+  for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
+  bool ok = true;
+  if (warp < kSoftmax && n > 0) {
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+    RowCheck check;
+    const float* q = w.q(row);
+#pragma unroll 1
+    for (int c = half * (DK / 2); c < (half + 1) * (DK / 2); c += 32) {  // 32 coordinates
+      uint32_t h[16], md[16], lo[16];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 v = q != nullptr && c + 4 * j < dim ? *reinterpret_cast<const float4*>(q + c + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        split_pair(v.x, v.y, h[2 * j], md[2 * j], lo[2 * j], check);
+        split_pair(v.z, v.w, h[2 * j + 1], md[2 * j + 1], lo[2 * j + 1], check);
+      }
+      tmem_st16(lanes + c / 2, h), tmem_st16(lanes + DK / 2 + c / 2, md), tmem_st16(lanes + DK + c / 2, lo);
+    }
+    if (check.special()) odd_query[row] = 1, odd[2] = 1;
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if (elect_one()) arrive(q_in);
+    int first, last;
+    w.seen(row, first, last);
+    // scores that are products times a positive number keep their order: that number enters with the exponents
+    const bool plain = w.plain();
+    const float factor2 = (plain ? w.factor() : 1.f) * 1.4426950408889634f;
+    float before = 0.f;  // what a tile's maximum takes off the sums so far
+    auto join = [&](int i) {  // adds tile i's output
+      ok = warp_wait(ok, smem_u32(out_in), i & 1, stop);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < COLS; c += 16) {
+        uint32_t r[16];
+        tmem_ld16(lanes + kColO + half * COLS + c, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(acc[c + j], before, __uint_as_float(r[j]));
+      }
+    };
+    for (int i = 0; i < n; ++i) {  // (a warp whose wait ran out still meets its partner at every barrier below)
+      const int k0 = w.tile(i) * kTileKeys + half * 32;
+      float* tops = top + (i & 1) * 2 * kTile;
+      float p[32];
+      {
+        uint32_t r[32];
+        ok = warp_wait(ok, smem_u32(&score_in[i % NS]), (i / NS) & 1, stop);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_ld32(lanes + kColS + (i % NS) * kTileKeys + half * 32, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (elect_one()) arrive(&score_out[i % NS]);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) p[j] = __uint_as_float(r[j]);
+      }
+      if (!plain) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) p[j] = w.score(p[j]);
+      }
+      if (!__all_sync(0xffffffffu, k0 + 31 <= last && k0 >= first)) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (k0 + j > last || (k0 + j < first && k0 + j >= w.keep())) p[j] = -INFINITY;
+      }
+      float most = m;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) most = fmaxf(most, p[j]);
+      tops[half * kTile + row] = most;
+      named_sync<64>(1 + quarter);  // the two warps of these rows
+      most = fmaxf(most, tops[(half ^ 1) * kTile + row]);
+      // a row that has seen nothing yet keeps max = -inf; subtracting 0 instead keeps 2^(-inf - 0) = 0 free of NaN
+      const float sub = most > -INFINITY ? most : 0.f, keep = ex2((m - sub) * factor2);
+      m = most;
+      float sum[2] = {0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) {
+        times_less(p[j], p[j + 1], sub, factor2);
+        p[j] = ex2(p[j]), p[j + 1] = ex2(p[j + 1]);
+        add_two(sum[0], sum[1], __float_as_uint(p[j]), __float_as_uint(p[j + 1]));
+      }
+      l = l * keep + (sum[0] + sum[1]);
+      const uint32_t at = lanes + kColP + half * 16;
+      if constexpr (COLS == 32) {  // the parts are ready when the products have read tile i - 1's weights
+        uint32_t h[16], md[16], lo[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) split_weight(p[2 * j], p[2 * j + 1], h[j], md[j], lo[j]);
+        if (i > 0) join(i - 1);
+        tmem_st16(at, h), tmem_st16(at + kTileKeys / 2, md), tmem_st16(at + kTileKeys, lo);
+      } else {  // (registers do not hold them)
+        if (i > 0) join(i - 1);
+#pragma unroll
+        for (int c = 0; c < 16; c += 8) {
+          uint32_t h[8], md[8], lo[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) split_weight(p[2 * (c + j)], p[2 * (c + j) + 1], h[j], md[j], lo[j]);
+          tmem_st8(at + c, h), tmem_st8(at + kTileKeys / 2 + c, md), tmem_st8(at + kTileKeys + c, lo);
+        }
+      }
+      before = keep;
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (elect_one()) arrive(weights_in);
+    }
+    join(n - 1);
+    sums[half * kTile + row] = l;
+    named_sync<64>(1 + quarter);
+    l = sums[row] + sums[kTile + row];
+    if (plain) m *= w.factor();
+  } else if (warp == kSoftmax) {
+    if (n > 0 && elect_one()) {
+      const uint32_t idesc_s = instr_desc(kTileKeys), idesc_o = instr_desc((vdim + 15) / 16 * 16) | (1u << 16);
+      const int steps = (dim + 15) / 16;
+      auto scores = [&](int i) {
+        if (!mbar_wait(smem_u32(&k_full[i % ST]), (i / ST) & 1, stop) ||
+            !mbar_wait(smem_u32(&score_out[i % NS]), ((i / NS) & 1) ^ 1u, stop))
+          return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t at = smem_u32(keys + (i % ST) * kParts<DK>), d = tmem + kColS + (i % NS) * kTileKeys;
+        auto products = [&](int qp, int kp, bool opens) {  // part qp of the queries with part kp of the keys
+#pragma unroll
+          for (int k = 0; k < DK / 16; ++k)  // 16 coordinates, inside the swizzle row
+            if (k < steps) mma_tmem(d, tmem + qp * (DK / 2) + k * 8, smem_desc(at + (kp * (DK / 64) + (k >> 2)) * kBlockBytes + (k & 3) * 32), idesc_s,
+                     opens && k == 0 ? 0u : 1u);
+        };
+        products(2, 0, true), products(0, 2, false), products(1, 1, false), products(1, 0, false), products(0, 1, false);
+        products(0, 0, false);
+        if (i + ST < n) mma_commit(smem_u32(&k_empty[i % ST]));  // (somebody waits for it)
+        mma_commit(smem_u32(&score_in[i % NS]));
+        return true;
+      };
+      bool go = mbar_wait(smem_u32(q_in), 0, stop) && scores(0);
+      for (int i = 0; i < n && go; ++i) {
+        if (i + 1 < n && !scores(i + 1)) break;
+        go = mbar_wait(smem_u32(&v_full[i % ST]), (i / ST) & 1, stop) && mbar_wait(smem_u32(weights_in), i & 1, stop);
+        if (!go) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t at = smem_u32(values + (i % ST) * kParts<DV>);
+        auto products = [&](int pp, int vp, bool opens) {
+#pragma unroll
+          for (int k = 0; k < kTileKeys / 16; ++k)  // 16 keys: 8 columns of weights, 16 rows of values
+            mma_tmem(tmem + kColO, tmem + kColP + pp * (kTileKeys / 2) + k * 8, value_desc(at + vp * (DV / 64) * kBlockBytes + k * 2048),
+                     idesc_o, opens && k == 0 ? 0u : 1u);
+        };
+        products(2, 0, true), products(0, 2, false), products(1, 1, false), products(1, 0, false), products(0, 1, false);
+        products(0, 0, false);
+        if (i + ST < n) mma_commit(smem_u32(&v_empty[i % ST]));
+        mma_commit(smem_u32(out_in));
+      }
+    }
+    __syncwarp();
+  } else if (n > 0) {
+    const int t = threadIdx.x - 32 * (kSoftmax + 1);
+    // a tile is 64 x D / 8 pieces of 8 coordinates of a key; this thread has piece t and every 224th after it
+    auto place = [&](auto width, bool by_key, int z, int& j, int& c) {
+      constexpr int C = decltype(width)::value / 8;
+      if (by_key) j = z % kTileKeys, c = z / kTileKeys;
+      else j = z / C, c = z % C;
+    };
+    auto count = [](int d) constexpr { return (8 * d + 32 * kLoaders - 1) / (32 * kLoaders); };
+    // where this thread's pieces lie inside a key's or value's coordinates (-1: there is none)
+    auto columns = [&](auto width, int used, bool by_key, auto column, auto& at) {
+      constexpr int D = decltype(width)::value;
+#pragma unroll
+      for (int x = 0; x < count(D); ++x) {
+        int j, c;
+        place(width, by_key, t + x * 32 * kLoaders, j, c);
+        at[x] = j < kTileKeys && c < D / 8 && 8 * c < used ? column(2 * c) : -1;
+      }
+    };
+    auto read = [&](auto width, int used, bool by_key, const float* from, auto row_of, auto column, int step, int i, const auto& at, auto& v) {
+      constexpr int D = decltype(width)::value;
+      const int j0 = w.tile(i) * kTileKeys;
+#pragma unroll
+      for (int x = 0; x < count(D); ++x) {
+        int j, c;
+        place(width, by_key, t + x * 32 * kLoaders, j, c);
+        const bool in = at[x] >= 0 && j0 + j <= w.last_key(), second = in && 8 * c + 4 < used;
+        const float* src = from + (in ? row_of(j0 + j) + at[x] : 0);
+        load16(v[x][0], src, in);
+        load16(v[x][1], src + (!second ? 0 : step ? step : column(2 * c + 1) - at[x]), second);
+      }
+    };
+    auto write = [&](auto width, bool by_key, int i, uint8_t* to, const auto& v) {
+      constexpr int D = decltype(width)::value;
+      auto dst = [&](int j, int c) { return reinterpret_cast<uint4*>(to + (c >> 3) * kBlockBytes + j * 128 + (((c & 7) ^ (j & 7)) << 4)); };
+      auto put = [&](uint4* p, const uint4& h, const uint4& md, const uint4& lo) {
+        p[0] = h, p[(D / 64) * kBlockBytes / 16] = md, p[2 * (D / 64) * kBlockBytes / 16] = lo;
+      };
+      auto split = [&](const float4& a, const float4& b, uint4& h, uint4& md, uint4& lo, RowCheck& check) {
+        split_pair(a.x, a.y, h.x, md.x, lo.x, check), split_pair(a.z, a.w, h.y, md.y, lo.y, check);
+        split_pair(b.x, b.y, h.z, md.z, lo.z, check), split_pair(b.z, b.w, h.w, md.w, lo.w, check);
+      };
+      RowCheck all;
+#pragma unroll
+      for (int x = 0; x < count(D); ++x) {
+        int j, c;
+        place(width, by_key, t + x * 32 * kLoaders, j, c);
+        uint4 h, md, lo;
+        split(v[x][0], v[x][1], h, md, lo, all);
+        if (j < kTileKeys && c < D / 8) put(dst(j, c), h, md, lo);
+      }
+      if (all.special()) {  // which ones?
+#pragma unroll 1
+        for (int z = t; z < 8 * D; z += 32 * kLoaders) {
+          int j, c;
+          place(width, by_key, z, j, c);
+          uint4 h, md, lo;
+          RowCheck check;
+#pragma unroll
+          for (int x = 0; x < count(D); ++x)
+            if (t + x * 32 * kLoaders == z) split(v[x][0], v[x][1], h, md, lo, check);
+          if (check.special()) {
+            put(dst(j, c), make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u));
+            const int key = w.tile(i) * kTileKeys + j;
+            atomicMin(&odd[0], key), atomicMax(&odd[1], key);
+          }
+        }
+      }
+    };
+    using KW = std::integral_constant<int, DK>;
+    using VW = std::integral_constant<int, DV>;
+    const bool by_key = w.keys_by_chunk();
+    auto key_row = [&](int j) { return w.key_row(j); };
+    auto value_row = [&](int j) { return w.value_row(j); };
+    auto key_column = [&](int c) { return w.key_column(c); };
+    auto value_column = [&](int c) { return w.value_column(c); };
+    int k_at[count(DK)], v_at[count(DV)];
+    columns(KW{}, dim, by_key, key_column, k_at);
+    columns(VW{}, vdim, false, value_column, v_at);
+    float4 k[count(DK)][2], v[count(DV)][2];
+    read(KW{}, dim, by_key, w.kb, key_row, key_column, w.key_step(), 0, k_at, k);
+    for (int i = 0; i < n; ++i) {
+      const int s = i % ST;
+      read(VW{}, vdim, false, w.vb, value_row, value_column, w.value_step(), i, v_at, v);
+      if (!warp_wait(true, smem_u32(&k_empty[s]), ((i / ST) & 1) ^ 1u, stop)) break;
+      write(KW{}, by_key, i, keys + s * kParts<DK>, k);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read what was written here
+      __syncwarp();
+      if (elect_one()) arrive(&k_full[s]);
+      if (i + 1 < n) read(KW{}, dim, by_key, w.kb, key_row, key_column, w.key_step(), i + 1, k_at, k);
+      if (!warp_wait(true, smem_u32(&v_empty[s]), ((i / ST) & 1) ^ 1u, stop)) break;
+      write(VW{}, false, i, values + s * kParts<DV>, v);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (elect_one()) arrive(&v_full[s]);
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();  // the last output has been joined: no product reads or writes anything any more
+  const bool again = odd[0] <= odd[1] || odd[2] != 0, stopped = *stop.here != 0;
+  auto redone = [&](int r) {
+    int first, last;
+    w.seen(r, first, last);
+    return odd_query[r] != 0 || (odd[0] <= last && (odd[1] >= first || odd[0] < w.keep()));
+  };
+  if (stopped)
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  if (warp == kSoftmax)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  if (warp < kSoftmax && !stopped && !(again && redone(row))) {
+#pragma unroll
+    for (int c = 0; c < COLS; c += 4)
+      if (half * COLS + c < vdim) w.store(row, m, l, half * COLS + c, make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]));
+  }
+  if (again) {
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    uint32_t mine = 0;  // of the rows that multiply-adds give this thread, in turn, those which take their result
+    for (int i = 0; i < kTile / 16; ++i) mine |= threadIdx.x < kThreads && redone(ty + 16 * i) ? 1u << i : 0u;
+    __syncthreads();  // everybody has read what shared memory holds
+    if (threadIdx.x < kThreads && !stopped) {
+      float* sm = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(raw_smem) + 15) & ~uintptr_t(15));
+      for (int from = 0; from < kTile; from += kRows) {
+        const Work part = w.at(from);
+        Sums<DV / 64> r;
+        f32attn::attend<DV / 64, Work, HalfBlock>(part, dim, vdim, sm, r);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int c = 0; c < DV / 64; ++c)
+            if ((mine >> (from / 16 + i) & 1u) && c * 64 + tx * 4 < vdim)
+              part.store(ty + 16 * i, r.m[i], r.l[i], c * 64 + tx * 4,
+                         make_float4(r.o[i][4 * c], r.o[i][4 * c + 1], r.o[i][4 * c + 2], r.o[i][4 * c + 3]));
+        HalfBlock::sync();  // its tiles are loaded again
+      }
+    }
+  }
+}
+
+}  // namespace umma
+}  // namespace f32attn
+}  // namespace kllm

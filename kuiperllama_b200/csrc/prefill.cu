@@ -18,7 +18,7 @@
 #include <cstdint>
 
 #include "../../include/kllm_b200.h"
-#include "f32_attention.cuh"
+#include "f32_attention_umma.cuh"
 #include "kllm_device.cuh"
 #include "kllm_host.h"
 
@@ -163,68 +163,82 @@ __global__ void attn_rows_kernel(const float* __restrict__ q, const float* __res
   }
 }
 
-// Causal attention of the block's queries over cache positions 0 .. start_pos + t (mha_kernel.cu:47-110 arithmetic, fp32
-// throughout), in tiles: a CTA takes 64 queries of one head against tiles of 64 keys (f32_attention.cuh).  The form before it was
-// one CTA per query and head whose threads each walked whole key rows: every key and value was read from L2 once per query, and
-// half the time one thread per column summed the values alone.  Here a key is read once per 64 queries and the FMA pipe bounds it.
+// Causal attention of the block's queries over cache positions 0 .. start_pos + t (fp32 throughout), on the tensor cores
+// (f32_attention_umma.cuh): a CTA takes 128 rows of one key head, row r = token r / rep, query head kvh * rep + r % rep, so that the
+// query heads that share keys share their tiles.  900 tokens, 32 heads of 64 on 4 key heads: 214 us a layer on multiply-adds with 64
+// queries of one head to a CTA, 46 here; with the key heads one after another instead of side by side in the grid the last one's long
+// tiles come last (90).
 struct CacheWork {
   const float *qb, *kb, *vb;
+  float* out;
   CacheLayout c;
-  int heads, head, kvh, start_pos, t0, rows, last, n_tiles;
+  int heads, rep, kvh, start_pos, r0, n_rows, last, n_tiles, v_pitch;
   float scale;
 
   // the persistent engine's keys lie chunk by chunk, the other layout's and all values row by row
   __device__ __forceinline__ bool keys_by_chunk() const { return c.mega != 0; }
   __device__ __forceinline__ const float* any() const { return kb; }
-  __device__ __forceinline__ const float* q(int row) const {
-    return row < rows ? qb + (static_cast<size_t>(t0 + row) * heads + head) * c.head_size : nullptr;
-  }
+  __device__ __forceinline__ size_t row_at(int r) const { return (static_cast<size_t>(r / rep) * heads + kvh * rep + r % rep) * c.head_size; }
+  __device__ __forceinline__ const float* q(int row) const { return r0 + row < n_rows ? qb + row_at(r0 + row) : nullptr; }
   __device__ __forceinline__ const float* key(int j, int ch) const { return j <= last ? kb + k_index(c, j, kvh, ch * 4) : nullptr; }
   __device__ __forceinline__ const float* value(int j, int ch) const { return j <= last ? vb + v_index(c, j, kvh, ch * 4) : nullptr; }
+  __device__ __forceinline__ int last_key() const { return last; }
+  __device__ __forceinline__ int key_row(int j) const { return j * (c.mega ? 4 : c.kv_dim); }
+  __device__ __forceinline__ int key_column(int ch) const { return static_cast<int>(k_index(c, 0, kvh, ch * 4)); }
+  __device__ __forceinline__ int key_step() const { return c.mega ? 4 * c.seq_len : 4; }
+  __device__ __forceinline__ int value_row(int j) const { return j * v_pitch; }
+  __device__ __forceinline__ int value_step() const { return v_pitch % 8 == 0 || !c.mega ? 4 : 0; }
+  __device__ __forceinline__ int value_column(int ch) const { return static_cast<int>(v_index(c, 0, kvh, ch * 4)); }
   __device__ __forceinline__ int tile(int i) const { return i; }
-  __device__ __forceinline__ bool hidden(int row, int j) const { return j > start_pos + t0 + row; }
-  __device__ __forceinline__ bool whole(int t) const { return t * f32attn::kKeys + f32attn::kKeys - 1 <= start_pos + t0; }
-  __device__ __forceinline__ float score(float s) const { return s * scale; }
-};
-template <int NV>  // head_size <= 64 NV, a multiple of 4
-__global__ void __launch_bounds__(f32attn::kThreads)
-attn_tile_kernel(const float* __restrict__ q, const float* __restrict__ kcache, const float* __restrict__ vcache,
-                 float* __restrict__ out, CacheLayout c, int heads, int kv_mul, int start_pos, int T) {
-  extern __shared__ __align__(16) float sm[];
-  const int hs = c.head_size, head = blockIdx.y;
-  const int t0 = (gridDim.x - 1 - blockIdx.x) * f32attn::kRows;  // the tiles with the most keys start first
-  const int rows = min(f32attn::kRows, T - t0), last = start_pos + t0 + rows - 1;
-  const CacheWork w{q, kcache, vcache, c, heads, head, head / kv_mul, start_pos, t0, rows, last, last / f32attn::kKeys + 1,
-                    1.f / sqrtf(static_cast<float>(hs))};
-  f32attn::Sums<NV> r;
-  f32attn::attend<NV>(w, hs, hs, sm, r);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int row = ty + 16 * i;
-    if (row >= rows) continue;
-    float* dst = out + (static_cast<size_t>(t0 + row) * heads + head) * hs;
-#pragma unroll
-    for (int n = 0; n < NV; ++n)
-      if (n * 64 + tx * 4 < hs)
-        *reinterpret_cast<float4*>(dst + n * 64 + tx * 4) =
-            make_float4(r.o[i][n * 4] / r.l[i], r.o[i][n * 4 + 1] / r.l[i], r.o[i][n * 4 + 2] / r.l[i], r.o[i][n * 4 + 3] / r.l[i]);
+  __device__ __forceinline__ int keep() const { return 0; }
+  __device__ __forceinline__ void seen(int row, int& first, int& to) const {
+    first = 0, to = r0 + row < n_rows ? start_pos + (r0 + row) / rep : -1;
   }
+  __device__ __forceinline__ bool hidden(int row, int j) const { return r0 + row >= n_rows || j > start_pos + (r0 + row) / rep; }
+  __device__ __forceinline__ bool whole(int t) const {
+    return r0 + f32attn::kRows <= n_rows && t * f32attn::kKeys + f32attn::kKeys - 1 <= start_pos + r0 / rep;
+  }
+  __device__ __forceinline__ float score(float s) const { return s * scale; }
+  __device__ __forceinline__ bool plain() const { return true; }
+  __device__ __forceinline__ float factor() const { return scale; }
+  __device__ __forceinline__ CacheWork at(int rows) const {
+    CacheWork w = *this;
+    w.r0 += rows;
+    return w;
+  }
+  __device__ __forceinline__ void store(int row, float, float l, int col, float4 o) const {
+    if (r0 + row < n_rows) *reinterpret_cast<float4*>(out + row_at(r0 + row) + col) = make_float4(o.x / l, o.y / l, o.z / l, o.w / l);
+  }
+};
+template <int D>  // head_size <= D, a multiple of 4
+__global__ void __launch_bounds__(f32attn::umma::kBlock, 1)
+attn_tile_kernel(const float* __restrict__ q, const float* __restrict__ kcache, const float* __restrict__ vcache,
+                 float* __restrict__ out, CacheLayout c, int heads, int rep, int start_pos, int T, int* report) {
+  extern __shared__ uint8_t raw_smem[];
+  const int r0 = (gridDim.y - 1 - blockIdx.y) * f32attn::umma::kTile;  // the tiles with the most keys start first
+  const int n_rows = T * rep, last = start_pos + (min(r0 + f32attn::umma::kTile, n_rows) - 1) / rep;
+  const CacheWork w{q, kcache, vcache, out, c, heads, rep, static_cast<int>(blockIdx.x), start_pos, r0, n_rows, last, last / f32attn::kKeys + 1,
+                    c.mega ? c.head_size / c.split : c.kv_dim, 1.f / sqrtf(static_cast<float>(c.head_size))};
+  f32attn::umma::attend<D, D>(w, c.head_size, c.head_size, raw_smem, report);
 }
 
 // heads of whole 16-byte chunks up to 128 coordinates, whose value slices are whole chunks too
 inline bool attn_tile_usable(const CacheLayout& c) {
   return c.head_size <= 128 && (c.head_size & 3) == 0 && ((c.head_size / c.split) & 3) == 0 && (c.kv_dim & 3) == 0;
 }
-template <int NV>
+template <int D>
 int launch_attn_tile(const float* q, const float* kcache, const float* vcache, float* out, const CacheLayout& c, int heads,
-                     int kv_mul, int start_pos, int T, cudaStream_t s) {
-  const cudaError_t e = cudaFuncSetAttribute(attn_tile_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(f32attn::smem_floats(64 * NV, NV) * sizeof(float)));
-  if (e != cudaSuccess) return static_cast<int>(e);
-  attn_tile_kernel<NV><<<dim3((T + f32attn::kRows - 1) / f32attn::kRows, heads), f32attn::kThreads,
-                         f32attn::smem_floats(c.head_size, NV) * sizeof(float), s>>>(
-      q, kcache, vcache, out, c, heads, kv_mul, start_pos, T);
+                     int rep, int start_pos, int T, cudaStream_t s, int* report) {
+  constexpr size_t smem = f32attn::umma::smem_bytes<D, D>();
+  static_assert(smem <= 232448, "shared memory of one CTA");
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(attn_tile_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = true;
+  }
+  const dim3 grid(heads / rep, (T * rep + f32attn::umma::kTile - 1) / f32attn::umma::kTile);
+  attn_tile_kernel<D><<<grid, f32attn::umma::kBlock, smem, s>>>(q, kcache, vcache, out, c, heads, rep, start_pos, T, report);
   return 0;
 }
 
@@ -285,9 +299,9 @@ int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* to
       const size_t sc_bytes = static_cast<size_t>(start_pos + T) * sizeof(float);  // (allowed by prefill_takes)
       attn_rows_kernel<<<dim3(heads, T), 128, sc_bytes, s>>>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos);
     } else if (hs <= 64) {
-      PF_TRY(launch_attn_tile<1>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos, T, s));
+      PF_TRY(launch_attn_tile<64>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos, T, s, wait));
     } else {
-      PF_TRY(launch_attn_tile<2>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos, T, s));
+      PF_TRY(launch_attn_tile<128>(ws.q, kc, vc, ws.att, cl, heads, heads / kvh, start_pos, T, s, wait));
     }
     PF_TRY(count());
     PF_TRY(prefill_product_add(ws.att, f32(m.wo[l]), ws.x, T, q_rows, dim, s, wait));  // llama3.cpp:683

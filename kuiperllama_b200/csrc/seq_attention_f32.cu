@@ -1,16 +1,14 @@
 // Prompt attention of the sequence-batch engine in fp32: the problem of attention_mma_kernel (seq_attention_mma.cu) -- a CTA takes
-// 64 consecutive rows of one entry and one key/value head, row r = token r / rep, query head g * rep + r % rep -- on fp32
-// multiply-adds, by the loop of f32_attention.cuh.  With one split the kernel divides by the sum, joins the sink and applies the
-// output gate itself; with several it leaves (max, sum, unnormalised output) per split for attention_merge_kernel.
+// 128 consecutive rows of one entry and one key/value head, row r = token r / rep, query head g * rep + r % rep -- by the loop of
+// f32_attention_umma.cuh.  With one split the kernel divides by the sum, joins the sink and applies the output gate itself; with several
+// it leaves (max, sum, unnormalised output) per split for attention_merge_kernel.
 //
-// The split-key kernel that these steps took before (attention_kernel, 32 rows against 64 keys) brings keys in by scalar loads
-// between two barriers and reads two 4-byte operands from shared memory for every four multiply-adds of a score; it stays for few
-// rows and for head sizes past 128.
+// Few rows, and head sizes past 128, stay with the split-key kernel (attention_kernel, 32 rows against 64 keys).
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
-#include "f32_attention.cuh"
+#include "f32_attention_umma.cuh"
 #include "seq_engine.h"
 #include "seq_mma.cuh"
 
@@ -25,7 +23,11 @@ struct PagedWork {
   const PagedKV& kv;
   int r0, n_rows, first, pos0, rep, g, gv, pmax;
   int keep_tiles, tile_first, tile_lo, n_tiles;
-  int pos_lo, seen_hi;  // the first row's position, the first key that the last row sees
+  int seen_hi;  // the first key that the last row sees
+  int splits, split;
+  float* ws;
+  const float* gates;
+  float* out;
 
   __device__ __forceinline__ bool keys_by_chunk() const { return false; }
   __device__ __forceinline__ const float* any() const { return kb; }
@@ -40,6 +42,15 @@ struct PagedWork {
   __device__ __forceinline__ const float* value(int j, int c) const {
     return j <= pmax ? vb + slot(j) * kv.v_row + gv * a.vdim + c * 4 : nullptr;
   }
+  __device__ __forceinline__ int last_key() const { return pmax; }
+  __device__ __forceinline__ size_t key_row(int j) const { return slot(j) * kv.k_row; }
+  __device__ __forceinline__ int key_column(int c) const { return g * a.dim + c * 4; }
+  __device__ __forceinline__ int key_step() const { return 4; }
+  __device__ __forceinline__ int value_step() const { return 4; }
+  __device__ __forceinline__ size_t value_row(int j) const { return slot(j) * kv.v_row; }
+  __device__ __forceinline__ int value_column(int c) const { return gv * a.vdim + c * 4; }
+  __device__ __forceinline__ bool plain() const { return !(a.softcap > 0.f) && a.scale > 0.f; }
+  __device__ __forceinline__ float factor() const { return a.scale; }
   __device__ __forceinline__ int tile(int i) const {
     const int li = tile_lo + i;
     return li < keep_tiles ? li : tile_first + (li - keep_tiles);
@@ -50,7 +61,39 @@ struct PagedWork {
     return r >= n_rows || j > p || (j < first_seen(a, p) && j >= a.keep_first);
   }
   __device__ __forceinline__ bool whole(int t) const {
-    return r0 + f32attn::kRows <= n_rows && t * f32attn::kKeys + f32attn::kKeys - 1 <= pos_lo && t * f32attn::kKeys >= seen_hi;
+    return r0 + f32attn::kRows <= n_rows && t * f32attn::kKeys + f32attn::kKeys - 1 <= pos0 + r0 / rep && t * f32attn::kKeys >= seen_hi;
+  }
+  __device__ __forceinline__ int keep() const { return a.keep_first; }
+  __device__ __forceinline__ void seen(int row, int& from, int& to) const {
+    const bool exists = r0 + row < n_rows;
+    to = exists ? pos0 + (r0 + row) / rep : -1, from = exists ? first_seen(a, to) : 0x7fffffff;
+  }
+  __device__ __forceinline__ PagedWork at(int rows) const {
+    PagedWork w = *this;
+    w.r0 += rows;
+    return w;
+  }
+  // (m: the row's maximum, l: the sum of its exponentials, o: not divided by it yet)
+  __device__ __forceinline__ void store(int row, float m, float l, int col, float4 o) const {
+    const int r = r0 + row, vdim = a.vdim;
+    if (r >= n_rows) return;
+    const size_t th = static_cast<size_t>(first + r / rep) * a.heads + g * rep + r % rep;
+    if (splits == 1 && !a.no_merge) {
+      if (a.sink != nullptr)  // exp(sink) joins the denominator
+        l = m > -INFINITY ? l + expf(a.sink[th % a.heads] - m) : 1.0f;
+      const bool per_element = gates != nullptr && a.gate == KLLM_SEQ_GATE_ELEMENT;
+      const float head_gate = gates && !per_element ? gates[th] : 1.0f;
+      float4 gt = make_float4(head_gate, head_gate, head_gate, head_gate);
+      if (per_element) {
+        const float* ge = gates + th * vdim + col;
+        gt = make_float4(ge[0], ge[1], ge[2], ge[3]);
+      }
+      *reinterpret_cast<float4*>(out + th * vdim + col) = make_float4(o.x / l * gt.x, o.y / l * gt.y, o.z / l * gt.z, o.w / l * gt.w);
+    } else {
+      float* p = ws + (th * splits + split) * (vdim + 2);
+      if (col == 0) p[0] = m, p[1] = l;
+      p[2 + col] = o.x, p[3 + col] = o.y, p[4 + col] = o.z, p[5 + col] = o.w;
+    }
   }
   __device__ __forceinline__ float score(float s) const {
     s *= a.scale;
@@ -58,19 +101,19 @@ struct PagedWork {
   }
 };
 
-template <int NV>
-__global__ void __launch_bounds__(f32attn::kThreads)
+template <int DK, int DV>
+__global__ void __launch_bounds__(f32attn::umma::kBlock, 1)
 attention_f32_kernel(AttnShape a, const float* __restrict__ q, PagedKV kv, const int32_t* __restrict__ ent_first,
                      const int32_t* __restrict__ ent_count, const int32_t* __restrict__ ent_seq,
                      const int32_t* __restrict__ ent_pos0, int splits, float* __restrict__ ws, const float* __restrict__ gates,
-                     float* __restrict__ out) {
-  extern __shared__ __align__(16) float sm[];
+                     float* __restrict__ out, int* report) {
+  extern __shared__ uint8_t raw_smem[];
   const int e = blockIdx.x / a.kv_heads, g = blockIdx.x % a.kv_heads, split = blockIdx.z;
   const int rep = a.heads / a.kv_heads;
   const int first = ent_first[e], pos0 = ent_pos0[e], n_rows = ent_count[e] * rep;
-  const int r0 = (gridDim.y - 1 - blockIdx.y) * f32attn::kRows;  // the tiles with the most keys start first
+  const int r0 = (gridDim.y - 1 - blockIdx.y) * f32attn::umma::kTile;  // the tiles with the most keys start first
   if (r0 >= n_rows) return;
-  const int last_row = min(r0 + f32attn::kRows, n_rows) - 1;
+  const int last_row = min(r0 + f32attn::umma::kTile, n_rows) - 1;
   const int pmax = pos0 + last_row / rep;  // last position any row of the tile sees
   const int n_tiles = pmax / f32attn::kKeys + 1;
   // with a window or chunks no row of the tile sees anything before what its first row sees; tiles before that which hold kept
@@ -81,46 +124,9 @@ attention_f32_kernel(AttnShape a, const float* __restrict__ q, PagedKV kv, const
   const int tile_lo = split * per, tile_hi = min(list_n, tile_lo + per);
   const PagedWork w{a, q, static_cast<const float*>(kv.k), static_cast<const float*>(kv.v),
                     kv.table + static_cast<size_t>(ent_seq[e]) * kv.table_stride, kv, r0, n_rows, first, pos0, rep, g,
-                    g / v_share_of(a), pmax, keep_tiles, tile_first, tile_lo, max(0, tile_hi - tile_lo), pos0 + r0 / rep,
-                    first_seen(a, pmax)};
-  f32attn::Sums<NV> r;
-  f32attn::attend<NV>(w, a.dim, a.vdim, sm, r);
-
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, vdim = a.vdim;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int rr = r0 + ty + 16 * i;
-    if (rr >= n_rows) continue;
-    const size_t th = static_cast<size_t>(first + rr / rep) * a.heads + g * rep + rr % rep;
-    if (splits == 1 && !a.no_merge) {
-      float l = r.l[i];
-      if (a.sink != nullptr)  // exp(sink) joins the denominator
-        l = r.m[i] > -INFINITY ? l + expf(a.sink[th % a.heads] - r.m[i]) : 1.0f;
-      const bool per_element = gates != nullptr && a.gate == KLLM_SEQ_GATE_ELEMENT;
-      const float head_gate = gates && !per_element ? gates[th] : 1.0f;
-#pragma unroll
-      for (int n = 0; n < NV; ++n) {
-        const int col = n * 64 + tx * 4;
-        if (col >= vdim) break;
-        float4 gt = make_float4(head_gate, head_gate, head_gate, head_gate);
-        if (per_element) {
-          const float* ge = gates + th * vdim + col;
-          gt = make_float4(ge[0], ge[1], ge[2], ge[3]);
-        }
-        *reinterpret_cast<float4*>(out + th * vdim + col) =
-            make_float4(r.o[i][n * 4] / l * gt.x, r.o[i][n * 4 + 1] / l * gt.y, r.o[i][n * 4 + 2] / l * gt.z,
-                        r.o[i][n * 4 + 3] / l * gt.w);
-      }
-    } else {
-      float* p = ws + (th * splits + split) * (vdim + 2);
-      if (tx == 0) p[0] = r.m[i], p[1] = r.l[i];
-#pragma unroll
-      for (int n = 0; n < NV; ++n)
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (n * 64 + tx * 4 + c < vdim) p[2 + n * 64 + tx * 4 + c] = r.o[i][n * 4 + c];
-    }
-  }
+                    g / v_share_of(a), pmax, keep_tiles, tile_first, tile_lo, max(0, tile_hi - tile_lo),
+                    first_seen(a, pmax), splits, split, ws, gates, out};
+  f32attn::umma::attend<DK, DV>(w, a.dim, a.vdim, raw_smem, report);
 }
 
 }  // namespace
@@ -133,29 +139,39 @@ bool attention_f32_usable(int dtype, const AttnShape& a, const PagedKV& kv, int 
   return dims && max_count >= 2 && max_count * (a.heads / a.kv_heads) >= 16;
 }
 
-template <int NV>
+template <int DK, int DV>
 static int launch_f32(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
                       const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0,
-                      int max_count, int splits, float* ws, void* out, cudaStream_t s) {
-  const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(f32attn::smem_floats(128, NV) * sizeof(float)));
-  if (e != cudaSuccess) return cuda_rc(e);
+                      int max_count, int splits, float* ws, void* out, int* report, cudaStream_t s) {
+  constexpr size_t smem = f32attn::umma::smem_bytes<DK, DV>();
+  static_assert(smem <= 232448, "shared memory of one CTA");
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return cuda_rc(e);
+    configured = true;
+  }
   const int rep = a.heads / a.kv_heads;
-  const dim3 grid(n_entries * a.kv_heads, (max_count * rep + f32attn::kRows - 1) / f32attn::kRows, splits);
+  const dim3 grid(n_entries * a.kv_heads, (max_count * rep + f32attn::umma::kTile - 1) / f32attn::umma::kTile, splits);
   if (grid.y > 65535u) return KLLM_E_UNSUPPORTED;
-  attention_f32_kernel<NV><<<grid, f32attn::kThreads, f32attn::smem_floats(a.dim, NV) * sizeof(float), s>>>(
+  attention_f32_kernel<DK, DV><<<grid, f32attn::umma::kBlock, smem, s>>>(
       a, static_cast<const float*>(q), kv, ent_first, ent_count, ent_seq, ent_pos0, splits, ws, a.gate ? gates : nullptr,
-      static_cast<float*>(out));
+      static_cast<float*>(out), report);
   count_launch();
   return cuda_rc(cudaGetLastError());
 }
 
 int launch_attention_f32(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
                          const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0,
-                         int max_count, int splits, float* ws, void* out, cudaStream_t s) {
-  if (a.vdim <= 64)
-    return launch_f32<1>(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, s);
-  return launch_f32<2>(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, s);
+                         int max_count, int splits, float* ws, void* out, cudaStream_t s, int* report) {
+  if (report == nullptr) return KLLM_E_STATE;
+#define KLLM_ATTN_F32(K, V) \
+  return launch_f32<K, V>(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, report, s)
+  if (a.dim <= 64 && a.vdim <= 64) KLLM_ATTN_F32(64, 64);
+  if (a.dim <= 64) KLLM_ATTN_F32(64, 128);
+  if (a.vdim <= 64) KLLM_ATTN_F32(128, 64);
+  KLLM_ATTN_F32(128, 128);
+#undef KLLM_ATTN_F32
 }
 
 }  // namespace seq

@@ -219,7 +219,7 @@ int launch_attention_umma(const AttnShape& a, const void* q, const float* gates,
 bool attention_f32_usable(int dtype, const AttnShape& a, const PagedKV& kv, int max_count);
 int launch_attention_f32(const AttnShape& a, const void* q, const float* gates, const PagedKV& kv, int n_entries,
                          const int32_t* ent_first, const int32_t* ent_count, const int32_t* ent_seq, const int32_t* ent_pos0,
-                         int max_count, int splits, float* ws, void* out, cudaStream_t s);
+                         int max_count, int splits, float* ws, void* out, cudaStream_t s, int* report);
 
 // bf16 steps of few rows per key head, or with fp32 queries (head sizes that are multiples of 8): partial results of every
 // split in `ws`, like the split-key kernel, or (`out` not null, one split) the finished rows.

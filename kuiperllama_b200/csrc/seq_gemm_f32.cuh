@@ -53,26 +53,6 @@ __device__ __forceinline__ void mma_tmem(uint32_t d, uint32_t a, uint64_t b, uin
   asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
                ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(joins) : "memory");
 }
-template <typename X>  // float, or its bits
-__device__ __forceinline__ void add_two(X& x, X& y, uint32_t a, uint32_t b) {  // x += a, y += b
-  uint32_t u, v;
-  memcpy(&u, &x, 4), memcpy(&v, &y, 4);
-  asm("{\n .reg .b64 p, q;\n mov.b64 p, {%0, %1};\n mov.b64 q, {%2, %3};\n add.rn.f32x2 p, p, q;\n mov.b64 {%0, %1}, p;\n}"
-      : "+r"(u), "+r"(v) : "r"(a), "r"(b));
-  memcpy(&x, &u, 4), memcpy(&y, &v, 4);
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  __syncwarp();
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  __syncwarp();
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
 __device__ __forceinline__ void arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }

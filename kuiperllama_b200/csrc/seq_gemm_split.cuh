@@ -60,6 +60,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
   return *reinterpret_cast<const uint32_t*>(&v);
 }
+template <typename X>  // float, or its bits
+__device__ __forceinline__ void add_two(X& x, X& y, uint32_t a, uint32_t b) {  // x += a, y += b
+  uint32_t u, v;
+  memcpy(&u, &x, 4), memcpy(&v, &y, 4);
+  asm("{\n .reg .b64 p, q;\n mov.b64 p, {%0, %1};\n mov.b64 q, {%2, %3};\n add.rn.f32x2 p, p, q;\n mov.b64 {%0, %1}, p;\n}"
+      : "+r"(u), "+r"(v) : "r"(a), "r"(b));
+  memcpy(&x, &u, 4), memcpy(&y, &v, 4);
+}
 // x -= the lower half of h, y -= its upper half
 __device__ __forceinline__ void take_off(float& x, float& y, uint32_t h) {
   asm("{\n .reg .b16 lo, hi, minus_one;\n mov.b32 {lo, hi}, %2;\n mov.b16 minus_one, 0xbf80;\n fma.rn.f32.bf16 %0, lo, minus_one, %0;\n"

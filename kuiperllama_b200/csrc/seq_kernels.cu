@@ -1748,7 +1748,8 @@ int launch_attention(int dtype, const AttnShape& a, const void* q, const float* 
                               out, s);
     if (rc || (splits == 1 && !a.no_merge)) return rc;
   } else if (attention_f32_usable(dtype, a, kv, max_count)) {
-    rc = launch_attention_f32(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, s);
+    rc = launch_attention_f32(a, q, gates, kv, n_entries, ent_first, ent_count, ent_seq, ent_pos0, max_count, splits, ws, out, s,
+                              report);
     if (rc || (splits == 1 && !a.no_merge)) return rc;
   } else if (attention_rows_mma_usable(dtype, a, kv, n_entries)) {
     const bool whole = splits == 1 && !a.no_merge;

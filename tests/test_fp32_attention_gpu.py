@@ -1,0 +1,53 @@
+"""fp32 attention on the tensor cores (csrc/f32_attention_umma.cuh): numbers that three bf16 parts do not hold.  Rows that see such a key or
+value are summed by multiply-adds, every other row keeps its bits.  (Edges of tiles, windows, kept positions, gates: test_attention_exact_gpu.py.)"""
+import numpy as np
+import pytest
+
+from test_attention_exact_gpu import VOCAB, assert_close, by_sequence, run_layer, softmax_attention
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("where", ["query", "key", "value"])
+@pytest.mark.parametrize("odd", [float("inf"), float("nan"), 2.0 ** -110])
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(4, 1, 64, 64), (2, 2, 128, 72)])
+def test_numbers_without_parts(where, odd, heads, kv, dim, vdim):
+    import torch
+    lens = [200, 70]
+    cuts = [heads * dim, kv * dim, kv * vdim]
+    width = max(sum(cuts), heads * vdim)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    embed = torch.randn(VOCAB, width, device="cuda", generator=g)
+    eye, scale = torch.eye(width, device="cuda")[:sum(cuts)].contiguous(), dim ** -0.5
+
+    def fill(L, w_out):
+        L.mixer_kind, a = 1, L.attn
+        a.heads, a.kv_heads, a.dim, a.vdim, a.scale, a.w_in, a.w_out = heads, kv, dim, vdim, scale, eye.data_ptr(), w_out.data_ptr()
+        return eye, w_out
+
+    ids = np.random.default_rng(3).integers(0, VOCAB, sum(lens)).astype(np.int32)  # run_layer's
+    token = int(ids[90])
+    at = {"query": dim + 3, "key": heads * dim + 5, "value": heads * dim + kv * dim + 9}[where] % width
+    if where == "query":
+        at = dim + 3  # of the second head
+    before, plain = run_layer("fp32", width, heads * vdim, fill, lens, embed)
+    changed = embed.clone()
+    changed[token, at] = odd
+    # the projections of a row that is not finite are not finite in every coordinate: only a tiny number stays where it was put
+    x, got = run_layer("fp32", width, heads * vdim, fill, lens, changed)
+    sees = torch.zeros(sum(lens), dtype=torch.bool, device="cuda")
+    start = 0
+    for n in lens:
+        hit = np.flatnonzero(ids[start:start + n] == token)
+        if len(hit):
+            sees[start + int(hit[0]):start + n] = True
+        start += n
+    assert torch.equal(got[~sees], plain[~sees])
+    if odd != 2.0 ** -110:
+        assert not got[sees].isfinite().all(1).any()  # as multiply-adds over such keys and values give
+        return
+    T = sum(lens)
+    q, k, v = x[:, :sum(cuts)].split(cuts, 1)
+    exact, size = by_sequence(lens, [q.reshape(T, heads, dim), k.reshape(T, kv, dim), v.reshape(T, kv, vdim)],
+                              lambda *p: softmax_attention(*p, scale))
+    assert_close(got.reshape(T, heads, vdim), exact, size, x, 2.0 ** -20, 2.0 ** -18)
