@@ -20,19 +20,20 @@ inline TileWaves tile_waves(bool gated, int T, int N) {
   return TileWaves{(features * ((T + 127) / 128) + kSms - 1) / kSms, (features * tokens + kSms - 1) / kSms,
                    ((features + 1) / 2 * tokens + kSms / 2 - 1) / (kSms / 2)};
 }
-// Measured with every form at 40 shapes from 900 to 6001 tokens and 4 to 6 lengths of K, bf16 and TF32 (a block of K is 128 bytes of a
-// row, 64 bf16 values).  us, wide / pair / narrow:
-//   plain, 32 blocks   one wide wave 21.2 / 23.2 / 29.3 (2048 x 2048); two 33.3 / 33.9 / 39.3 (2048 x 3072), 35.3 / 34.4 / 49.9 (x 4352);
-//                      three 50.3 / 45.7 / 72.1 (x 6144); five 75.7 / 69.1 / 102.6 (6001 x 3456)
-//   plain, 16 blocks   one 15.3 / 17.3 / 19.4; two 23.1 / 23.2 / 25.3; three 31.1 / 30.0 / 41.6
-//   plain, 8 blocks    one 14.5 / 16.2 / 16.3; two 18.5 / 20.4 / 18.8; three 23.3 / 24.0 / 27.2; five 33.7 / 33.9 / 37.2
-//   a pair too many    an odd number of feature tiles can cost pairs a wave more: 900 x 4736 21.5 / 33.4 / 29.5 (32 blocks), 33.2 / 53.8 /
-//                      49.8 (64), 2048 x 4736 35.5 / 45.7 / 50.1
-//   all narrow tiles at once    520 x 3072: - / 18.6 / 16.5 (32 blocks), - / 32.9 / 30.2 (64)
-//   gated, 8 to 32     the way out of a tile bounds it, and a pair's CTAs wait for one another: one 33.7 / 35.6 / 38.9 (2048 x 1024, 32 blocks),
-//                      eleven 232 / 244 / 266 (6001 x 4096); two and three 54.3 / 50.9 / 51.0 (2048 x 1536), 79.1 / 75.4 / 88.1 (x 3328);
-//                      16 blocks 47.8 / 45.4 / 40.5 (x 1536), 103.9 / 108.7 / 99.5 (6001 x 1728)
-//   gated, 64 blocks   one 48.0 / 48.9 / 64.3; two 71.8 / 68.7 / 86.1; five 147 / 142 / 215
+// Measured with every form at 72 plain and 44 gated shapes from 300 to 6001 tokens and K = 512 to 4096, bf16 (a block of K is 128 bytes of a
+// row, 64 bf16 values); the form that the rule takes is the fastest or within 10 % of it but for 300 to 700 tokens in 48 narrow tiles, which
+// stay split (their sums are closer there).  us, wide / pair / narrow:
+//   plain, 32 blocks   one wide wave 16.8 / 18.7 / 20.9 (2048 x 2048); two 28.9 / 29.0 / 28.9 (2048 x 3072), 28.9 / 29.3 / 36.9 (x 4352);
+//                      three 45.3 / 41.7 / 54.0 (x 6144); five 80.8 / 74.0 / 93.2 (6001 x 3456)
+//   plain, 16 blocks   one 12.5 / 14.5 / 14.5; two 18.6 / 18.7 / 18.6; three 26.8 / 25.5 / 30.9
+//   plain, 8 blocks    one 10.5 / 12.5 / 10.4; two 14.5 / 15.6 / 13.3; three 18.9 / 20.6 / 20.9; five 29.9 / 30.9 / 31.9
+//   a pair too many    an odd number of feature tiles can cost pairs a wave more: 900 x 4736 18.7 / 29.0 / 22.9 (32 blocks), 30.4 / 49.4 /
+//                      37.1 (64), 2048 x 4736 31.0 / 39.1 / 38.1
+//   all narrow tiles at once    520 x 3072: 18.6 / 20.7 / 14.5 (32 blocks), 26.8 / 28.9 / 20.7 (64)
+//   gated, 8 to 32     a pair's CTAs wait for one another on the way out: one 21.1 / 24.8 / 23.9 (2048 x 1024, 32 blocks), eleven 144 / 148 /
+//                      195 (6001 x 4096); two and three 31.3 / 32.9 / 31.0 (2048 x 1536), 41.8 / 41.4 / 51.6 (x 3328);
+//                      16 blocks 21.8 / 24.8 / 18.6 (x 1536), 41.9 / 47.3 / 41.3 (6001 x 1728)
+//   gated, 64 blocks   one 31.0 / 33.0 / 37.1; two 50.9 / 53.5 / 51.5; five 160 / 154 / 189
 inline TileForm tile_form(bool gated, int T, int N, int kblocks) {
   const TileWaves w = tile_waves(gated, T, N);
   // a narrow tile takes this many hundredths of a wide one's time
