@@ -145,6 +145,15 @@ __device__ __forceinline__ void split_reduce(const SplitArgs& p, const float* pa
 #pragma unroll 1
   for (int g = 0; g < PER; g += GROUP) {
     float v[GROUP][S], u[two ? GROUP : 1][S];
+    // what is added is on its way too: behind a store to `out`, which may be the same memory, each would wait for the one before it
+    float add[OUT == kAdd ? GROUP : 1];
+    if constexpr (OUT == kAdd) {
+#pragma unroll
+      for (int j = 0; j < GROUP; ++j) {
+        const int t = t0 + c0 + (g + j) * STEP;
+        add[j] = t < p.T ? p.add[static_cast<size_t>(t) * p.N + row] : 0.f;
+      }
+    }
 #pragma unroll
     for (int q = 0; q < S; ++q) {
       const uint32_t from = (S > 1 ? peer_smem(mine, static_cast<uint32_t>(q)) : mine) + (c0 + g * STEP) * BM * 4;
@@ -164,7 +173,7 @@ __device__ __forceinline__ void split_reduce(const SplitArgs& p, const float* pa
         a += v[j][q];
         if constexpr (two) b += u[j][q];
       }
-      split_store<MODE, OUT>(p, t, row, a, b);
+      split_store<MODE, OUT>(p, t, row, a, OUT == kAdd ? add[OUT == kAdd ? j : 0] : b);
     }
   }
 }
@@ -405,9 +414,18 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   if (epilogue && ok) {
     if (!two && S == 1) {
       if (n0 + mine < p.N) {
+        constexpr int GROUP = BN < 32 ? BN : 32;
 #pragma unroll
-        for (int j = 0; j < BN; ++j)
-          if (t0 + j < p.T) split_store<MODE, OUT>(p, t0 + j, n0 + mine, acc[j], 0.f);
+        for (int c = 0; c < BN; c += GROUP) {
+          float add[OUT == kAdd ? GROUP : 1];
+          if constexpr (OUT == kAdd) {
+#pragma unroll
+            for (int j = 0; j < GROUP; ++j) add[j] = t0 + c + j < p.T ? p.add[static_cast<size_t>(t0 + c + j) * p.N + n0 + mine] : 0.f;
+          }
+#pragma unroll
+          for (int j = 0; j < GROUP; ++j)
+            if (t0 + c + j < p.T) split_store<MODE, OUT>(p, t0 + c + j, n0 + mine, acc[c + j], OUT == kAdd ? add[OUT == kAdd ? j : 0] : 0.f);
+        }
       }
     } else {
       if (S == 8) split_reduce<MODE, BN, OUT, 8>(p, part, rank, t0, n0, mine);

@@ -291,6 +291,7 @@ __device__ __forceinline__ void with_act(const GatedAct& a, F f) {
 
 template <typename OT> __device__ __forceinline__ OT to_type(float v) { return v; }
 template <> __device__ __forceinline__ __nv_bfloat16 to_type<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+// u: the up rows' sum, or what is added (kAdd)
 template <int MODE, int OUT>
 __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, float v, float u) {
   const size_t at = static_cast<size_t>(t) * p.N + row;
@@ -299,7 +300,7 @@ __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, 
     if constexpr (MODE == kBf16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(y);
     else static_cast<float*>(p.out)[at] = y;
   } else if constexpr (OUT == kAdd) {
-    static_cast<float*>(p.out)[at] = p.add[at] + v;
+    static_cast<float*>(p.out)[at] = u + v;
   } else {
     static_cast<float*>(p.out)[at] = p.bias ? v + p.bias[row] : v;
   }
@@ -506,12 +507,14 @@ umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
           } else if (ok && row < N) {
             const size_t at = static_cast<size_t>(t0 + c) * N + row;
             float* out = static_cast<float*>(p.out) + at;
+            float old[OUT == kAdd ? 32 : 1];  // (all on their way before the first store: `add` may be `out`)
+            if constexpr (OUT == kAdd) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) old[j] = t0 + c + j < T ? p.add[at + static_cast<size_t>(j) * N] : 0.f;
+            }
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (t0 + c + j < T) {
-                if constexpr (OUT == kAdd) out[static_cast<size_t>(j) * N] = p.add[at + static_cast<size_t>(j) * N] + __uint_as_float(r[j]);
-                else out[static_cast<size_t>(j) * N] = __uint_as_float(r[j]) + add;
-              }
+              if (t0 + c + j < T) out[static_cast<size_t>(j) * N] = __uint_as_float(r[j]) + (OUT == kAdd ? old[OUT == kAdd ? j : 0] : add);
           }
         }
       } else {
