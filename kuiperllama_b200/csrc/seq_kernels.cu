@@ -733,50 +733,36 @@ __global__ void qk_prepare_kernel(AttnShape a, RopeArgs rope, const float* qkvg,
 // The same with 16-byte accesses for heads that turn (halves paired) or are unit-normed, sizes multiples of 4: G lanes share a head,
 // a lane owns four coordinates of its first half and the four they turn with (or four that do not turn).  The angles of the
 // token's position are taken once, into shared memory; all heads read them from there.
+// What bounds it is latency -- frequencies (powf), angles, the row's loads, the page's entry, one behind the other -- and then instructions.
+// So a CTA takes every gridDim.x-th token, its frequencies once, the first heads' loads run under the angles, a step's first angles under
+// the kernel ahead, and a warp without heads in a round leaves it out
+// (6001 tokens, 16 + 8 heads of 128: 49 us with a CTA a token and its loads behind the angles, 39 here; 24 chats of 4 layers, 12 steps 3591 -> 3553).
+constexpr int kTurnCtas = 148 * 4;  // as many as run at once
 template <typename AT, int G>
 __global__ void __launch_bounds__(512)
 qk_turn_kernel(AttnShape a, RopeArgs rope, const float* qkvg, int stride, const float* __restrict__ qnorm_w,
                const float* __restrict__ knorm_w, float eps, const int32_t* tok_seq,
-               const int32_t* tok_pos, AT* q, float* gates, PagedKV kv) {
+               const int32_t* tok_pos, AT* q, float* gates, PagedKV kv, int T) {
+  extern __shared__ __align__(16) float turns_of[];  // [2][cos, sin][half]: of a token, and of the next
+  __shared__ float red_of[2][2][32];
   next_may_start();
-  after_previous();
-  extern __shared__ __align__(16) float turn[];  // [half] cos, [half] sin
-  __shared__ float red[2][32];
-  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int qn = a.heads * a.dim, kn = a.kv_heads * a.dim, vn = a.kv_heads * a.vdim, gn = gate_floats(a);
-  const float* row = qkvg + static_cast<size_t>(t) * stride;
-  const int seq = tok_seq[t], pos = tok_pos[t];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int half = rope.dims / 2;
-  float* co = turn;
-  float* si = turn + half;
-  for (int i = threadIdx.x; i < half; i += blockDim.x) {
-    const float freq = rope.freq ? rope.freq[i] : powf(rope.base, -2.0f * static_cast<float>(i) / static_cast<float>(rope.dims));
-    const float ang = static_cast<float>(pos) * freq;
-    co[i] = cosf(ang) * rope.mag, si[i] = sinf(ang) * rope.mag;
-  }
-  const bool whole = a.qk_norm == KLLM_SEQ_QKNORM_PROJECTION, weighted = whole || a.qk_norm == KLLM_SEQ_QKNORM_WEIGHTED;
-  float sq = 0.f, sk = 0.f;
-  if (whole) {
-    for (int i = threadIdx.x * 4; i < qn + kn; i += blockDim.x * 4) {
-      const float4 v = *reinterpret_cast<const float4*>(row + i);
-      const float ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
-      if (i < qn) sq += ss;
-      else sk += ss;
+  auto frequency = [&](int i) {
+    return rope.freq ? rope.freq[i] : powf(rope.base, -2.0f * static_cast<float>(i) / static_cast<float>(rope.dims));
+  };
+  const float first_freq = threadIdx.x < half ? frequency(threadIdx.x) : 0.f;
+  auto angles = [&](int t, float* co) {
+    const float pos = static_cast<float>(tok_pos[t]);
+    for (int i = threadIdx.x; i < half; i += blockDim.x) {
+      const float ang = pos * (i < static_cast<int>(blockDim.x) ? first_freq : frequency(i));
+      co[i] = cosf(ang) * rope.mag, co[half + i] = sinf(ang) * rope.mag;
     }
-    sq = warp_sum(sq), sk = warp_sum(sk);
-    if (lane == 0) red[0][warp] = sq, red[1][warp] = sk;
-  }
-  __syncthreads();
-  float rq = 1.0f, rk = 1.0f;
-  if (whole) {
-    sq = 0.f, sk = 0.f;
-    for (int i = 0; i < nw; ++i) sq += red[0][i], sk += red[1][i];
-    rq = 1.0f / sqrtf(sq / static_cast<float>(qn) + eps);
-    rk = 1.0f / sqrtf(sk / static_cast<float>(kn) + eps);
-  }
-  const float temp = a.temp_every > 0 ? 1.0f + a.temp_coef * logf(static_cast<float>((pos + 1) / a.temp_every) + 1.0f) : 1.0f;
-  AT* krow = page_row(static_cast<AT*>(kv.k), kv, seq, pos, a.kv_heads, a.dim);
-  AT* vrow = page_row(static_cast<AT*>(kv.v), kv, seq, pos, a.kv_heads, a.vdim);
+  };
+  angles(blockIdx.x, turns_of);  // (positions are the step's index arrays, complete before its first kernel)
+  after_previous();
+  const int qn = a.heads * a.dim, kn = a.kv_heads * a.dim, vn = a.kv_heads * a.vdim, gn = gate_floats(a);
+  const bool whole = a.qk_norm == KLLM_SEQ_QKNORM_PROJECTION, weighted = whole || a.qk_norm == KLLM_SEQ_QKNORM_WEIGHTED;
   const float inv_dim = 1.0f / static_cast<float>(a.dim);
   const int pairs = half / 4, rest = (a.dim - 2 * half) / 4;  // units of a head: pairs of quads, then quads
   const int gl = threadIdx.x % G, group = threadIdx.x / G, groups = blockDim.x / G;
@@ -784,48 +770,89 @@ qk_turn_kernel(AttnShape a, RopeArgs rope, const float* qkvg, int stride, const 
   const bool turns = gl < pairs;
   const int d0 = turns ? 4 * gl : (gl - pairs < rest ? 2 * half + 4 * (gl - pairs) : -1), d1 = turns ? half + 4 * gl : -1;
   const int total = a.heads + a.kv_heads;
-  for (int u0 = 0; u0 < total; u0 += groups) {  // every lane of a warp walks the same rounds: the shuffles need them all
-    const int u = u0 + group;
-    const bool live = u < total, is_q = u < a.heads;
-    const float* src = row + (is_q ? u * a.dim : qn + (u - a.heads) * a.dim);
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
-    if (live && d0 >= 0) x = *reinterpret_cast<const float4*>(src + d0);
-    if (live && d1 >= 0) y = *reinterpret_cast<const float4*>(src + d1);
-    auto head_ss = [&]() {
-      float ss = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w))) + fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, y.w * y.w)));
-#pragma unroll
-      for (int o = G / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(kAll, ss, o);
-      return ss;
+  int parity = 0;
+  for (int t = blockIdx.x; t < T; t += gridDim.x, parity ^= 1) {
+    const float* co = turns_of + parity * 2 * half;
+    const float* si = co + half;
+    float(&red)[2][32] = red_of[parity];
+    const float* row = qkvg + static_cast<size_t>(t) * stride;
+    const int seq = tok_seq[t], pos = tok_pos[t];
+    auto load_head = [&](int u, float4& x, float4& y) {
+      x = y = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (u >= total) return;
+      const float* src = row + (u < a.heads ? u * a.dim : qn + (u - a.heads) * a.dim);
+      if (d0 >= 0) x = *reinterpret_cast<const float4*>(src + d0);
+      if (d1 >= 0) y = *reinterpret_cast<const float4*>(src + d1);
     };
-    float rinv = is_q ? rq : rk;
-    if (a.qk_norm == KLLM_SEQ_QKNORM_WEIGHTED) rinv = 1.0f / sqrtf(head_ss() * inv_dim + eps);
-    if (weighted && live) {
-      const float* w = (is_q ? qnorm_w : knorm_w) + (whole ? (is_q ? u : u - a.heads) * a.dim : 0);
-      if (d0 >= 0) {
-        const float4 g = *reinterpret_cast<const float4*>(w + d0);
-        x = make_float4(x.x * rinv * g.x, x.y * rinv * g.y, x.z * rinv * g.z, x.w * rinv * g.w);
+    float4 x, y;
+    load_head(group, x, y);
+    AT* krow = page_row(static_cast<AT*>(kv.k), kv, seq, pos, a.kv_heads, a.dim);
+    AT* vrow = page_row(static_cast<AT*>(kv.v), kv, seq, pos, a.kv_heads, a.vdim);
+    float sq = 0.f, sk = 0.f;
+    if (whole) {
+      for (int i = threadIdx.x * 4; i < qn + kn; i += blockDim.x * 4) {
+        const float4 v = *reinterpret_cast<const float4*>(row + i);
+        const float ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
+        if (i < qn) sq += ss;
+        else sk += ss;
       }
-      if (d1 >= 0) {
-        const float4 g = *reinterpret_cast<const float4*>(w + d1);
-        y = make_float4(y.x * rinv * g.x, y.y * rinv * g.y, y.z * rinv * g.z, y.w * rinv * g.w);
+      sq = warp_sum(sq), sk = warp_sum(sk);
+      if (lane == 0) red[0][warp] = sq, red[1][warp] = sk;
+    }
+    __syncthreads();  // (also: everybody is done with the other buffers)
+    if (t + gridDim.x < T) angles(t + gridDim.x, turns_of + (parity ^ 1) * 2 * half);
+    float rq = 1.0f, rk = 1.0f;
+    if (whole) {
+      sq = 0.f, sk = 0.f;
+      for (int i = 0; i < nw; ++i) sq += red[0][i], sk += red[1][i];
+      rq = 1.0f / sqrtf(sq / static_cast<float>(qn) + eps);
+      rk = 1.0f / sqrtf(sk / static_cast<float>(kn) + eps);
+    }
+    const float temp = a.temp_every > 0 ? 1.0f + a.temp_coef * logf(static_cast<float>((pos + 1) / a.temp_every) + 1.0f) : 1.0f;
+    // every lane of a warp walks the same rounds (the shuffles need them all): as long as one of its heads exists
+    for (int u0 = 0; u0 + warp * (32 / G) < total; u0 += groups) {
+      const int u = u0 + group;
+      const bool live = u < total, is_q = u < a.heads;
+      float4 next_x, next_y;
+      load_head(u + groups, next_x, next_y);
+      auto head_ss = [&]() {
+        float ss = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w))) + fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, y.w * y.w)));
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(kAll, ss, o);
+        return ss;
+      };
+      float rinv = is_q ? rq : rk;
+      if (a.qk_norm == KLLM_SEQ_QKNORM_WEIGHTED) rinv = 1.0f / sqrtf(head_ss() * inv_dim + eps);
+      if (weighted && live) {
+        const float* w = (is_q ? qnorm_w : knorm_w) + (whole ? (is_q ? u : u - a.heads) * a.dim : 0);
+        if (d0 >= 0) {
+          const float4 g = *reinterpret_cast<const float4*>(w + d0);
+          x = make_float4(x.x * rinv * g.x, x.y * rinv * g.y, x.z * rinv * g.z, x.w * rinv * g.w);
+        }
+        if (d1 >= 0) {
+          const float4 g = *reinterpret_cast<const float4*>(w + d1);
+          y = make_float4(y.x * rinv * g.x, y.y * rinv * g.y, y.z * rinv * g.z, y.w * rinv * g.w);
+        }
       }
+      if (turns) {
+        const float4 c = *reinterpret_cast<const float4*>(co + d0), z = *reinterpret_cast<const float4*>(si + d0);
+        const float4 n = make_float4(x.x * c.x - y.x * z.x, x.y * c.y - y.y * z.y, x.z * c.z - y.z * z.z, x.w * c.w - y.w * z.w);
+        y = make_float4(y.x * c.x + x.x * z.x, y.y * c.y + x.y * z.y, y.z * c.z + x.z * z.z, y.w * c.w + x.w * z.w);
+        x = n;
+      }
+      float post = is_q ? temp : 1.0f;
+      if (a.qk_norm == KLLM_SEQ_QKNORM_UNIT) post *= 1.0f / sqrtf(head_ss() * inv_dim + eps);
+      if (live) {
+        AT* dst = is_q ? q + (static_cast<size_t>(t) * a.heads + u) * a.dim : krow + (u - a.heads) * a.dim;
+        if (d0 >= 0) put4(dst + d0, scaled(post, x));
+        if (d1 >= 0) put4(dst + d1, scaled(post, y));
+      }
+      x = next_x, y = next_y;
     }
-    if (turns) {
-      const float4 c = *reinterpret_cast<const float4*>(co + d0), z = *reinterpret_cast<const float4*>(si + d0);
-      const float4 n = make_float4(x.x * c.x - y.x * z.x, x.y * c.y - y.y * z.y, x.z * c.z - y.z * z.z, x.w * c.w - y.w * z.w);
-      y = make_float4(y.x * c.x + x.x * z.x, y.y * c.y + x.y * z.y, y.z * c.z + x.z * z.z, y.w * c.w + x.w * z.w);
-      x = n;
-    }
-    float post = is_q ? temp : 1.0f;
-    if (a.qk_norm == KLLM_SEQ_QKNORM_UNIT) post *= 1.0f / sqrtf(head_ss() * inv_dim + eps);
-    if (!live) continue;
-    AT* dst = is_q ? q + (static_cast<size_t>(t) * a.heads + u) * a.dim : krow + (u - a.heads) * a.dim;
-    if (d0 >= 0) put4(dst + d0, scaled(post, x));
-    if (d1 >= 0) put4(dst + d1, scaled(post, y));
+    for (int i = threadIdx.x * 4; i < vn; i += blockDim.x * 4) put4(vrow + i, *reinterpret_cast<const float4*>(row + qn + kn + i));
+    for (int i = threadIdx.x; i < gn; i += blockDim.x)
+      gates[static_cast<size_t>(t) * gn + i] = 1.0f / (1.0f + expf(-row[qn + kn + vn + i]));
   }
-  for (int i = threadIdx.x * 4; i < vn; i += blockDim.x * 4) put4(vrow + i, *reinterpret_cast<const float4*>(row + qn + kn + i));
-  for (int i = threadIdx.x; i < gn; i += blockDim.x)
-    gates[static_cast<size_t>(t) * gn + i] = 1.0f / (1.0f + expf(-row[qn + kn + vn + i]));
 }
 
 // The same for heads without rotation, temperature or maps, normed over the whole projection or not at all: nothing is done
@@ -1648,10 +1675,11 @@ int launch_qk_prepare(int dtype, const AttnShape& a, const RopeArgs& rope_, cons
       (rope.dims == 0 || rope.pairing == KLLM_SEQ_ROPE_HALVES) && units <= 32 && stride % 4 == 0 &&
       (reinterpret_cast<uintptr_t>(qkvg) & 15) == 0) {
     const int threads = T <= 64 ? 512 : 256;
-    const size_t smem = std::max<size_t>(16, 2 * static_cast<size_t>(half) * sizeof(float));
+    const size_t smem = std::max<size_t>(16, 4 * static_cast<size_t>(half) * sizeof(float));
+    const int ctas = std::min(T, kTurnCtas);
 #define KLLM_QK_TURN(G)                                                                                                   \
-  KLLM_SEQ_DISPATCH(dtype, (launch_ahead(qk_turn_kernel<AT, G>, dim3(T), dim3(threads), smem, s, a, rope, qkvg, stride, qnorm_w, knorm_w, eps, tok_seq, \
-                                                                          tok_pos, static_cast<AT*>(q), gates, kv)))
+  KLLM_SEQ_DISPATCH(dtype, (launch_ahead(qk_turn_kernel<AT, G>, dim3(ctas), dim3(threads), smem, s, a, rope, qkvg, stride, qnorm_w, knorm_w, eps, tok_seq, \
+                                                                          tok_pos, static_cast<AT*>(q), gates, kv, T)))
     if (units <= 8) KLLM_QK_TURN(8);
     else if (units <= 16) KLLM_QK_TURN(16);
     else KLLM_QK_TURN(32);

@@ -49,7 +49,7 @@ def test_only_weights_take_the_read_only_path(name, parameters, code):
 
 # what a kernel reads ahead of its wait: weights, and what was complete before the step's first kernel began
 EARLY = {"rows_kernel": {"w"}, "rows_gated_kernel": {"w"}, "umma_split_kernel": {"map_w", "map_w2", "p"},
-         "umma_f32_kernel": {"map_w", "map_w2", "p"},
+         "umma_f32_kernel": {"map_w", "map_w2", "p"}, "qk_turn_kernel": {"rope", "tok_pos"},
          "attention_rows_mma_kernel": {"ent_first", "ent_count", "ent_seq", "ent_pos0", "kv"}}
 
 
