@@ -67,6 +67,8 @@ int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* to
 // (ahead: may read its weights before the kernels ahead of it on the stream have finished)
 int prefill_product(const float* x, const float* w, const float* bias, float* out, int T, int K, int N, cudaStream_t s,
                     int* wait, bool ahead = true);
+int prefill_product_three(const float* x, const float* const (&w)[3], const float* const (&bias)[3], float* const (&out)[3], int T, int K,
+                          const int (&N)[3], cudaStream_t s, int* wait);
 int prefill_product_add(const float* x, const float* w, float* residual, int T, int K, int N, cudaStream_t s, int* wait);
 int prefill_product_gated(const float* x, const float* w1, const float* w3, float* out, int T, int K, int N, cudaStream_t s,
                           int* wait);

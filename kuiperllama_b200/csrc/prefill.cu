@@ -288,9 +288,9 @@ int prefill_block(const PrefillModel& m, PrefillWorkspace& ws, const int32_t* to
     const size_t layer_off = static_cast<size_t>(l) * m.seq_len * kvd;
     rmsnorm_rows_kernel<<<T, 256, 0, s>>>(ws.x, m.attn_norm[l], ws.xn, dim, m.eps);
     PF_TRY(count());
-    PF_TRY(prefill_product(ws.xn, f32(m.wq[l]), m.bq ? m.bq[l] : nullptr, ws.q, T, dim, q_rows, s, wait));
-    PF_TRY(prefill_product(ws.xn, f32(m.wk[l]), m.bq ? m.bk[l] : nullptr, ws.k, T, dim, kvd, s, wait));
-    PF_TRY(prefill_product(ws.xn, f32(m.wv[l]), m.bq ? m.bv[l] : nullptr, ws.v, T, dim, kvd, s, wait));
+    PF_TRY(prefill_product_three(ws.xn, {f32(m.wq[l]), f32(m.wk[l]), f32(m.wv[l])},
+                                 {m.bq ? m.bq[l] : nullptr, m.bq ? m.bk[l] : nullptr, m.bq ? m.bv[l] : nullptr}, {ws.q, ws.k, ws.v}, T, dim,
+                                 {q_rows, kvd, kvd}, s, wait));
     rope_scatter_kernel<<<T, 256, 0, s>>>(ws.q, ws.k, ws.v, m.sin_cache, m.cos_cache, m.key_cache + layer_off,
                                           m.value_cache + layer_off, cl, heads, kvh, m.flavour, start_pos);
     PF_TRY(count());

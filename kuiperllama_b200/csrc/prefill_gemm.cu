@@ -30,7 +30,8 @@ namespace {
 template <int OUT>
 int product(const seq::umma::SplitArgs& p, cudaStream_t s, bool ahead = true) {
   using namespace seq::umma;
-  if (fills_chip(p.T, p.N)) return launch_tiles<kTf32, OUT>(p, s);
+  if constexpr (OUT != kThree)
+    if (fills_chip(p.T, p.N)) return launch_tiles<kTf32, OUT>(p, s);
   if (p.T <= 16) return launch_split<kTf32, 16, OUT, 5>(p, s, ahead);
   if (p.T <= 32) return launch_split<kTf32, 32, OUT, 5>(p, s, ahead);
   if (p.T <= 64) return launch_split<kTf32, 64, OUT, 4>(p, s, ahead);
@@ -48,6 +49,21 @@ int prefill_product(const float* x, const float* w, const float* bias, float* ou
                     int* wait, bool ahead) {
   if (!aligned(x, w, K)) return KLLM_E_UNSUPPORTED;
   return product<seq::umma::kPlain>({x, w, nullptr, bias, nullptr, out, T, N, K, 1, kSwiglu, wait}, s, ahead);
+}
+// Queries, keys and values: one launch while the queries alone do not fill the chip (900 x 2048 against 2048 + 256 + 256 rows: one after the
+// other 25 + 15 + 15 us, the last two bound by the way to and through a cluster of eight; together 32).
+int prefill_product_three(const float* x, const float* const (&w)[3], const float* const (&bias)[3], float* const (&out)[3], int T, int K,
+                          const int (&N)[3], cudaStream_t s, int* wait) {
+  using namespace seq::umma;
+  if (fills_chip(T, N[0])) {
+    for (int i = 0; i < 3; ++i)
+      if (const int rc = prefill_product(x, w[i], bias[i], out[i], T, K, N[i], s, wait)) return rc;
+    return 0;
+  }
+  for (int i = 0; i < 3; ++i)
+    if (!aligned(x, w[i], K)) return KLLM_E_UNSUPPORTED;
+  return product<kThree>({x, w[0], w[1], bias[0], nullptr, out[0], T, N[0], K, 1, kSwiglu, wait, w[2], bias[1], bias[2], out[1], out[2],
+                          N[1], N[2]}, s);
 }
 int prefill_product_add(const float* x, const float* w, float* residual, int T, int K, int N, cudaStream_t s, int* wait) {
   if (!aligned(x, w, K)) return KLLM_E_UNSUPPORTED;

@@ -235,10 +235,23 @@ constexpr int split_ctas_per_sm() { return split_smem<MODE, BN, ST>() <= 113 * 1
 template <int MODE, int BN, int OUT, int ST>
 __global__ void __launch_bounds__(split_threads<MODE>(), split_ctas_per_sm<MODE, BN, ST>())
 umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
-                  const __grid_constant__ CUtensorMap map_a, const SplitArgs p) {
+                  const __grid_constant__ CUtensorMap map_w3, const __grid_constant__ CUtensorMap map_a, const SplitArgs args) {
   using M = ModeOf<MODE>;
   constexpr bool two = OUT == kGated;
   constexpr int FEATURES = two ? BM / 2 : BM;
+  SplitArgs p = args;
+  int feature_tile = blockIdx.x;
+  const CUtensorMap* map_own = &map_w;  // of the matrix that this CTA has a tile of
+  if constexpr (OUT == kThree) {
+    const int tiles = (args.N + BM - 1) / BM, tiles2 = (args.N2 + BM - 1) / BM;
+    if (feature_tile >= tiles + tiles2) {
+      feature_tile -= tiles + tiles2, map_own = &map_w3;
+      p.N = args.N3, p.out = args.out3, p.bias = args.bias3;
+    } else if (feature_tile >= tiles) {
+      feature_tile -= tiles, map_own = &map_w2;
+      p.N = args.N2, p.out = args.out2, p.bias = args.bias2;
+    }
+  }
   constexpr int W_BYTES = A_BYTES, B_BYTES = BN * 128;
   constexpr int HALF = W_BYTES + B_BYTES;                  // the tiles as they arrive
   constexpr int STAGE = kSplitStage<MODE, BN>;           // kFp32: h and m take the tiles' place, l follows
@@ -263,7 +276,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   float* special_row = special + 1;
 
   const int warp = warp_number(), lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * FEATURES, t0 = blockIdx.z * BN;
+  const int n0 = feature_tile * FEATURES, t0 = blockIdx.z * BN;
   const int S = p.S, rank = S > 1 ? static_cast<int>(cluster_rank()) : 0;
   const int all_blocks = (p.K + M::BKE - 1) / M::BKE;
   const int kb0 = static_cast<int>(static_cast<long long>(all_blocks) * rank / S);
@@ -303,7 +316,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const uint32_t bar = smem_u32(&full[i % ST]);
         uint8_t* st = base + (i % ST) * STAGE;
         mbar_expect_tx(bar, HALF);
-        tma_load_2d(smem_u32(st), &map_w, bar, (kb0 + i) * M::BKE, n0);
+        tma_load_2d(smem_u32(st), map_own, bar, (kb0 + i) * M::BKE, n0);
         if (two) tma_load_2d(smem_u32(st + A_BYTES / 2), &map_w2, bar, (kb0 + i) * M::BKE, n0);
       };
       // the ring's first weights are on their way before the rows they meet are there
@@ -473,11 +486,15 @@ template <int MODE, int BN, int OUT, int ST>
 inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
   constexpr bool two = OUT == kGated;
   constexpr int FEATURES = two ? BM / 2 : BM;
+  constexpr bool three = OUT == kThree;
   CUtensorMap map_w, map_w2, map_a;
   if (p.report == nullptr) return KLLM_E_STATE;
   if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, FEATURES)) return rc;
-  if (int rc = make_map_of<MODE>(&map_w2, two ? p.w2 : p.w, p.N, p.K, FEATURES)) return rc;
+  if (int rc = make_map_of<MODE>(&map_w2, two || three ? p.w2 : p.w, three ? p.N2 : p.N, p.K, FEATURES)) return rc;
   if (int rc = make_map_of<MODE>(&map_a, p.a, p.T, p.K, BN)) return rc;
+  CUtensorMap map_w3 = map_w;
+  if constexpr (three)
+    if (int rc = make_map_of<MODE>(&map_w3, p.w3, p.N3, p.K, FEATURES)) return rc;
   constexpr size_t smem = split_smem<MODE, BN, ST>();
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kernel = umma_split_kernel<MODE, BN, OUT, ST>;
@@ -487,7 +504,9 @@ inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
-  const int feature_tiles = (p.N + FEATURES - 1) / FEATURES, token_tiles = (p.T + BN - 1) / BN;
+  int feature_tiles = (p.N + FEATURES - 1) / FEATURES;
+  if constexpr (three) feature_tiles += (p.N2 + FEATURES - 1) / FEATURES + (p.N3 + FEATURES - 1) / FEATURES;
+  const int token_tiles = (p.T + BN - 1) / BN;
   p.S = split_count(feature_tiles * token_tiles, (p.K + ModeOf<MODE>::BKE - 1) / ModeOf<MODE>::BKE, split_ctas_per_sm<MODE, BN, ST>() * kSms);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(feature_tiles, p.S, token_tiles);
@@ -501,7 +520,7 @@ inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ahead ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_w2, map_a, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_w2, map_w3, map_a, p);
   count_launch();
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }

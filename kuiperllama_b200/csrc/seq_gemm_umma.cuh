@@ -248,7 +248,8 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 enum Out {
   kPlain = 0,  // out = sum + bias (fp32)
   kGated = 1,  // out = gated_act(sum of w + bias[n], sum of w2 + bias[N + n]) in the operands' type
-  kAdd = 2     // out = add + sum (fp32; add may be out itself)
+  kAdd = 2,    // out = add + sum (fp32; add may be out itself)
+  kThree = 3   // kPlain for three matrices side by side: w to out, w2 to out2, w3 to out3
 };
 
 // operand pointers (kFp32 sums rows that hold infinities through them) and what joins the sums
@@ -260,6 +261,11 @@ struct SplitArgs {
   int T, N, K, S;
   GatedAct act;
   int* report;  // where a wait that ran out is noted
+  // kThree
+  const void* w3;
+  const float *bias2, *bias3;
+  void *out2, *out3;
+  int N2, N3;
 };
 
 // gated_act without branches, for results that 16 bits or TF32 products round far more: 1 / (1 + exp(-x)) from ex2.approx and rcp.approx,
