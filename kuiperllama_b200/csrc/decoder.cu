@@ -126,7 +126,8 @@ struct kllm_decoder {
   StepState* st = nullptr;
   int32_t* out_tokens = nullptr;  // device [seq_len]
   int32_t* teacher = nullptr;     // device [seq_len]
-  StepState* st_host = nullptr;   // pinned
+  StepState* st_host = nullptr;   // pinned; the persistent engine writes it itself
+  float* logits_host = nullptr;   // pinned [vocab_size]
   int32_t* io_host = nullptr;     // pinned scratch
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;       // out_tokens recorded, no teacher
@@ -361,7 +362,8 @@ int kllm_decoder_create(const kllm_decoder_desc* desc, void* stream, kllm_decode
       cudaMalloc(&dc->out_tokens, sizeof(int32_t) * d.seq_len) != cudaSuccess ||
       cudaMalloc(&dc->teacher, sizeof(int32_t) * d.seq_len) != cudaSuccess ||
       cudaMallocHost(&dc->st_host, sizeof(StepState)) != cudaSuccess ||
-      cudaMallocHost(&dc->io_host, sizeof(int32_t) * d.seq_len) != cudaSuccess)
+      cudaMallocHost(&dc->io_host, sizeof(int32_t) * d.seq_len) != cudaSuccess ||
+      cudaMallocHost(&dc->logits_host, sizeof(float) * d.vocab_size) != cudaSuccess)
     return fail(static_cast<int>(cudaErrorMemoryAllocation));
   cudaMemsetAsync(dc->st, 0, sizeof(StepState), dc->stream);
 
@@ -405,7 +407,7 @@ int kllm_decoder_create(const kllm_decoder_desc* desc, void* stream, kllm_decode
     mm.bv = dc->bv.empty() ? nullptr : dc->bv.data();
     mm.x = dc->x, mm.q = dc->q, mm.k_raw = dc->k_raw, mm.attn_out = dc->attn, mm.h = dc->h;
     mm.logits = dc->logits, mm.score = dc->score, mm.key_cache = dc->kcache, mm.value_cache = dc->vcache;
-    mm.sin_cache = dc->sin_t, mm.cos_cache = dc->cos_t, mm.state = dc->st, mm.out_tokens = dc->out_tokens;
+    mm.sin_cache = dc->sin_t, mm.cos_cache = dc->cos_t, mm.state = dc->st_host, mm.out_tokens = dc->out_tokens;
     rc = dc->mega.init(mm, dc->stream);
     if (rc == 0) {
       dc->use_mega = true;
@@ -443,8 +445,22 @@ void kllm_decoder_destroy(kllm_decoder* dc) {
   if (dc->pf_buf) cudaFree(dc->pf_buf);
   if (dc->st_host) cudaFreeHost(dc->st_host);
   if (dc->io_host) cudaFreeHost(dc->io_host);
+  if (dc->logits_host) cudaFreeHost(dc->logits_host);
   if (dc->own_stream && dc->stream) cudaStreamDestroy(dc->stream);
   delete dc;
+}
+
+// The graph engine reads and writes its state in device memory.  The persistent engine takes the first token and its position as
+// parameters and writes the state to pinned memory by itself.  The two copies of a step, and logits that went to the caller's memory without
+// a pinned stop on the way, were 18 of the 50 us that a token of stories15M and its logits spent outside of the kernel (164 -> 146).
+static int state_in(kllm_decoder* dc, int32_t token, int32_t pos) {
+  *dc->st_host = StepState{token, pos, 0, -1};
+  if (dc->use_mega) return 0;
+  return static_cast<int>(cudaMemcpyAsync(dc->st, dc->st_host, sizeof(StepState), cudaMemcpyHostToDevice, dc->stream));
+}
+static int state_out(kllm_decoder* dc) {  // there once the stream has been waited for
+  if (dc->use_mega) return 0;
+  return static_cast<int>(cudaMemcpyAsync(dc->st_host, dc->st, sizeof(StepState), cudaMemcpyDeviceToHost, dc->stream));
 }
 
 int kllm_decoder_step(kllm_decoder* dc, int32_t token_host, int32_t pos, int is_prompt,
@@ -452,19 +468,15 @@ int kllm_decoder_step(kllm_decoder* dc, int32_t token_host, int32_t pos, int is_
   if (!dc || !next_host) return KLLM_E_INVALID;
   if (pos < 0 || pos >= dc->d.seq_len) return KLLM_E_INVALID;
   StepState* hs = dc->st_host;
-  hs->token = token_host;
-  hs->pos = pos;
-  hs->step = 0;
-  hs->next = -1;
-  KLLM_TRY(cudaMemcpyAsync(dc->st, hs, sizeof(StepState), cudaMemcpyHostToDevice, dc->stream));
+  KLLM_TRY(state_in(dc, token_host, pos));
   if (dc->use_mega) {
     // a prompt position needs no logits (llama3.cpp:738-739 returns -1): the classifier is skipped
-    KLLM_TRY(dc->mega.run(1, nullptr, nullptr, -1, is_prompt ? 1 : 0));
+    KLLM_TRY(dc->mega.run(token_host, pos, 1, nullptr, nullptr, -1, is_prompt ? 1 : 0));
   } else {
     KLLM_TRY(cudaGraphLaunch(dc->exec, dc->stream));
     count_launch(static_cast<uint64_t>(dc->launches_per_step));
   }
-  KLLM_TRY(cudaMemcpyAsync(hs, dc->st, sizeof(StepState), cudaMemcpyDeviceToHost, dc->stream));
+  KLLM_TRY(state_out(dc));
   KLLM_TRY(cudaStreamSynchronize(dc->stream));
   *next_host = is_prompt ? -1 : hs->next;
   return 0;
@@ -475,22 +487,18 @@ int kllm_decoder_prompt(kllm_decoder* dc, const int32_t* tokens_host, int32_t n_
   if (!dc || !tokens_host || !next_host || n_tokens <= 0 || start_pos < 0) return KLLM_E_INVALID;
   if (start_pos + n_tokens > dc->d.seq_len) return KLLM_E_INVALID;
   StepState* hs = dc->st_host;
-  hs->token = tokens_host[0];
-  hs->pos = start_pos;
-  hs->step = 0;
-  hs->next = -1;
-  KLLM_TRY(cudaMemcpyAsync(dc->st, hs, sizeof(StepState), cudaMemcpyHostToDevice, dc->stream));
+  KLLM_TRY(state_in(dc, tokens_host[0], start_pos));
   std::memcpy(dc->io_host, tokens_host, sizeof(int32_t) * n_tokens);
   KLLM_TRY(cudaMemcpyAsync(dc->teacher, dc->io_host, sizeof(int32_t) * n_tokens, cudaMemcpyHostToDevice,
                            dc->stream));
   if (dc->use_mega) {
     // ONE launch for the whole prompt; only the last position runs the classifier
-    KLLM_TRY(dc->mega.run(n_tokens, dc->teacher, nullptr, -1, n_tokens - 1));
+    KLLM_TRY(dc->mega.run(tokens_host[0], start_pos, n_tokens, dc->teacher, nullptr, -1, n_tokens - 1));
   } else {
     for (int i = 0; i < n_tokens; ++i) KLLM_TRY(cudaGraphLaunch(dc->exec_tf, dc->stream));
     count_launch(static_cast<uint64_t>(dc->launches_per_step) * n_tokens);
   }
-  KLLM_TRY(cudaMemcpyAsync(hs, dc->st, sizeof(StepState), cudaMemcpyDeviceToHost, dc->stream));
+  KLLM_TRY(state_out(dc));
   KLLM_TRY(cudaStreamSynchronize(dc->stream));
   *next_host = hs->next;
   return 0;
@@ -591,19 +599,15 @@ int kllm_decoder_generate(kllm_decoder* dc, int32_t first_token, int32_t start_p
                           int32_t* out_tokens_host) {
   if (!dc || n_steps <= 0 || start_pos < 0) return KLLM_E_INVALID;
   if (start_pos + n_steps > dc->d.seq_len) return KLLM_E_INVALID;
-  StepState* hs = dc->st_host;
-  hs->token = teacher_host ? teacher_host[0] : first_token;
-  hs->pos = start_pos;
-  hs->step = 0;
-  hs->next = -1;
-  KLLM_TRY(cudaMemcpyAsync(dc->st, hs, sizeof(StepState), cudaMemcpyHostToDevice, dc->stream));
+  const int32_t first = teacher_host ? teacher_host[0] : first_token;
+  KLLM_TRY(state_in(dc, first, start_pos));
   if (teacher_host) {
     std::memcpy(dc->io_host, teacher_host, sizeof(int32_t) * n_steps);
     KLLM_TRY(cudaMemcpyAsync(dc->teacher, dc->io_host, sizeof(int32_t) * n_steps,
                              cudaMemcpyHostToDevice, dc->stream));
   }
   if (dc->use_mega) {
-    KLLM_TRY(dc->mega.run(n_steps, teacher_host ? dc->teacher : nullptr));
+    KLLM_TRY(dc->mega.run(first, start_pos, n_steps, teacher_host ? dc->teacher : nullptr));
   } else {
     cudaGraphExec_t exec = teacher_host ? dc->exec_tf : dc->exec;
     for (int i = 0; i < n_steps; ++i) KLLM_TRY(cudaGraphLaunch(exec, dc->stream));
@@ -632,10 +636,7 @@ int kllm_decoder_profile(kllm_decoder* dc, int32_t first_token, int32_t start_po
   unsigned long long* d_prof = nullptr;
   KLLM_TRY(cudaMalloc(&d_prof, n * sizeof(unsigned long long)));
   cudaMemsetAsync(d_prof, 0, n * sizeof(unsigned long long), dc->stream);
-  StepState* hs = dc->st_host;
-  hs->token = first_token, hs->pos = start_pos, hs->step = 0, hs->next = -1;
-  cudaMemcpyAsync(dc->st, hs, sizeof(StepState), cudaMemcpyHostToDevice, dc->stream);
-  int rc = dc->mega.run(n_steps, nullptr, d_prof, profiled_step);
+  int rc = dc->mega.run(first_token, start_pos, n_steps, nullptr, d_prof, profiled_step);
   if (rc == 0) rc = static_cast<int>(cudaStreamSynchronize(dc->stream));
   if (rc == 0)
     rc = static_cast<int>(cudaMemcpy(stamps_host, d_prof, n * sizeof(unsigned long long),
@@ -646,9 +647,11 @@ int kllm_decoder_profile(kllm_decoder* dc, int32_t first_token, int32_t start_po
 
 int kllm_decoder_logits(kllm_decoder* dc, float* logits_host) {
   if (!dc || !logits_host) return KLLM_E_INVALID;
+  const size_t bytes = sizeof(float) * dc->d.vocab_size;
+  KLLM_TRY(cudaMemcpyAsync(dc->logits_host, dc->logits, bytes, cudaMemcpyDeviceToHost, dc->stream));
   KLLM_TRY(cudaStreamSynchronize(dc->stream));
-  return static_cast<int>(cudaMemcpy(logits_host, dc->logits, sizeof(float) * dc->d.vocab_size,
-                                     cudaMemcpyDeviceToHost));
+  std::memcpy(logits_host, dc->logits_host, bytes);
+  return 0;
 }
 
 const float* kllm_decoder_logits_device(const kllm_decoder* dc) { return dc ? dc->logits : nullptr; }

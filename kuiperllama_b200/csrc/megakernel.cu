@@ -1791,7 +1791,7 @@ __device__ __forceinline__ void epilogue_role(const Params& P, int lane) {
   const Phase& ph = g_ph_epi;
   const int cta = blockIdx.x, G = gridDim.x;
   unsigned groups = 0;
-  int pos = P.state->pos;
+  int pos = P.start_pos;
   for (int tok = 0; tok < P.n_tokens; ++tok, ++pos) {
     ArgBest best{0.f, -1};
     for (int pi = 0; pi < P.n_phases; ++pi) {
@@ -2408,7 +2408,7 @@ __global__ void __launch_bounds__(mega_threads(CW, KIND), 1) decode_megakernel(c
     const uint64_t policy = policy_evict_first();  // weights: streamed once per token
     const uint64_t policy_kv = policy_evict_last();  // KV tiles: re-read every token, keep in L2
     unsigned filled = 0u;
-    int ppos = P.state->pos;
+    int ppos = P.start_pos;
     for (int tok = 0; tok < P.n_tokens; ++tok, ++ppos) {
       const int n_run = tok < P.skip_cls_tokens ? P.n_phases - P.n_cls_phases : P.n_phases;  // prompt token: no classifier
       for (int pi = 0; pi < n_run; ++pi) {
@@ -2594,7 +2594,7 @@ __global__ void __launch_bounds__(mega_threads(CW, KIND), 1) decode_megakernel(c
   if (warp == CW + 1) {
     if (P.pf_stages <= 0) return;
     unsigned ahead = 0u;  // stages walked by this warp (same counting as the producer's `filled`)
-    int ppos = P.state->pos;
+    int ppos = P.start_pos;
     for (int tok = 0; tok < P.n_tokens; ++tok, ++ppos) {
       const int n_run = tok < P.skip_cls_tokens ? P.n_phases - P.n_cls_phases : P.n_phases;
       for (int pi = 0; pi < n_run; ++pi) {
@@ -2675,10 +2675,10 @@ __global__ void __launch_bounds__(mega_threads(CW, KIND), 1) decode_megakernel(c
   // =============================== consumer warps ===============================================
   unsigned groups = 0u;
   unsigned bar_target = P.barrier_base;
-  int token = P.state->token;
+  int token = P.start_token;
   if (static_cast<unsigned>(token) >= static_cast<unsigned>(P.vocab_size)) token = 0;
-  int pos = P.state->pos;
-  int step = P.state->step;
+  int pos = P.start_pos;
+  int step = 0;
   float4* xres4 = reinterpret_cast<float4*>(xres);
   constexpr int kPhaseWords = static_cast<int>(sizeof(Phase) / 4);
   static_assert(kPhaseWords <= CT, "phase copy: one word per consumer thread");
@@ -3343,7 +3343,7 @@ void MegaEngine::destroy() {
   ready_ = false;
 }
 
-int MegaEngine::run(int n_tokens, const int32_t* teacher_dev, unsigned long long* prof_dev,
+int MegaEngine::run(int first_token, int start_pos, int n_tokens, const int32_t* teacher_dev, unsigned long long* prof_dev,
                     int prof_token, int skip_cls_tokens) {
   if (!ready_) return KLLM_E_STATE;
   Params P{};
@@ -3351,6 +3351,7 @@ int MegaEngine::run(int n_tokens, const int32_t* teacher_dev, unsigned long long
   P.phases = static_cast<const Phase*>(d_phases_);
   P.n_phases = n_phases_;
   P.n_tokens = n_tokens;
+  P.start_token = first_token, P.start_pos = start_pos;
   P.skip_cls_tokens = skip_cls_tokens;
   P.n_cls_phases = n_cls_phases_;
   P.int8_fast = int8_fast_;

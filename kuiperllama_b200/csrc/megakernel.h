@@ -95,6 +95,7 @@ struct State {  // == StepState in decoder.cu
 struct Params {
   const Phase* phases;
   int n_phases, n_tokens;
+  int start_token, start_pos;
   int attn_vsplit;      // V cache layout [L][kv_head][attn_vsplit][seq_len][head_size / attn_vsplit]
   int attn_parts;       // flash attention: threads per timestep in the scores pass
   int int8_fast;        // int8 weights: 1 = fixed-point activations on dp4a (toleranced), 0 = the reference's per-element order
@@ -178,7 +179,7 @@ class MegaEngine {
   int init(const MegaModel& m, cudaStream_t stream);
   void destroy();
   // Run n_tokens consecutive positions starting from the device-resident state.
-  int run(int n_tokens, const int32_t* teacher_dev, unsigned long long* prof_dev = nullptr,
+  int run(int first_token, int start_pos, int n_tokens, const int32_t* teacher_dev, unsigned long long* prof_dev = nullptr,
           int prof_token = -1, int skip_cls_tokens = 0);
   int grid() const { return grid_; }
   bool ready() const { return ready_; }
