@@ -222,6 +222,9 @@ __device__ __forceinline__ void split_sum_special(const SplitArgs& p, int rank, 
 template <int MODE>
 constexpr int split_threads() { return MODE == kFp32 ? THREADS + kSplitWarps * 32 : THREADS; }
 
+struct MoreMaps {  // of the up rows, or (kThree) of the second and the third matrix
+  CUtensorMap second, third;
+};
 // grid: (feature tiles, S, token tiles), clusters of (1, S, 1)
 template <int MODE, int BN>
 constexpr int kSplitStage = (A_BYTES + BN * 128) * (MODE == kFp32 ? 3 : 2) / 2;  // bytes
@@ -234,22 +237,21 @@ template <int MODE, int BN, int ST>
 constexpr int split_ctas_per_sm() { return split_smem<MODE, BN, ST>() <= 113 * 1024 ? 2 : 1; }
 template <int MODE, int BN, int OUT, int ST>
 __global__ void __launch_bounds__(split_threads<MODE>(), split_ctas_per_sm<MODE, BN, ST>())
-umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
-                  const __grid_constant__ CUtensorMap map_w3, const __grid_constant__ CUtensorMap map_a, const SplitArgs args) {
+umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ MoreMaps map_w2,
+                  const __grid_constant__ CUtensorMap map_a, SplitArgs p) {
   using M = ModeOf<MODE>;
   constexpr bool two = OUT == kGated;
   constexpr int FEATURES = two ? BM / 2 : BM;
-  SplitArgs p = args;
   int feature_tile = blockIdx.x;
   const CUtensorMap* map_own = &map_w;  // of the matrix that this CTA has a tile of
   if constexpr (OUT == kThree) {
-    const int tiles = (args.N + BM - 1) / BM, tiles2 = (args.N2 + BM - 1) / BM;
+    const int tiles = (p.N + BM - 1) / BM, tiles2 = (p.N2 + BM - 1) / BM;
     if (feature_tile >= tiles + tiles2) {
-      feature_tile -= tiles + tiles2, map_own = &map_w3;
-      p.N = args.N3, p.out = args.out3, p.bias = args.bias3;
+      feature_tile -= tiles + tiles2, map_own = &map_w2.third;
+      p.N = p.N3, p.out = p.out3, p.bias = p.bias3;
     } else if (feature_tile >= tiles) {
-      feature_tile -= tiles, map_own = &map_w2;
-      p.N = args.N2, p.out = args.out2, p.bias = args.bias2;
+      feature_tile -= tiles, map_own = &map_w2.second;
+      p.N = p.N2, p.out = p.out2, p.bias = p.bias2;
     }
   }
   constexpr int W_BYTES = A_BYTES, B_BYTES = BN * 128;
@@ -317,7 +319,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         uint8_t* st = base + (i % ST) * STAGE;
         mbar_expect_tx(bar, HALF);
         tma_load_2d(smem_u32(st), map_own, bar, (kb0 + i) * M::BKE, n0);
-        if (two) tma_load_2d(smem_u32(st + A_BYTES / 2), &map_w2, bar, (kb0 + i) * M::BKE, n0);
+        if (two) tma_load_2d(smem_u32(st + A_BYTES / 2), &map_w2.second, bar, (kb0 + i) * M::BKE, n0);
       };
       // the ring's first weights are on their way before the rows they meet are there
       for (int i = 0; i < ST && i < blocks; ++i) weights(i);
@@ -487,14 +489,15 @@ inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
   constexpr bool two = OUT == kGated;
   constexpr int FEATURES = two ? BM / 2 : BM;
   constexpr bool three = OUT == kThree;
-  CUtensorMap map_w, map_w2, map_a;
+  CUtensorMap map_w, map_a;
+  MoreMaps map_w2;
   if (p.report == nullptr) return KLLM_E_STATE;
   if (int rc = make_map_of<MODE>(&map_w, p.w, p.N, p.K, FEATURES)) return rc;
-  if (int rc = make_map_of<MODE>(&map_w2, two || three ? p.w2 : p.w, three ? p.N2 : p.N, p.K, FEATURES)) return rc;
+  if (int rc = make_map_of<MODE>(&map_w2.second, two || three ? p.w2 : p.w, three ? p.N2 : p.N, p.K, FEATURES)) return rc;
   if (int rc = make_map_of<MODE>(&map_a, p.a, p.T, p.K, BN)) return rc;
-  CUtensorMap map_w3 = map_w;
+  map_w2.third = map_w;
   if constexpr (three)
-    if (int rc = make_map_of<MODE>(&map_w3, p.w3, p.N3, p.K, FEATURES)) return rc;
+    if (int rc = make_map_of<MODE>(&map_w2.third, p.w3, p.N3, p.K, FEATURES)) return rc;
   constexpr size_t smem = split_smem<MODE, BN, ST>();
   static_assert(smem <= 232448, "shared memory of one CTA");
   auto kernel = umma_split_kernel<MODE, BN, OUT, ST>;
@@ -520,7 +523,7 @@ inline int launch_split(SplitArgs p, cudaStream_t stream, bool ahead) {
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ahead ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_w2, map_w3, map_a, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_w, map_w2, map_a, p);
   count_launch();
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
