@@ -324,7 +324,8 @@ __device__ __forceinline__ void split_store(const SplitArgs& p, int t, int row, 
 // Plain results leave through shared memory by TMA, 32 features x 16 tokens at a time: stored from registers, 32 features of a token per
 // instruction, a tile took 10 us to leave, which the products of a short K do not cover and the last tile never does.
 // 2048 x K x 8192 in us, calls back to back, one CTA to a tile of 256 tokens / pairs / and stores by TMA: K = 2048 64.5 / 61.2 / 57.4,
-// K = 512 - / 35.1 / 26.8; 4096 x 4096 x 4096 110 / 105 / 102, 1501 x 2048 x 3072 20.6 / 22.7 / 20.5.  A block of K lasts some 560
+// K = 512 - / 35.1 / 26.8; 4096 x 4096 x 4096 110 / 105 / 102, 1501 x 2048 x 3072 20.6 / 22.7 / 20.5.  With an elected lane (elect_one) pairs
+// take 55.3, 25.5 and 98.5, K = 8192 200 instead of 210, and 900 x 2048 x 2048 in narrow tiles 14.5 instead of 18.6.  A block of K lasts some 560
 // cycles of a tile wherever a CTA takes in 32 KB for it (256 x 256 on a pair, 256 x 128 on a pair, 128 x 128 on a CTA; the slope of the time
 // over K = 512 to 16384), the products of a tile of 256 x 256 take 512.  What bounds pairs now is what lies around that: for 2048 x 2048 x
 // 8192 the tensor pipe is busy in 57 % of the cycles and the SMs' read port in 28 % (ncu): 3.46 waves of tiles, the ring's start, the last
